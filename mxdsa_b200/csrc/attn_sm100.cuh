@@ -6,20 +6,23 @@
 //   the pair holds the 64 rows of token 2p+c.  All MMAs are tcgen05 cta_group::2, M = 128:
 //     QK : P[128 x 128 keys]  += Q[128 x 32] . K[128 keys x 32]^T      16 steps over the 512 dims
 //     PV : O[128 x 256 dims]  += S[128 x 32 keys] . V[32 keys x 256]   4 key steps x 2 dim chunks
-//   K rows are split between the CTAs by key (CTA c stages keys 64c..64c+63 of the tile, all 512
-//   bytes), V rows by dimension (CTA c stages all 128 keys, bytes 256c..256c+255).  The
+//   K rows are split between the CTAs by key (CTA c holds keys 64c..64c+63 of the tile, all 512
+//   bytes), V rows by dimension (CTA c holds all 128 keys, bytes 256c..256c+255).  K and V are the
+//   same bytes, so a tile is staged ONCE: after QK the half of the K tile that this CTA's V does not
+//   contain is overwritten with the half that it lacks.  The
 //   accumulators live in tensor memory: per CTA 128 lanes x (256 O + 2 x 64 P) columns; lane L
 //   holds row L%64, and column half L/64 (P: keys 64*(L/64).., O: dims 256*(L/64)..).
 //
 // Roles (warp-specialised, 28 warps per CTA; the launch gives every thread 72 registers, re-balanced with
 // setmaxnreg to 48 / 32 / 64 / 104 / 48 for the five kinds of warp below)
 //   warps 0-3   K producers: read key indices one tile ahead and copy the selected rows of this CTA's 64 keys
-//               into the K ring with 16-byte cp.async; one warp instruction moves one 512-byte row straight
+//               into the tile ring with 16-byte cp.async; one warp instruction moves one 512-byte row straight
 //               into the 128-byte-swizzled operand layout.  The same warps gather the 8 scale bytes of all 128
 //               keys of the tile into the row layout that tcgen05.cp wants, and vote the validity bits.
-//   warps 4-7   V producers: TMA gather4 (four rows x 128 bytes per request) of the 256-byte halves of all 128
-//               keys into the V ring; every lane works out one key's row coordinate, eight lanes per warp
-//               collect four each and issue.  The bytes of both CTAs complete on one barrier of CTA 0.
+//   warps 4-7   V producers: once a tile's QK is done, TMA gather4 (four rows x 128 bytes per request) of this
+//               CTA's 256 bytes of the PEER's 64 keys over the 256 bytes of its own keys that belong to the peer;
+//               every lane works out one key's row coordinate, eight lanes per warp collect four each and issue
+//               one request.  The bytes of both CTAs complete on one barrier of CTA 0.
 //               (cp.async carrying V as well makes the K rows -- which the next QK waits for -- land late; the
 //               copy engine alone is the slower of the two paths, which is why K is not on it.)
 //   warp 8      CTA 0: QK issuer for even tiles      (issuers run as converged warps, one elected lane
@@ -74,10 +77,6 @@
 #ifndef MXDSA_OUT_TILES
 #define MXDSA_OUT_TILES 2
 #endif
-#ifndef MXDSA_K_STAGES
-#define MXDSA_K_STAGES 2
-#define MXDSA_V_STAGES 2
-#endif
 #ifndef MXDSA_S_BUFS
 #define MXDSA_S_BUFS 3
 #endif
@@ -90,8 +89,7 @@ static constexpr int kHeads = 64;
 static constexpr int kDim = 512;
 static constexpr int kRowBytes = 528;
 static constexpr int kTileKeys = 128;    // keys per tensor-core tile
-static constexpr int kKStages = MXDSA_K_STAGES;       // K ring depth (32 KB per stage and CTA); freed as soon as QK is done
-static constexpr int kVStages = MXDSA_V_STAGES;       // V ring depth (32 KB per stage and CTA); held until PV is done
+static constexpr int kStages = 4;        // ring of KV tiles (32 KB per stage and CTA); held until PV is done
 static constexpr int kOutTiles = MXDSA_OUT_TILES;   // staging tiles per epilogue warp: stores in flight while the next tile is filled
 static constexpr int kSBufs = MXDSA_S_BUFS;      // S (quantised probabilities) ring: how far the softmax may run ahead of PV
 #ifndef MXDSA_SC_STAGES
@@ -180,15 +178,14 @@ struct WorkItem {
 
 struct __align__(1024) SmemPlan {
     uint8_t q[4 * 64 * 128];                       // [chunk][head][128 B], 128-byte swizzle
-    uint8_t k[kKStages][4 * 64 * 128];             // [chunk][key of this CTA][128 B]
-    uint8_t v[kVStages][2 * 128 * 128];            // [chunk of this CTA][key][128 B]
+    uint8_t kv[kStages][4 * 64 * 128];             // K: [chunk][key of this CTA][128 B]; V after the exchange of one half
     uint8_t s[kSBufs][64 * 128];                        // [row][128 keys], 128-byte swizzle
 #if MXDSA_TMA_EPILOGUE
     uint8_t o_stage[4][kOutTiles][32 * 64];        // per epilogue warp: tiles of 32 rows x 32 bf16 on their way out, 64-byte swizzle
 #endif
-    __align__(16) uint16_t kvalid[kKStages][8];     // validity bits of the tile's keys, 16 per entry (K ring)
+    __align__(16) uint16_t kvalid[kStages][8];      // validity bits of the tile's keys, 16 per entry
     __align__(128) uint32_t q_sf[64 * 4];          // scale rows for tcgen05.cp (64 rows x 16 B)
-    __align__(128) uint32_t k_sf[kKStages][64 * 4];   // per K stage: K scale rows for tcgen05.cp, gathered by the producers with the rows
+    __align__(128) uint32_t k_sf[kStages][64 * 4];    // per stage: K scale rows for tcgen05.cp, gathered by the producers with the rows
     __align__(128) uint32_t s_sf[kSBufs][64 * 4];
     __align__(16) float tok_scale[kScStages][kTileKeys];
     __align__(16) uint32_t valid[kScStages][4];
@@ -198,8 +195,8 @@ struct __align__(1024) SmemPlan {
     uint64_t bar_q_landed;                         // local: Q bytes landed
     uint64_t bar_q_full;                           // CTA0: Q data + scale rows of both CTAs ready
     uint64_t bar_q_empty;                          // both: every QK of the pair finished (2 arrivals)
-    uint64_t bar_k_landed[kKStages];               // local: this CTA's K rows landed (128 arrivals)
-    uint64_t bar_v_full[kVStages];                 // CTA0: V rows of both CTAs landed (8 arrivals + 64 KB of gather4 bytes)
+    uint64_t bar_k_landed[kStages];                // local: this CTA's K rows landed (128 arrivals)
+    uint64_t bar_v_full[kStages];                  // CTA0: the exchanged halves of both CTAs landed (8 arrivals + 32 KB of gather4 bytes)
     uint64_t bar_qk_done[kScStages];               // both: QK of tile g finished (ring by g % 4)
     uint64_t bar_pv_done[kScStages];               // both: PV of tile g finished
     uint64_t bar_pv_half[kSBufs];                       // both: first key half accumulated (64-key tiles)
@@ -553,10 +550,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         mbar_init(smem_u32(&sm.bar_q_landed), 1);
         mbar_init(smem_u32(&sm.bar_q_full), 2);
         mbar_init(smem_u32(&sm.bar_q_empty), 2);
-        for (int i = 0; i < kKStages; ++i) {
+        for (int i = 0; i < kStages; ++i) {
             mbar_init(smem_u32(&sm.bar_k_landed[i]), 128 + 4);   // 128 copy completions + one plain arrival per producer warp
-        }
-        for (int i = 0; i < kVStages; ++i) {
             mbar_init(smem_u32(&sm.bar_v_full[i]), 8);
         }
         for (int i = 0; i < kScStages; ++i) {
@@ -611,7 +606,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     tc_fence_after();
 
     const uint64_t desc_k128 = smem_desc_base(16, 1024, 2);   // K-major, 128-byte swizzle
-    const uint64_t desc_v = smem_desc_base(16384, 1024, 2);   // MN-major, 128-byte swizzle
+    const uint64_t desc_v = smem_desc_base(8192, 1024, 2);    // MN-major, 128-byte swizzle
     const uint64_t desc_sf = smem_desc_base(0, 128, 0);       // scale rows, 16 bytes each
 
     // ------------------------------------------------------------------ roles
@@ -644,7 +639,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             TileCursor<DECODE, NT> ck(p);
             uint32_t kt = 0;
             int idx = ck.live ? key_index<DECODE>(p, ck.w, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64) : -1;
-            const uint32_t k_stage0 = smem_u32(sm.k[0]) + (lane / 8) * 8192;
+            const uint32_t k_stage0 = smem_u32(sm.kv[0]) + (lane / 8) * 8192;
             // Where the key's row and scale slot are is worked out as soon as the tile's index is back, before the
             // wait for a free stage: the wait then covers what is left of the index load's latency.
             const uint8_t* cur = nullptr;
@@ -658,10 +653,10 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             if (ck.live) resolve_tile();
 #pragma unroll 1
             while (ck.live) {
-                const uint32_t s = kt % kKStages;
-                if (kt >= (uint32_t)kKStages) {   // stage s was last used by tile kt-2: its QK must be done
-                    const uint32_t g = kt - kKStages;
-                    MXDSA_WAIT(sm.bar_qk_done[g % kScStages], (g / kScStages) & 1, 10);
+                const uint32_t s = kt % kStages;
+                if (kt >= (uint32_t)kStages) {   // stage s was last used by tile kt-4: its PV must be done
+                    const uint32_t g = kt - kStages;
+                    MXDSA_WAIT(sm.bar_pv_done[g % kScStages], (g / kScStages) & 1, 10);
                 }
                 // The index rows are read once, front to back, and never fit in L2 as a whole: four lanes of one
                 // warp ask for the 512 bytes that a tile further on will need, so that the index loads of all three
@@ -700,57 +695,53 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         } else {
             if constexpr (kRebalanceRegs) setmaxnreg_dec<kRegsGather>();
             // ===================== V producers (warps 4-7): TMA gather4 =====================
-            // CTA c stages bytes 256c .. 256c+255 of all 128 keys of a tile as [chunk of 128 B][key][128 B].
-            // Warp pw takes keys 32*pw .. 32*pw+31; its lanes 0-7 own four keys each and issue two gather4
-            // copies (one per chunk) of four rows (measured: the copy engine takes requests fastest from a few
-            // lanes of several warps -- 4 warps x 8 lanes reach 21 B/clk, one warp of 32 lanes 8 B/clk).  Rows
-            // that do not exist (index -1, position beyond the list, row outside the store) get a coordinate
-            // outside the tensor map, which the copy engine fills with zeros.  The bytes of both CTAs complete
-            // on ONE barrier of CTA 0, where the PV issuer waits; nothing else needs to know that V has landed.
+            // V of CTA c = bytes 256c .. 256c+255 of all 128 keys.  Its own 64 keys are in shared memory already: the
+            // 128-byte chunks 2c, 2c+1 of the K tile.  Chunks 2(1-c), 2(1-c)+1 belong to the peer and are free once the
+            // tile's QK is done in both CTAs; the peer's 64 keys go there.  In both CTAs chunks 0, 1 then hold keys
+            // 0-63 and chunks 2, 3 keys 64-127, so one descriptor serves the pair.  Against gathering all 128 keys into
+            // a ring of their own this halves the requests and a quarter of the L2 reads disappear (64 -> 48 KB per
+            // tile and CTA), and the same 128 KB of shared memory hold four tiles in flight instead of two and two:
+            // 65 536 tokens at topk 4096 21.0 -> 20.2 ms, decode of 128 requests at 4224 keys 374 -> 359 us.
+            // Lanes 0-7 of every warp request four keys x 128 bytes each (measured: the copy engine takes requests
+            // fastest from a few lanes of several warps).  Rows that do not exist (index -1, position beyond the list,
+            // row outside the store) get a coordinate outside the tensor map, which the copy engine fills with zeros.
+            // The bytes of both CTAs complete on ONE barrier of CTA 0, where the PV issuer waits; nothing else needs
+            // to know that V has landed.  Every lane turns one index into a row coordinate, ahead of the wait for
+            // "QK done", and the index load it needs is issued before the requests of the tile before it.
             const int pw = warp - 4;
-            const int jl = 32 * pw + lane;               // the key whose row this lane works out
-            const int j0 = 32 * pw + 4 * (lane & 7);     // first of the four keys this lane requests (lanes 0-7)
+            const int other = 1 - (int)cta;              // the 64-key half of a tile that the peer CTA holds
+            const int jl = 16 * pw + (lane & 15);        // the key of that half whose row this lane works out
             TileCursor<DECODE, NT> cv(p);
             uint32_t vt = 0;
             const uint32_t v_full0 = map_to_cta(smem_u32(&sm.bar_v_full[0]), 0);
-            const uint32_t v_dst0 = smem_u32(sm.v[0]) + j0 * 128;
-            // Every lane turns ONE index into a row coordinate and the requesting lanes collect four of them: the
-            // warp's instructions are issued between those of six other warps of its scheduler, and a chain of
-            // address arithmetic four keys long per lane cost about 1000 cycles per tile.  The coordinates of a
-            // tile are worked out right after the requests of the tile before it, ahead of the wait for a free
-            // stage, and the index load they need is issued before those requests, which hold the warp long
-            // enough for it to come back.
+            const int col = 256 * (int)cta + 128 * (lane & 1);
+            const uint32_t v_dst0 = smem_u32(sm.kv[0]) + (2 * other + (lane & 1)) * 8192 + (16 * pw + 4 * ((lane >> 1) & 3)) * 128;
             int row = -1;
             const void* map = &maps.kv;
             auto locate = [&](int idx) {
-                const int blk = cv.w.blk_begin + 2 * cv.t + jl / 64;   // the same block for the warp's 32 keys
-                row = key_row<DECODE>(p, cv.w, blk, jl % 64, idx);
+                const int blk = cv.w.blk_begin + 2 * cv.t + other;
+                row = key_row<DECODE>(p, cv.w, blk, jl, idx);
                 map = key_map<DECODE>(p, maps, cv.w, blk);
             };
             bool live = cv.live;
-            if (live) locate(key_index<DECODE>(p, cv.w, cv.w.blk_begin + 2 * cv.t + jl / 64, jl % 64));
+            if (live) locate(key_index<DECODE>(p, cv.w, cv.w.blk_begin + 2 * cv.t + other, jl));
 #pragma unroll 1
             while (live) {
-                const uint32_t s = vt % kVStages;
-                if (vt >= (uint32_t)kVStages) {   // stage s was last used by tile vt-3: its PV must be done
-                    const uint32_t g = vt - kVStages;
-                    MXDSA_WAIT(sm.bar_pv_done[g % kScStages], (g / kScStages) & 1, 11);
-                }
+                const uint32_t s = vt % kStages;
                 const void* map_cur = map;
                 int r[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) r[i] = __shfl_sync(0xffffffffu, row, 4 * (lane & 7) + i);
+                for (int i = 0; i < 4; ++i) r[i] = __shfl_sync(0xffffffffu, row, 4 * ((lane >> 1) & 3) + i);
                 cv.advance();
                 live = cv.live;
                 int idx = -1;
-                if (live) idx = key_index<DECODE>(p, cv.w, cv.w.blk_begin + 2 * cv.t + jl / 64, jl % 64);
-                if (lane == 0) mbar_expect_tx_cluster(v_full0 + s * 8, 2 * 32 * 128);
+                if (live) idx = key_index<DECODE>(p, cv.w, cv.w.blk_begin + 2 * cv.t + other, jl);
+                // the half that is about to be overwritten has been read once the tile's QK is done
+                MXDSA_WAIT(sm.bar_qk_done[vt % kScStages], (vt / kScStages) & 1, 11);
+                if (lane == 0) mbar_expect_tx_cluster(v_full0 + s * 8, 16 * 256);
                 __syncwarp();
-                if (lane < 8) {
-                    const uint32_t dst = v_dst0 + s * 32768;
-                    tma_gather4_pair(dst, map_cur, 256 * (int)cta, r[0], r[1], r[2], r[3], v_full0 + s * 8, MXDSA_V_HINT);
-                    tma_gather4_pair(dst + 16384, map_cur, 256 * (int)cta + 128, r[0], r[1], r[2], r[3], v_full0 + s * 8, MXDSA_V_HINT);
-                }
+                if (lane < 8)
+                    tma_gather4_pair(v_dst0 + s * 32768, map_cur, col, r[0], r[1], r[2], r[3], v_full0 + s * 8, MXDSA_V_HINT);
                 __syncwarp();
                 ++vt;
                 if (live) locate(idx);
@@ -785,7 +776,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
 #pragma unroll 1
                 for (int t = 0; t < ntiles; ++t, ++gt) {
                     if ((gt & 1) != e) continue;
-                    const uint32_t s = gt % kKStages;
+                    const uint32_t s = gt % kStages;
                     const uint32_t sc = gt % kScStages, sph = (gt / kScStages) & 1;
                     const uint32_t bph = (gt >> 1) & 1;
                     MXDSA_WAIT_TIGHT(sm.bar_sc_full[sc], sph, 21);
@@ -799,7 +790,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                         if (!mine)   // first own tile of this pair: the pair's Q scale rows
                             tmem_cp_sf_pair(sfa0, smem_desc(desc_sf, smem_u32(sm.q_sf)));
                         tmem_cp_sf_pair(sfb0, smem_desc(desc_sf, smem_u32(sm.k_sf[s])));
-                        const uint64_t b_base = smem_desc(desc_k128, smem_u32(sm.k[s]));
+                        const uint64_t b_base = smem_desc(desc_k128, smem_u32(sm.kv[s]));
 #pragma unroll
                         for (int kk = 0; kk < 16; ++kk) {
                             // Q bytes (kk%8)*64 + (kk/8)*32 of the row meet K bytes 32*kk
@@ -845,12 +836,12 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 tc_fence_after();
 #pragma unroll 1
                 for (int t = 0; t < ntiles; ++t, ++gt) {
-                    const uint32_t s = gt % kVStages, ph = (gt / kVStages) & 1;
+                    const uint32_t s = gt % kStages, ph = (gt / kStages) & 1;
                     const uint32_t b = gt % kSBufs, bph = (gt / kSBufs) & 1;   // S buffer and the phase of its barriers
                     const uint32_t sc = gt % kScStages;
                     MXDSA_WAIT_TIGHT(sm.bar_v_full[s], ph, 34);
                     const uint64_t a_base = smem_desc(desc_k128, smem_u32(sm.s[b]));
-                    const uint64_t b_base = smem_desc(desc_v, smem_u32(sm.v[s]));
+                    const uint64_t b_base = smem_desc(desc_v, smem_u32(sm.kv[s]));
                     const uint32_t sfa = tmem + kColSs + 4 * b;
                     const bool fresh = t == 0;
 #pragma unroll
@@ -865,7 +856,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                             for (int i = (NT == 64 ? 4 * h : 0); i < 4 * h + 4; ++i) {
                                 const int ks = i >> 1, n = i & 1;   // key step (32 keys), dim chunk (128 dims of each CTA)
                                 mma_mxf8<2>(tmem + kColO + n * 128, a_base + ((ks * 32) >> 4),
-                                            b_base + ((n * 16384 + ks * 4096) >> 4),
+                                            b_base + (((ks >> 1) * 16384 + n * 8192 + (ks & 1) * 4096) >> 4),
                                             mx_idesc(128, 256, true, ks, NT == 64 ? (ks & 1) : ks), sfa,
                                             tmem + kColVs + 4 * n, !(fresh && ks == 0));
                             }
@@ -935,8 +926,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
 #pragma unroll 1
             for (int t = 0; t < ntiles; ++t) {
                 const uint32_t sc = gt % kScStages, sph = (gt / kScStages) & 1;
-                const uint32_t ks = gt % kKStages;
-                MXDSA_WAIT_TIGHT(sm.bar_k_landed[ks], (gt / kKStages) & 1, 44);
+                const uint32_t ks = gt % kStages;
+                MXDSA_WAIT_TIGHT(sm.bar_k_landed[ks], (gt / kStages) & 1, 44);
                 // The K rows, the scale rows and the validity bits of this CTA have landed.  Publish at once (the
                 // fence makes what cp.async wrote visible to the tensor core), then derive what the softmax reads.
                 fence_proxy_async_smem();
