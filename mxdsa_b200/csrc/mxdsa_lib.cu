@@ -129,9 +129,6 @@ int make_out_map(CUtensorMap* map, void* base, uint64_t tokens) {
 
 constexpr size_t kSmemBytes = sizeof(mxdsa::SmemPlan) + 1024;
 
-#ifndef MXDSA_COMBINE_PDL
-#define MXDSA_COMBINE_PDL 1
-#endif
 #ifndef MXDSA_GROUPS_PREFILL
 #define MXDSA_GROUPS_PREFILL 3
 #endif
@@ -278,26 +275,38 @@ __global__ void __launch_bounds__(32) mxdsa_sched_whole_kernel(int b, int topk, 
 
 // ------------------------------------------------------------------------------------------
 // Split combine.  A request whose key blocks were divided between sm-parts has one fp32 partial
-// (O/l, log2 l + m) per split.  Every split request ends some part while continuing into the
-// next one; the part in which it STARTS (split 0) owns its merge.  One CTA per (part, token,
-// group of 8 heads), one warp per head:
+// (O/l, log2 l + m) per split:
 //   g = log2 sum_i 2^lse_i ; lse = g / log2e ; with a sink g += log2(1 + 2^(sink*log2e - g));
 //   out = sum_i 2^(lse_i - g) * o_i                       (reference csrc/split_kv/combine.cu:66-160)
+// A unit of work is a divided request.  With no more requests than parts the grid counts requests; otherwise it
+// counts parts, and the part in which a divided request STARTS (split 0) owns its merge (every divided request ends
+// some part while continuing into the next one).  WPH warps share a head, 512 / WPH dims each; a lane keeps eight
+// 16-byte loads in flight, the first of them issued before the weights are worked out.
+// Bound: latency while few requests are divided -- one request of one token over 34 splits is 64 heads x 34 rows, which
+// a warp per head with one row in flight took 14.5 us to walk, four warps per head with eight rows in flight 4.9 us --
+// and L2 bandwidth when every part ends inside a request: then a warp per head (WPH = 1) has all the parallelism the
+// SMs hold, and more warps only add latency chains (128 requests of 6 tokens on 24 parts: 9.9 us, WPH = 4 22 us).
 // ------------------------------------------------------------------------------------------
 constexpr int kMaxSplits = 192;
+constexpr int kCombineWarps = 8;
 
-__global__ void __launch_bounds__(256) mxdsa_combine_kernel(int b, int s_q, int parts, const int* meta,
-                                                           const int* num_splits, const float* o_accum,
-                                                           const float* lse_accum, const float* sink,
-                                                           __nv_bfloat16* out, float* lse) {
-    __shared__ float weight[8][kMaxSplits];
-    const int part = blockIdx.x / s_q, tok = blockIdx.x % s_q;
+template <int WPH>
+__global__ void __launch_bounds__(kCombineWarps * 32)
+mxdsa_combine_kernel(int b, int s_q, int by_request, const int* meta, const int* num_splits, const float* o_accum,
+                     const float* lse_accum, const float* sink, __nv_bfloat16* out, float* lse) {
+    constexpr int kVec = 4 / WPH;        // 16-byte pieces of a partial row per lane
+    constexpr int kAhead = 8 / kVec;     // partial rows in flight
+    const int unit = blockIdx.x / s_q, tok = blockIdx.x % s_q;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    const int head = blockIdx.y * 8 + warp;
-    const int* rec = meta + 8 * part;
-    const int begin_req = rec[0], r = rec[1];
-    if (begin_req >= b || r < 0 || r >= b) return;
-    if (!(begin_req < r || rec[2] == 0)) return;           // the request started in an earlier part
+    const int head = blockIdx.y * (kCombineWarps / WPH) + warp / WPH, dim = (warp % WPH) * (512 / WPH) + lane * 4;
+    int r = unit;
+    if (!by_request) {
+        const int* rec = meta + 8 * unit;
+        const int begin_req = rec[0];
+        r = rec[1];
+        if (begin_req >= b || r < 0 || r >= b) return;
+        if (!(begin_req < r || rec[2] == 0)) return;       // the request started in an earlier part
+    }
     const int s0 = num_splits[r], n = num_splits[r + 1] - s0;
     if (n <= 1) return;
     // Launched as a programmatic dependent of the attention kernel (mxdsa_decode_fwd), this grid may start while
@@ -306,45 +315,93 @@ __global__ void __launch_bounds__(256) mxdsa_combine_kernel(int b, int s_q, int 
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const float* lse_in = lse_accum + ((long long)s0 * s_q + tok) * 64 + head;
     const long long lse_stride = (long long)s_q * 64;
+    const float* o_in = o_accum + (((long long)s0 * s_q + tok) * 64 + head) * 512 + dim;
+    const long long o_stride = (long long)s_q * 64 * 512;
+    float4 v[kAhead][kVec];
+    auto load = [&](int i0) {            // rows i0 .. i0 + kAhead - 1
+#pragma unroll
+        for (int j = 0; j < kAhead; ++j)
+            if (i0 + j < n) {
+#pragma unroll
+                for (int c = 0; c < kVec; ++c) v[j][c] = *reinterpret_cast<const float4*>(o_in + (i0 + j) * o_stride + c * 128);
+            }
+    };
+    load(0);
+    float w[kMaxSplits / 32];            // lane i holds the splits i, i + 32, ...: first their lse, then their weight
     float mx = -CUDART_INF_F;
-    for (int i = lane; i < n; i += 32) mx = fmaxf(mx, lse_in[i * lse_stride]);
+#pragma unroll
+    for (int k = 0; k < kMaxSplits / 32; ++k) {
+        const int i = 32 * k + lane;
+        w[k] = i < n ? lse_in[i * lse_stride] : -CUDART_INF_F;
+        mx = fmaxf(mx, w[k]);
+    }
     for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
     if (mx == -CUDART_INF_F) mx = 0.f;
     float sum = 0.f;
-    for (int i = lane; i < n; i += 32) sum += sm100::ex2_approx(lse_in[i * lse_stride] - mx);
+#pragma unroll
+    for (int k = 0; k < kMaxSplits / 32; ++k) sum += sm100::ex2_approx(w[k] - mx);
     for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     float g = sum == 0.f ? CUDART_INF_F : sm100::lg2_approx(sum) + mx;
-    if (lane == 0) lse[((long long)r * s_q + tok) * 64 + head] = g / 1.4426950408889634f;
+    if (lane == 0 && warp % WPH == 0) lse[((long long)r * s_q + tok) * 64 + head] = g / 1.4426950408889634f;
     if (sink != nullptr) {
         const float sk = sink[head];
         if (g != CUDART_INF_F) g += sm100::lg2_approx(1.f + sm100::ex2_approx(sk * CUDART_L2E_F - g));
         else g = sk == -CUDART_INF_F ? CUDART_INF_F : sk * CUDART_L2E_F;
     }
-    for (int i = lane; i < n; i += 32) weight[warp][i] = sm100::ex2_approx(lse_in[i * lse_stride] - g);
-    __syncwarp();
-    const float* o_in = o_accum + (((long long)s0 * s_q + tok) * 64 + head) * 512;
-    const long long o_stride = (long long)s_q * 64 * 512;
-    float4 acc[4];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (int i = 0; i < n; ++i) {
-        const float wgt = weight[warp][i];
+    for (int k = 0; k < kMaxSplits / 32; ++k) w[k] = sm100::ex2_approx(w[k] - g);
+    float4 acc[kVec];
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float4 v = *reinterpret_cast<const float4*>(o_in + i * o_stride + j * 128 + lane * 4);
-            acc[j].x += wgt * v.x;
-            acc[j].y += wgt * v.y;
-            acc[j].z += wgt * v.z;
-            acc[j].w += wgt * v.w;
+    for (int c = 0; c < kVec; ++c) acc[c] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int k = 0; k < kMaxSplits / 32; ++k) {
+        if (32 * k >= n) break;
+        const int last = min(n, 32 * k + 32);
+        for (int i0 = 32 * k; i0 < last; i0 += kAhead) {
+            if (i0 > 0) load(i0);
+#pragma unroll
+            for (int j = 0; j < kAhead; ++j) {
+                const float wgt = __shfl_sync(0xffffffffu, w[k], (i0 + j) & 31);
+                if (i0 + j < last) {
+#pragma unroll
+                    for (int c = 0; c < kVec; ++c) {
+                        acc[c].x += wgt * v[j][c].x;
+                        acc[c].y += wgt * v[j][c].y;
+                        acc[c].z += wgt * v[j][c].z;
+                        acc[c].w += wgt * v[j][c].w;
+                    }
+                }
+            }
         }
     }
-    __nv_bfloat16* dst = out + (((long long)r * s_q + tok) * 64 + head) * 512;
+    __nv_bfloat16* dst = out + (((long long)r * s_q + tok) * 64 + head) * 512 + dim;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        __nv_bfloat162 lo = __floats2bfloat162_rn(acc[j].x, acc[j].y), hi = __floats2bfloat162_rn(acc[j].z, acc[j].w);
-        uint2 pk = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
-        *reinterpret_cast<uint2*>(dst + j * 128 + lane * 4) = pk;
+    for (int c = 0; c < kVec; ++c) {
+        const __nv_bfloat162 lo = __floats2bfloat162_rn(acc[c].x, acc[c].y), hi = __floats2bfloat162_rn(acc[c].z, acc[c].w);
+        *reinterpret_cast<uint2*>(dst + c * 128) =
+            make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
     }
+}
+
+int launch_combine(int b, int s_q, int parts, const int* meta, const int* num_splits, const float* o_accum,
+                   const float* lse_accum, const float* sink, __nv_bfloat16* out, float* lse, bool dependent, int sms,
+                   cudaStream_t stream) {
+    const int by_request = b <= parts;
+    const int units = (by_request ? b : parts) * s_q;
+    // 64 heads a unit: from 16 warps an SM on a warp per head fills the SMs
+    const bool wide = units * MXDSA_HEADS < 16 * sms;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)units, MXDSA_HEADS / kCombineWarps * (wide ? 4 : 1), 1);
+    cfg.blockDim = dim3(kCombineWarps * 32, 1, 1);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = dependent ? 1 : 0;
+    MX_CUDA(cudaLaunchKernelEx(&cfg, wide ? mxdsa_combine_kernel<4> : mxdsa_combine_kernel<1>, b, s_q, by_request, meta,
+                               num_splits, o_accum, lse_accum, sink, out, lse));
+    return MXDSA_OK;
 }
 
 }  // namespace
@@ -638,24 +695,10 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     st = launch_pairs(mxdsa::mxdsa_attn_kernel<true, 64, MXDSA_GROUPS_DECODE>, MXDSA_GROUPS_DECODE, grid, stream, ap, maps);
     if (st != MXDSA_OK) return st;
     if (!combine) return MXDSA_OK;
-    const dim3 cgrid(p->num_sm_parts * p->s_q, MXDSA_HEADS / 8, 1);
     // programmatic dependent launch: the combine grid is set up while the attention grid drains (the attention
     // kernel releases its dependents as soon as it has started; the combine kernel waits before it reads)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = cgrid;
-    cfg.blockDim = dim3(256, 1, 1);
-    cfg.dynamicSmemBytes = 0;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = MXDSA_COMBINE_PDL;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    MX_CUDA(cudaLaunchKernelEx(&cfg, mxdsa_combine_kernel, (int)p->b, (int)p->s_q, (int)p->num_sm_parts,
-                               (const int*)p->sched_meta, (const int*)p->num_splits, (const float*)o_accum,
-                               (const float*)lse_accum, (const float*)p->attn_sink,
-                               static_cast<__nv_bfloat16*>(p->out), (float*)p->lse));
-    return MXDSA_OK;
+    return launch_combine(p->b, p->s_q, p->num_sm_parts, p->sched_meta, p->num_splits, o_accum, lse_accum, p->attn_sink,
+                          static_cast<__nv_bfloat16*>(p->out), p->lse, true, d->sm_count, stream);
 }
 
 extern "C" int mxdsa_decode_fwd(const mxdsa_decode_params* p) { return decode_impl(p, true); }
@@ -682,12 +725,12 @@ extern "C" int mxdsa_decode_combine(const mxdsa_combine_params* p) {
     const size_t slots = (size_t)(p->b + p->num_sm_parts) * p->s_q * MXDSA_HEADS;
     const float* o_accum = static_cast<const float*>(p->workspace);
     const float* lse_accum = o_accum + slots * MXDSA_DIM;
-    const dim3 cgrid(p->num_sm_parts * p->s_q, MXDSA_HEADS / 8, 1);
-    mxdsa_combine_kernel<<<cgrid, 256, 0, static_cast<cudaStream_t>(p->stream)>>>(
-        p->b, p->s_q, p->num_sm_parts, p->sched_meta, p->num_splits, o_accum, lse_accum, p->attn_sink,
-        static_cast<__nv_bfloat16*>(p->out), p->lse);
-    MX_CUDA(cudaGetLastError());
-    return MXDSA_OK;
+    DeviceInfo* d = nullptr;
+    const int st = device_info(&d);
+    if (st != MXDSA_OK) return st;
+    return launch_combine(p->b, p->s_q, p->num_sm_parts, p->sched_meta, p->num_splits, o_accum, lse_accum, p->attn_sink,
+                          static_cast<__nv_bfloat16*>(p->out), p->lse, false, d->sm_count,
+                          static_cast<cudaStream_t>(p->stream));
 }
 
 // ------------------------------------------------------------------------------------------
