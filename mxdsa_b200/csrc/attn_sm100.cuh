@@ -100,6 +100,7 @@ static constexpr int kScStages = MXDSA_SC_STAGES;      // scale/validity ring de
 // registers per thread that a launch of 512 + 128 G threads gets (65536 / threads, rounded down to a multiple of 8)
 __host__ __device__ constexpr int launch_regs(int g) { return g == 2 ? 80 : 72; }
 static constexpr int kBaseThreads = 512;   // warps 0-11: K producers, V producers, control; then G x 4 softmax warps; then 4 epilogue warps
+static constexpr uint32_t kBarTmem = 7;    // named barrier: tensor memory allocated (warp 10 -> warps 12-15)
 static constexpr int kMaxGroups = 3;     // softmax groups of four warps (template parameter G = 2 or 3); tile g is handled by group g % G
 
 // tensor-memory columns
@@ -172,6 +173,9 @@ struct WorkItem {
     int len, elen;      // attended lengths
     int n_main_blocks;  // 64-key blocks of the main part
     int blk_begin, blk_end;
+};
+// Where a work item's result goes.
+struct WorkOutput {
     int split;          // decode: 1 -> write fp32 partials for the combine step
     int split_idx;
 };
@@ -210,30 +214,35 @@ struct __align__(1024) SmemPlan {
     uint64_t bar_os_empty[2];                      // local: the epilogue warps have read it (4 arrivals)
     uint64_t bar_o_empty;                          // CTA0: epilogue has drained O (4 warps of each CTA)
     uint64_t bar_m_ready[kMaxGroups];                 // local: group g published the running max of its tile
+    uint64_t bar_tmem_ready;                       // CTA0: tensor memory allocated and V scales written in both CTAs (4 warps each)
     uint32_t tmem_base;
     int abort_word;
     DeviceFault* fault;                            // copy of the kernel parameter, for the out-of-line wait path
 };
 
 // ----------------------------------------------------------------------------------------------
+// The roles walk the schedule independently.  What an iterator keeps in registers is its position alone: the schedule
+// record is read again (from L1) where it is needed, because every role holds its iterator across the tile loop.
 template <bool DECODE> struct WorkIter {
     const AttnParams& p;
     int next_pair, pair_step;      // prefill
     int req, end_req;              // decode
-    int meta[8];
-    bool started;
 
-    __device__ WorkIter(const AttnParams& params) : p(params), started(false) {
+    __device__ static int4 record(const AttnParams& p, int half) {
+        int4 v;
+        asm volatile("ld.global.nc.v4.s32 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+                     : "l"(p.sched_meta + 8 * blockIdx.y + 4 * half));
+        return v;
+    }
+    __device__ WorkIter(const AttnParams& params) : p(params) {
         if constexpr (!DECODE) {
             next_pair = blockIdx.x / 2;
             pair_step = gridDim.x / 2;
         } else {
-            const int4* m = reinterpret_cast<const int4*>(p.sched_meta + 8 * blockIdx.y);
-            int4 a = __ldg(m), b2 = __ldg(m + 1);
-            meta[0] = a.x; meta[1] = a.y; meta[2] = a.z; meta[3] = a.w;
-            meta[4] = b2.x; meta[5] = b2.y; meta[6] = b2.z; meta[7] = b2.w;
-            req = meta[0];
-            end_req = meta[0] >= p.b ? -1 : meta[1];
+            const int4 a = record(p, 0);
+            req = a.x;
+            end_req = a.x >= p.b ? -1 : a.y;
         }
     }
     template <int NT> __device__ bool next(WorkItem& w) {
@@ -250,12 +259,11 @@ template <bool DECODE> struct WorkIter {
             w.n_main_blocks = ntiles * (NT / 64);
             w.blk_begin = 0;
             w.blk_end = w.n_main_blocks;
-            w.split = 0;
-            w.split_idx = 0;
             return true;
         } else {
             if (req > end_req) return false;
             const int r = req++;
+            const int4 a = record(p, 0);
             w.req = r;
             w.pair = blockIdx.x / 2;
             w.row = p.indices + (long long)r * p.idx_stride_b + (long long)w.pair * p.idx_stride_row;
@@ -266,19 +274,26 @@ template <bool DECODE> struct WorkIter {
             w.elen = p.extra_topk > 0 ? (p.extra_topk_length ? __ldg(p.extra_topk_length + r) : p.extra_topk) : 0;
             w.n_main_blocks = max((w.len + 63) / 64, 1);
             const int total = w.n_main_blocks + (w.elen + 63) / 64;
-            w.blk_begin = r == meta[0] ? meta[2] : 0;
-            w.blk_end = r == meta[1] ? meta[3] : total;
-            w.split = r == meta[0] ? meta[5] : (r == meta[1] ? meta[6] : 0);
-            w.split_idx = __ldg(p.num_splits + r) + (r == meta[0] ? meta[4] : 0);
-            if (w.split && p.o_accum == nullptr) {
+            w.blk_begin = r == a.x ? a.z : 0;
+            w.blk_end = r == a.y ? a.w : total;
+            return true;
+        }
+    }
+    __device__ WorkOutput output(const WorkItem& w) const {
+        WorkOutput o = {0, 0};
+        if constexpr (DECODE) {
+            const int4 a = record(p, 0), c = record(p, 1);
+            o.split = w.req == a.x ? c.y : (w.req == a.y ? c.z : 0);
+            o.split_idx = __ldg(p.num_splits + w.req) + (w.req == a.x ? c.x : 0);
+            if (o.split && p.o_accum == nullptr) {
                 // a divided request in a launch without partials (decode without a combine pass needs a schedule of
                 // whole requests): flag it and write what this part has straight to `out` rather than through a
                 // null pointer
                 if (atomicCAS(&p.fault->flag, 0, 1) == 0) p.fault->where = 71;
-                w.split = 0;
+                o.split = 0;
             }
-            return true;
         }
+        return o;
     }
 };
 
@@ -543,71 +558,70 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     const uint32_t cta = cluster_cta_rank();
 
     // ------------------------------------------------------------------ set-up
-    // decode: the combine grid that follows may be set up from now on (it waits for this grid's completion
-    // before it reads the partials)
-    if constexpr (DECODE) asm volatile("griddepcontrol.launch_dependents;");
-    if (threadIdx.x == 0) {
-        mbar_init(smem_u32(&sm.bar_q_landed), 1);
-        mbar_init(smem_u32(&sm.bar_q_full), 2);
-        mbar_init(smem_u32(&sm.bar_q_empty), 2);
-        for (int i = 0; i < kStages; ++i) {
-            mbar_init(smem_u32(&sm.bar_k_landed[i]), 128 + 4);   // 128 copy completions + one plain arrival per producer warp
-            mbar_init(smem_u32(&sm.bar_v_full[i]), 8);
+    // A programmatic dependent of whatever precedes it on the stream: set-up overlaps that grid's tail, and nothing
+    // in global memory is touched before the wait.  Its own dependents may be set up from now on (they wait for this
+    // grid's completion in the same way).
+    // What bounds a small call is this start, not the tiles: with one thread initialising sixty barriers, three
+    // cluster barriers in a row, the schedule and index loads behind them and parts without work going through all of
+    // it, the first row was asked for 8 000 cycles after the start; now 4 500.  With the launch overlap: 256 tokens at
+    // topk 128 18.4 -> 14.4 us per call, 37 requests of 2 tokens 25.3 -> 21.7 us, one request of one token 19.8 -> 15.7.
+    grid_launch_dependents();
+    if constexpr (DECODE) {
+        // parts without work (few requests on many parts) leave before they set anything up; the schedule is read
+        // while the barriers are initialised
+        grid_dependency_wait();
+        const int2 rec = __ldg(reinterpret_cast<const int2*>(p.sched_meta + 8 * blockIdx.y));
+        if (rec.x >= p.b || rec.x > rec.y) return;   // the same for both CTAs of the pair
+    }
+    if (warp == 0) {   // one lane per ring slot: a handful of initialisations in a row instead of sixty
+        if (lane < kStages) {
+            mbar_init(smem_u32(&sm.bar_k_landed[lane]), 128 + 4);   // 128 copy completions + one plain arrival per producer warp
+            mbar_init(smem_u32(&sm.bar_v_full[lane]), 8);
         }
-        for (int i = 0; i < kScStages; ++i) {
-            mbar_init(smem_u32(&sm.bar_qk_done[i]), 1);
-            mbar_init(smem_u32(&sm.bar_pv_done[i]), 1);
-            mbar_init(smem_u32(&sm.bar_sc_full[i]), 2);
-            mbar_init(smem_u32(&sm.bar_tok_full[i]), 1);
-            mbar_init(smem_u32(&sm.bar_tok_empty[i]), 4);
+        if (lane < kScStages) {
+            mbar_init(smem_u32(&sm.bar_qk_done[lane]), 1);
+            mbar_init(smem_u32(&sm.bar_pv_done[lane]), 1);
+            mbar_init(smem_u32(&sm.bar_sc_full[lane]), 2);
+            mbar_init(smem_u32(&sm.bar_tok_full[lane]), 1);
+            mbar_init(smem_u32(&sm.bar_tok_empty[lane]), 4);
         }
-        for (int i = 0; i < 2; ++i) mbar_init(smem_u32(&sm.bar_p_empty[i]), 8);
-        for (int i = 0; i < kSBufs; ++i) {
-            mbar_init(smem_u32(&sm.bar_s_full[i][0]), 8);
-            mbar_init(smem_u32(&sm.bar_s_full[i][1]), 8);
-            mbar_init(smem_u32(&sm.bar_pv_half[i]), 1);
+        if (lane < kSBufs) {
+            mbar_init(smem_u32(&sm.bar_s_full[lane][0]), 8);
+            mbar_init(smem_u32(&sm.bar_s_full[lane][1]), 8);
+            mbar_init(smem_u32(&sm.bar_pv_half[lane]), 1);
         }
-        mbar_init(smem_u32(&sm.bar_o_empty), 8);
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(smem_u32(&sm.bar_os_full[i]), 2);
-            mbar_init(smem_u32(&sm.bar_os_empty[i]), 4);
+        if (lane < 2) {
+            mbar_init(smem_u32(&sm.bar_p_empty[lane]), 8);
+            mbar_init(smem_u32(&sm.bar_os_full[lane]), 2);
+            mbar_init(smem_u32(&sm.bar_os_empty[lane]), 4);
         }
-        for (int i = 0; i < kMaxGroups; ++i) mbar_init(smem_u32(&sm.bar_m_ready[i]), 4);
-        sm.abort_word = 0;
-        sm.fault = p.fault;
+        if (lane < kMaxGroups) mbar_init(smem_u32(&sm.bar_m_ready[lane]), 4);
+        if (lane == 8) {
+            mbar_init(smem_u32(&sm.bar_q_landed), 1);
+            mbar_init(smem_u32(&sm.bar_q_full), 2);
+            mbar_init(smem_u32(&sm.bar_q_empty), 2);
+            mbar_init(smem_u32(&sm.bar_o_empty), 8);
+            mbar_init(smem_u32(&sm.bar_tmem_ready), 8);
+        }
+        if (lane == 9) {
+            sm.abort_word = 0;
+            sm.fault = p.fault;
+        }
         fence_mbar_init();
     }
     if (warp == 11 && lane == 0) prefetch_tensormap(&maps.q);
     __syncthreads();
-    cluster_sync();
-    if (warp == 10) {
-        tmem_alloc<2>(smem_u32(&sm.tmem_base), kTmemCols);
-        tmem_relinquish<2>();
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync();
-    tc_fence_after();
-    const uint32_t tmem = sm.tmem_base;
-    if (warp >= 12 && warp < 16) {
-        // V dimension scales (B-operand scale columns of every PV): lanes 0-63 hold the dims of CTA 0's half
-        // (w1), lanes 64-127 those of CTA 1's half (w2); column c = word c.  Written once, straight from
-        // registers; the barriers below order it before the first MMA of either CTA.
-        const uint32_t* wv = (warp & 3) < 2 ? p.w1 : p.w2;
-        uint32_t v[8];
-#pragma unroll
-        for (int c = 0; c < 8; ++c) v[c] = wv[c];
-        tmem_st8(tmem + (uint32_t((warp & 3) * 32) << 16) + kColVs, v);
-        tmem_wait_st();
-    }
-    tc_fence_before();
-    __syncthreads();
-    cluster_sync();
-    tc_fence_after();
+    // From here a role may use this CTA's barriers; the peer's, and its tensor memory, only after cluster_wait().
+    // Every role makes its first global loads (schedule, lengths, indices: three dependent latencies) in between.
+    cluster_arrive();
+    if constexpr (!DECODE) grid_dependency_wait();
 
     const uint64_t desc_k128 = smem_desc_base(16, 1024, 2);   // K-major, 128-byte swizzle
     const uint64_t desc_v = smem_desc_base(8192, 1024, 2);    // MN-major, 128-byte swizzle
     const uint64_t desc_sf = smem_desc_base(0, 128, 0);       // scale rows, 16 bytes each
+
+    uint32_t tmem;
+    asm volatile("mov.u32 %0, 0;" : "=r"(tmem));
 
     // ------------------------------------------------------------------ roles
     // Register budget.  The launch gives every thread kLaunchRegs (the most that 640 or 768 threads can have),
@@ -651,6 +665,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 vbits = __ballot_sync(0xffffffffu, valid);
             };
             if (ck.live) resolve_tile();
+            cluster_wait();
 #pragma unroll 1
             while (ck.live) {
                 const uint32_t s = kt % kStages;
@@ -725,6 +740,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             };
             bool live = cv.live;
             if (live) locate(key_index<DECODE>(p, cv.w, cv.w.blk_begin + 2 * cv.t + other, jl));
+            cluster_wait();
 #pragma unroll 1
             while (live) {
                 const uint32_t s = vt % kStages;
@@ -750,7 +766,9 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     } else if (warp < 12) {
     if constexpr (kRebalanceRegs) setmaxnreg_dec<kRegsCtl>();
     if (warp == 8 || warp == 9) {
-        if (cta == 0) {
+        if (cta != 0) {
+            cluster_wait();
+        } else {
             // ===================== QK issuers (CTA 0): warp 8 even tiles, warp 9 odd tiles ==========
             // The whole warp walks the schedule and waits; one elected lane issues.  Keeping the warp
             // converged lets the descriptor arithmetic run on the uniform datapath, and the 16 steps
@@ -765,6 +783,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             const uint32_t q_empty_peer = map_to_cta(smem_u32(&sm.bar_q_empty), 1);
             const uint64_t a_base = smem_desc(desc_k128, smem_u32(sm.q));
             const uint32_t d_p = tmem + kColP + e * 64, sfa0 = tmem + kColQs + 4 * e, sfb0 = tmem + kColKs + 4 * e;
+            cluster_wait();
+            MXDSA_WAIT_TIGHT(sm.bar_tmem_ready, 0, 23);
 #pragma unroll 1
             while (it.template next<NT>(w)) {
                 const int ntiles = (w.blk_end - w.blk_begin + 1) / 2;
@@ -821,6 +841,11 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             }
         }
     } else if (warp == 10) {
+        cluster_wait();
+        tmem_alloc<2>(smem_u32(&sm.tmem_base), kTmemCols);
+        tmem_relinquish<2>();
+        if (lane == 0 && *(volatile uint32_t*)&sm.tmem_base != tmem) raise_fault(sm, 72);
+        named_bar_arrive(kBarTmem, 160);   // warps 12-15 write the V scales into it
         if (cta == 0) {
             // ===================== PV issuer (CTA 0): converged warp, one elected lane issues ==========
             WorkIter<DECODE> it(p);
@@ -828,6 +853,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             uint32_t gt = 0, gw = 0;
             const uint32_t pv_half_peer = map_to_cta(smem_u32(&sm.bar_pv_half[0]), 1);
             const uint32_t pv_done_peer = map_to_cta(smem_u32(&sm.bar_pv_done[0]), 1);
+            MXDSA_WAIT_TIGHT(sm.bar_tmem_ready, 0, 24);
 #pragma unroll 1
             while (it.template next<NT>(w)) {
                 const int ntiles = (w.blk_end - w.blk_begin + 1) / 2;
@@ -898,7 +924,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 }
             }
             __syncwarp();
-            MXDSA_WAIT(sm.bar_q_empty, (gw & 1) ^ 1, 40);
+            if (gw > 0) MXDSA_WAIT(sm.bar_q_empty, (gw & 1) ^ 1, 40);
             if (lane == 0) {
                 mbar_expect_tx(smem_u32(&sm.bar_q_landed), 4 * 64 * 128);
                 asm volatile(
@@ -920,6 +946,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 fence_proxy_async_smem();
                 __syncwarp();
             }
+            if (gw == 0) cluster_wait();   // ahead of the first arrival on a barrier of the peer
             // ---- per tile: K scale rows, key token scales, validity.  Everything arrives in shared memory with the
             // K rows (the producers gather the scale slots and vote the validity bits), so no global load sits
             // between "K landed" and "QK may start".  lane L looks after keys L, L+32 (block 0) and L+64, L+96.
@@ -954,6 +981,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             }
             ++gw;
         }
+        if (gw == 0) cluster_wait();
     }
     } else if (warp < 12 + 4 * G) {
         if constexpr (kRebalanceRegs) setmaxnreg_inc<kRegsSoftmax>();
@@ -973,6 +1001,23 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         const uint32_t p_empty0 = map_to_cta(smem_u32(&sm.bar_p_empty[0]), 0);
         const uint32_t s_full0 = map_to_cta(smem_u32(&sm.bar_s_full[0][0]), 0);
         const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+        cluster_wait();
+        if (grp == 0) {
+            // V dimension scales (B-operand scale columns of every PV): lanes 0-63 hold the dims of CTA 0's half
+            // (w1), lanes 64-127 those of CTA 1's half (w2); column c = word c.  Written once, straight from
+            // registers, as soon as the tensor memory has been allocated; the MMA issuers wait for both CTAs' four warps.
+            named_bar_sync(kBarTmem, 160);
+            tc_fence_after();
+            const uint32_t* wv = q4 < 2 ? p.w1 : p.w2;
+            uint32_t v[8];
+#pragma unroll
+            for (int c = 0; c < 8; ++c) v[c] = wv[c];
+            tmem_st8(lane_addr + kColVs, v);
+            tmem_wait_st();
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(&sm.bar_tmem_ready), 0));
+        }
         WorkIter<DECODE> it(p);
         WorkItem w;
         uint32_t gt = 0, gw = 0;
@@ -1163,20 +1208,21 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     m = -CUDART_INF_F;
                 }
                 const int tok_idx = 2 * w.pair + (int)cta;
+                const WorkOutput wo = it.output(w);
                 const float sink = p.attn_sink ? __ldg(p.attn_sink + row) : -CUDART_INF_F;
                 float oscale;
-                if (!DECODE || !w.split) oscale = __fdividef(1.0f, l_tot + ex2_approx(fmaf(sink, CUDART_L2E_F, -m)));
+                if (!DECODE || !wo.split) oscale = __fdividef(1.0f, l_tot + ex2_approx(fmaf(sink, CUDART_L2E_F, -m)));
                 else oscale = __fdividef(1.0f, l_tot);
                 if (l_tot == 0.f) oscale = 0.f;
                 if (tok_idx < p.s_q) {
-                    if (!DECODE || !w.split) {
+                    if (!DECODE || !wo.split) {
                         float lse = fmaf(m, CUDART_LN2_F, CUDART_LN2_F * lg2_approx(l_tot));
                         if (l_tot == 0.f || lse == -CUDART_INF_F) lse = CUDART_INF_F;
                         const long long o = ((long long)w.req * p.s_q + tok_idx) * kHeads + row;
                         p.lse[o] = lse;
                         if (!DECODE) p.max_logits[o] = real_all * CUDART_LN2_F;
                     } else {
-                        p.lse_accum[((long long)w.split_idx * p.s_q + tok_idx) * kHeads + row] = lg2_approx(l_tot) + m;
+                        p.lse_accum[((long long)wo.split_idx * p.s_q + tok_idx) * kHeads + row] = lg2_approx(l_tot) + m;
                     }
                 }
                 // oscale is handed over through a two-deep buffer: slot gw & 1 was last used by pair gw - 2
@@ -1200,6 +1246,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         const int half = L / 64;
         const uint32_t lane_addr = tmem + (uint32_t(q4 * 32) << 16);
         const uint32_t o_empty0 = map_to_cta(smem_u32(&sm.bar_o_empty), 0);
+        cluster_wait();
         // O is free for the next pair's first PV as soon as this warp has READ its last columns; the stores of
         // those columns (which may have to wait for a staging tile) follow after the release.
         auto release_o = [&]() {
@@ -1225,7 +1272,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             tc_fence_after();
             const int tok_idx = 2 * w.pair + (int)cta;
             const bool store = tok_idx < p.s_q;
-            if (!DECODE || !w.split) {
+            const WorkOutput wo = it.output(w);
+            if (!DECODE || !wo.split) {
 #if MXDSA_TMA_EPILOGUE
                 // 32 columns at a time: one load becomes 32 rows x 64 bytes of the warp's staging area (16-byte
                 // chunk c of row r sits at chunk c ^ ((r / 2) % 4), the 64-byte swizzle that the tensor map undoes
@@ -1290,7 +1338,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 }
 #endif
             } else {
-                float* dst = p.o_accum + (((long long)w.split_idx * p.s_q + tok_idx) * kHeads + row) * kDim + half * 256;
+                float* dst = p.o_accum + (((long long)wo.split_idx * p.s_q + tok_idx) * kHeads + row) * kDim + half * 256;
 #pragma unroll 1
                 for (int c = 0; c < 256; c += 32) {
                     float o[32];
@@ -1328,8 +1376,11 @@ done:
         named_bar_arrive(1 + kGroups, kGroups * 128);
     }
     tc_fence_before();
-    __syncthreads();
-    cluster_sync();
+    // Nobody leaves while the peer may still signal it.  The epilogue warps arrive without a release: there is
+    // nothing for the peer to read, and a release would wait for the global stores of the last pair.
+    if (warp >= 12 + 4 * G) cluster_arrive_relaxed();
+    else cluster_arrive();
+    cluster_wait();
     if (warp == 10) tmem_dealloc<2>(tmem, kTmemCols);
 }
 

@@ -154,11 +154,13 @@ int launch_pairs(K kernel, int groups, dim3 grid, cudaStream_t stream, const mxd
     cfg.blockDim = dim3(mxdsa::kBaseThreads + 128 * groups);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = stream;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim = {2, 1, 1};
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[2]{};
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim = {2, 1, 1};
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // the kernel waits before it touches global memory
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
     MX_CUDA(cudaLaunchKernelEx(&cfg, kernel, ap, maps));
     return MXDSA_OK;
 }
@@ -300,19 +302,25 @@ mxdsa_combine_kernel(int b, int s_q, int by_request, const int* meta, const int*
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int head = blockIdx.y * (kCombineWarps / WPH) + warp / WPH, dim = (warp % WPH) * (512 / WPH) + lane * 4;
     int r = unit;
+    bool mine = true;
     if (!by_request) {
         const int* rec = meta + 8 * unit;
         const int begin_req = rec[0];
         r = rec[1];
-        if (begin_req >= b || r < 0 || r >= b) return;
-        if (!(begin_req < r || rec[2] == 0)) return;       // the request started in an earlier part
+        // the part in which the request started
+        mine = begin_req < b && r >= 0 && r < b && (begin_req < r || rec[2] == 0);
     }
-    const int s0 = num_splits[r], n = num_splits[r + 1] - s0;
-    if (n <= 1) return;
+    int s0 = 0, n = 0;
+    if (mine) {
+        s0 = num_splits[r];
+        n = num_splits[r + 1] - s0;
+    }
     // Launched as a programmatic dependent of the attention kernel (mxdsa_decode_fwd), this grid may start while
     // that one is still running: everything above reads the schedule only, everything below reads the partials,
-    // which are complete and visible once the wait returns.  After a plain launch the wait returns at once.
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    // which are complete and visible once the wait returns.  After a plain launch the wait returns at once.  Blocks
+    // without work wait as well: the next grid on the stream may count on this grid's end for the attention grid's.
+    sm100::grid_dependency_wait();
+    if (n <= 1) return;
     const float* lse_in = lse_accum + ((long long)s0 * s_q + tok) * 64 + head;
     const long long lse_stride = (long long)s_q * 64;
     const float* o_in = o_accum + (((long long)s0 * s_q + tok) * 64 + head) * 512 + dim;

@@ -127,6 +127,7 @@ SM100_DEVICE void fence_proxy_async_smem() {
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 SM100_DEVICE void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+SM100_DEVICE void cluster_arrive_relaxed() { asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory"); }
 SM100_DEVICE void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 SM100_DEVICE void cluster_sync() {
     cluster_arrive();
@@ -135,6 +136,11 @@ SM100_DEVICE void cluster_sync() {
 SM100_DEVICE void named_bar_sync(uint32_t id, uint32_t threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
+
+// Programmatic dependent launch: dependents of this grid may be set up from now on / wait until the grids that this
+// one depends on have completed and their writes are visible (returns at once after a plain launch).
+SM100_DEVICE void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+SM100_DEVICE void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ----------------------------------------------------------------------------------------------
 // TMA
