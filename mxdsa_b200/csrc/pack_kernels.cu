@@ -5,10 +5,13 @@
 //
 // Same arithmetic as the reference's Python packers (reference tests/mxfp8_test_utils.py:11-27):
 //   scale = 2^ceil(log2(max(amax/448, 2^-126)));  code = e4m3(clamp(x / scale, -448, 448))
-// with the ceil(log2()) taken exactly from the bits of the float (exponent, +1 when the mantissa is
-// not zero).  Compiled WITHOUT fast-math: amax/448 must be the correctly rounded quotient.
+// with the ceil(log2()) taken exactly from the bits of amax (see scale_byte).
 //
-// Bound: HBM.  Algorithmic bytes per row: 512 * sizeof(input element) read + 528 written.
+// Bound: HBM.  Algorithmic bytes per row: 512 * sizeof(input element) read + 528 written.  A warp takes two
+// adjacent rows at a time: both rows' loads are in flight together, and the 1056 bytes it writes for queries begin
+// and end on whole 32-byte sectors.  What used to come before the memory was the instruction count -- a 64-bit
+// division and remainder per row, a rounded float division, two clamps per value, byte stores of the slot; see the
+// comments below for what stands in their place.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -19,13 +22,19 @@ namespace {
 
 constexpr int kDim = 512;
 constexpr int kWarpsPerBlock = 8;
+constexpr int kRowsPerWarp = 2;
 
-// UE8M0 byte of 2^ceil(log2(max(amax/448, 2^-126))) and the factor 2^-e to multiply by
+// UE8M0 byte of 2^ceil(log2(max(amax/448, 2^-126))) and the factor 2^-e to multiply by, without the division.
+// Write amax = m * 2^e, 1 <= m < 2, and 448 = 1.75 * 2^8.  The correctly rounded quotient is at most 2^(e-8) for
+// m <= 1.75 (the value below 1.75 next to it gives 2 - 1.14 ulp, which rounds to 2 - 1 ulp) and above 2^(e-8) for
+// m > 1.75 (the next value above gives 1 + 0.57 ulp, which rounds to 1 + 1 ulp), so the exponent is e - 8 or e - 7:
+// adding 0x1FFFFF to the bits carries into the exponent field exactly when the mantissa field exceeds 0x600000.
+// Quotients up to 2^-126 end at byte 1; an infinite amax gives byte 255 as the quotient's own bits would.
 __device__ __forceinline__ uint32_t scale_byte(float amax, float& inv_scale) {
-    float s = __fdiv_rn(amax, 448.0f);
-    s = fmaxf(s, 1.17549435e-38f);                       // 2^-126
-    const uint32_t bits = __float_as_uint(s);
-    const uint32_t byte = (bits >> 23) + ((bits & 0x7FFFFFu) != 0u ? 1u : 0u);   // e + 127, 1..254
+    const uint32_t bits = __float_as_uint(amax);
+    const uint32_t up = (bits + 0x1FFFFFu) >> 23;
+    uint32_t byte = up > 9u ? up - 8u : 1u;
+    if (bits == 0x7F800000u) byte = 255u;
     inv_scale = __uint_as_float((254u - byte) << 23);    // 2^(127 - byte) = 2^-e
     return byte;
 }
@@ -36,23 +45,49 @@ __device__ __forceinline__ uint16_t e4m3x2(float lo, float hi) {
     return r;
 }
 
-template <typename T> __device__ __forceinline__ void load16(const T* src, float (&x)[16]);
-template <> __device__ __forceinline__ void load16<__nv_bfloat16>(const __nv_bfloat16* src, float (&x)[16]) {
-    const uint4 a = __ldg(reinterpret_cast<const uint4*>(src));
-    const uint4 b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-    const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        x[2 * i] = __uint_as_float(w[i] << 16);
-        x[2 * i + 1] = __uint_as_float(w[i] & 0xFFFF0000u);
+// Sixteen values of a row as they come from memory, and what is needed of them.
+template <typename T> struct Raw16;
+template <> struct Raw16<__nv_bfloat16> {
+    uint32_t w[8];
+    __device__ __forceinline__ void load(const __nv_bfloat16* src) {
+        const uint4 a = __ldg(reinterpret_cast<const uint4*>(src));
+        const uint4 b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
     }
-}
-template <> __device__ __forceinline__ void load16<float>(const float* src, float (&x)[16]) {
+    // largest magnitude, NaNs passed over: two values per instruction
+    __device__ __forceinline__ float amax() const {
+        uint32_t m = w[0] & 0x7FFF7FFFu;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float4 v = __ldg(reinterpret_cast<const float4*>(src) + i);
-        x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
+        for (int i = 1; i < 8; ++i) asm("max.bf16x2 %0, %0, %1;" : "+r"(m) : "r"(w[i] & 0x7FFF7FFFu));
+        return fmaxf(fmaxf(__uint_as_float(m << 16), __uint_as_float(m & 0xFFFF0000u)), 0.f);
     }
+    __device__ __forceinline__ float2 pair(int i) const {
+        return make_float2(__uint_as_float(w[i] << 16), __uint_as_float(w[i] & 0xFFFF0000u));
+    }
+};
+template <> struct Raw16<float> {
+    float4 v[4];
+    __device__ __forceinline__ void load(const float* src) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) v[i] = __ldg(reinterpret_cast<const float4*>(src) + i);
+    }
+    __device__ __forceinline__ float amax() const {
+        float m = 0.f;
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+        return m;
+    }
+    __device__ __forceinline__ float2 pair(int i) const {
+        return i & 1 ? make_float2(v[i >> 1].z, v[i >> 1].w) : make_float2(v[i >> 1].x, v[i >> 1].y);
+    }
+};
+
+// e4m3(clamp(x * inv, -448, 448)) of two values.  The conversion saturates by itself; the maximum is there for NaN,
+// which becomes -448.
+__device__ __forceinline__ uint32_t codes(float2 x, float inv) {
+    return e4m3x2(fmaxf(x.x * inv, -448.0f), fmaxf(x.y * inv, -448.0f));
 }
 
 // QGROUPS: true  -> Q rows: scale g covers dims [32g,32g+32) and [256+32g,256+32g+32)
@@ -66,40 +101,58 @@ mxdsa_pack_rows_kernel(const T* __restrict__ src, long long src_stride, long lon
     const int lane = threadIdx.x & 31;
     const long long warp0 = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     const long long nwarps = (long long)gridDim.x * kWarpsPerBlock;
-    for (long long r = warp0; r < rows; r += nwarps) {
-        float x[16];
-        load16<T>(src + r * src_stride + 16 * lane, x);
-        float amax = 0.f;
+    int off = 16 * lane;
+    if (QGROUPS && paired_storage) {   // [g][half][32]: natural chunk c = lane/2 -> chunk 2*(c%8) + c/8
+        const int c = lane >> 1;
+        off = (2 * (c & 7) + (c >> 3)) * 32 + (lane & 1) * 16;
+    }
+    // where this lane's scale byte goes in the two slot words (each group's first lane contributes)
+    const bool leader = QGROUPS ? (lane < 16 && (lane & 1) == 0) : ((lane & 3) == 0);
+    const int g = QGROUPS ? (lane >> 1) : (lane >> 2);
+    for (long long r0 = kRowsPerWarp * warp0; r0 < rows; r0 += kRowsPerWarp * nwarps) {
+        Raw16<T> x[kRowsPerWarp];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(x[i]));
-        // the group's four lanes: Q {2g, 2g+1, 2g+16, 2g+17}; KV {4g .. 4g+3}
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, QGROUPS ? 16 : 2));
-        float inv;
-        const uint32_t byte = scale_byte(amax, inv);
-        uint32_t w[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            float v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = fminf(fmaxf(x[4 * i + j] * inv, -448.0f), 448.0f);
-            w[i] = (uint32_t)e4m3x2(v[0], v[1]) | ((uint32_t)e4m3x2(v[2], v[3]) << 16);
+        for (int u = 0; u < kRowsPerWarp; ++u) {
+            const long long r = r0 + u < rows ? r0 + u : r0;     // past the end: the row before once more, not stored
+            x[u].load(src + r * src_stride + 16 * lane);
         }
-        // page addressing: rows_per_page rows of data, then their slots (prefill plane: one page of all rows)
-        const long long page = r / rows_per_page, in_page = r % rows_per_page;
-        uint8_t* drow = data + page * page_stride + in_page * data_stride;
-        uint8_t* srow = slots + page * page_stride + in_page * slot_stride;
-        int off = 16 * lane;
-        if (QGROUPS && paired_storage) {   // [g][half][32]: natural chunk c = lane/2 -> chunk 2*(c%8) + c/8
-            const int c = lane >> 1;
-            off = (2 * (c & 7) + (c >> 3)) * 32 + (lane & 1) * 16;
-        }
-        *reinterpret_cast<uint4*>(drow + off) = make_uint4(w[0], w[1], w[2], w[3]);
-        const bool leader = QGROUPS ? (lane < 16 && (lane & 1) == 0) : ((lane & 3) == 0);
-        if (leader) {
-            const int g = QGROUPS ? (lane >> 1) : (lane >> 2);
-            srow[g] = (uint8_t)byte;
-            srow[8 + g] = (uint8_t)byte;
+#pragma unroll
+        for (int u = 0; u < kRowsPerWarp; ++u) {
+            const long long r = r0 + u;
+            float amax = x[u].amax();
+            // the group's four lanes: Q {2g, 2g+1, 2g+16, 2g+17}; KV {4g .. 4g+3}
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, QGROUPS ? 16 : 2));
+            float inv;
+            const uint32_t byte = scale_byte(amax, inv);
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = codes(x[u].pair(2 * i), inv) | (codes(x[u].pair(2 * i + 1), inv) << 16);
+            const uint32_t mine = leader ? byte << (8 * (g & 3)) : 0u;
+            const uint32_t lo = __reduce_or_sync(0xffffffffu, g < 4 ? mine : 0u);
+            const uint32_t hi = __reduce_or_sync(0xffffffffu, g < 4 ? 0u : mine);
+            if (r >= rows) break;
+            uint8_t* drow;
+            uint8_t* srow;
+            if (QGROUPS) {             // data and slot of a row are adjacent
+                drow = data + r * data_stride;
+                srow = slots + r * slot_stride;
+            } else {                   // rows_per_page rows of data, then their slots (prefill plane: one page of all rows)
+                long long page = 0, in_page = r;
+                if (r >= rows_per_page) {
+                    if (r <= 0xffffffffLL) {
+                        page = (unsigned)r / (unsigned)rows_per_page;
+                        in_page = (unsigned)r % (unsigned)rows_per_page;
+                    } else {
+                        page = r / rows_per_page;
+                        in_page = r % rows_per_page;
+                    }
+                }
+                drow = data + page * page_stride + in_page * data_stride;
+                srow = slots + page * page_stride + in_page * slot_stride;
+            }
+            *reinterpret_cast<uint4*>(drow + off) = make_uint4(w[0], w[1], w[2], w[3]);
+            if (lane == 0) *reinterpret_cast<uint4*>(srow) = make_uint4(lo, hi, lo, hi);
         }
     }
 }
@@ -112,7 +165,7 @@ int launch(const T* src, long long src_stride, long long rows, uint8_t* data, lo
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return MXDSA_ERR_CUDA;
-    const long long want = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
+    const long long want = (rows + kRowsPerWarp * kWarpsPerBlock - 1) / (kRowsPerWarp * kWarpsPerBlock);
     const int grid = (int)(want < (long long)sms * 8 ? want : (long long)sms * 8);   // 8 resident CTAs of 256 threads per SM
     mxdsa_pack_rows_kernel<T, Q><<<grid, kWarpsPerBlock * 32, 0, stream>>>(src, src_stride, rows, data, data_stride, slots,
                                                                            slot_stride, rows_per_page, page_stride, paired);
@@ -137,12 +190,10 @@ extern "C" int mxdsa_pack_q(const mxdsa_pack_q_params* p) {
         return MXDSA_ERR_ALIGN;
     uint8_t* dst = static_cast<uint8_t*>(p->dst);
     const cudaStream_t s = static_cast<cudaStream_t>(p->stream);
-    // Q rows: data and slot of a row are adjacent; one "page" holds every row
-    const int big = 0x7fffffff;
     if (p->src_dtype == MXDSA_DTYPE_BF16)
-        return launch<__nv_bfloat16, true>(static_cast<const __nv_bfloat16*>(p->src), st, p->rows, dst, dt, dst + kDim, dt, big,
+        return launch<__nv_bfloat16, true>(static_cast<const __nv_bfloat16*>(p->src), st, p->rows, dst, dt, dst + kDim, dt, 1,
                                            0, p->paired_storage, s);
-    return launch<float, true>(static_cast<const float*>(p->src), st, p->rows, dst, dt, dst + kDim, dt, big, 0,
+    return launch<float, true>(static_cast<const float*>(p->src), st, p->rows, dst, dt, dst + kDim, dt, 1, 0,
                                p->paired_storage, s);
 }
 

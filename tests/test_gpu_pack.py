@@ -61,6 +61,33 @@ def test_pack_prefill_kv_matches_oracle_and_torch_packer(dtype):
     assert torch.equal(got, P.pack_dual_prefill_kv64(t)[0])
 
 
+@pytest.mark.parametrize("rows", [1, 2, 3, 15, 16, 17, 130])
+def test_scale_bytes_at_every_exponent_and_odd_row_counts(rows):
+    """amax = 1.75 * 2^e and its neighbours (where ceil(log2(amax / 448)) steps), tiny and infinite ones, NaN beside
+    them: scale bytes and codes against the formula in numpy."""
+    from mxdsa_b200 import quantize as Z
+    rng = np.random.default_rng(rows)
+    x = rng.standard_normal((rows, 8, 64)).astype(np.float32)
+    e = rng.integers(-149, 128, size=(rows, 8))
+    amax = np.ldexp(np.float64(1.75), e).astype(np.float32)
+    amax = np.where(rng.random((rows, 8)) < 0.3, np.nextafter(amax, np.float32(0)), amax)
+    amax = np.where(rng.random((rows, 8)) < 0.3, np.nextafter(amax, np.float32(np.inf)), amax).astype(np.float32)
+    x = (np.clip(x / 4, -1, 1) * amax[..., None]).astype(np.float32)
+    x[..., 11] = -amax
+    x[..., 12] = np.where(rng.random((rows, 8)) < 0.1, np.nan, x[..., 12])
+    x[0, 0, 5] = np.inf if rows > 2 else 1.0
+    with np.errstate(all="ignore"):
+        top = np.nanmax(np.abs(x), axis=2)
+        s = np.maximum(top / np.float32(448), np.float32(2.0 ** -126)).astype(np.float32).view(np.uint32)
+        byte = ((s >> 23) + ((s & 0x7FFFFF) != 0)).astype(np.uint32)
+        inv = ((254 - byte.astype(np.int64)).astype(np.uint32) << 23).view(np.float32)
+        v = np.fmin(np.fmax(x * inv[..., None], np.float32(-448)), np.float32(448))
+    want = torch.from_numpy(v).to(torch.float8_e4m3fn).view(torch.uint8).numpy().reshape(rows, 512)
+    got = Z.pack_dual_prefill_kv64(torch.from_numpy(x.reshape(rows, 1, 512)).cuda()).cpu().numpy().reshape(-1)
+    assert np.array_equal(got[: rows * 512].reshape(rows, 512), want)
+    assert np.array_equal(got[rows * 512:].reshape(rows, 2, 8), np.repeat(byte[:, None], 2, axis=1).astype(np.uint8))
+
+
 def test_pack_decode_pages_matches_oracle():
     from mxdsa_b200 import quantize as Z
     rng = np.random.default_rng(13)
