@@ -16,7 +16,12 @@
 //     (-0 and +0 tie);
 //   * written in ascending j (+ row_offset[r]), then -1 up to topk; topk_length[r] = number selected.
 //
-// Method: exact radix selection on the order-preserving 32-bit image of the float, three histogram
+// Two kernels.  mxdsa_topk_rows_kernel counts every key.  mxdsa_topk_pivot_kernel, for rows of more than 16 384 keys,
+// finds a score that a little more than topk keys reach from a sample of every eighth key, lists the keys at or above
+// it in one sweep of the row and selects exactly among those; where there are fewer rows than SMs it divides a row
+// among the CTAs of a cluster.
+//
+// Counting every key: exact radix selection on the order-preserving 32-bit image of the float, three histogram
 // passes (11 + 11 + 10 bits) with shared-memory atomics, keys of a row held in registers (one HBM read
 // per score for rows of up to 16 384 keys; longer rows are swept again from L2).  No pass branches per
 // key: the first counts every key, the later ones send keys outside the current prefix to a per-lane
@@ -24,9 +29,11 @@
 // position; the row is staged in shared memory and written in whole lines.  No sort, no global atomics,
 // deterministic.
 //
-// Bound: HBM on paper (group * s_kv * 4 bytes read + topk * 4 written per row); in practice the integer
-// pipe (about 25 instructions per key), so every step is written to save instructions, not bytes.
+// Bound: HBM on paper (group * s_kv * 4 bytes read + topk * 4 written per row); in practice the integer and
+// shared-memory pipes (counting every key: about 25 instructions and three shared atomics per key), so every step is
+// written to save instructions, not bytes.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <math_constants.h>
 #include <stdint.h>
 
@@ -110,7 +117,8 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int lane) {
 // After a histogram is complete: the bin that holds the k-th largest entry (k counted from the top,
 // 1 <= k <= total), the mass above that bin and the bin's own count.  Returns the histogram total.
 // Ends with a barrier; the result is in sm.sel_*.
-__device__ __forceinline__ uint32_t find_bin(TopkShared& sm, uint32_t k_or_cap, bool cap_to_total, uint32_t& k_out, int nbins) {
+template <typename Shared>
+__device__ __forceinline__ uint32_t find_bin(Shared& sm, uint32_t k_or_cap, bool cap_to_total, uint32_t& k_out, int nbins) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint4 h = *reinterpret_cast<const uint4*>(&sm.hist[4 * tid]);
     if (cap_to_total && tid == 0) h = make_uint4(0u, 0u, 0u, 0u);   // pass 0: bins 0-3 collect the non-candidates
@@ -304,6 +312,538 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
     }
 }
 
+// ------------------------------------------------------------------------------------------------ selection by pivot
+//
+// For rows of more than 16 384 keys the kernel above sweeps the row four times and spends three shared-memory atomics
+// on every key.  Here
+//   1. every eighth key (four per thread) is a sample; two histogram passes over the samples give a pivot: the lower
+//      edge, to 22 bits, of the rank'th largest, rank = topk/8 + 5 sqrt(topk/8) + 8, so that about 1.2 to 1.4 topk keys
+//      reach it and fewer than topk do with a probability of less than 1e-6 for samples that are independent;
+//   2. one sweep compares every score with the pivot (as floats: NaN, -inf and keys past the length fail by
+//      themselves) and lists key and position of those that reach it, in ascending position, in shared memory;
+//   3. the topk-th largest of the list is found by histogram passes over the list alone, whose digits start at the
+//      pivot and span just the range up to the list's maximum, so that the entries spread over the bins and the first
+//      or second pass usually decides; the list is compacted to the output with ballots.
+// A row where the list overflows or falls short (a sample that misled, heavy ties) is counted key by key.  Rows of up
+// to kShortRow keys skip the sampling: every usable key is listed.
+//
+// Measured against the kernel above (cold L2, us): 2048 rows of 32 768 keys, topk 2048 195.6 -> 134.2 (pairs 257 -> 183),
+// of 65 536 keys 355 -> 196; 64 rows of 65 536 keys, half to full length 28.7 -> 20.5; one pair of 131 072 keys 72.7 -> 24.6.
+// Bound: latency of the phases between barriers and, with many rows, instruction issue (54 % of the slots, about 1 650
+// instructions per warp and 16 384 keys of a pair), not HBM.
+//
+// CLUSTER: the CTAs of a cluster divide a row's keys in order; they add up their sample histograms through distributed
+// shared memory, each lists its own part, and the first one gathers the lists and finishes the row.
+//
+constexpr int kList = 8192;                        // capacity of the list (64 KB of shared memory; two CTAs per SM)
+constexpr int kShortRow = 4096;
+constexpr int kMaxSweeps = 8;                      // a CTA's part of a row: samples stay in registers (4 per sweep)
+constexpr uint32_t kMinKey = 0x00800000u;          // score_key(-FLT_MAX): every usable key reaches it
+
+struct PivotShared {
+    uint32_t hist[2 * kBins];                      // one per sample pass (peers read them); the list uses the first
+    uint32_t warp_tot[kWarps];
+    uint32_t chunk_tot[kChunks * kWarps];
+    uint32_t sel_bin, sel_above, sel_count;
+    uint32_t list_n;                               // entries of this CTA's list; kList + 1: it did not fit
+    uint32_t key_max;                              // largest key of this CTA's part
+    uint32_t warp_gt[kWarps], warp_eq[kWarps];
+    uint32_t few_n;                                // entries of the last bin when they are few, gathered
+    uint2 few[32];                                 // (key, place in the list)
+    uint2 list[kList];                             // (score, later its key; position in the row)
+};
+
+__device__ __forceinline__ uint32_t cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ uint32_t cluster_size() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t peer_address(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ uint32_t peer_load(uint32_t a) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint4 peer_load4(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ uint2 peer_load2(uint32_t a) {
+    uint2 v;
+    asm volatile("ld.shared::cluster.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ float fmax3(float a, float b, float c) {
+    float d;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+// the float whose score_key is `key`
+__device__ __forceinline__ float key_score(uint32_t key) {
+    return __uint_as_float(key & 0x80000000u ? key ^ 0x80000000u : ~key);
+}
+
+// The bin of the k-th largest entry, from this thread's four bins; sel_* as in find_bin.  Returns the total; nothing is
+// selected where it is below k.  Ends with a barrier.
+__device__ __forceinline__ uint32_t locate(PivotShared& sm, uint4 h, uint32_t k) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t local = h.x + h.y + h.z + h.w;
+    const uint32_t inc = warp_inclusive_scan(local, lane);
+    if (lane == 31) sm.warp_tot[warp] = inc;
+    __syncthreads();
+    const uint32_t wt = lane < kWarps ? sm.warp_tot[lane] : 0u;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, wt);
+    const uint32_t below_warps = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u);
+    uint32_t run = total - (below_warps + inc);
+    if (run < k && run + local >= k) {
+        const uint32_t hh[4] = {h.x, h.y, h.z, h.w};
+#pragma unroll
+        for (int b = 3; b >= 0; --b) {
+            if (run < k && run + hh[b] >= k) {
+                sm.sel_bin = 4 * tid + b;
+                sm.sel_above = run;
+                sm.sel_count = hh[b];
+            }
+            run += hh[b];
+        }
+    }
+    __syncthreads();
+    return total;
+}
+
+// Four scores of the row from position j on: the larger of the pair's, -inf from `end` on.
+template <int GROUP>
+__device__ __forceinline__ float4 load_scores4(const float* __restrict__ row0, const float* __restrict__ row1, int j, int end) {
+    float4 v = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+    if (j < end) {
+        v = __ldg(reinterpret_cast<const float4*>(row0 + j));
+        if (GROUP == 2) {
+            const float4 b = __ldg(reinterpret_cast<const float4*>(row1 + j));
+            v = make_float4(fmaxf(v.x, b.x), fmaxf(v.y, b.y), fmaxf(v.z, b.z), fmaxf(v.w, b.w));
+        }
+        const int nin = end - j;
+        if (nin < 4) {
+            v.w = -CUDART_INF_F;
+            if (nin < 3) v.z = -CUDART_INF_F;
+            if (nin < 2) v.y = -CUDART_INF_F;
+        }
+    }
+    return v;
+}
+template <int GROUP>
+__device__ __forceinline__ void load_scores(const float* __restrict__ row0, const float* __restrict__ row1, int j0, int end,
+                                            float (&s)[kKpt]) {
+    constexpr int kBatch = GROUP == 2 ? kChunks / 4 : kChunks / 2;      // 16-byte loads in flight, per row
+#pragma unroll
+    for (int c0 = 0; c0 < kChunks; c0 += kBatch) {
+        const int jb = j0 + (c0 * kThreads + (int)threadIdx.x) * 4;
+        if (j0 + (c0 + kBatch) * kThreads * 4 <= end) {             // all of the batch is there: no bounds per key
+            float4 a[kBatch], b[GROUP == 2 ? kBatch : 1];
+#pragma unroll
+            for (int c = 0; c < kBatch; ++c) {
+                a[c] = __ldg(reinterpret_cast<const float4*>(row0 + jb + c * kThreads * 4));
+                if (GROUP == 2) b[c] = __ldg(reinterpret_cast<const float4*>(row1 + jb + c * kThreads * 4));
+            }
+#pragma unroll
+            for (int c = 0; c < kBatch; ++c) {
+                float* o = &s[4 * (c0 + c)];
+                o[0] = a[c].x; o[1] = a[c].y; o[2] = a[c].z; o[3] = a[c].w;
+                if (GROUP == 2) {
+                    o[0] = fmaxf(o[0], b[c].x); o[1] = fmaxf(o[1], b[c].y);
+                    o[2] = fmaxf(o[2], b[c].z); o[3] = fmaxf(o[3], b[c].w);
+                }
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < kBatch; ++c) {
+                const float4 v = load_scores4<GROUP>(row0, row1, jb + c * kThreads * 4, end);
+                float* o = &s[4 * (c0 + c)];
+                o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+            }
+        }
+    }
+}
+
+// one list entry at shared address `to` where `on` is not zero; predicated, not branched: 32 of these follow one another
+__device__ __forceinline__ void append(uint32_t& to, uint32_t on, float score, uint32_t pos) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, 0;\n@p st.shared.v2.b32 [%0], {%2, %3};\n@p add.u32 %0, %0, 8;\n}"
+                 : "+r"(to) : "r"(on), "r"(__float_as_uint(score)), "r"(pos) : "memory");
+}
+
+// Appends the scores of one sweep that reach the pivot to the list and raises sm.key_max; false (for all threads) where
+// they do not fit.  What reaches the pivot is one bit per key, so that the scores are all that a thread keeps of it.
+__device__ __forceinline__ bool list_sweep(PivotShared& sm, const float (&s)[kKpt], float pivot, int j0, int end, uint32_t& n) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t mask = 0u;
+    float top = -CUDART_INF_F;
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+        if (j0 + c * kThreads * 4 < end) {         // the same for all threads: nothing is done for chunks past the row's end
+#pragma unroll
+            for (int i = 4 * c; i < 4 * c + 4; i += 2) {
+                mask |= s[i] >= pivot ? 1u << i : 0u;
+                mask |= s[i + 1] >= pivot ? 2u << i : 0u;
+                top = fmax3(top, s[i], s[i + 1]);
+            }
+        }
+    }
+    const uint32_t mx = __reduce_max_sync(0xffffffffu, score_key(top));
+    // counts per chunk (four keys), a nibble each, spread over two words of bytes: chunks 0, 2, 4, 6 and 1, 3, 5, 7
+    uint32_t nib = mask - ((mask >> 1) & 0x55555555u);
+    nib = (nib & 0x33333333u) + ((nib >> 2) & 0x33333333u);
+    const uint32_t own[2] = {nib & 0x0f0f0f0fu, (nib >> 4) & 0x0f0f0f0fu};
+    uint32_t ex[2];                                // a warp's exclusive total per chunk is at most 124
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t inc = warp_inclusive_scan(own[h], lane);
+        if (lane == 31) {
+#pragma unroll
+            for (int i = 0; i < kChunks / 2; ++i) sm.chunk_tot[(2 * i + h) * kWarps + warp] = (inc >> (8 * i)) & 0xffu;
+        }
+        ex[h] = inc - own[h];
+    }
+    if (lane == 0) atomicMax(&sm.key_max, mx);
+    __syncthreads();
+    // every warp scans the 128 (chunk, warp) totals for itself: cheaper than one warp and a barrier
+    const uint4 t = *reinterpret_cast<const uint4*>(&sm.chunk_tot[4 * lane]);
+    const uint32_t sum = t.x + t.y + t.z + t.w;
+    const uint32_t incl = warp_inclusive_scan(sum, lane);
+    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
+    uint32_t first = n + incl - sum;               // where this warp's piece of the chunk lane * 4 / kWarps begins
+    if ((warp & 3) > 0) first += t.x;
+    if ((warp & 3) > 1) first += t.y;
+    if ((warp & 3) > 2) first += t.z;
+    const bool fits = n + total <= (uint32_t)kList;
+    if (fits) {
+        const uint32_t j = (uint32_t)(j0 + tid * 4), list0 = (uint32_t)__cvta_generic_to_shared(sm.list);
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+            if (j0 + c * kThreads * 4 >= end) break;
+            uint32_t to = list0 + 8u * (__shfl_sync(0xffffffffu, first, (c * kWarps + warp) >> 2) + ((ex[c & 1] >> (8 * (c >> 1))) & 0xffu));
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+                append(to, mask & (1u << (4 * c + e)), s[4 * c + e], j + (uint32_t)(c * kThreads * 4 + e));
+        }
+    }
+    n += total;
+    __syncthreads();
+    return fits;
+}
+
+// The min(topk, n) largest of the list (ties: first come), in list order, to `out`, then -1.
+__device__ __forceinline__ void select_from_list(PivotShared& sm, uint32_t n, uint32_t pivot_key, uint32_t key_max, int topk,
+                                                 int32_t* __restrict__ out, int32_t off, int32_t* __restrict__ count) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t n_sel = min((uint32_t)topk, n);
+    // Selected in the end: keys above `key_t`, and those equal to it up to place `at_t` of the list -- or, with `ties`,
+    // the first `need` of them.
+    uint32_t key_t = 0u, at_t = 0xffffffffu, need = 0u, above = 0u;    // above: the warps count keys >= this
+    bool ties = false, few = false;
+    if (n > (uint32_t)topk) {
+        uint32_t base = pivot_key, in_bin;
+        uint32_t span = key_max - base;            // keys of the current interval: base .. base + span
+        int sh = max(21 - __clz(span), 0);         // the interval in at most 2048 bins
+        need = (uint32_t)topk;
+#pragma unroll 1
+        for (bool first = true;; first = false) {
+            *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+            if (tid == 0) sm.few_n = 0u;
+            __syncthreads();
+            // entries below the interval wrap to distances beyond it: keys lie in [2^23, 2^32 - 2^23]
+#pragma unroll 4
+            for (uint32_t i = tid; i < n; i += kThreads) {
+                uint32_t key = sm.list[i].x;
+                if (first) {
+                    key = score_key(__uint_as_float(key));
+                    sm.list[i].x = key;
+                }
+                if (key - base <= span) atomicAdd(&sm.hist[(key - base) >> sh], 1u);
+            }
+            __syncthreads();
+            locate(sm, *reinterpret_cast<const uint4*>(&sm.hist[4 * tid]), need);
+            base += sm.sel_bin << sh;
+            need -= sm.sel_above;
+            in_bin = sm.sel_count;
+            if (in_bin == need || in_bin <= 32u || sh == 0) break;
+            span = (1u << sh) - 1u;
+            sh = max(sh - 11, 0);
+            // (the next pass's barriers stand between these reads of sel_* and their next writes)
+        }
+        key_t = above = base;                      // the whole bin is taken ...
+        if (in_bin != need) {
+            above = base + (1u << sh);             // ... or need of its entries: a few, or equal ones
+            few = in_bin <= 32u;
+            ties = !few;
+        }
+    }
+    // a warp compacts a contiguous piece of the list
+    const uint32_t seg = ((n + kThreads - 1) / kThreads) * 32;
+    const uint32_t lo = warp * seg, hi = min(lo + seg, n);
+    uint32_t a, q = 0u;
+    {
+        uint32_t gt = 0, eq = 0;
+#pragma unroll 4
+        for (uint32_t i = lo; i < hi; i += 32) {
+            const bool in = i + lane < hi;
+            const uint32_t key = in ? sm.list[i + lane].x : 0u;
+            gt += __popc(__ballot_sync(0xffffffffu, in && key >= above));
+            if (few && key >= key_t && key < above) sm.few[atomicAdd(&sm.few_n, 1u)] = make_uint2(key, i + lane);
+            if (ties) eq += __popc(__ballot_sync(0xffffffffu, key == key_t));
+        }
+        if (lane == 0) {
+            sm.warp_gt[warp] = gt;
+            sm.warp_eq[warp] = eq;
+        }
+        __syncthreads();
+        a = __reduce_add_sync(0xffffffffu, lane < warp ? sm.warp_gt[lane & (kWarps - 1)] : 0u);
+        if (ties) {
+            q = __reduce_add_sync(0xffffffffu, lane < warp ? sm.warp_eq[lane & (kWarps - 1)] : 0u);
+            a += min(q, need);
+        } else if (few) {                          // rank the few among themselves; every warp for itself
+            const uint32_t m = sm.few_n;
+            const uint2 own = lane < m ? sm.few[lane] : make_uint2(0u, 0xffffffffu);
+            uint32_t better = 0;
+            for (uint32_t i = 0; i < m; ++i) {
+                const uint2 o = sm.few[i];
+                better += (o.x > own.x || (o.x == own.x && o.y < own.y)) ? 1u : 0u;
+            }
+            const bool taken = lane < m && better < need;
+            a += __popc(__ballot_sync(0xffffffffu, taken && own.y < lo));
+            const int last = __ffs(__ballot_sync(0xffffffffu, lane < m && better == need - 1u)) - 1;
+            key_t = __shfl_sync(0xffffffffu, own.x, last);
+            at_t = __shfl_sync(0xffffffffu, own.y, last);
+        }
+    }
+    const uint32_t before = (1u << lane) - 1u;
+#pragma unroll 4
+    for (uint32_t i = lo; i < hi; i += 32) {
+        const bool in = i + lane < hi;
+        const uint2 en = in ? sm.list[i + lane] : make_uint2(0u, 0u);
+        bool sel = en.x > key_t || (en.x == key_t && i + lane <= at_t);
+        if (ties) {
+            const uint32_t me = __ballot_sync(0xffffffffu, en.x == key_t);
+            sel = en.x > key_t || (en.x == key_t && q + __popc(me & before) < need);
+            q += __popc(me);
+        }
+        sel = sel && in;
+        const uint32_t ms = __ballot_sync(0xffffffffu, sel);
+        if (sel) out[a + __popc(ms & before)] = (int32_t)en.y + off;
+        a += __popc(ms);
+    }
+    for (uint32_t pos = n_sel + tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = -1;
+    if (count != nullptr && tid == 0) *count = (int32_t)n_sel;
+    __syncthreads();
+}
+
+// A row in which the list did not work out, by counting every key, straight from memory: the rare case, written for few
+// registers (in the form of mxdsa_topk_rows_kernel, inlined or called, it made the whole kernel spill).
+template <int GROUP>
+__device__ __forceinline__ void misled_row(PivotShared& sm, const float* __restrict__ row0, const float* __restrict__ row1,
+                                           int len, int topk, int32_t* __restrict__ out, int32_t off,
+                                           int32_t* __restrict__ count) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t prefix = 0, k = (uint32_t)topk, n_sel = 0;
+#pragma unroll 1
+    for (int pass = 0; pass < 3; ++pass) {
+        const int lo = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
+        const int hi = pass == 0 ? 32 : (pass == 1 ? 21 : 10);
+        const uint32_t first = pass == 0 ? 0u : prefix << hi;
+        const uint32_t spare = (uint32_t)((pass == 2 ? kBins / 2 : kBins) + lane);
+        *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+#pragma unroll 2
+        for (int j = 4 * tid; j < len; j += 4 * kThreads) {
+            const float4 v = load_scores4<GROUP>(row0, row1, j, len);
+            atomicAdd(&sm.hist[min((score_key(v.x) - first) >> lo, spare)], 1u);
+            atomicAdd(&sm.hist[min((score_key(v.y) - first) >> lo, spare)], 1u);
+            atomicAdd(&sm.hist[min((score_key(v.z) - first) >> lo, spare)], 1u);
+            atomicAdd(&sm.hist[min((score_key(v.w) - first) >> lo, spare)], 1u);
+        }
+        __syncthreads();
+        uint32_t k_now;
+        const uint32_t total = find_bin(sm, k, pass == 0, k_now, pass == 2 ? kBins / 2 : kBins);
+        if (pass == 0) n_sel = k_now;
+        if (total == 0u || k_now == 0u) { n_sel = 0; break; }
+        prefix = pass == 0 ? sm.sel_bin : ((prefix << (hi - lo)) | sm.sel_bin);
+        k = k_now - sm.sel_above;
+    }
+    uint32_t base_gt = 0, base_eq = 0;
+#pragma unroll 1
+    for (int j0 = 0; n_sel > 0u && j0 < len; j0 += 4 * kThreads) {
+        const int j = j0 + 4 * tid;
+        const float4 v = load_scores4<GROUP>(row0, row1, j, len);
+        const uint32_t key[4] = {score_key(v.x), score_key(v.y), score_key(v.z), score_key(v.w)};
+        uint32_t own = 0;                          // keys above the threshold | equal to it << 16
+#pragma unroll
+        for (int e = 0; e < 4; ++e) own += key[e] > prefix ? 1u : (key[e] == prefix ? 1u << 16 : 0u);
+        const uint32_t inc = warp_inclusive_scan(own, lane);
+        if (lane == 31) sm.warp_tot[warp] = inc;
+        __syncthreads();
+        const uint32_t wt = lane < kWarps ? sm.warp_tot[lane] : 0u;
+        const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u) + inc - own;
+        const uint32_t total = __reduce_add_sync(0xffffffffu, wt);
+        uint32_t a = base_gt + (before & 0xffffu), q = base_eq + (before >> 16);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const bool is_gt = key[e] > prefix, is_eq = key[e] == prefix;
+            if (is_gt || (is_eq && q < k)) out[a + min(q, k)] = j + e + off;
+            a += is_gt ? 1u : 0u;
+            q += is_eq ? 1u : 0u;
+        }
+        base_gt += total & 0xffffu;
+        base_eq += total >> 16;
+        __syncthreads();
+    }
+    for (uint32_t pos = n_sel + tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = -1;
+    if (count != nullptr && tid == 0) *count = (int32_t)n_sel;
+    __syncthreads();
+}
+
+template <int GROUP, bool MULTI, bool CLUSTER>
+__global__ void __launch_bounds__(kThreads, 2)
+mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
+                        const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
+                        int32_t* __restrict__ topk_length, int rows, int s_kv, int topk, uint32_t sample_rank) {
+    extern __shared__ __align__(16) uint8_t topk_smem[];
+    PivotShared& sm = *reinterpret_cast<PivotShared*>(topk_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t parts = CLUSTER ? cluster_size() : 1u, part = CLUSTER ? cluster_rank() : 0u;
+    const int step = (int)(gridDim.x / parts);
+    if (tid == 0) sm.key_max = 0u;
+    __syncthreads();
+    for (int r = (int)(blockIdx.x / parts); r < rows; r += step) {
+        const float* row0 = scores + (long long)r * GROUP * score_stride;
+        const float* row1 = row0 + score_stride;
+        int len = s_kv;
+        if (lengths != nullptr) len = min(max(__ldg(lengths + r), 0), s_kv);
+        // this CTA's keys: the row's own length is divided, in whole groups of four
+        int begin = 0, end = len;
+        if (CLUSTER) {
+            const int each = ((len + (int)parts - 1) / (int)parts + 3) & ~3;
+            begin = min((int)part * each, len);      // an empty part begins at len, multiple of four or not: it loads nothing
+            end = min(begin + each, len);
+        }
+        const int nsweeps = MULTI ? (end - begin + kSweep - 1) / kSweep : 1;
+
+        // ---- 1. the pivot
+        float s[kKpt];                                // MULTI: the samples first, then a sweep at a time
+        if (!MULTI) load_scores<GROUP>(row0, row1, begin, end, s);
+        uint32_t pivot_key = kMinKey;
+        if (len > kShortRow) {                        // the same for all CTAs of the cluster
+#pragma unroll
+            for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(&sm.hist[i * kBins + 4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+            constexpr int kSamples = MULTI ? 4 * kMaxSweeps : 4;
+            uint32_t smp[kSamples];
+            if (MULTI) {                              // a chunk of four per thread and sweep, another one for each warp
+#pragma unroll
+                for (int sw = 0; sw < kMaxSweeps; ++sw) {
+                    const int j = begin + sw * kSweep + (((warp + sw) & (kChunks - 1)) * kThreads + tid) * 4;
+                    const float4 v = load_scores4<GROUP>(row0, row1, j, end);
+                    s[4 * sw] = v.x; s[4 * sw + 1] = v.y; s[4 * sw + 2] = v.z; s[4 * sw + 3] = v.w;
+                }
+#pragma unroll
+                for (int i = 0; i < kSamples; ++i) smp[i] = score_key(s[i % kKpt]);
+            } else {                                  // one of four keys of every other chunk, even or odd by warp
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const float* c0 = &s[8 * i];
+                    const float a = warp & 1 ? c0[4] : c0[0], b = warp & 1 ? c0[5] : c0[1];
+                    const float c = warp & 1 ? c0[6] : c0[2], d = warp & 1 ? c0[7] : c0[3];
+                    smp[i] = score_key(lane & 2 ? (lane & 1 ? d : c) : (lane & 1 ? b : a));
+                }
+            }
+            __syncthreads();
+            uint32_t prefix = 0, k = sample_rank;
+            bool found = true;
+#pragma unroll 1
+            for (int pass = 0; pass < 2; ++pass) {
+                uint32_t* hist = &sm.hist[pass * kBins];
+                const int lo = pass == 0 ? 21 : 10;
+                const uint32_t first = pass == 0 ? 0u : prefix << 21;
+#pragma unroll
+                for (int i = 0; i < kSamples; ++i) {
+                    const uint32_t bin = (smp[i] - first) >> lo;
+                    if (smp[i] >= kMinKey && bin < (uint32_t)kBins) atomicAdd(&hist[bin], 1u);
+                }
+                uint4 h;
+                if (CLUSTER) {
+                    cluster_barrier();
+                    h = make_uint4(0u, 0u, 0u, 0u);
+                    for (uint32_t c = 0; c < parts; ++c) {
+                        const uint4 o = peer_load4(peer_address(&hist[4 * tid], c));
+                        h.x += o.x; h.y += o.y; h.z += o.z; h.w += o.w;
+                    }
+                } else {
+                    __syncthreads();
+                    h = *reinterpret_cast<const uint4*>(&hist[4 * tid]);
+                }
+                if (locate(sm, h, k) < k) {               // fewer usable samples than that: list every usable key
+                    found = false;                        // (decided in the first pass, by all CTAs of the cluster alike)
+                    break;
+                }
+                prefix = pass == 0 ? sm.sel_bin : (prefix << 11) | sm.sel_bin;
+                k -= sm.sel_above;
+            }
+            if (found) pivot_key = max(prefix << 10, kMinKey);
+        }
+        const float pivot = key_score(pivot_key);
+
+        // ---- 2. the list
+        uint32_t n = 0;
+        bool fits = true;
+#pragma unroll 1
+        for (int sw = 0; sw < nsweeps && fits; ++sw) {
+            if (MULTI) load_scores<GROUP>(row0, row1, begin + sw * kSweep, end, s);
+            fits = list_sweep(sm, s, pivot, begin + sw * kSweep, end, n);
+        }
+        uint32_t key_max = sm.key_max;
+        if (CLUSTER) {
+            if (tid == 0) sm.list_n = fits ? n : (uint32_t)kList + 1u;
+            cluster_barrier();
+            if (part == 0) {
+                for (uint32_t c = 1; c < parts; ++c) {
+                    const uint32_t m = peer_load(peer_address(&sm.list_n, c));
+                    fits = fits && n + m <= (uint32_t)kList;
+                    if (!fits) break;
+                    const uint32_t src = peer_address(sm.list, c);
+                    for (uint32_t i = tid; i < m; i += kThreads) sm.list[n + i] = peer_load2(src + 8 * i);
+                    n += m;
+                    key_max = max(key_max, peer_load(peer_address(&sm.key_max, c)));
+                }
+            }
+            cluster_barrier();
+        } else {
+            __syncthreads();
+        }
+        if (tid == 0) sm.key_max = 0u;               // everybody has read it; a barrier follows before it is raised again
+        if (CLUSTER && part != 0) {
+            __syncthreads();
+            continue;
+        }
+
+        // ---- 3. the selection
+        int32_t* out = indices + (long long)r * index_stride;
+        const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
+        int32_t* count = topk_length != nullptr ? topk_length + r : nullptr;
+        if (fits && (n >= (uint32_t)topk || pivot_key == kMinKey)) select_from_list(sm, n, pivot_key, key_max, topk, out, off, count);
+        else misled_row<GROUP>(sm, row0, row1, len, topk, out, off, count);
+    }
+}
+
 thread_local int tl_topk_cuda_error = 0;
 
 }  // namespace
@@ -318,13 +858,53 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return MXDSA_ERR_CUDA;
-    const int grid = p->rows < sms * 2 ? p->rows : sms * 2;      // two resident CTAs of 512 threads per SM
     const cudaStream_t s = static_cast<cudaStream_t>(p->stream);
-    auto kern = p->topk <= kStage ? (p->group == 2 ? mxdsa_topk_rows_kernel<2, true> : mxdsa_topk_rows_kernel<1, true>)
-                                  : (p->group == 2 ? mxdsa_topk_rows_kernel<2, false> : mxdsa_topk_rows_kernel<1, false>);
-    kern<<<grid, kThreads, 0, s>>>(p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows, p->s_kv,
-                                   p->topk);
-    const cudaError_t e = cudaGetLastError();
+    // By pivot where a row does not fit the registers of a CTA (16 384 keys) and the list fits with its margin.  Shorter
+    // rows are read and counted once by the other kernel, which is the faster one there for the lists in use: 2048 rows of
+    // 16 384 keys, topk 2048 81 us against 84 by pivot (pairs 101 against 120); 20 rows of 16 384 keys 11 against 19.
+    // Few rows are divided among CTAs as long as these find SMs: four of them, eight where each still has 16 384 keys
+    // (20 rows of 32 768 keys: 29 us by eights, 20 rows of 20 480 keys 19 us by fours).  The steps between the CTAs of a
+    // row cost more than a second sweep (one row of 32 768 keys, topk 2048: 20.5 us counted, 24.5 divided), less than the
+    // further ones (65 536 keys: 32.8 against 22.6), hence the two lines.
+    int parts = 1;
+    while (parts < 8 && (long long)p->rows * parts * 2 <= sms * 2 && p->s_kv / (parts * 2) >= (parts < 4 ? kShortRow : kSweep)) parts *= 2;
+    const int each = (int)((((long long)p->s_kv + parts - 1) / parts + 3) & ~3LL);      // the longest part of a row
+    const bool pivot = p->topk <= kStage && p->s_kv > (parts > 1 ? 2 : 1) * kSweep && each <= kMaxSweeps * kSweep;
+    cudaError_t e = cudaSuccess;
+    if (pivot) {
+        const bool multi = each > kSweep;
+        const float mean = p->topk * 0.125f;
+        const uint32_t rank = (uint32_t)(mean + 5.0f * sqrtf(mean) + 8.0f);
+        auto kern = p->group == 2 ? (parts == 1 ? mxdsa_topk_pivot_kernel<2, true, false>
+                                     : multi ? mxdsa_topk_pivot_kernel<2, true, true> : mxdsa_topk_pivot_kernel<2, false, true>)
+                                  : (parts == 1 ? mxdsa_topk_pivot_kernel<1, true, false>
+                                     : multi ? mxdsa_topk_pivot_kernel<1, true, true> : mxdsa_topk_pivot_kernel<1, false, true>);
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PivotShared));
+        if (e == cudaSuccess) {
+            const long long want = (long long)p->rows * parts;
+            cudaLaunchAttribute attr[1];
+            attr[0].id = cudaLaunchAttributeClusterDimension;
+            attr[0].val.clusterDim.x = parts;
+            attr[0].val.clusterDim.y = 1;
+            attr[0].val.clusterDim.z = 1;
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3((unsigned)(want < sms * 2 ? want : sms * 2 / parts * parts));
+            cfg.blockDim = dim3(kThreads);
+            cfg.dynamicSmemBytes = sizeof(PivotShared);
+            cfg.stream = s;
+            cfg.attrs = attr;
+            cfg.numAttrs = parts > 1 ? 1 : 0;
+            e = cudaLaunchKernelEx(&cfg, kern, p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length,
+                                   p->rows, p->s_kv, p->topk, rank);
+        }
+    } else {
+        const int grid = p->rows < sms * 2 ? p->rows : sms * 2;      // two resident CTAs of 512 threads per SM
+        auto kern = p->topk <= kStage ? (p->group == 2 ? mxdsa_topk_rows_kernel<2, true> : mxdsa_topk_rows_kernel<1, true>)
+                                      : (p->group == 2 ? mxdsa_topk_rows_kernel<2, false> : mxdsa_topk_rows_kernel<1, false>);
+        kern<<<grid, kThreads, 0, s>>>(p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows,
+                                       p->s_kv, p->topk);
+    }
+    if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
         tl_topk_cuda_error = (int)e;
         return MXDSA_ERR_CUDA;

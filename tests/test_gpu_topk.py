@@ -93,6 +93,38 @@ def test_pair_sharing_and_pool_offsets():
     _check(s, 2048, pair=True, row_offset=off, lengths=rng.integers(1, 16385, size=12).astype(np.int32))
 
 
+# Rows of more than 16 384 keys (divided ones: 32 768), selected by a pivot from a sample: parts of a cluster that end inside a group of four or
+# are empty, one sweep and several, the longest row of a CTA and one beyond, lists as long as the row's candidates.
+@pytest.mark.parametrize("rows,s_kv,topk,pair", [
+    (1, 32772, 64, False), (2, 40004, 1, False), (3, 32772, 4096, True), (1, 131072, 2048, True), (300, 16392, 1500, True),
+    (5, 131076, 4096, False), (75, 65544, 2048, True), (149, 20480, 300, False), (149, 131072, 64, False), (150, 131080, 33, False)])
+def test_rows_selected_by_pivot(rows, s_kv, topk, pair):
+    rng = np.random.default_rng(rows + s_kv)
+    s = rng.standard_normal((rows * (2 if pair else 1), s_kv), dtype=np.float32)
+    lengths = rng.integers(0, s_kv + 1, size=rows).astype(np.int32)
+    lengths[: min(rows, 3)] = [s_kv, 4097, 4096][: min(rows, 3)]
+    _check(s, topk, pair=pair)
+    _check(s, topk, lengths=lengths, pair=pair, row_offset=np.arange(rows) * 7)
+
+
+@pytest.mark.parametrize("rows", [4, 160])     # a row divided among CTAs, and a CTA for each
+@pytest.mark.parametrize("s_kv", [33000, 70000])
+def test_samples_that_mislead(rows, s_kv):
+    rng = np.random.default_rng(rows + s_kv)
+    s = rng.standard_normal((rows, s_kv), dtype=np.float32)
+    s[0] = rng.integers(0, 3, size=s_kv)                       # ties by the thousand: the list overflows
+    s[1] = np.arange(s_kv) * 1e-3                              # ascending: the best keys are neighbours
+    s[2, :] = np.where(np.arange(s_kv) % 1024 < 200, 9.0 + s[2], s[2] - 9.0)   # blocks of good keys
+    s[3] = np.nan
+    s[3, 5000:5010] = 1.0                                      # fewer usable keys than sampled ranks
+    if rows > 4:
+        s[4] = 100.0 + rng.random(s_kv, dtype=np.float32)      # one exponent
+        s[5, rng.choice(s_kv, 1900, replace=False)] = np.inf   # +inf keys are usable
+        s[6] = -np.abs(s[6])
+        s[7] = -0.0
+    _check(s, 1500)
+
+
 def test_argument_rules():
     from mxdsa_b200.indexer import select_topk_indices
     dev = torch.device("cuda:0")
