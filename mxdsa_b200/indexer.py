@@ -10,12 +10,9 @@ fallback.
 """
 from __future__ import annotations
 
-import ctypes as C
 from typing import Optional, Tuple
 
 import torch
-
-from . import capi
 
 
 def select_topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch.Tensor] = None,
@@ -39,7 +36,6 @@ def select_topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch
     if s_kv <= 0 or s_kv % 4 or topk <= 0:
         raise RuntimeError("s_kv must be a positive multiple of 4 and topk positive")
     rows = n // group
-    dev = scores.device
 
     def opt(t, name):
         if t is None:
@@ -49,15 +45,5 @@ def select_topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch
         return t.contiguous()
 
     lengths, row_offset = opt(lengths, "lengths"), opt(row_offset, "row_offset")
-    indices = torch.empty((rows, topk), dtype=torch.int32, device=dev)
-    count = torch.empty((rows,), dtype=torch.int32, device=dev)
-    if rows:
-        p = capi.TopkParams(scores=scores.data_ptr(), score_stride=scores.stride(0),
-                            lengths=lengths.data_ptr() if lengths is not None else None,
-                            row_offset=row_offset.data_ptr() if row_offset is not None else None,
-                            indices=indices.data_ptr(), index_stride=topk, topk_length=count.data_ptr(),
-                            rows=rows, group=group, s_kv=s_kv, topk=topk,
-                            stream=torch.cuda.current_stream(dev).cuda_stream)
-        with torch.cuda.device(dev):
-            capi.check(capi.lib().mxdsa_topk_select(C.byref(p)), "mxdsa_topk_select")
-    return indices, count
+    from . import ext
+    return ext().topk_rows(scores, topk, lengths, group, row_offset)

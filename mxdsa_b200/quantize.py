@@ -9,39 +9,31 @@ fallback.
 """
 from __future__ import annotations
 
-import ctypes as C
-
 import torch
-
-from . import capi
 
 D = 512
 ROW = 528
 
 
-def _src(t: torch.Tensor, name: str):
+def _src(t: torch.Tensor, name: str) -> torch.Tensor:
     if not t.is_cuda:
         raise RuntimeError(f"{name} must be on CUDA")
     if t.dtype not in (torch.bfloat16, torch.float32):
         raise RuntimeError(f"{name} must be bf16 or fp32")
     if t.dim() < 2 or t.size(-1) != D:
         raise RuntimeError(f"{name} must have a last dimension of {D}")
-    t = t.contiguous()
-    return t, (capi.DTYPE_BF16 if t.dtype == torch.bfloat16 else capi.DTYPE_F32)
+    return t.contiguous()
+
+
+def _ext():
+    from . import ext      # the package binds it after this module may have been imported
+    return ext()
 
 
 def pack_dual_q64(q: torch.Tensor, paired_storage: bool = False) -> torch.Tensor:
     """q [..., 64, 512] -> u8 [..., 64, 528]: 512 E4M3 bytes + 8 UE8M0 scale bytes stored twice; scale g is
     shared by dims [32g,32g+32) and [256+32g,256+32g+32) (reference pack_dual_q64)."""
-    src, dt = _src(q, "q")
-    out = torch.empty((*src.shape[:-1], ROW), dtype=torch.uint8, device=src.device)
-    rows = src.numel() // D
-    p = capi.PackQParams(rows=rows, src=src.data_ptr(), src_dtype=dt, src_stride_row=D, dst=out.data_ptr(),
-                         dst_stride_row=ROW, paired_storage=int(bool(paired_storage)),
-                         stream=torch.cuda.current_stream(src.device).cuda_stream)
-    with torch.cuda.device(src.device):
-        capi.check(capi.lib().mxdsa_pack_q(C.byref(p)), "mxdsa_pack_q")
-    return out
+    return _ext().pack_q_rows(_src(q, "q"), bool(paired_storage))
 
 
 def pack_dual_prefill_kv64(kv: torch.Tensor) -> torch.Tensor:
@@ -49,16 +41,8 @@ def pack_dual_prefill_kv64(kv: torch.Tensor) -> torch.Tensor:
     slots; scale g covers dims [64g,64g+64) (reference pack_dual_prefill_kv64)."""
     if kv.dim() != 3 or kv.size(1) != 1:
         raise RuntimeError("kv must have shape [s_kv, 1, 512]")
-    src, dt = _src(kv, "kv")
-    n = src.size(0)
-    out = torch.empty(n * ROW, dtype=torch.uint8, device=src.device)
-    if n:
-        p = capi.PackKVParams(rows=n, src=src.data_ptr(), src_dtype=dt, src_stride_row=D, dst=out.data_ptr(),
-                              rows_per_page=n, dst_stride_page=0,
-                              stream=torch.cuda.current_stream(src.device).cuda_stream)
-        with torch.cuda.device(src.device):
-            capi.check(capi.lib().mxdsa_pack_kv(C.byref(p)), "mxdsa_pack_kv")
-    return out.view(n, 1, ROW)
+    n = kv.size(0)
+    return _ext().pack_kv_rows(_src(kv, "kv"), 1, n).view(n, 1, ROW)
 
 
 def pack_dual_decode_kv_pages(kv: torch.Tensor) -> torch.Tensor:
@@ -66,13 +50,5 @@ def pack_dual_decode_kv_pages(kv: torch.Tensor) -> torch.Tensor:
     then page_size 16-byte scale slots (reference pack_dual_decode_kv_pages)."""
     if kv.dim() != 4 or kv.size(2) != 1:
         raise RuntimeError("kv must have shape [pages, page_size, 1, 512]")
-    src, dt = _src(kv, "kv")
-    pages, psz = src.size(0), src.size(1)
-    out = torch.empty((pages, psz * ROW), dtype=torch.uint8, device=src.device)
-    if pages * psz:
-        p = capi.PackKVParams(rows=pages * psz, src=src.data_ptr(), src_dtype=dt, src_stride_row=D,
-                              dst=out.data_ptr(), rows_per_page=psz, dst_stride_page=psz * ROW,
-                              stream=torch.cuda.current_stream(src.device).cuda_stream)
-        with torch.cuda.device(src.device):
-            capi.check(capi.lib().mxdsa_pack_kv(C.byref(p)), "mxdsa_pack_kv")
-    return out.view(pages, psz, 1, ROW)
+    pages, psz = kv.size(0), kv.size(1)
+    return _ext().pack_kv_rows(_src(kv, "kv"), pages, psz).view(pages, psz, 1, ROW)
