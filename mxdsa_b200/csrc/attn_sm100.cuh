@@ -558,19 +558,19 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     const uint32_t cta = cluster_cta_rank();
 
     // ------------------------------------------------------------------ set-up
-    // A programmatic dependent of whatever precedes it on the stream: set-up overlaps that grid's tail, and nothing
-    // in global memory is touched before the wait.  Its own dependents may be set up from now on (they wait for this
-    // grid's completion in the same way).
+    // A programmatic dependent of whatever precedes it on the stream: its CTAs may be resident before that grid has ended,
+    // and nothing in global memory is touched before the wait.  Prefill sets up its barriers ahead of the wait; decode
+    // waits first, because a part without work (few requests on many parts) leaves before it sets anything up.
+    // Dependents of this grid are released by warp 10, once the CTA has passed the wait AND holds its tensor memory: a
+    // dependent that reads data older than this grid ahead of its own wait then finds it complete, and one that
+    // allocates tensor memory cannot take what this grid still needs.
     // What bounds a small call is this start, not the tiles: with one thread initialising sixty barriers, three
     // cluster barriers in a row, the schedule and index loads behind them and parts without work going through all of
     // it, the first row was asked for 8 000 cycles after the start; now 4 500.  With the launch overlap: 256 tokens at
     // topk 128 18.4 -> 14.4 us per call, 37 requests of 2 tokens 25.3 -> 21.7 us, one request of one token 19.8 -> 15.7.
-    grid_launch_dependents();
     if constexpr (DECODE) {
-        // parts without work (few requests on many parts) leave before they set anything up; the schedule is read
-        // while the barriers are initialised
         grid_dependency_wait();
-        const int2 rec = __ldg(reinterpret_cast<const int2*>(p.sched_meta + 8 * blockIdx.y));
+        const int4 rec = WorkIter<DECODE>::record(p, 0);   // a volatile load: it stays behind the wait
         if (rec.x >= p.b || rec.x > rec.y) return;   // the same for both CTAs of the pair
     }
     if (warp == 0) {   // one lane per ring slot: a handful of initialisations in a row instead of sixty
@@ -844,6 +844,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         cluster_wait();
         tmem_alloc<2>(smem_u32(&sm.tmem_base), kTmemCols);
         tmem_relinquish<2>();
+        grid_launch_dependents();   // behind this thread's grid_dependency_wait() and the allocation, see the set-up
         if (lane == 0 && *(volatile uint32_t*)&sm.tmem_base != tmem) raise_fault(sm, 72);
         named_bar_arrive(kBarTmem, 160);   // warps 12-15 write the V scales into it
         if (cta == 0) {

@@ -301,6 +301,12 @@ mxdsa_combine_kernel(int b, int s_q, int by_request, const int* meta, const int*
     const int unit = blockIdx.x / s_q, tok = blockIdx.x % s_q;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int head = blockIdx.y * (kCombineWarps / WPH) + warp / WPH, dim = (warp % WPH) * (512 / WPH) + lane * 4;
+    // Launched as a programmatic dependent of the attention kernel (mxdsa_decode_fwd), this grid may start while that
+    // one is still running.  Everything it reads lies behind the wait: the partials are the attention grid's, and the
+    // schedule may come from a kernel directly ahead of the attention grid, whose completion only the wait carries over.
+    // After a plain launch the wait returns at once.  Blocks without work wait as well: the next grid on the stream may
+    // count on this grid's end for the attention grid's.
+    sm100::grid_dependency_wait();
     int r = unit;
     bool mine = true;
     if (!by_request) {
@@ -315,11 +321,6 @@ mxdsa_combine_kernel(int b, int s_q, int by_request, const int* meta, const int*
         s0 = num_splits[r];
         n = num_splits[r + 1] - s0;
     }
-    // Launched as a programmatic dependent of the attention kernel (mxdsa_decode_fwd), this grid may start while
-    // that one is still running: everything above reads the schedule only, everything below reads the partials,
-    // which are complete and visible once the wait returns.  After a plain launch the wait returns at once.  Blocks
-    // without work wait as well: the next grid on the stream may count on this grid's end for the attention grid's.
-    sm100::grid_dependency_wait();
     if (n <= 1) return;
     const float* lse_in = lse_accum + ((long long)s0 * s_q + tok) * 64 + head;
     const long long lse_stride = (long long)s_q * 64;
@@ -704,7 +705,7 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     if (st != MXDSA_OK) return st;
     if (!combine) return MXDSA_OK;
     // programmatic dependent launch: the combine grid is set up while the attention grid drains (the attention
-    // kernel releases its dependents as soon as it has started; the combine kernel waits before it reads)
+    // kernel releases its dependents once it runs; the combine kernel waits before it reads anything)
     return launch_combine(p->b, p->s_q, p->num_sm_parts, p->sched_meta, p->num_splits, o_accum, lse_accum, p->attn_sink,
                           static_cast<__nv_bfloat16*>(p->out), p->lse, true, d->sm_count, stream);
 }

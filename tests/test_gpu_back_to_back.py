@@ -1,0 +1,64 @@
+"""Calls of different kinds queued one behind the other without a synchronisation give what each gives alone: the grids
+are programmatic dependents of one another, so each is set up while the one ahead of it still runs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+SCALE = 512 ** -0.5
+
+
+def _decode_inputs(b, s_q, topk, extra, g):
+    from mxdsa_b200 import packing, quantize
+    q = quantize.pack_dual_q64(torch.randn(b * s_q, 64, 512, device="cuda", generator=g)).view(b, s_q, 64, 528)
+    kvf, w1, w2 = packing.make_rank1_kv((2 * b + 16, 64, 1), device="cuda", generator=g)
+    kv = quantize.pack_dual_decode_kv_pages(kvf)
+    pick = lambda n, k: torch.rand(b * s_q, n, device="cuda", generator=g).argsort(1)[:, :k].sort(1).values.int().view(b, s_q, k)
+    main = pick(128, topk) + torch.arange(b, device="cuda", dtype=torch.int32).view(b, 1, 1) * 128
+    return dict(q=q, kv=kv[: 2 * b].contiguous(), idx=main, ekv=kv[2 * b:].contiguous(), eidx=pick(1024, extra), w1=w1, w2=w2)
+
+
+def _decode(d, lengths, op, meta=None, splits=None):
+    return op(d["q"], d["kv"], d["idx"], None, None, meta, splits, d["ekv"], d["eidx"], lengths, 512, 512, SCALE, d["w1"], d["w2"])
+
+
+@pytest.mark.parametrize("b,s_q", [(3, 6), (30, 6), (16, 5), (1, 8), (40, 1)])
+def test_schedule_then_decode_then_others(b, s_q):
+    import mxdsa_b200 as M
+    from mxdsa_b200 import packing, quantize
+    g = torch.Generator(device="cuda").manual_seed(100 * b + s_q)
+    d = _decode_inputs(b, s_q, 128, 512, g)
+    # two sets of lengths whose schedules divide different requests
+    short = torch.randint(0, 65, (b,), device="cuda", generator=g).int()
+    long = torch.full((b,), 512, device="cuda").int()
+    q = quantize.pack_dual_q64(torch.randn(64, 64, 512, device="cuda", generator=g))
+    kvf, w1, w2 = packing.make_rank1_kv((512, 1), device="cuda", generator=g)
+    kv = quantize.pack_dual_prefill_kv64(kvf)
+    idx = torch.rand(32, 512, device="cuda", generator=g).argsort(1)[:, :128].int().view(32, 1, 128)
+    prefill = lambda: M.dual_mxfp8_head64_sparse_prefill_fwd(q, kv, idx, SCALE, w1, w2, None, None)
+    split, whole = M.dual_mxfp8_sparse_decode_fwd, M.dual_mxfp8_sparse_decode_fwd_whole
+
+    alone = {}
+    for name, lengths in (("short", short), ("long", long)):
+        for kind, op in (("split", split), ("whole", whole)):
+            alone[kind, name] = _decode(d, lengths, op)
+            torch.cuda.synchronize()
+    alone["prefill"] = prefill()
+    torch.cuda.synchronize()
+    assert not torch.equal(alone["split", "short"][2], alone["split", "long"][2])       # two different schedules
+
+    meta, splits = (torch.empty_like(t) for t in alone["split", "short"][2:])
+    got = []
+    for _ in range(6):
+        for name, lengths in (("short", short), ("long", long)):
+            got.append((("split", name), _decode(d, lengths, split)))          # the schedule is made in the call
+            got.append(("prefill", prefill()))
+            got.append((("whole", name), _decode(d, lengths, whole)))
+            meta.copy_(alone["split", name][2])                                # the schedule is written right ahead of the call
+            splits.copy_(alone["split", name][3])
+            got.append((("split", name), _decode(d, lengths, split, meta, splits)))
+    torch.cuda.synchronize()
+    M.device_fault()
+    for key, out in got:
+        n = 3 if key == "prefill" else 2
+        assert all(torch.equal(a, r) for a, r in zip(out[:n], alone[key][:n])), key

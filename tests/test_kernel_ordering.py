@@ -1,0 +1,36 @@
+"""Orders between grids and between the CTAs of a pair that no run on a GPU can be relied on to show when they are lost.
+They are read off the kernels' source: what a grid reads stands behind its wait for the grids ahead of it, and its
+dependents are released behind that wait."""
+import os
+import re
+
+CSRC = os.path.join(os.path.dirname(os.path.abspath(__file__)), "..", "mxdsa_b200", "csrc")
+
+
+def body(name: str, kernel: str) -> str:
+    """The kernel's function body, comments taken out."""
+    with open(os.path.join(CSRC, name)) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    at = text.index("{", re.search(r"__launch_bounds__\([^{;]*\)\s*" + kernel + r"\(", text).end())
+    depth, end = 1, at + 1
+    while depth:
+        depth += {"{": 1, "}": -1}.get(text[end], 0)
+        end += 1
+    return text[at:end]
+
+
+def test_combine_reads_schedule_and_partials_behind_its_wait():
+    b = body("mxdsa_lib.cu", "mxdsa_combine_kernel")
+    ahead = b[: b.index("grid_dependency_wait()")]
+    assert not re.search(r"\b(meta|num_splits|o_accum|lse_accum|sink)\b", ahead), ahead
+
+
+def test_attention_releases_its_dependents_behind_its_wait():
+    b = body("attn_sm100.cuh", "mxdsa_attn_kernel")
+    waits = [m.start() for m in re.finditer(r"grid_dependency_wait\(\)", b)]
+    release = [m.start() for m in re.finditer(r"grid_launch_dependents\(\)", b)]
+    assert len(waits) == 2 and len(release) == 1        # one wait for each instantiation
+    assert max(waits) < release[0]
+    assert b.index("tmem_alloc<2>") < release[0]        # the CTA holds its tensor memory before a dependent may start
+    ahead = b[: waits[0]]
+    assert not re.search(r"\bp\.|__ldg|WorkIter", ahead), ahead      # decode: nothing at all is touched ahead of the wait
