@@ -279,6 +279,7 @@ template <bool DECODE> struct WorkIter {
             return true;
         }
     }
+    __device__ bool done() const { return DECODE ? req > end_req : next_pair >= p.num_pairs; }
     __device__ WorkOutput output(const WorkItem& w) const {
         WorkOutput o = {0, 0};
         if constexpr (DECODE) {
@@ -542,6 +543,8 @@ template <typename Plan> __device__ __noinline__ void raise_fault(Plan& sm, int 
     // tell the peer CTA so that its roles stop waiting as well
     const uint32_t peer = map_to_cta(smem_u32(&sm.abort_word), cluster_cta_rank() ^ 1u);
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(peer), "r"(1) : "memory");
+    // an epilogue warp arrives at the tear-down's cluster barrier without a release: this store must not outlive the peer
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
     if (atomicCAS(&sm.fault->flag, 0, 1) == 0) sm.fault->where = code;
 }
 
@@ -852,6 +855,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             WorkIter<DECODE> it(p);
             WorkItem w;
             uint32_t gt = 0, gw = 0;
+            bool released = false;
             const uint32_t pv_half_peer = map_to_cta(smem_u32(&sm.bar_pv_half[0]), 1);
             const uint32_t pv_done_peer = map_to_cta(smem_u32(&sm.bar_pv_done[0]), 1);
             MXDSA_WAIT_TIGHT(sm.bar_tmem_ready, 0, 24);
@@ -898,8 +902,11 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                         __syncwarp();
                     }
                 }
+                released = !it.done();
                 ++gw;
             }
+            // "O drained" is not signalled for a role's last work item; where only empty ones follow it has been
+            if (released) MXDSA_WAIT(sm.bar_o_empty, (gw & 1) ^ 1, 31);
         }
     } else if (warp == 11) {
         // ===================== operand stager =====================
@@ -983,6 +990,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             ++gw;
         }
         if (gw == 0) cluster_wait();
+        else MXDSA_WAIT(sm.bar_q_empty, (gw & 1) ^ 1, 42);   // CTA 0's issuers signal it for the last pair too
     }
     } else if (warp < 12 + 4 * G) {
         if constexpr (kRebalanceRegs) setmaxnreg_inc<kRegsSoftmax>();
@@ -1248,15 +1256,16 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         const uint32_t lane_addr = tmem + (uint32_t(q4 * 32) << 16);
         const uint32_t o_empty0 = map_to_cta(smem_u32(&sm.bar_o_empty), 0);
         cluster_wait();
+        WorkIter<DECODE> it(p);
+        WorkItem w;
         // O is free for the next pair's first PV as soon as this warp has READ its last columns; the stores of
-        // those columns (which may have to wait for a staging tile) follow after the release.
+        // those columns (which may have to wait for a staging tile) follow after the release.  Nothing is signalled where
+        // no pair follows: CTA 0 may be gone before an arrival that nobody waits for has come.
         auto release_o = [&]() {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(o_empty0);
+            if (lane == 0 && !it.done()) mbar_arrive_cluster(o_empty0);
         };
-        WorkIter<DECODE> it(p);
-        WorkItem w;
         uint32_t gt = 0, gw = 0;
         uint32_t round = 0;   // output rounds of this warp so far (staging tile = round % kOutTiles)
 #pragma unroll 1
@@ -1361,6 +1370,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             }
             ++gw;
         }
+        // CTA 0 signals this one for every tile, whether a maximum grew or not
+        if (NT == 64 && gt > 0) MXDSA_WAIT(sm.bar_pv_half[(gt - 1) % kSBufs], ((gt - 1) / kSBufs) & 1, 57);
     }
 
 done:
@@ -1377,8 +1388,9 @@ done:
         named_bar_arrive(1 + kGroups, kGroups * 128);
     }
     tc_fence_before();
-    // Nobody leaves while the peer may still signal it.  The epilogue warps arrive without a release: there is
-    // nothing for the peer to read, and a release would wait for the global stores of the last pair.
+    // Nobody leaves while the peer may still signal it: the cluster barrier's release orders every arrival on a barrier of
+    // the peer ahead of the peer's exit.  The epilogue warps arrive without a release, which would wait for their global
+    // stores of the last pair: all that they signal the peer, "O drained", is waited for by CTA 0's PV issuer.
     if (warp >= 12 + 4 * G) cluster_arrive_relaxed();
     else cluster_arrive();
     cluster_wait();

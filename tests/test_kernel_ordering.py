@@ -34,3 +34,20 @@ def test_attention_releases_its_dependents_behind_its_wait():
     assert b.index("tmem_alloc<2>") < release[0]        # the CTA holds its tensor memory before a dependent may start
     ahead = b[: waits[0]]
     assert not re.search(r"\bp\.|__ldg|WorkIter", ahead), ahead      # decode: nothing at all is touched ahead of the wait
+
+
+def test_nobody_leaves_ahead_of_the_peers_last_arrivals():
+    """An arrival on a barrier of a CTA that has ended is a write to memory that is no longer its own.  The tear-down's
+    cluster barrier orders what was signalled by warps that release at it.  The epilogue warps do not: they signal nothing
+    for their last work item, and what they have signalled is waited for.  What the tensor core's commits signal for the
+    last item is waited for by the CTA that is signalled."""
+    b = body("attn_sm100.cuh", "mxdsa_attn_kernel")
+    assert "cluster_arrive_relaxed()" in b[b.index("done:"):]
+    release = b[b.index("release_o = ["):]
+    assert re.search(r"!it\.done\(\)\) mbar_arrive_cluster\(o_empty0\)", release[: release.index("};")])
+    for barrier, role_from, role_to in (("bar_o_empty", "else if (warp == 10)", "else if (warp == 11)"),
+                                        ("bar_q_empty", "else if (warp == 11)", "else if (warp < 12 + 4 * G)"),
+                                        (r"bar_pv_half\[", "release_o = ", "done:")):
+        role = b[b.index(role_from): b.index(role_to)]
+        last_item = role.rindex("++gw;")        # a role's loop over its work items ends by counting one
+        assert re.search(r"MXDSA_WAIT\(sm\." + barrier, role[last_item:]), barrier
