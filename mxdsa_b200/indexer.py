@@ -15,6 +15,17 @@ from typing import Optional, Tuple
 import torch
 
 
+def _score_rows(scores: torch.Tensor) -> torch.Tensor:
+    """`scores` [n, s_kv] with the strides that the kernel is to read it by.  It takes a row stride of 0 for s_kv, so a
+    row that is broadcast over n is copied out; the stride of a single row means nothing and is set to s_kv."""
+    n, s_kv = scores.shape
+    if scores.stride(1) != 1 or (n > 1 and scores.stride(0) == 0):
+        scores = scores.contiguous()
+    if n == 1:
+        scores = scores.as_strided((1, s_kv), (s_kv, 1))
+    return scores
+
+
 def select_topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch.Tensor] = None,
                         pair: bool = False, row_offset: Optional[torch.Tensor] = None
                         ) -> Tuple[torch.Tensor, torch.Tensor]:
@@ -27,8 +38,6 @@ def select_topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch
     """
     if not scores.is_cuda or scores.dtype != torch.float32 or scores.dim() != 2:
         raise RuntimeError("scores must be a CUDA float32 tensor of shape [n, s_kv]")
-    if scores.stride(1) != 1:
-        scores = scores.contiguous()
     n, s_kv = scores.shape
     group = 2 if pair else 1
     if n % group:
@@ -36,6 +45,7 @@ def select_topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch
     if s_kv <= 0 or s_kv % 4 or topk <= 0:
         raise RuntimeError("s_kv must be a positive multiple of 4 and topk positive")
     rows = n // group
+    scores = _score_rows(scores)
 
     def opt(t, name):
         if t is None:

@@ -125,6 +125,18 @@ def test_samples_that_mislead(rows, s_kv):
     _check(s, 1500)
 
 
+def test_broadcast_and_single_rows():
+    from mxdsa_b200.indexer import select_topk_indices
+    x = torch.randn(1, 20480, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
+    want = select_topk_indices(x, 300)
+    for n, pair in ((5, False), (6, True)):
+        got = select_topk_indices(x.expand(n, -1), 300, None, pair)
+        rows = n // (2 if pair else 1)
+        assert torch.equal(got[0], want[0].expand(rows, -1)) and torch.equal(got[1], want[1].expand(rows))
+    got = select_topk_indices(x.view(20480, 1).t(), 300)       # one row whose stride is 1
+    assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+
+
 def test_argument_rules():
     from mxdsa_b200.indexer import select_topk_indices
     dev = torch.device("cuda:0")
