@@ -7,11 +7,11 @@
 //   scale = 2^ceil(log2(max(amax/448, 2^-126)));  code = e4m3(clamp(x / scale, -448, 448))
 // with the ceil(log2()) taken exactly from the bits of amax (see scale_byte).
 //
-// Bound: HBM.  Algorithmic bytes per row: 512 * sizeof(input element) read + 528 written.  A warp takes two
-// adjacent rows at a time: both rows' loads are in flight together, and the 1056 bytes it writes for queries begin
-// and end on whole 32-byte sectors.  What used to come before the memory was the instruction count -- a 64-bit
-// division and remainder per row, a rounded float division, two clamps per value, byte stores of the slot; see the
-// comments below for what stands in their place.
+// Bound: HBM.  Algorithmic bytes per row: 512 * sizeof(input element) read + 528 written.  In a long call a warp takes
+// two adjacent rows at a time: both rows' loads are in flight together, and the 1056 bytes it writes for queries begin
+// and end on whole 32-byte sectors.  A short call takes one, see launch().  What used to come before the memory was the
+// instruction count -- a 64-bit division and remainder per row, a rounded float division, two clamps per value, byte
+// stores of the slot; see the comments below for what stands in their place.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -22,7 +22,6 @@ namespace {
 
 constexpr int kDim = 512;
 constexpr int kWarpsPerBlock = 8;
-constexpr int kRowsPerWarp = 2;
 
 // UE8M0 byte of 2^ceil(log2(max(amax/448, 2^-126))) and the factor 2^-e to multiply by, without the division.
 // Write amax = m * 2^e, 1 <= m < 2, and 448 = 1.75 * 2^8.  The correctly rounded quotient is at most 2^(e-8) for
@@ -92,8 +91,8 @@ __device__ __forceinline__ uint32_t codes(float2 x, float inv) {
 
 // QGROUPS: true  -> Q rows: scale g covers dims [32g,32g+32) and [256+32g,256+32g+32)
 //          false -> KV rows: scale g covers dims [64g,64g+64)
-// Lane L owns dims [16L, 16L+16).
-template <typename T, bool QGROUPS>
+// Lane L owns dims [16L, 16L+16) of the ROWS rows that its warp takes at a time.
+template <typename T, bool QGROUPS, int ROWS>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 mxdsa_pack_rows_kernel(const T* __restrict__ src, long long src_stride, long long rows, uint8_t* __restrict__ data,
                        long long data_stride, uint8_t* __restrict__ slots, long long slot_stride, int rows_per_page,
@@ -109,15 +108,15 @@ mxdsa_pack_rows_kernel(const T* __restrict__ src, long long src_stride, long lon
     // where this lane's scale byte goes in the two slot words (each group's first lane contributes)
     const bool leader = QGROUPS ? (lane < 16 && (lane & 1) == 0) : ((lane & 3) == 0);
     const int g = QGROUPS ? (lane >> 1) : (lane >> 2);
-    for (long long r0 = kRowsPerWarp * warp0; r0 < rows; r0 += kRowsPerWarp * nwarps) {
-        Raw16<T> x[kRowsPerWarp];
+    for (long long r0 = ROWS * warp0; r0 < rows; r0 += ROWS * nwarps) {
+        Raw16<T> x[ROWS];
 #pragma unroll
-        for (int u = 0; u < kRowsPerWarp; ++u) {
+        for (int u = 0; u < ROWS; ++u) {
             const long long r = r0 + u < rows ? r0 + u : r0;     // past the end: the row before once more, not stored
             x[u].load(src + r * src_stride + 16 * lane);
         }
 #pragma unroll
-        for (int u = 0; u < kRowsPerWarp; ++u) {
+        for (int u = 0; u < ROWS; ++u) {
             const long long r = r0 + u;
             float amax = x[u].amax();
             // the group's four lanes: Q {2g, 2g+1, 2g+16, 2g+17}; KV {4g .. 4g+3}
@@ -165,10 +164,16 @@ int launch(const T* src, long long src_stride, long long rows, uint8_t* data, lo
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return MXDSA_ERR_CUDA;
-    const long long want = (rows + kRowsPerWarp * kWarpsPerBlock - 1) / (kRowsPerWarp * kWarpsPerBlock);
-    const int grid = (int)(want < (long long)sms * 8 ? want : (long long)sms * 8);   // 8 resident CTAs of 256 threads per SM
-    mxdsa_pack_rows_kernel<T, Q><<<grid, kWarpsPerBlock * 32, 0, stream>>>(src, src_stride, rows, data, data_stride, slots,
-                                                                           slot_stride, rows_per_page, page_stride, paired);
+    // Two rows at a time pay where every warp has many: 262 144 rows of bf16 72.2 us (one at a time 72.7), 1 048 576 272
+    // (287); f32 106 (122) and 410 (478).  Below that the longer code and the higher register count (42 to 59 against 32 to
+    // 40: 4 or 5 resident CTAs of the 8 per SM that are launched, against 6 to 8) cost more: 65 536 rows of bf16 20.9 us
+    // (19.1), 4 096 4.1 (3.4), 64 2.4 (1.6); f32 16 384 rows 9.5 (9.3), 4 096 4.5 (4.2), 64 3.0 (2.3).  All from a cold L2.
+    const long long most = (long long)sms * 8, full = most * kWarpsPerBlock;     // warps of a full grid
+    const int each = rows <= full * (sizeof(T) == 2 ? 16 : 2) ? 1 : 2;
+    const long long want = (rows + each * kWarpsPerBlock - 1) / (each * kWarpsPerBlock);
+    (each == 1 ? mxdsa_pack_rows_kernel<T, Q, 1> : mxdsa_pack_rows_kernel<T, Q, 2>)
+        <<<(unsigned)(want < most ? want : most), kWarpsPerBlock * 32, 0, stream>>>(src, src_stride, rows, data, data_stride, slots,
+                                                                                    slot_stride, rows_per_page, page_stride, paired);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) {
         tl_pack_cuda_error = (int)e;

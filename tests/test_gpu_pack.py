@@ -139,3 +139,22 @@ def test_argument_rules():
     assert L.mxdsa_pack_q(ctypes.byref(p)) == 2          # unknown dtype
     k = capi.PackKVParams(rows=10, src=buf.data_ptr(), src_dtype=0, dst=buf.data_ptr(), rows_per_page=4)
     assert L.mxdsa_pack_kv(ctypes.byref(k)) == 2         # rows not a multiple of the page size
+
+
+@pytest.mark.parametrize("dtype,per_warp", [(torch.bfloat16, 16), (torch.float32, 2)])
+@pytest.mark.parametrize("kind", ["q", "kv", "pages"])
+def test_both_sides_of_the_row_count_at_which_a_warp_takes_two_rows(dtype, per_warp, kind):
+    """The rows around the line, packed in one call, equal the same rows packed in small calls."""
+    from mxdsa_b200 import quantize as Z
+    line = torch.cuda.get_device_properties(0).multi_processor_count * 64 * per_warp
+    step = 1 if kind == "kv" else 64           # whole tokens of 64 heads, whole pages of 64 rows
+    g = torch.Generator(device="cuda").manual_seed(17)
+    x = torch.randn(line + step, 512, device="cuda", generator=g, dtype=dtype)
+    pack = {"q": lambda t: Z.pack_dual_q64(t.view(-1, 64, 512)).view(-1, 528),
+            "kv": lambda t: Z.pack_dual_prefill_kv64(t.view(-1, 1, 512)).view(-1),
+            "pages": lambda t: Z.pack_dual_decode_kv_pages(t.view(-1, 64, 1, 512)).view(-1, 64 * 528)}[kind]
+    for rows in (line, line + step):
+        got, parts = pack(x[:rows]), [pack(x[i: min(i + 4096, rows)]) for i in range(0, rows, 4096)]
+        if kind == "kv":                       # all data rows, then all slots
+            parts = [torch.cat([p[: p.numel() // 528 * 512] for p in parts]), torch.cat([p[p.numel() // 528 * 512:] for p in parts])]
+        assert torch.equal(got, torch.cat(parts))
