@@ -18,8 +18,8 @@
 //
 // Two kernels.  mxdsa_topk_rows_kernel counts every key.  mxdsa_topk_pivot_kernel, for rows of more than 16 384 keys,
 // finds a score that a little more than topk keys reach from a sample of every eighth key, lists the keys at or above
-// it in one sweep of the row and selects exactly among those; where there are fewer rows than SMs it divides a row
-// among the CTAs of a cluster.
+// it in one sweep of the row and selects exactly among those (rows of many equal scores are counted instead); where there
+// are fewer rows than SMs it divides a row among the CTAs of a cluster.
 //
 // Counting every key: exact radix selection on the order-preserving 32-bit image of the float, three histogram
 // passes (11 + 11 + 10 bits) with shared-memory atomics, keys of a row held in registers (one HBM read
@@ -317,15 +317,16 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 // For rows of more than 16 384 keys the kernel above sweeps the row four times and spends three shared-memory atomics
 // on every key.  Here
 //   1. every eighth key (four per thread) is a sample; two histogram passes over the samples give a pivot: the lower
-//      edge, to 22 bits, of the rank'th largest, rank = topk/8 + 5 sqrt(topk/8) + 8, so that about 1.2 to 1.4 topk keys
-//      reach it and fewer than topk do with a probability of less than 1e-6 for samples that are independent;
+//      edge, to 22 bits, of the rank'th largest, rank = topk/8 + 5 sqrt(topk/8) + 8, so that about 8 rank keys reach it
+//      (1.24 topk of them at topk 4096, 1.34 at 2048, 3.75 at 64) and fewer than topk do with a probability of less than
+//      1e-6 for samples that are independent;
 //   2. one sweep compares every score with the pivot (as floats: NaN, -inf and keys past the length fail by
 //      themselves) and lists key and position of those that reach it, in ascending position, in shared memory;
 //   3. the topk-th largest of the list is found by histogram passes over the list alone, whose digits start at the
 //      pivot and span just the range up to the list's maximum, so that the entries spread over the bins and the first
 //      or second pass usually decides; the list is compacted to the output with ballots.
-// A row where the list overflows or falls short (a sample that misled, heavy ties) is counted key by key.  Rows of up
-// to kShortRow keys skip the sampling: every usable key is listed.
+// A row where the list overflows or falls short (heavy ties, a sample that misled) is counted, see recount_row.  Rows of
+// up to kShortRow keys skip the sampling: every usable key is listed.
 //
 // Measured against the kernel above (cold L2, us): 2048 rows of 32 768 keys, topk 2048 195.6 -> 134.2 (pairs 257 -> 183),
 // of 65 536 keys 355 -> 196; 64 rows of 65 536 keys, half to full length 28.7 -> 20.5; one pair of 131 072 keys 72.7 -> 24.6.
@@ -334,7 +335,6 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 //
 // CLUSTER: the CTAs of a cluster divide a row's keys in order; they add up their sample histograms through distributed
 // shared memory, each lists its own part, and the first one gathers the lists and finishes the row.
-//
 constexpr int kList = 8192;                        // capacity of the list (64 KB of shared memory; two CTAs per SM)
 constexpr int kShortRow = 4096;
 constexpr int kMaxSweeps = 8;                      // a CTA's part of a row: samples stay in registers (4 per sweep)
@@ -348,6 +348,7 @@ struct PivotShared {
     uint32_t list_n;                               // entries of this CTA's list; kList + 1: it did not fit
     uint32_t key_max;                              // largest key of this CTA's part
     uint32_t warp_gt[kWarps], warp_eq[kWarps];
+    uint4 part_count[2];                           // recount: this CTA's keys above | inside an interval, smallest and largest inside
     uint32_t few_n;                                // entries of the last bin when they are few, gathered
     uint2 few[32];                                 // (key, place in the list)
     uint2 list[kList];                             // (score, later its key; position in the row)
@@ -444,12 +445,12 @@ __device__ __forceinline__ float4 load_scores4(const float* __restrict__ row0, c
     }
     return v;
 }
-template <int GROUP>
+template <int GROUP, int CHUNKS>
 __device__ __forceinline__ void load_scores(const float* __restrict__ row0, const float* __restrict__ row1, int j0, int end,
-                                            float (&s)[kKpt]) {
-    constexpr int kBatch = GROUP == 2 ? kChunks / 4 : kChunks / 2;      // 16-byte loads in flight, per row
+                                            float (&s)[4 * CHUNKS]) {
+    constexpr int kBatch = GROUP == 2 ? 2 : 4;                          // 16-byte loads in flight, per row
 #pragma unroll
-    for (int c0 = 0; c0 < kChunks; c0 += kBatch) {
+    for (int c0 = 0; c0 < CHUNKS; c0 += kBatch) {
         const int jb = j0 + (c0 * kThreads + (int)threadIdx.x) * 4;
         if (j0 + (c0 + kBatch) * kThreads * 4 <= end) {             // all of the batch is there: no bounds per key
             float4 a[kBatch], b[GROUP == 2 ? kBatch : 1];
@@ -649,68 +650,217 @@ __device__ __forceinline__ void select_from_list(PivotShared& sm, uint32_t n, ui
     __syncthreads();
 }
 
-// A row in which the list did not work out, by counting every key, straight from memory: the rare case, written for few
-// registers (in the form of mxdsa_topk_rows_kernel, inlined or called, it made the whole kernel spill).
+// ---- A row whose keys the list cannot hold, or whose sample misled: by counting its keys, straight from memory.
+//
+// The CTAs of a cluster share the sweeps, each over its own part of the row.  One sweep counts the keys above the pivot's
+// interval of 1024 keys and inside it.  As a rule that settles it: thousands of equal scores reach the pivot, the
+// threshold is their value, and a second sweep writes the indices.  Otherwise a histogram of the interval, or three of
+// all keys, finds the threshold; and where the keys above the interval alone are enough, the row is listed once more from
+// there.  Rows of which the sample says that the list cannot hold them are not listed in the first place.
+// Against counting every key three times (us, cold L2: mxdsa_topk_rows_kernel / a misled row counted by one CTA, as it was
+// for a while / now): 64 rows of 65 536 keys, topk 2048, all but 1.4 % of them zero 34.8 / 79.2 / 22.4; the same key
+// throughout 34.7 / 75.3 / 22.2; 300 rows of 32 768 48.2 / 63.8 / 36.1; 2048 rows of 65 536 423 / 518 / 289.
+constexpr int kRecountChunks = 4;                  // chunks of keys per step: half a sweep, to stay inside the register budget
+constexpr int kRecountStep = kRecountChunks * kThreads * 4;
+
+// Sum over the CTAs of the row of this thread's four bins; a barrier (of the cluster) stands ahead of it.
+template <bool CLUSTER>
+__device__ __forceinline__ uint4 row_bins(const uint32_t* hist, uint32_t parts) {
+    const int tid = threadIdx.x;
+    uint4 h;
+    if (CLUSTER) {
+        cluster_barrier();
+        h = make_uint4(0u, 0u, 0u, 0u);
+        for (uint32_t c = 0; c < parts; ++c) {
+            const uint4 o = peer_load4(peer_address(&hist[4 * tid], c));
+            h.x += o.x; h.y += o.y; h.z += o.z; h.w += o.w;
+        }
+    } else {
+        __syncthreads();
+        h = *reinterpret_cast<const uint4*>(&hist[4 * tid]);
+    }
+    return h;
+}
+
+// Counts this CTA's keys from `hi` on and those in [lo, hi) into sm.part_count[slot], with the smallest and largest of the
+// latter.  (`hi` beyond +inf is a NaN, which no key reaches.)
 template <int GROUP>
-__device__ __forceinline__ void misled_row(PivotShared& sm, const float* __restrict__ row0, const float* __restrict__ row1,
-                                           int len, int topk, int32_t* __restrict__ out, int32_t off,
-                                           int32_t* __restrict__ count) {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    uint32_t prefix = 0, k = (uint32_t)topk, n_sel = 0;
-#pragma unroll 1
-    for (int pass = 0; pass < 3; ++pass) {
-        const int lo = pass == 0 ? 21 : (pass == 1 ? 10 : 0);
-        const int hi = pass == 0 ? 32 : (pass == 1 ? 21 : 10);
-        const uint32_t first = pass == 0 ? 0u : prefix << hi;
-        const uint32_t spare = (uint32_t)((pass == 2 ? kBins / 2 : kBins) + lane);
-        *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
-        __syncthreads();
-#pragma unroll 2
-        for (int j = 4 * tid; j < len; j += 4 * kThreads) {
-            const float4 v = load_scores4<GROUP>(row0, row1, j, len);
-            atomicAdd(&sm.hist[min((score_key(v.x) - first) >> lo, spare)], 1u);
-            atomicAdd(&sm.hist[min((score_key(v.y) - first) >> lo, spare)], 1u);
-            atomicAdd(&sm.hist[min((score_key(v.z) - first) >> lo, spare)], 1u);
-            atomicAdd(&sm.hist[min((score_key(v.w) - first) >> lo, spare)], 1u);
-        }
-        __syncthreads();
-        uint32_t k_now;
-        const uint32_t total = find_bin(sm, k, pass == 0, k_now, pass == 2 ? kBins / 2 : kBins);
-        if (pass == 0) n_sel = k_now;
-        if (total == 0u || k_now == 0u) { n_sel = 0; break; }
-        prefix = pass == 0 ? sm.sel_bin : ((prefix << (hi - lo)) | sm.sel_bin);
-        k = k_now - sm.sel_above;
-    }
-    uint32_t base_gt = 0, base_eq = 0;
-#pragma unroll 1
-    for (int j0 = 0; n_sel > 0u && j0 < len; j0 += 4 * kThreads) {
-        const int j = j0 + 4 * tid;
-        const float4 v = load_scores4<GROUP>(row0, row1, j, len);
-        const uint32_t key[4] = {score_key(v.x), score_key(v.y), score_key(v.z), score_key(v.w)};
-        uint32_t own = 0;                          // keys above the threshold | equal to it << 16
-#pragma unroll
-        for (int e = 0; e < 4; ++e) own += key[e] > prefix ? 1u : (key[e] == prefix ? 1u << 16 : 0u);
-        const uint32_t inc = warp_inclusive_scan(own, lane);
-        if (lane == 31) sm.warp_tot[warp] = inc;
-        __syncthreads();
-        const uint32_t wt = lane < kWarps ? sm.warp_tot[lane] : 0u;
-        const uint32_t before = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u) + inc - own;
-        const uint32_t total = __reduce_add_sync(0xffffffffu, wt);
-        uint32_t a = base_gt + (before & 0xffffu), q = base_eq + (before >> 16);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const bool is_gt = key[e] > prefix, is_eq = key[e] == prefix;
-            if (is_gt || (is_eq && q < k)) out[a + min(q, k)] = j + e + off;
-            a += is_gt ? 1u : 0u;
-            q += is_eq ? 1u : 0u;
-        }
-        base_gt += total & 0xffffu;
-        base_eq += total >> 16;
-        __syncthreads();
-    }
-    for (uint32_t pos = n_sel + tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = -1;
-    if (count != nullptr && tid == 0) *count = (int32_t)n_sel;
+__device__ __forceinline__ void count_part(PivotShared& sm, int slot, const float* __restrict__ row0,
+                                           const float* __restrict__ row1, int begin, int end, float lo, float hi) {
+    uint4& total = sm.part_count[slot];
+    if (threadIdx.x == 0) total = make_uint4(0u, 0u, 0xffffffffu, 0u);
     __syncthreads();
+    uint32_t above = 0u, from = 0u;
+    float least = CUDART_INF_F, most = -CUDART_INF_F;
+#pragma unroll 1
+    for (int j0 = begin; j0 < end; j0 += kRecountStep) {
+        float s[4 * kRecountChunks];
+        load_scores<GROUP, kRecountChunks>(row0, row1, j0, end, s);
+#pragma unroll
+        for (int i = 0; i < 4 * kRecountChunks; ++i) {
+            const bool ge = s[i] >= lo, gt = s[i] >= hi;
+            from += ge ? 1u : 0u;
+            above += gt ? 1u : 0u;
+            if (ge && !gt) {
+                least = fminf(least, s[i]);
+                most = fmaxf(most, s[i]);
+            }
+        }
+    }
+    above = __reduce_add_sync(0xffffffffu, above);
+    from = __reduce_add_sync(0xffffffffu, from);
+    const uint32_t key_lo = __reduce_min_sync(0xffffffffu, score_key(least)), key_hi = __reduce_max_sync(0xffffffffu, score_key(most));
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&total.x, above);
+        atomicAdd(&total.y, from - above);
+        atomicMin(&total.z, key_lo);
+        atomicMax(&total.w, key_hi);
+    }
+}
+// The counts of the whole row, and what of them lies in the parts ahead of this one.
+template <bool CLUSTER>
+__device__ __forceinline__ uint4 row_counts(PivotShared& sm, int slot, uint32_t parts, uint32_t part, uint2& ahead) {
+    ahead = make_uint2(0u, 0u);
+    if (!CLUSTER) {
+        __syncthreads();
+        return sm.part_count[slot];
+    }
+    cluster_barrier();
+    uint4 all = make_uint4(0u, 0u, 0xffffffffu, 0u);
+    for (uint32_t c = 0; c < parts; ++c) {
+        const uint4 o = peer_load4(peer_address(&sm.part_count[slot], c));
+        if (c < part) ahead = make_uint2(ahead.x + o.x, ahead.y + o.y);
+        all = make_uint4(all.x + o.x, all.y + o.y, min(all.z, o.z), max(all.w, o.w));
+    }
+    return all;
+}
+
+// Histogram of the row's keys in base .. base + span by (key - base) >> sh, and the bin of the k-th largest (sel_*).
+// Returns the number of keys; where it is below k, the bin of the smallest.
+template <int GROUP, bool CLUSTER>
+__device__ __forceinline__ uint32_t count_bins(PivotShared& sm, int slot, const float* __restrict__ row0,
+                                               const float* __restrict__ row1, int begin, int end, uint32_t parts,
+                                               uint32_t base, uint32_t span, int sh, uint32_t k) {
+    uint32_t* hist = &sm.hist[slot * kBins];
+    *reinterpret_cast<uint4*>(&hist[4 * threadIdx.x]) = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+#pragma unroll 1
+    for (int j0 = begin; j0 < end; j0 += kRecountStep) {
+        float s[4 * kRecountChunks];
+        load_scores<GROUP, kRecountChunks>(row0, row1, j0, end, s);
+#pragma unroll
+        for (int i = 0; i < 4 * kRecountChunks; ++i) {
+            const uint32_t d = score_key(s[i]) - base;       // not usable, or below base: beyond the span
+            if (d <= span) atomicAdd(&hist[d >> sh], 1u);
+        }
+    }
+    const uint4 h = row_bins<CLUSTER>(hist, parts);
+    const uint32_t total = locate(sm, h, k);
+    if (total < k && total > 0u) locate(sm, h, total);
+    return total;
+}
+
+// Writes the positions of this CTA's keys from `hi` on and of the first `need` of the row's keys in [lo, hi), in
+// ascending position; `ahead`: how many of either lie in the parts before this one.
+template <int GROUP>
+__device__ __forceinline__ void emit_part(PivotShared& sm, const float* __restrict__ row0, const float* __restrict__ row1,
+                                          int begin, int end, float lo, float hi, uint32_t need, uint2 ahead,
+                                          int32_t* __restrict__ out, int32_t off) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll 1
+    for (int j0 = begin; j0 < end; j0 += kRecountStep) {
+        float s[4 * kRecountChunks];
+        load_scores<GROUP, kRecountChunks>(row0, row1, j0, end, s);
+        uint32_t above = 0u, inside = 0u;          // a bit per key
+        uint32_t own_a = 0u, own_i = 0u;           // counts, a byte per chunk (a warp's total per chunk is at most 128)
+#pragma unroll
+        for (int i = 0; i < 4 * kRecountChunks; ++i) {
+            const bool ge = s[i] >= lo, gt = s[i] >= hi;
+            above |= gt ? 1u << i : 0u;
+            inside |= ge && !gt ? 1u << i : 0u;
+        }
+#pragma unroll
+        for (int c = 0; c < kRecountChunks; ++c) {
+            own_a |= __popc(above & (15u << (4 * c))) << (8 * c);
+            own_i |= __popc(inside & (15u << (4 * c))) << (8 * c);
+        }
+        const uint32_t inc_a = warp_inclusive_scan(own_a, lane), inc_i = warp_inclusive_scan(own_i, lane);
+        if (lane == 31) {
+#pragma unroll
+            for (int c = 0; c < kRecountChunks; ++c)
+                sm.chunk_tot[c * kWarps + warp] = ((inc_a >> (8 * c)) & 0xffu) | (((inc_i >> (8 * c)) & 0xffu) << 16);
+        }
+        __syncthreads();
+        const uint2 t = *reinterpret_cast<const uint2*>(&sm.chunk_tot[2 * lane]);      // 64 (chunk, warp) totals
+        const uint32_t incl = warp_inclusive_scan(t.x + t.y, lane);
+        const uint32_t first = incl - t.x - t.y + (warp & 1 ? t.x : 0u);
+#pragma unroll
+        for (int c = 0; c < kRecountChunks; ++c) {
+            const uint32_t before = __shfl_sync(0xffffffffu, first, (c * kWarps + warp) >> 1);
+            uint32_t a = ahead.x + (before & 0xffffu) + ((inc_a - own_a) >> (8 * c) & 0xffu);
+            uint32_t q = ahead.y + (before >> 16) + ((inc_i - own_i) >> (8 * c) & 0xffu);
+            const int j = j0 + (c * kThreads + tid) * 4 + off;
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const bool is_a = above >> (4 * c + e) & 1u, is_i = inside >> (4 * c + e) & 1u;
+                if (is_a || (is_i && q < need)) out[a + min(q, need)] = j + e;
+                a += is_a ? 1u : 0u;
+                q += is_i ? 1u : 0u;
+            }
+        }
+        const uint32_t all = __shfl_sync(0xffffffffu, incl, 31);
+        ahead = make_uint2(ahead.x + (all & 0xffffu), ahead.y + (all >> 16));
+        __syncthreads();
+    }
+}
+
+// All CTAs of the row call it; pivot_key: the lower edge, to 22 bits, of the interval the sample pointed at.  True, with
+// nothing written, where the keys above the interval are enough and the list can hold them (RELIST).  Out of line: inlined, the
+// kernel spills and the rows that never come here take 3 to 6 % longer.
+template <int GROUP, bool RELIST, bool CLUSTER>
+__device__ __noinline__ bool recount_row(const float* __restrict__ row0, const float* __restrict__ row1, int begin, int end,
+                                         uint32_t parts, uint32_t part, uint32_t pivot_key, int topk,
+                                         int32_t* __restrict__ out, int32_t off, int32_t* __restrict__ count) {
+    extern __shared__ __align__(16) uint8_t topk_smem[];
+    PivotShared& sm = *reinterpret_cast<PivotShared*>(topk_smem);
+    uint2 ahead;
+    count_part<GROUP>(sm, 0, row0, row1, begin, end, key_score(pivot_key), key_score(pivot_key + 1024u));
+    const uint4 all = row_counts<CLUSTER>(sm, 0, parts, part, ahead);
+    uint32_t n_sel = (uint32_t)topk, need = n_sel - all.x, key = all.z;
+    const bool inside = all.x < n_sel && all.x + all.y >= n_sel, list = RELIST && all.x >= n_sel && all.x <= (uint32_t)kList;
+    if (list) n_sel = 0u;
+    else if (!inside || all.z != all.w) {
+        // digits of 11, 11 and 10 bits of the distance from the smallest usable key, or the last one alone; the histograms
+        // take turns, so that no CTA clears one that a peer may still read
+        uint32_t base = inside ? pivot_key : kMinKey, span = inside ? 1023u : 0xff000000u;
+        uint32_t k = inside ? need : n_sel;
+#pragma unroll 1
+        for (int sh = inside ? 0 : 21, slot = 0; sh >= 0; slot ^= 1) {
+            const uint32_t total = count_bins<GROUP, CLUSTER>(sm, slot, row0, row1, begin, end, parts, base, span, sh, k);
+            if (total < k) n_sel = k = total;      // fewer candidates than topk (known after the first digit)
+            if (total == 0u) break;
+            base += sm.sel_bin << sh;
+            k -= sm.sel_above;
+            span = (1u << sh) - 1u;
+            sh = sh == 21 ? 10 : (sh == 10 ? 0 : -1);
+            __syncthreads();                       // sel_* have been read
+        }
+        key = base;
+        need = k;
+        ahead = make_uint2(0u, 0u);
+        if (CLUSTER) {
+            count_part<GROUP>(sm, 1, row0, row1, begin, end, key_score(key), key_score(key + 1u));
+            row_counts<CLUSTER>(sm, 1, parts, part, ahead);
+        }
+    }
+    if (n_sel > 0u) emit_part<GROUP>(sm, row0, row1, begin, end, key_score(key), key_score(key + 1u), need, ahead, out, off);
+    if (part == 0u && !list) {
+        for (uint32_t pos = n_sel + threadIdx.x; pos < (uint32_t)topk; pos += kThreads) out[pos] = -1;
+        if (count != nullptr && threadIdx.x == 0) *count = (int32_t)n_sel;
+    }
+    if (CLUSTER) cluster_barrier();                // nobody leaves, or starts on another row, while a peer reads its counts
+    else __syncthreads();
+    return list;
 }
 
 template <int GROUP, bool MULTI, bool CLUSTER>
@@ -741,17 +891,21 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 
         // ---- 1. the pivot
         float s[kKpt];                                // MULTI: the samples first, then a sweep at a time
-        if (!MULTI) load_scores<GROUP>(row0, row1, begin, end, s);
+        if (!MULTI) load_scores<GROUP, kChunks>(row0, row1, begin, end, s);
         uint32_t pivot_key = kMinKey;
+        bool listed = true;                           // the list is expected to hold what reaches the pivot
         if (len > kShortRow) {                        // the same for all CTAs of the cluster
 #pragma unroll
             for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(&sm.hist[i * kBins + 4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
             constexpr int kSamples = MULTI ? 4 * kMaxSweeps : 4;
             uint32_t smp[kSamples];
-            if (MULTI) {                              // a chunk of four per thread and sweep, another one for each warp
+            if (MULTI) {                              // four adjacent keys per thread and sweep, of another chunk for each warp
 #pragma unroll
                 for (int sw = 0; sw < kMaxSweeps; ++sw) {
-                    const int j = begin + sw * kSweep + (((warp + sw) & (kChunks - 1)) * kThreads + tid) * 4;
+                    const int j0 = begin + sw * kSweep;
+                    int in_sweep = ((warp + sw) & (kChunks - 1)) * kThreads + tid;
+                    if (j0 + kSweep > end) in_sweep = 8 * tid + ((5 * tid) & 7);      // a sweep cut short: its chunks would not
+                    const int j = j0 + 4 * in_sweep;                                  // all be sampled by as many warps
                     const float4 v = load_scores4<GROUP>(row0, row1, j, end);
                     s[4 * sw] = v.x; s[4 * sw + 1] = v.y; s[4 * sw + 2] = v.z; s[4 * sw + 3] = v.w;
                 }
@@ -779,68 +933,68 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
                     const uint32_t bin = (smp[i] - first) >> lo;
                     if (smp[i] >= kMinKey && bin < (uint32_t)kBins) atomicAdd(&hist[bin], 1u);
                 }
-                uint4 h;
-                if (CLUSTER) {
-                    cluster_barrier();
-                    h = make_uint4(0u, 0u, 0u, 0u);
-                    for (uint32_t c = 0; c < parts; ++c) {
-                        const uint4 o = peer_load4(peer_address(&hist[4 * tid], c));
-                        h.x += o.x; h.y += o.y; h.z += o.z; h.w += o.w;
-                    }
-                } else {
-                    __syncthreads();
-                    h = *reinterpret_cast<const uint4*>(&hist[4 * tid]);
-                }
-                if (locate(sm, h, k) < k) {               // fewer usable samples than that: list every usable key
+                if (locate(sm, row_bins<CLUSTER>(hist, parts), k) < k) {               // fewer usable samples than that: list every usable key
                     found = false;                        // (decided in the first pass, by all CTAs of the cluster alike)
                     break;
                 }
                 prefix = pass == 0 ? sm.sel_bin : (prefix << 11) | sm.sel_bin;
                 k -= sm.sel_above;
             }
-            if (found) pivot_key = max(prefix << 10, kMinKey);
-        }
-        const float pivot = key_score(pivot_key);
-
-        // ---- 2. the list
-        uint32_t n = 0;
-        bool fits = true;
-#pragma unroll 1
-        for (int sw = 0; sw < nsweeps && fits; ++sw) {
-            if (MULTI) load_scores<GROUP>(row0, row1, begin + sw * kSweep, end, s);
-            fits = list_sweep(sm, s, pivot, begin + sw * kSweep, end, n);
-        }
-        uint32_t key_max = sm.key_max;
-        if (CLUSTER) {
-            if (tid == 0) sm.list_n = fits ? n : (uint32_t)kList + 1u;
-            cluster_barrier();
-            if (part == 0) {
-                for (uint32_t c = 1; c < parts; ++c) {
-                    const uint32_t m = peer_load(peer_address(&sm.list_n, c));
-                    fits = fits && n + m <= (uint32_t)kList;
-                    if (!fits) break;
-                    const uint32_t src = peer_address(sm.list, c);
-                    for (uint32_t i = tid; i < m; i += kThreads) sm.list[n + i] = peer_load2(src + 8 * i);
-                    n += m;
-                    key_max = max(key_max, peer_load(peer_address(&sm.key_max, c)));
-                }
+            if (found) {
+                pivot_key = max(prefix << 10, kMinKey);
+                listed = 8u * (sample_rank - k + sm.sel_count) <= (uint32_t)kList;     // samples above the interval and inside it
             }
-            cluster_barrier();
-        } else {
-            __syncthreads();
         }
-        if (tid == 0) sm.key_max = 0u;               // everybody has read it; a barrier follows before it is raised again
-        if (CLUSTER && part != 0) {
-            __syncthreads();
-            continue;
-        }
-
-        // ---- 3. the selection
         int32_t* out = indices + (long long)r * index_stride;
         const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
         int32_t* count = topk_length != nullptr ? topk_length + r : nullptr;
-        if (fits && (n >= (uint32_t)topk || pivot_key == kMinKey)) select_from_list(sm, n, pivot_key, key_max, topk, out, off, count);
-        else misled_row<GROUP>(sm, row0, row1, len, topk, out, off, count);
+
+        // ---- 2. the list, and 3. the selection.  All CTAs of the cluster decide alike.
+#pragma unroll 1
+        while (true) {
+            uint32_t n = 0, key_max = 0u;
+            if (listed) {
+                const float pivot = key_score(pivot_key);
+                bool fits = true;
+#pragma unroll 1
+                for (int sw = 0; sw < nsweeps && fits; ++sw) {
+                    if (MULTI) load_scores<GROUP, kChunks>(row0, row1, begin + sw * kSweep, end, s);
+                    fits = list_sweep(sm, s, pivot, begin + sw * kSweep, end, n);
+                }
+                key_max = sm.key_max;
+                if (CLUSTER) {
+                    if (tid == 0) sm.list_n = fits ? n : (uint32_t)kList + 1u;
+                    cluster_barrier();
+                    const uint32_t entries = lane < (int)parts ? peer_load(peer_address(&sm.list_n, lane)) : 0u;
+                    const uint32_t upto = warp_inclusive_scan(entries, lane);
+                    n = __shfl_sync(0xffffffffu, upto, 31);
+                    fits = n <= (uint32_t)kList;
+                    if (part == 0 && fits) {          // the first CTA gathers the others' lists behind its own
+                        key_max = __reduce_max_sync(0xffffffffu, lane < (int)parts ? peer_load(peer_address(&sm.key_max, lane)) : 0u);
+                        for (uint32_t c = 1; c < parts; ++c) {
+                            const uint32_t m = __shfl_sync(0xffffffffu, entries, c), at = __shfl_sync(0xffffffffu, upto, c) - m;
+                            const uint32_t src = peer_address(sm.list, c);
+                            for (uint32_t i = tid; i < m; i += kThreads) sm.list[at + i] = peer_load2(src + 8 * i);
+                        }
+                    }
+                    cluster_barrier();
+                } else {
+                    __syncthreads();
+                }
+                if (tid == 0) sm.key_max = 0u;        // everybody has read it; a barrier follows before it is raised again
+                listed = fits && (n >= (uint32_t)topk || pivot_key == kMinKey);
+            }
+            if (listed) {
+                if (part == 0) select_from_list(sm, n, pivot_key, key_max, topk, out, off, count);
+                else __syncthreads();
+                break;
+            }
+            // (a row that is held in registers is not listed twice: it would have to be kept there across the call)
+            if (!recount_row<GROUP, MULTI, CLUSTER>(row0, row1, begin, end, parts, part, pivot_key, topk, out, off, count)) break;
+            if (!MULTI) break;
+            pivot_key += 1024u;
+            listed = true;
+        }
     }
 }
 

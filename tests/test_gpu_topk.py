@@ -125,6 +125,50 @@ def test_samples_that_mislead(rows, s_kv):
     _check(s, 1500)
 
 
+def _crowded_rows(s_kv, topk, rng):
+    """Rows that the list of a pivot cannot hold or that fall short of it, one per way of finding their threshold."""
+    ulps = lambda base, n: (np.float32(base).view(np.uint32) + n.astype(np.uint32)).view(np.float32)
+    normal = lambda: rng.standard_normal(s_kv, dtype=np.float32)
+    rows = [np.full(s_kv, 1.5, np.float32), np.full(s_kv, np.finfo(np.float32).min, np.float32), np.full(s_kv, np.inf, np.float32)]
+    r = np.maximum(normal() - np.float32(2.2), 0)                  # a few positive, the rest zeros of either sign
+    rows.append(np.where(rng.random(s_kv) < 0.5, r, np.where(r == 0, np.float32(-0.0), r)))
+    rows.append(ulps(1.5, rng.integers(0, 900, s_kv)))             # one interval of 1024 keys, many values
+    rows.append(ulps(-1.5, rng.integers(0, 5000, s_kv)))           # several intervals
+    rows.append(np.where(rng.random(s_kv) < 0.4, np.float32(np.inf), normal()))
+    for above in (0, 1, topk - 1, topk):                           # so many above the tied value
+        r = np.full(s_kv, -3.0, np.float32)
+        r[rng.choice(s_kv, above, replace=False)] = 2.0
+        rows.append(r)
+    r = np.full(s_kv, 0.25, np.float32)
+    r[rng.random(s_kv) < 0.6] = np.nan
+    rows.append(r)
+    r = np.full(s_kv, -np.inf, np.float32)                         # ties in the last keys of the row alone
+    r[-(s_kv // 3):] = 7.0
+    rows.append(r)
+    j = np.arange(s_kv)
+    warp, chunk = j % 2048 // 128, j // 2048                       # usable keys where a sample looks and nowhere else
+    rows.append(np.where((warp < 4) & (chunk == warp % 8), normal(), np.float32(-np.inf)))
+    rows.append(np.where(j % 1024 < 200, normal() + 9, normal() - 9))
+    return np.stack(rows).astype(np.float32)
+
+
+@pytest.mark.parametrize("topk", [1500, 4096])
+@pytest.mark.parametrize("s_kv,pair,rows", [(33000, False, 0), (33000, False, 160), (49156, True, 0), (70004, True, 160), (280004, False, 0)])
+def test_crowded_rows_are_recounted(s_kv, pair, rows, topk):
+    """A row divided among the CTAs of a cluster (rows == 0: only the crowded ones) and a CTA for each (160)."""
+    rng = np.random.default_rng(s_kv + topk)
+    s = _crowded_rows(s_kv, topk, rng)
+    s = np.concatenate([s, rng.standard_normal((max(rows - len(s), 0), s_kv), dtype=np.float32)])
+    if pair:                                                       # the other token's scores: below, equal or not usable
+        other = np.where(rng.random(s.shape) < 0.3, np.float32(np.nan), np.where(rng.random(s.shape) < 0.5, s, np.float32(-np.inf)))
+        s = np.stack([s, other], 1)
+        s[::2] = s[::2, ::-1]
+        s = np.ascontiguousarray(s.reshape(-1, s_kv))
+    n = len(s) // (2 if pair else 1)
+    _check(s, topk, pair=pair)
+    _check(s, topk, pair=pair, lengths=rng.integers(s_kv // 2, s_kv + 1, size=n).astype(np.int32), row_offset=np.arange(n) * 11)
+
+
 def test_broadcast_and_single_rows():
     from mxdsa_b200.indexer import select_topk_indices
     x = torch.randn(1, 20480, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
