@@ -1016,14 +1016,27 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     // By pivot where a row does not fit the registers of a CTA (16 384 keys) and the list fits with its margin.  Shorter
     // rows are read and counted once by the other kernel, which is the faster one there for the lists in use: 2048 rows of
     // 16 384 keys, topk 2048 81 us against 84 by pivot (pairs 101 against 120); 20 rows of 16 384 keys 11 against 19.
-    // Few rows are divided among CTAs as long as these find SMs: four of them, eight where each still has 16 384 keys
-    // (20 rows of 32 768 keys: 29 us by eights, 20 rows of 20 480 keys 19 us by fours).  The steps between the CTAs of a
-    // row cost more than a second sweep (one row of 32 768 keys, topk 2048: 20.5 us counted, 24.5 divided), less than the
-    // further ones (65 536 keys: 32.8 against 22.6), hence the two lines.
+    // Few rows are divided among CTAs.  A division in two, four or eight is taken while every CTA of the call finds an SM of
+    // its own; clusters of four and eight leave some SMs over (33 rows by four, 15 by eight are resident at once, one more
+    // makes a second wave: 34 rows of 36 864 keys 15.3 -> 17.6 us).  With two CTAs on an SM a division gains only where the
+    // parts stay long: 148 rows by two, topk 2048, of 65 536 keys 24.8 us against 23.7 undivided, of 131 072 35.7 against
+    // 38.7; 16 rows by eight of 262 144 31.0 against 28.3 by four, of 524 288 40.6 against 41.6.  There, too, what does not
+    // fit at once must not be started: 74 rows by four of 49 152 keys 31.2 us, by two 20.2, counted 23.6.  A row is divided in
+    // any case where a CTA could not hold the samples of its part.
+    // The steps between the CTAs of a row cost more than a second sweep (one row of 32 768 keys, topk 2048, events around the
+    // call: 20.5 us counted, 24.5 divided), less than the further ones (65 536 keys: 32.8 against 22.6), hence the two lines.
     int parts = 1;
-    while (parts < 8 && (long long)p->rows * parts * 2 <= sms * 2 && p->s_kv / (parts * 2) >= (parts < 4 ? kShortRow : kSweep)) parts *= 2;
+    while (parts < 8) {
+        const int next = 2 * parts, over = next == 8 ? 28 : (next == 4 ? 16 : 0);      // SMs left over
+        const long long ctas = (long long)p->rows * next;
+        const bool own_sm = ctas <= sms - over && p->s_kv / next >= (next < 8 ? kShortRow : kSweep);
+        const bool shared_sm = ctas <= 2 * sms - over && (long long)p->s_kv * p->group > (next < 8 ? 4 : 31) * kSweep;
+        const bool too_long = ctas <= 2 * sms && p->s_kv > parts * kMaxSweeps * kSweep;
+        if (!own_sm && !shared_sm && !too_long) break;
+        parts = next;
+    }
     const int each = (int)((((long long)p->s_kv + parts - 1) / parts + 3) & ~3LL);      // the longest part of a row
-    const bool pivot = p->topk <= kStage && p->s_kv > (parts > 1 ? 2 : 1) * kSweep && each <= kMaxSweeps * kSweep;
+    const bool pivot = p->topk <= kStage && p->s_kv > (p->rows <= sms ? 2 : 1) * kSweep && each <= kMaxSweeps * kSweep;
     cudaError_t e = cudaSuccess;
     if (pivot) {
         const bool multi = each > kSweep;

@@ -125,6 +125,15 @@ def test_samples_that_mislead(rows, s_kv):
     _check(s, 1500)
 
 
+@pytest.mark.parametrize("rows,s_kv,pair", [(15, 131072, True), (16, 131072, False), (33, 65540, False), (34, 65540, False), (70, 65540, True),
+                                            (71, 65540, True), (74, 40004, False), (75, 40004, False), (3, 1048576, False)])
+def test_rows_on_both_sides_of_a_division(rows, s_kv, pair):
+    """Divided by eight, four, two or not: the row counts up to which the CTAs of a call are resident at once."""
+    rng = np.random.default_rng(rows)
+    s = rng.standard_normal((rows * (2 if pair else 1), s_kv), dtype=np.float32)
+    _check(s, 700, pair=pair, lengths=rng.integers(s_kv // 2, s_kv + 1, size=rows).astype(np.int32))
+
+
 def _crowded_rows(s_kv, topk, rng):
     """Rows that the list of a pivot cannot hold or that fall short of it, one per way of finding their threshold."""
     ulps = lambda base, n: (np.float32(base).view(np.uint32) + n.astype(np.uint32)).view(np.float32)
