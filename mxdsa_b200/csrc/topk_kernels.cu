@@ -117,8 +117,7 @@ __device__ __forceinline__ uint32_t warp_inclusive_scan(uint32_t v, int lane) {
 // After a histogram is complete: the bin that holds the k-th largest entry (k counted from the top,
 // 1 <= k <= total), the mass above that bin and the bin's own count.  Returns the histogram total.
 // Ends with a barrier; the result is in sm.sel_*.
-template <typename Shared>
-__device__ __forceinline__ uint32_t find_bin(Shared& sm, uint32_t k_or_cap, bool cap_to_total, uint32_t& k_out, int nbins) {
+__device__ __forceinline__ uint32_t find_bin(TopkShared& sm, uint32_t k_or_cap, bool cap_to_total, uint32_t& k_out, int nbins) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint4 h = *reinterpret_cast<const uint4*>(&sm.hist[4 * tid]);
     if (cap_to_total && tid == 0) h = make_uint4(0u, 0u, 0u, 0u);   // pass 0: bins 0-3 collect the non-candidates
@@ -316,10 +315,13 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 //
 // For rows of more than 16 384 keys the kernel above sweeps the row four times and spends three shared-memory atomics
 // on every key.  Here
-//   1. every eighth key (four per thread) is a sample; two histogram passes over the samples give a pivot: the lower
-//      edge, to 22 bits, of the rank'th largest, rank = topk/8 + 5 sqrt(topk/8) + 8, so that about 8 rank keys reach it
-//      (1.24 topk of them at topk 4096, 1.34 at 2048, 3.75 at 64) and fewer than topk do with a probability of less than
-//      1e-6 for samples that are independent;
+//   1. every eighth key is a sample; two histogram passes over the samples give a pivot: the lower edge, to 22 bits, of the
+//      rank'th largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that about 8 rank keys reach it (1.46 topk of them at
+//      topk 4096, 1.66 at 2048, 5.5 at 64).  Independent scores would do with half the margin; but neighbouring keys have
+//      similar scores in earnest, a sample of 16 adjacent keys then tells little more than one of them, and a row that
+//      falls short costs a second time.  (With 128 adjacent keys per sample and the smaller margin, 64 rows of 65 536
+//      keys, topk 2048, equal in runs of 128, took 59.9 us, by counting 29.4, now 20.5; in runs of 64 60.6, 29.3, 21.1;
+//      independent ones 21.7, 29.3, 21.0.)
 //   2. one sweep compares every score with the pivot (as floats: NaN, -inf and keys past the length fail by
 //      themselves) and lists key and position of those that reach it, in ascending position, in shared memory;
 //   3. the topk-th largest of the list is found by histogram passes over the list alone, whose digits start at the
@@ -899,13 +901,12 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
             for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(&sm.hist[i * kBins + 4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
             constexpr int kSamples = MULTI ? 4 * kMaxSweeps : 4;
             uint32_t smp[kSamples];
-            if (MULTI) {                              // four adjacent keys per thread and sweep, of another chunk for each warp
+            if (MULTI) {
+                // Four threads take 16 adjacent keys (64 bytes) out of 128, another eighth in each 128 and sweep: a row is looked
+                // at evenly wherever it ends, where good scores come with a period, and where they are neighbours.
 #pragma unroll
                 for (int sw = 0; sw < kMaxSweeps; ++sw) {
-                    const int j0 = begin + sw * kSweep;
-                    int in_sweep = ((warp + sw) & (kChunks - 1)) * kThreads + tid;
-                    if (j0 + kSweep > end) in_sweep = 8 * tid + ((5 * tid) & 7);      // a sweep cut short: its chunks would not
-                    const int j = j0 + 4 * in_sweep;                                  // all be sampled by as many warps
+                    const int j = begin + sw * kSweep + (tid >> 2) * 128 + ((5 * (tid >> 2) + 3 * warp + sw) & 7) * 16 + 4 * (tid & 3);
                     const float4 v = load_scores4<GROUP>(row0, row1, j, end);
                     s[4 * sw] = v.x; s[4 * sw + 1] = v.y; s[4 * sw + 2] = v.z; s[4 * sw + 3] = v.w;
                 }
@@ -1041,7 +1042,7 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     if (pivot) {
         const bool multi = each > kSweep;
         const float mean = p->topk * 0.125f;
-        const uint32_t rank = (uint32_t)(mean + 5.0f * sqrtf(mean) + 8.0f);
+        const uint32_t rank = (uint32_t)(mean + 10.0f * sqrtf(mean) + 8.0f);
         auto kern = p->group == 2 ? (parts == 1 ? mxdsa_topk_pivot_kernel<2, true, false>
                                      : multi ? mxdsa_topk_pivot_kernel<2, true, true> : mxdsa_topk_pivot_kernel<2, false, true>)
                                   : (parts == 1 ? mxdsa_topk_pivot_kernel<1, true, false>

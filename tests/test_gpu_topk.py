@@ -178,6 +178,17 @@ def test_crowded_rows_are_recounted(s_kv, pair, rows, topk):
     _check(s, topk, pair=pair, lengths=rng.integers(s_kv // 2, s_kv + 1, size=n).astype(np.int32), row_offset=np.arange(n) * 11)
 
 
+@pytest.mark.parametrize("rows,s_kv,run", [(3, 50000, 64), (160, 36864, 128), (160, 20484, 16), (2, 140004, 300)])
+def test_neighbouring_keys_with_similar_scores(rows, s_kv, run):
+    rng = np.random.default_rng(rows + run)
+    s = np.repeat(rng.standard_normal((rows, s_kv // run + 1), dtype=np.float32), run, axis=1)[:, :s_kv]
+    s = s + 0.1 * rng.standard_normal((rows, s_kv), dtype=np.float32)
+    s[0] = np.arange(s_kv) * 1e-3                                   # the best are the last
+    s[1] = 3 * np.sin(np.arange(s_kv) * (6.283 / 700)) + 0.1 * s[1]
+    for topk in (64, 2048):
+        _check(np.ascontiguousarray(s), topk, lengths=rng.integers(s_kv // 2, s_kv + 1, size=rows).astype(np.int32))
+
+
 def test_broadcast_and_single_rows():
     from mxdsa_b200.indexer import select_topk_indices
     x = torch.randn(1, 20480, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3))
