@@ -387,13 +387,6 @@ __device__ __forceinline__ const uint8_t* key_resolve(const AttnParams& p, const
         return pg + in_page * kDim;
     }
 }
-template <bool DECODE>
-__device__ __forceinline__ const uint8_t* key_lookup(const AttnParams& p, const WorkItem& w, int blk, int j,
-                                                     bool& valid, const uint8_t*& slot) {
-    return key_resolve<DECODE>(p, w, blk, j, key_index<DECODE>(p, w, blk, j), valid, slot);
-}
-
-
 // Row coordinate of one key in the 2-D view {512 B, rows} of its KV store (-1 = no row: the copy engine fills
 // zeros), from the key's raw index.
 template <bool DECODE>
@@ -449,10 +442,7 @@ __device__ __forceinline__ float2 f2_add(float2 a, float2 b) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
-// 8-byte flavour (through L1; the 16-byte one is the only size that may bypass it)
-__device__ __forceinline__ void cp_async8(uint32_t dst, const void* src, uint32_t bytes) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
-}
+// 4-byte flavour (through L1; the 16-byte one is the only size that may bypass it)
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
 }
@@ -570,7 +560,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     // What bounds a small call is this start, not the tiles: with one thread initialising sixty barriers, three
     // cluster barriers in a row, the schedule and index loads behind them and parts without work going through all of
     // it, the first row was asked for 8 000 cycles after the start; now 4 500.  With the launch overlap: 256 tokens at
-    // topk 128 18.4 -> 14.4 us per call, 37 requests of 2 tokens 25.3 -> 21.7 us, one request of one token 19.8 -> 15.7.
+    // topk 128 18.4 -> 14.2 us per call, 37 requests of 2 tokens 25.3 -> 21.7 us, one request of one token 19.8 -> 15.7, each
+    // among calls of its own kind; a single pass on new inputs gains factors of 1.06 and 1.07.
     if constexpr (DECODE) {
         grid_dependency_wait();
         const int4 rec = WorkIter<DECODE>::record(p, 0);   // a volatile load: it stays behind the wait
@@ -719,7 +710,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             // 0-63 and chunks 2, 3 keys 64-127, so one descriptor serves the pair.  Against gathering all 128 keys into
             // a ring of their own this halves the requests and a quarter of the L2 reads disappear (64 -> 48 KB per
             // tile and CTA), and the same 128 KB of shared memory hold four tiles in flight instead of two and two:
-            // 65 536 tokens at topk 4096 21.0 -> 20.2 ms, decode of 128 requests at 4224 keys 374 -> 359 us.
+            // 65 536 tokens at topk 4096 21.9 -> 21.0 ms, both trees timed in turn; decode of 128 requests at 4224 keys 386 ->
+            // 370 us, within the spread of either's runs.
             // Lanes 0-7 of every warp request four keys x 128 bytes each (measured: the copy engine takes requests
             // fastest from a few lanes of several warps).  Rows that do not exist (index -1, position beyond the list,
             // row outside the store) get a coordinate outside the tensor map, which the copy engine fills with zeros.
@@ -995,11 +987,11 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     } else if (warp < 12 + 4 * G) {
         if constexpr (kRebalanceRegs) setmaxnreg_inc<kRegsSoftmax>();
         // ===================== softmax + epilogue (warps 12 ..) =====================
-        // Two groups of four warps take alternate tiles (group = tile parity = P buffer), so one
-        // group's exp / quantise / store phase overlaps the other group's load / max phase.  Inside a
+        // G groups of four warps take tiles in turn (tile g: group g % G, P buffer g & 1), so one
+        // group's exp / quantise / store phase overlaps another group's load / max phase.  Inside a
         // group a thread owns one row and one 64-key half of the tile (two UE8M0 scale groups of S).
         // The only serial link between consecutive tiles is the running maximum: after deciding m_t a
-        // group publishes it (sm.m_pub) and the other group picks it up before deciding m_{t+1}.
+        // group publishes it (sm.m_pub) and the next group picks it up before deciding m_{t+1}.
         const int grp = (warp - 12) >> 2;
         const int prev_grp = (grp + kGroups - 1) % kGroups;
         const int q4 = warp & 3;                 // lane quadrant of tensor memory
@@ -1070,7 +1062,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 xm[L] = own_max;
                 named_bar_sync(1 + grp, 128);
                 const float peer_max = xm[L ^ 64];
-                // the running maximum handed over by the other group (value ignored on a pair's first
+                // the running maximum handed over by the group before (value ignored on a pair's first
                 // tile, but every phase of that barrier is observed)
                 if (gt > 0) MXDSA_WAIT_POLL(sm.bar_m_ready[prev_grp], ((gt - 1) / kGroups) & 1, 58);
                 const float m_prev = t == 0 ? -1e30f : sm.m_pub[prev_grp][row];

@@ -285,7 +285,8 @@ __global__ void __launch_bounds__(32) mxdsa_sched_whole_kernel(int b, int topk, 
 // some part while continuing into the next one).  WPH warps share a head, 512 / WPH dims each; a lane keeps eight
 // 16-byte loads in flight, the first of them issued before the weights are worked out.
 // Bound: latency while few requests are divided -- one request of one token over 34 splits is 64 heads x 34 rows, which
-// a warp per head with one row in flight took 14.5 us to walk, four warps per head with eight rows in flight 4.9 us --
+// a warp per head with one row in flight took 14.5 us to walk, four warps per head with eight rows in flight 3.9 us (taken
+// while the schedule was still read ahead of the wait for the attention grid) --
 // and L2 bandwidth when every part ends inside a request: then a warp per head (WPH = 1) has all the parallelism the
 // SMs hold, and more warps only add latency chains (128 requests of 6 tokens on 24 parts: 9.9 us, WPH = 4 22 us).
 // ------------------------------------------------------------------------------------------
