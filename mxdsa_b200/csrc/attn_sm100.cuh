@@ -323,17 +323,24 @@ template <bool DECODE, int NT> struct TileCursor {
 
 // Key at position `j` (0..63) of 64-key block `blk` of a work item, in two steps so that callers can
 // keep the index load and the loads that depend on it in flight for different tiles.
-// Step 1: the raw index (-1 when the position does not exist).
+// Step 1: the raw index (-1 when the position does not exist, or nothing `exists`).  The load is predicated by hand: as a
+// conditional expression it became a load, a wait for it and a selection, which held the copying warps for its latency.
+__device__ __forceinline__ int load_index_if(bool exists, const int* at) {
+    int v = -1;
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, 0;\n@p ld.global.nc.s32 %0, [%2];\n}"
+                 : "+r"(v) : "r"((uint32_t)exists), "l"(at));
+    return v;
+}
 template <bool DECODE>
-__device__ __forceinline__ int key_index(const AttnParams& p, const WorkItem& w, int blk, int j) {
-    if (blk >= w.blk_end) return -1;
+__device__ __forceinline__ int key_index(const AttnParams& p, const WorkItem& w, bool exists, int blk, int j) {
+    exists = exists && blk < w.blk_end;
     if constexpr (!DECODE) {
         const int pos = blk * 64 + j;
-        return pos < p.topk ? __ldg(w.row + pos) : -1;
+        return load_index_if(exists && pos < p.topk, w.row + pos);
     } else {
         const bool extra = blk >= w.n_main_blocks;
         const int pos = (extra ? blk - w.n_main_blocks : blk) * 64 + j;
-        return pos < (extra ? p.extra_topk : p.topk) ? __ldg((extra ? w.erow : w.row) + pos) : -1;
+        return load_index_if(exists && pos < (extra ? p.extra_topk : p.topk), (extra ? w.erow : w.row) + pos);
     }
 }
 // Ask for the index lines of the two 64-key blocks blk, blk + 1 into L2: lane 0..3 takes 128-byte line lane % 2 of
@@ -351,41 +358,41 @@ __device__ __forceinline__ void prefetch_index_lines(const AttnParams& p, const 
         if (pos < (extra ? p.extra_topk : p.topk)) prefetch_l2((extra ? w.erow : w.row) + pos);
     }
 }
-// Step 2: is the key attended, where are its 512 data bytes (nullptr = no row, the operand rows are
-// zero-filled) and its 16-byte scale slot.
+// Step 2: is the key attended, where is its 16-byte scale slot, and -- returned -- the coordinate of its data in the view
+// of the KV store as rows of 512 bytes (kNoRow = no row: the operand rows are zero-filled, the slot is null).
+static constexpr uint32_t kNoRow = 0xffffffffu;
 template <bool DECODE>
-__device__ __forceinline__ const uint8_t* key_resolve(const AttnParams& p, const WorkItem& w, int blk, int j, int idx,
-                                                      bool& valid, const uint8_t*& slot) {
+__device__ __forceinline__ uint32_t key_resolve(const AttnParams& p, const WorkItem& w, int blk, int j, int idx, bool& valid,
+                                                const uint8_t*& slot) {
     valid = false;
     slot = nullptr;
-    if (blk >= w.blk_end) return nullptr;
+    if (blk >= w.blk_end) return kNoRow;
     if constexpr (!DECODE) {
         const int pos = blk * 64 + j;
-        if (idx < 0 || idx >= p.s_kv) return nullptr;
+        if (idx < 0 || idx >= p.s_kv) return kNoRow;
         valid = pos < w.len;
         slot = p.kv_scales + (long long)idx * 16;
-        return p.kv + (long long)idx * kDim;
+        return (uint32_t)idx;
     } else {
         const bool extra = blk >= w.n_main_blocks;
         const int pos = (extra ? blk - w.n_main_blocks : blk) * 64 + j;
         // an index outside the pool (stale or corrupt) is treated like -1: not attended, nothing dereferenced
         // (one unsigned compare: a negative index is a huge unsigned one)
         valid = (unsigned)idx < (extra ? p.extra_pool_rows32 : p.pool_rows32) && pos < (extra ? w.elen : w.len);
-        if (!valid) return nullptr;
+        if (!valid) return kNoRow;
         const unsigned psz = extra ? p.extra_page_size : p.page_size;
         const int sh = extra ? p.extra_page_shift : p.page_shift;   // pages are powers of two as a rule: no division then
-        unsigned page, in_page;
-        if (__builtin_expect(sh >= 0, 1)) {
-            page = (unsigned)idx >> sh;
-            in_page = (unsigned)idx & (psz - 1);
-        } else {
-            page = (unsigned)idx / psz;
-            in_page = (unsigned)idx - page * psz;
-        }
-        const uint8_t* pg = (extra ? p.extra_kv : p.kv) + (long long)page * (extra ? p.extra_stride_block : p.stride_block);
-        slot = pg + psz * kDim + in_page * 16;
-        return pg + in_page * kDim;
+        const unsigned page = __builtin_expect(sh >= 0, 1) ? (unsigned)idx >> sh : (unsigned)idx / psz;
+        const unsigned in_page = (unsigned)idx - page * psz;
+        slot = (extra ? p.extra_kv : p.kv) + (long long)page * (extra ? p.extra_stride_block : p.stride_block) + psz * kDim + in_page * 16;
+        return (unsigned)idx + page * (extra ? p.extra_row_gap : p.row_gap);
     }
+}
+// Base of the store that the rows of 64-key block `blk` come from.
+template <bool DECODE>
+__device__ __forceinline__ const uint8_t* key_store(const AttnParams& p, const WorkItem& w, int blk) {
+    if constexpr (!DECODE) return p.kv;
+    else return (blk >= w.n_main_blocks && p.extra_topk > 0) ? p.extra_kv : p.kv;
 }
 // Row coordinate of one key in the 2-D view {512 B, rows} of its KV store (-1 = no row: the copy engine fills
 // zeros), from the key's raw index.
@@ -441,6 +448,9 @@ __device__ __forceinline__ float2 f2_add(float2 a, float2 b) {
 // 16-byte asynchronous copy global -> shared; `bytes` = 16 copies, 0 writes zeros.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, uint32_t bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 // 4-byte flavour (through L1; the 16-byte one is the only size that may bypass it)
 __device__ __forceinline__ void cp_async4(uint32_t dst, const void* src, uint32_t bytes) {
@@ -646,16 +656,20 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             const int key = lane < 16 ? 64 * (int)cta + 16 * pw + lane : 64 * (1 - (int)cta) + 16 * pw + (lane - 16);
             TileCursor<DECODE, NT> ck(p);
             uint32_t kt = 0;
-            int idx = ck.live ? key_index<DECODE>(p, ck.w, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64) : -1;
-            const uint32_t k_stage0 = smem_u32(sm.kv[0]) + (lane / 8) * 8192;
+            int idx = key_index<DECODE>(p, ck.w, ck.live, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64);
+            // row 16 pw of chunk lane/8, 16-byte column lane%8; bits 4-6 are free for the swizzle's exclusive or
+            const uint32_t k_dst0 = smem_u32(sm.kv[0]) + (lane / 8) * 8192 + 16 * pw * 128 + (lane & 7) * 16;
             // Where the key's row and scale slot are is worked out as soon as the tile's index is back, before the
             // wait for a free stage: the wait then covers what is left of the index load's latency.
-            const uint8_t* cur = nullptr;
+            uint32_t krow = kNoRow;
+            const uint8_t* src0 = p.kv;      // lane's column of row 0 of the store that this warp's rows come from
             const uint8_t* slot = nullptr;
             uint32_t vbits = 0;
             auto resolve_tile = [&]() {
                 bool valid;
-                cur = key_resolve<DECODE>(p, ck.w, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64, idx, valid, slot);
+                const int blk = ck.w.blk_begin + 2 * ck.t;
+                krow = key_resolve<DECODE>(p, ck.w, blk + key / 64, key % 64, idx, valid, slot);
+                src0 = key_store<DECODE>(p, ck.w, blk + (int)cta) + lane * 16;
                 vbits = __ballot_sync(0xffffffffu, valid);
             };
             if (ck.live) resolve_tile();
@@ -676,21 +690,27 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 }
                 // the next tile's indices: the loads run while this tile's rows are issued
                 ck.advance();
-                idx = ck.live ? key_index<DECODE>(p, ck.w, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64) : -1;
-                const uint32_t base = k_stage0 + s * 32768;
-#pragma unroll 4
-                for (int i = 0; i < 16; ++i) {
-                    const uint8_t* src = reinterpret_cast<const uint8_t*>(
-                        __shfl_sync(0xffffffffu, reinterpret_cast<unsigned long long>(cur), i));
-                    const int r = 16 * pw + i;
-                    cp_async16(base + r * 128 + (((lane & 7) ^ (r & 7)) << 4), src ? src + lane * 16 : p.kv, src ? 16u : 0u);
+                idx = key_index<DECODE>(p, ck.w, ck.live, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64);
+                // Four instructions a row: the coordinate by shuffle, one multiply-add to its address, one exclusive or
+                // for the swizzle, the copy.
+                const uint32_t dst = k_dst0 + s * 32768;
+                if ((__ballot_sync(0xffffffffu, krow != kNoRow) & 0xffffu) == 0xffffu) {
+#pragma unroll
+                    for (int i = 0; i < 16; ++i)
+                        cp_async16((dst ^ ((i & 7) << 4)) + i * 128, src0 + (unsigned long long)__shfl_sync(0xffffffffu, krow, i) * kDim);
+                } else {
+#pragma unroll 1
+                    for (int i = 0; i < 16; ++i) {
+                        const uint32_t r = __shfl_sync(0xffffffffu, krow, i);
+                        cp_async16((dst ^ ((i & 7) << 4)) + i * 128, r != kNoRow ? src0 + (unsigned long long)r * kDim : p.kv, r != kNoRow ? 16u : 0u);
+                    }
                 }
                 // the key's 8 scale bytes go straight into the row layout that tcgen05.cp wants: row (key/64)*32 +
                 // key%32 holds {bytes0-3[k], bytes0-3[k+32], bytes4-7[k], bytes4-7[k+32]} of keys k and k+32
                 {
-                    const uint32_t dst = smem_u32(&sm.k_sf[s][((key >> 6) * 32 + (key & 31)) * 4 + ((key >> 5) & 1)]);
-                    cp_async4(dst, slot ? slot : p.kv, slot ? 4u : 0u);
-                    cp_async4(dst + 8, slot ? slot + 4 : p.kv, slot ? 4u : 0u);
+                    const uint32_t sf = smem_u32(&sm.k_sf[s][((key >> 6) * 32 + (key & 31)) * 4 + ((key >> 5) & 1)]);
+                    cp_async4(sf, slot ? slot : p.kv, slot ? 4u : 0u);
+                    cp_async4(sf + 8, slot ? slot + 4 : p.kv, slot ? 4u : 0u);
                 }
                 cp_async_arrive(smem_u32(&sm.bar_k_landed[s]));
                 if (lane == 0) {   // validity of the warp's 32 keys: a plain store, released by a plain arrival
@@ -734,7 +754,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 map = key_map<DECODE>(p, maps, cv.w, blk);
             };
             bool live = cv.live;
-            if (live) locate(key_index<DECODE>(p, cv.w, cv.w.blk_begin + 2 * cv.t + other, jl));
+            if (live) locate(key_index<DECODE>(p, cv.w, true, cv.w.blk_begin + 2 * cv.t + other, jl));
             cluster_wait();
 #pragma unroll 1
             while (live) {
@@ -745,8 +765,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 for (int i = 0; i < 4; ++i) r[i] = __shfl_sync(0xffffffffu, row, 4 * ((lane >> 1) & 3) + i);
                 cv.advance();
                 live = cv.live;
-                int idx = -1;
-                if (live) idx = key_index<DECODE>(p, cv.w, cv.w.blk_begin + 2 * cv.t + other, jl);
+                const int idx = key_index<DECODE>(p, cv.w, live, cv.w.blk_begin + 2 * cv.t + other, jl);
                 // the half that is about to be overwritten has been read once the tile's QK is done
                 MXDSA_WAIT(sm.bar_qk_done[vt % kScStages], (vt / kScStages) & 1, 11);
                 if (lane == 0) mbar_expect_tx_cluster(v_full0 + s * 8, 16 * 256);
