@@ -13,8 +13,8 @@
 //   accumulators live in tensor memory: per CTA 128 lanes x (256 O + 2 x 64 P) columns; lane L
 //   holds row L%64, and column half L/64 (P: keys 64*(L/64).., O: dims 256*(L/64)..).
 //
-// Roles (warp-specialised, 28 warps per CTA; the launch gives every thread 72 registers, re-balanced with
-// setmaxnreg to 48 / 32 / 64 / 104 / 48 for the five kinds of warp below)
+// Roles (warp-specialised, 32 warps per CTA; the launch gives every thread 64 registers, re-balanced with
+// setmaxnreg to 48 / 32 / 48 / 72 / 96 for the five kinds of warp below)
 //   warps 0-3   K producers: read key indices one tile ahead and copy the selected rows of this CTA's 64 keys
 //               into the tile ring with 16-byte cp.async; one warp instruction moves one 512-byte row straight
 //               into the 128-byte-swizzled operand layout.  The same warps gather the 8 scale bytes of all 128
@@ -32,13 +32,23 @@
 //               L2 a pair ahead); per tile it waits for "K landed", fences and publishes "scale rows ready"
 //               to CTA 0 -- no global load sits between a landed K tile and its QK -- then derives the key
 //               token scales and validity words that the softmax reads.
-//   warps 12-23 softmax: three groups of four warps take tiles in turn (each thread one row and one 64-key
-//               half of its tile): P -> registers, running max with lazy rescale handed from group to group,
-//               exp2, token scale, per-32-key UE8M0 requantisation to E4M3 S (ring of three), O rescale.
+//   warps 12-27 softmax: two groups of eight warps take tiles in turn (each thread one row and 32 keys of its tile):
+//               P -> registers, running max with lazy rescale handed from group to group, exp2, token scale,
+//               UE8M0 requantisation of the thread's 32 keys to E4M3 S (ring of three).
 //               At the end of a pair the groups add up their row sums and hand 1/l to the epilogue warps.
-//   warps 24-27 epilogue: drain O (tensor memory -> bf16 `out` through small staging tiles and tiled TMA
-//               stores, or fp32 split partials) while the other warps are already working on the next pair;
-//               only that pair's first PV waits, and only until the last columns have been read.
+//   warps 28-31 epilogue: while a pair's tiles are worked on they watch the published maxima, rescale O where one has
+//               grown and tell the PV issuer; at the pair's end they drain O (tensor memory -> bf16 `out` through small
+//               staging tiles and tiled TMA stores, or fp32 split partials) while the other warps are already working
+//               on the next pair; only that pair's first PV waits, and only until the last columns have been read.
+//
+// What bounds a tile: latency.  A tile's way (K rows, QK, softmax, PV, its stage freed) is longer than four stages of the
+// ring at the tensor core's pace, and a warp gets to issue an instruction every 7 cycles or so (four to eight warps of a
+// scheduler are at work, 50 to 60 % of the issue slots taken).  Hence warps with little to do each: with three groups of
+// four warps, 64 keys a thread, and O rescaled by the softmax warps the softmax of a tile took 3 050 cycles from P to S
+// and a rescale 1 250 more; now 2 400 and none.  Per pass, that form / now, timed in turn: 256 tokens at topk 128 14.1 /
+// 12.9 us, decode of 64 requests at 640 keys 46.6 / 44.2, of 128 requests at 4224 keys 354 / 336, of 37 requests of two
+// tokens 22.7 / 21.6; prefill of 4 096 tokens at topk 2048 unchanged (672 / 680): there the chip is at its power limit
+// (990 W, 1 590 of 1 965 MHz), fewer cycles buy a lower clock.
 //
 // Numerical contract (identical to the reference kernels, reference file:line in brackets)
 //   * keys are consumed in numerical tiles of NT = 128 (prefill, topk >= 512) or 64 keys
@@ -97,11 +107,13 @@ static constexpr int kSBufs = MXDSA_S_BUFS;      // S (quantised probabilities) 
 #endif
 static constexpr int kScStages = MXDSA_SC_STAGES;      // scale/validity ring depth; also the depth of the
                                          // per-tile "QK done" / "PV done" barrier rings
-// registers per thread that a launch of 512 + 128 G threads gets (65536 / threads, rounded down to a multiple of 8)
-__host__ __device__ constexpr int launch_regs(int g) { return g == 2 ? 80 : 72; }
-static constexpr int kBaseThreads = 512;   // warps 0-11: K producers, V producers, control; then G x 4 softmax warps; then 4 epilogue warps
+static constexpr int kGroups = 2;          // softmax groups; tile g is handled by group g % kGroups
+static constexpr int kGroupWarps = 8;      // warps of a softmax group: a thread has one row and 32 keys of a tile
+static constexpr int G = kGroups * kGroupWarps / 4;   // softmax warps in fours: one for each lane quadrant of tensor memory
+static constexpr int kThreads = 32 * (12 + 4 * G + 4);   // warps 0-11: K producers, V producers, control; then softmax; then four epilogue warps
+static constexpr int kLaunchRegs = 64;     // registers per thread of the launch: 65536 / kThreads
 static constexpr uint32_t kBarTmem = 7;    // named barrier: tensor memory allocated (warp 10 -> warps 12-15)
-static constexpr int kMaxGroups = 3;     // softmax groups of four warps (template parameter G = 2 or 3); tile g is handled by group g % G
+static constexpr int kMRing = 6;         // ring of running maxima by tile, see the epilogue warps
 
 // tensor-memory columns
 static constexpr uint32_t kColO = 0;      // 256 columns
@@ -193,9 +205,10 @@ struct __align__(1024) SmemPlan {
     __align__(128) uint32_t s_sf[kSBufs][64 * 4];
     __align__(16) float tok_scale[kScStages][kTileKeys];
     __align__(16) uint32_t valid[kScStages][4];
-    float xmax[kMaxGroups][2][128];                   // [group][parity of the group's tile count][lane]: row max of the lane's 64 keys
-    float m_pub[kMaxGroups][64];                      // [group][row]: running max after the group's latest tile
-    float xl[kMaxGroups * 128], xr[kMaxGroups * 128];    // [group*128 + lane]: partial l and true max at the end of a pair
+    float xmax[kGroups][2][4][64];                 // [group][parity of the group's tile count][32-key quarter][row]: row max of the quarter
+    float m_pub[kMRing][64];                       // [tile % kMRing][row]: running max after the tile
+    float m_mid[kMRing][64];                       // 64-key tiles: after the tile's first half
+    float xl[kGroups][4][64], xr[kGroups][64];     // partial l by quarter and true max at the end of a pair
     uint64_t bar_q_landed;                         // local: Q bytes landed
     uint64_t bar_q_full;                           // CTA0: Q data + scale rows of both CTAs ready
     uint64_t bar_q_empty;                          // both: every QK of the pair finished (2 arrivals)
@@ -203,17 +216,18 @@ struct __align__(1024) SmemPlan {
     uint64_t bar_v_full[kStages];                  // CTA0: the exchanged halves of both CTAs landed (8 arrivals + 32 KB of gather4 bytes)
     uint64_t bar_qk_done[kScStages];               // both: QK of tile g finished (ring by g % 4)
     uint64_t bar_pv_done[kScStages];               // both: PV of tile g finished
-    uint64_t bar_pv_half[kSBufs];                       // both: first key half accumulated (64-key tiles)
+    uint64_t bar_pv_half[kScStages];              // both: first step of PV of tile g finished (128-key tiles: dim chunk 0; 64-key tiles: key half 0)
     uint64_t bar_sc_full[kScStages];               // CTA0: K scale rows of both CTAs written
     uint64_t bar_tok_full[kScStages];              // local: token scales + validity written
     uint64_t bar_tok_empty[kScStages];             // local: softmax has read the stage
     uint64_t bar_p_empty[2];                       // CTA0: P buffer copied to registers
-    uint64_t bar_s_full[kSBufs][2];                     // CTA0: [buffer][key half]
+    uint64_t bar_s_full[kSBufs];                        // CTA0: S tile and its scale rows written
     float oscale[2][64];                           // [pair parity][row]: 1 / (l + sink term), what the epilogue multiplies O by
     uint64_t bar_os_full[2];                       // local: oscale of the pair written (2 arrivals)
     uint64_t bar_os_empty[2];                      // local: the epilogue warps have read it (4 arrivals)
     uint64_t bar_o_empty;                          // CTA0: epilogue has drained O (4 warps of each CTA)
-    uint64_t bar_m_ready[kMaxGroups];                 // local: group g published the running max of its tile
+    uint64_t bar_o_ready[2][kScStages];            // CTA0: O is rescaled for step 0, 1 of PV; rings: step 0 by tiles after their pair's first, step 1 of 64-key tiles by all tiles
+    uint64_t bar_m_ready[kMRing];                  // local: the running max of tile g is published
     uint64_t bar_tmem_ready;                       // CTA0: tensor memory allocated and V scales written in both CTAs (4 warps each)
     uint32_t tmem_base;
     int abort_word;
@@ -467,19 +481,24 @@ template <int N> __device__ __forceinline__ void setmaxnreg_dec() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// multiply the 256 O columns of this thread's tensor-memory lane by f (out of line: one copy)
-__device__ __noinline__ void rescale_o(uint32_t lane_addr, float f) {
-    // 64 columns per round: half as many exposed load latencies
+// multiply `cols` columns of this thread's tensor-memory lane by f, 64 columns a round (16 a round, one batch loaded
+// while another is multiplied, takes 665 cycles alone against 379)
+__device__ __forceinline__ void rescale_o(uint32_t addr, int cols, float f) {
+    const float2 f2 = make_float2(f, f);
 #pragma unroll 1
-    for (int c = 0; c < 256; c += 64) {
+    for (int c = 0; c < cols; c += 64) {
         uint32_t v[64];
-        tmem_ld32(lane_addr + kColO + c, v);
-        tmem_ld32(lane_addr + kColO + c + 32, v + 32);
+        tmem_ld32(addr + c, v);
+        tmem_ld32(addr + c + 32, v + 32);
         tmem_wait_ld();
 #pragma unroll
-        for (int i = 0; i < 64; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * f);
-        tmem_st32(lane_addr + kColO + c, v);
-        tmem_st32(lane_addr + kColO + c + 32, v + 32);
+        for (int i = 0; i < 64; i += 2) {
+            const float2 r = f2_mul(make_float2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), f2);
+            v[i] = __float_as_uint(r.x);
+            v[i + 1] = __float_as_uint(r.y);
+        }
+        tmem_st32(addr + c, v);
+        tmem_st32(addr + c + 32, v + 32);
     }
     tmem_wait_st();
 }
@@ -548,8 +567,8 @@ template <typename Plan> __device__ __noinline__ void raise_fault(Plan& sm, int 
     if (atomicCAS(&sm.fault->flag, 0, 1) == 0) sm.fault->where = code;
 }
 
-template <bool DECODE, int NT, int G>
-__global__ void __launch_bounds__(kBaseThreads + 128 * G, 1)
+template <bool DECODE, int NT>
+__global__ void __launch_bounds__(kThreads, 1)
 mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ TensorMaps maps) {
     extern __shared__ uint8_t smem_raw[];
     // The plan starts at the first 1024-byte boundary.  The pointer is formed by adding an offset to
@@ -587,19 +606,20 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             mbar_init(smem_u32(&sm.bar_pv_done[lane]), 1);
             mbar_init(smem_u32(&sm.bar_sc_full[lane]), 2);
             mbar_init(smem_u32(&sm.bar_tok_full[lane]), 1);
-            mbar_init(smem_u32(&sm.bar_tok_empty[lane]), 4);
-        }
-        if (lane < kSBufs) {
-            mbar_init(smem_u32(&sm.bar_s_full[lane][0]), 8);
-            mbar_init(smem_u32(&sm.bar_s_full[lane][1]), 8);
+            mbar_init(smem_u32(&sm.bar_tok_empty[lane]), kGroupWarps);
+            mbar_init(smem_u32(&sm.bar_o_ready[0][lane]), 8);
+            mbar_init(smem_u32(&sm.bar_o_ready[1][lane]), 8);
             mbar_init(smem_u32(&sm.bar_pv_half[lane]), 1);
         }
+        if (lane < kSBufs) {
+            mbar_init(smem_u32(&sm.bar_s_full[lane]), 2 * kGroupWarps);
+        }
         if (lane < 2) {
-            mbar_init(smem_u32(&sm.bar_p_empty[lane]), 8);
+            mbar_init(smem_u32(&sm.bar_p_empty[lane]), 2 * kGroupWarps);
             mbar_init(smem_u32(&sm.bar_os_full[lane]), 2);
             mbar_init(smem_u32(&sm.bar_os_empty[lane]), 4);
         }
-        if (lane < kMaxGroups) mbar_init(smem_u32(&sm.bar_m_ready[lane]), 4);
+        if (lane < kMRing) mbar_init(smem_u32(&sm.bar_m_ready[lane]), 2);
         if (lane == 8) {
             mbar_init(smem_u32(&sm.bar_q_landed), 1);
             mbar_init(smem_u32(&sm.bar_q_full), 2);
@@ -628,23 +648,18 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     asm volatile("mov.u32 %0, 0;" : "=r"(tmem));
 
     // ------------------------------------------------------------------ roles
-    // Register budget.  The launch gives every thread kLaunchRegs (the most that 640 or 768 threads can have),
+    // Register budget.  The launch gives every thread kLaunchRegs (the most that 1024 threads can have),
     // and that allocation -- not the SM's whole file -- is the pool setmaxnreg draws from: an increase beyond
     // what the other warps have released would block for ever, hence the static_assert, and the host refuses
     // to launch unless the compiled kernel really has kLaunchRegs registers.  The copy and control warps hand
-    // most of theirs back so that the softmax warps (64 logits per thread in registers) work without spilling.
+    // most of theirs back so that the softmax warps (32 logits per thread in registers) work without spilling.
     // Each setmaxnreg is executed by the four warps of one aligned warp group with the same value.
-    constexpr int kGroups = G;
-    constexpr int kThreads = kBaseThreads + 128 * G;
-    constexpr int kLaunchRegs = launch_regs(G);
-    constexpr bool kRebalanceRegs = true;
-    constexpr int kRegsCopy = G == 2 ? 64 : 48, kRegsGather = G == 2 ? 40 : 32, kRegsCtl = 64, kRegsEpi = G == 2 ? 56 : 48;
-    constexpr int kRegsSoftmax = G == 2 ? 128 : 104;
-    static_assert(4 * 32 * (kRegsCopy + kRegsGather + kRegsCtl + kRegsEpi) + 4 * G * 32 * kRegsSoftmax <= kThreads * kLaunchRegs,
+    constexpr int kRegsCopy = 48, kRegsGather = 32, kRegsCtl = 48, kRegsEpi = 96, kRegsSoftmax = 72;
+    static_assert(4 * 32 * (kRegsCopy + kRegsGather + kRegsCtl + kRegsEpi) + kGroups * kGroupWarps * 32 * kRegsSoftmax <= kThreads * kLaunchRegs,
                   "register budget must fit in the launch allocation");
     if (warp < 8) {
         if (warp < 4) {
-            if constexpr (kRebalanceRegs) setmaxnreg_dec<kRegsCopy>();
+            setmaxnreg_dec<kRegsCopy>();
             // ===================== K producers (warps 0-3): 16-byte cp.async =====================
             // Warp pw copies rows 64*cta + 16*pw + i (i < 16) of every tile, whole 512-byte rows, one row per
             // instruction: lane L writes byte chunk L of the row -> chunk tile L/8, 16-byte column (L%8) ^ (row%8).
@@ -722,7 +737,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 if (ck.live) resolve_tile();
             }
         } else {
-            if constexpr (kRebalanceRegs) setmaxnreg_dec<kRegsGather>();
+            setmaxnreg_dec<kRegsGather>();
             // ===================== V producers (warps 4-7): TMA gather4 =====================
             // V of CTA c = bytes 256c .. 256c+255 of all 128 keys.  Its own 64 keys are in shared memory already: the
             // 128-byte chunks 2c, 2c+1 of the K tile.  Chunks 2(1-c), 2(1-c)+1 belong to the peer and are free once the
@@ -778,7 +793,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             }
         }
     } else if (warp < 12) {
-    if constexpr (kRebalanceRegs) setmaxnreg_dec<kRegsCtl>();
+    setmaxnreg_dec<kRegsCtl>();
     if (warp == 8 || warp == 9) {
         if (cta != 0) {
             cluster_wait();
@@ -793,7 +808,6 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             WorkIter<DECODE> it(p);
             WorkItem w;
             uint32_t gt = 0, gw = 0;
-            const uint32_t qk_done_peer = map_to_cta(smem_u32(&sm.bar_qk_done[0]), 1);
             const uint32_t q_empty_peer = map_to_cta(smem_u32(&sm.bar_q_empty), 1);
             const uint64_t a_base = smem_desc(desc_k128, smem_u32(sm.q));
             const uint32_t d_p = tmem + kColP + e * 64, sfa0 = tmem + kColQs + 4 * e, sfb0 = tmem + kColKs + 4 * e;
@@ -834,8 +848,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                                         mx_idesc(128, 128, false, kk & 3, (kk >> 1) & 3), sfa0 + 2 * ((kk >> 2) & 1),
                                         sfb0 + 2 * (kk >> 3), kk != 0);
                         }
-                        mma_commit<2>(smem_u32(&sm.bar_qk_done[sc]));
-                        mma_commit<2>(qk_done_peer + sc * 8);
+                        mma_commit_both(smem_u32(&sm.bar_qk_done[sc]));
                     }
                     __syncwarp();
                     mine = true;
@@ -843,8 +856,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 // Q may be overwritten once both issuers' QKs of this pair have finished
                 if (elect_one()) {
                     if (mine) {
-                        mma_commit<2>(smem_u32(&sm.bar_q_empty));
-                        mma_commit<2>(q_empty_peer);
+                        mma_commit_both(smem_u32(&sm.bar_q_empty));
                     } else {
                         mbar_arrive(smem_u32(&sm.bar_q_empty));
                         mbar_arrive_cluster(q_empty_peer);
@@ -865,17 +877,14 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             // ===================== PV issuer (CTA 0): converged warp, one elected lane issues ==========
             WorkIter<DECODE> it(p);
             WorkItem w;
-            uint32_t gt = 0, gw = 0;
+            uint32_t gt = 0, gw = 0, later = 0;   // tiles, pairs, tiles that were not their pair's first
             bool released = false;
-            const uint32_t pv_half_peer = map_to_cta(smem_u32(&sm.bar_pv_half[0]), 1);
-            const uint32_t pv_done_peer = map_to_cta(smem_u32(&sm.bar_pv_done[0]), 1);
             MXDSA_WAIT_TIGHT(sm.bar_tmem_ready, 0, 24);
 #pragma unroll 1
             while (it.template next<NT>(w)) {
                 const int ntiles = (w.blk_end - w.blk_begin + 1) / 2;
                 if (ntiles <= 0) continue;  // never produced by the scheduler; keeps the roles in step
                 MXDSA_WAIT_TIGHT(sm.bar_o_empty, (gw & 1) ^ 1, 30);
-                tc_fence_after();
 #pragma unroll 1
                 for (int t = 0; t < ntiles; ++t, ++gt) {
                     const uint32_t s = gt % kStages, ph = (gt / kStages) & 1;
@@ -886,32 +895,32 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     const uint64_t b_base = smem_desc(desc_v, smem_u32(sm.kv[s]));
                     const uint32_t sfa = tmem + kColSs + 4 * b;
                     const bool fresh = t == 0;
+                    MXDSA_WAIT_TIGHT(sm.bar_s_full[b], bph, 33);
+                    // Two steps, each of which waits for its part of O.  128-key tiles: dim chunk 0, then 1, so that one chunk is
+                    // rescaled while the other is being accumulated.  64-key tiles: key half 0, then 1, O being rescaled in between.
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
-                        if (NT == 128 && h == 0) continue;   // 128-key tiles: one wait, after both halves are in
-                        MXDSA_WAIT_TIGHT(sm.bar_s_full[b][h], bph, 32 + h);
+                        if (t > 0 || (NT == 64 && h == 1)) {
+                            const uint32_t n = NT == 64 && h == 1 ? gt : later;
+                            MXDSA_WAIT_TIGHT(sm.bar_o_ready[h][n % kScStages], (n / kScStages) & 1, 32 + 3 * h);
+                        }
                         tc_fence_after();
                         __syncwarp();
                         if (elect_one()) {
-                            tmem_cp_sf_pair(sfa, smem_desc(desc_sf, smem_u32(sm.s_sf[b])));
+                            if (h == 0) tmem_cp_sf_pair(sfa, smem_desc(desc_sf, smem_u32(sm.s_sf[b])));
 #pragma unroll
-                            for (int i = (NT == 64 ? 4 * h : 0); i < 4 * h + 4; ++i) {
-                                const int ks = i >> 1, n = i & 1;   // key step (32 keys), dim chunk (128 dims of each CTA)
+                            for (int i = 0; i < 4; ++i) {
+                                const int ks = NT == 64 ? 2 * h + (i >> 1) : i, n = NT == 64 ? i & 1 : h;   // key step (32 keys), dim chunk (128 dims of each CTA)
                                 mma_mxf8<2>(tmem + kColO + n * 128, a_base + ((ks * 32) >> 4),
                                             b_base + (((ks >> 1) * 16384 + n * 8192 + (ks & 1) * 4096) >> 4),
                                             mx_idesc(128, 256, true, ks, NT == 64 ? (ks & 1) : ks), sfa,
                                             tmem + kColVs + 4 * n, !(fresh && ks == 0));
                             }
-                            if (NT == 64 && h == 0) {
-                                mma_commit<2>(smem_u32(&sm.bar_pv_half[b]));
-                                mma_commit<2>(pv_half_peer + b * 8);
-                            } else {
-                                mma_commit<2>(smem_u32(&sm.bar_pv_done[sc]));
-                                mma_commit<2>(pv_done_peer + sc * 8);
-                            }
+                            mma_commit_both(smem_u32(h == 0 ? &sm.bar_pv_half[sc] : &sm.bar_pv_done[sc]));
                         }
                         __syncwarp();
                     }
+                    if (t > 0) ++later;
                 }
                 released = !it.done();
                 ++gw;
@@ -1004,25 +1013,26 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         else MXDSA_WAIT(sm.bar_q_empty, (gw & 1) ^ 1, 42);   // CTA 0's issuers signal it for the last pair too
     }
     } else if (warp < 12 + 4 * G) {
-        if constexpr (kRebalanceRegs) setmaxnreg_inc<kRegsSoftmax>();
-        // ===================== softmax + epilogue (warps 12 ..) =====================
-        // G groups of four warps take tiles in turn (tile g: group g % G, P buffer g & 1), so one
-        // group's exp / quantise / store phase overlaps another group's load / max phase.  Inside a
-        // group a thread owns one row and one 64-key half of the tile (two UE8M0 scale groups of S).
+        setmaxnreg_inc<kRegsSoftmax>();
+        // ===================== softmax (warps 12 ..) =====================
+        // Two groups of eight warps take tiles in turn (tile g: group and P buffer g & 1), so one group's exp / quantise /
+        // store phase overlaps the other's load / max phase.  Inside a group a thread owns one row and one 32-key quarter of
+        // the tile, a UE8M0 scale group of S.
         // The only serial link between consecutive tiles is the running maximum: after deciding m_t a
         // group publishes it (sm.m_pub) and the next group picks it up before deciding m_{t+1}.
-        const int grp = (warp - 12) >> 2;
-        const int prev_grp = (grp + kGroups - 1) % kGroups;
+        const int grp = (warp - 12) / kGroupWarps;
         const int q4 = warp & 3;                 // lane quadrant of tensor memory
         const int L = q4 * 32 + lane;            // tensor-memory lane
         const int row = L % 64;                  // head
-        const int half = L / 64;                 // key half of a tile / dim half of O
+        const int half = L / 64;                 // key half of a tile
+        const int part = ((warp - 12) % kGroupWarps) >> 2;   // which 32 keys of the half
+        const int qtr = 2 * half + part;
         const uint32_t lane_addr = tmem + (uint32_t(q4 * 32) << 16);
         const uint32_t p_empty0 = map_to_cta(smem_u32(&sm.bar_p_empty[0]), 0);
-        const uint32_t s_full0 = map_to_cta(smem_u32(&sm.bar_s_full[0][0]), 0);
+        const uint32_t s_full0 = map_to_cta(smem_u32(&sm.bar_s_full[0]), 0);
         const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
         cluster_wait();
-        if (grp == 0) {
+        if (warp < 16) {
             // V dimension scales (B-operand scale columns of every PV): lanes 0-63 hold the dims of CTA 0's half
             // (w1), lanes 64-127 those of CTA 1's half (w2); column c = word c.  Written once, straight from
             // registers, as soon as the tensor memory has been allocated; the MMA issuers wait for both CTAs' four warps.
@@ -1052,117 +1062,112 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 if ((int)(gt % kGroups) != grp) continue;
                 const uint32_t sc = gt % kScStages, sph = (gt / kScStages) & 1;
                 const uint32_t pb = gt & 1;                              // P buffer
-                const uint32_t b = gt % kSBufs, bph = (gt / kSBufs) & 1;   // S buffer and the phase of its barriers
+                const uint32_t b = gt % kSBufs;                          // S buffer
+                const uint32_t mr = gt % kMRing, mr_prev = (gt + kMRing - 1) % kMRing;
                 MXDSA_WAIT_POLL(sm.bar_tok_full[sc], sph, 50);
-                const uint32_t v0 = sm.valid[sc][2 * half], v1 = sm.valid[sc][2 * half + 1];
+                const uint32_t vbits = sm.valid[sc][qtr];
                 MXDSA_WAIT_POLL(sm.bar_qk_done[sc], sph, 51);
                 tc_fence_after();
-                float x[64];
-                tmem_ld32(lane_addr + kColP + pb * 64, reinterpret_cast<uint32_t*>(x));
-                tmem_ld32(lane_addr + kColP + pb * 64 + 32, reinterpret_cast<uint32_t*>(x + 32));
+                float x[32];
+                tmem_ld32(lane_addr + kColP + pb * 64 + part * 32, reinterpret_cast<uint32_t*>(x));
                 tmem_wait_ld();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_cluster(p_empty0 + pb * 8);
-                if ((v0 & v1) != 0xffffffffu) {
+                if (vbits != 0xffffffffu) {
 #pragma unroll
-                    for (int i = 0; i < 64; ++i) x[i] = (((i < 32 ? v0 : v1) >> (i & 31)) & 1u) ? x[i] : -CUDART_INF_F;
+                    for (int i = 0; i < 32; ++i) x[i] = ((vbits >> i) & 1u) ? x[i] : -CUDART_INF_F;
                 }
-                float mx8[8];
+                float mx4[4];
 #pragma unroll
-                for (int i = 0; i < 8; ++i) mx8[i] = x[i];
+                for (int i = 0; i < 4; ++i) mx4[i] = fmax3(x[i], x[4 + i], x[8 + i]);
 #pragma unroll
-                for (int i = 8; i < 64; i += 16) {
+                for (int i = 12; i < 28; i += 8) {
 #pragma unroll
-                    for (int j = 0; j < 8; ++j) mx8[j] = fmax3(mx8[j], x[i + j], x[i + 8 + j < 64 ? i + 8 + j : i + j]);
+                    for (int j = 0; j < 4; ++j) mx4[j] = fmax3(mx4[j], x[i + j], x[i + 4 + j]);
                 }
-                const float own_max = fmaxf(fmax3(mx8[0], mx8[1], mx8[2]), fmaxf(fmax3(mx8[3], mx8[4], mx8[5]), fmaxf(mx8[6], mx8[7]))) * p.scale_log2;
-                float* xm = sm.xmax[grp][(gt / kGroups) & 1];
-                xm[L] = own_max;
-                named_bar_sync(1 + grp, 128);
-                const float peer_max = xm[L ^ 64];
+                const float own_max = fmaxf(fmax3(fmaxf(mx4[0], x[28]), fmaxf(mx4[1], x[29]), fmaxf(mx4[2], x[30])), fmaxf(mx4[3], x[31])) * p.scale_log2;
+                float (*xm)[64] = sm.xmax[grp][(gt / kGroups) & 1];
+                xm[qtr][row] = own_max;
+                named_bar_sync(1 + grp, 32 * kGroupWarps);
+                const float half0_max = fmaxf(xm[0][row], xm[1][row]), half1_max = fmaxf(xm[2][row], xm[3][row]);
                 // the running maximum handed over by the group before (value ignored on a pair's first
                 // tile, but every phase of that barrier is observed)
-                if (gt > 0) MXDSA_WAIT_POLL(sm.bar_m_ready[prev_grp], ((gt - 1) / kGroups) & 1, 58);
-                const float m_prev = t == 0 ? -1e30f : sm.m_pub[prev_grp][row];
+                if (gt > 0) MXDSA_WAIT_POLL(sm.bar_m_ready[mr_prev], ((gt - 1) / kMRing) & 1, 58);
+                const float m_prev = t == 0 ? -1e30f : sm.m_pub[mr_prev][row];
                 const float sprev = (m_own == m_prev) ? 1.f : ex2_approx(m_own - m_prev);
                 // numerical tiles: NT = 128 -> one per tensor-core tile; NT = 64 -> key half 0 then 1
                 float m_used, scale0 = 1.f, scale1 = 1.f;
-                bool grow0, grow1 = false;
                 if constexpr (NT == 128) {
-                    const float tmax = fmaxf(own_max, peer_max);
+                    const float tmax = fmaxf(half0_max, half1_max);
                     real_m = fmaxf(real_m, tmax);
-                    grow0 = __any_sync(0xffffffffu, tmax - m_prev > 6.0f);
+                    const bool grow0 = __any_sync(0xffffffffu, tmax - m_prev > 6.0f);
                     const float nm = grow0 ? fmaxf(m_prev, tmax) : m_prev;
                     scale0 = grow0 ? ex2_approx(m_prev - nm) : 1.f;
                     m_own = nm;
                     m_used = nm;
                 } else {
-                    const float t0 = half == 0 ? own_max : peer_max;
-                    const float t1 = half == 0 ? peer_max : own_max;
+                    const float t0 = half0_max, t1 = half1_max;
                     real_m = fmaxf(real_m, fmaxf(t0, t1));
-                    grow0 = __any_sync(0xffffffffu, t0 - m_prev > 6.0f);
+                    const bool grow0 = __any_sync(0xffffffffu, t0 - m_prev > 6.0f);
                     const float m1 = grow0 ? fmaxf(m_prev, t0) : m_prev;
                     scale0 = grow0 ? ex2_approx(m_prev - m1) : 1.f;
-                    grow1 = __any_sync(0xffffffffu, t1 - m1 > 6.0f);
+                    const bool grow1 = __any_sync(0xffffffffu, t1 - m1 > 6.0f);
                     const float m2 = grow1 ? fmaxf(m1, t1) : m1;
                     scale1 = grow1 ? ex2_approx(m1 - m2) : 1.f;
                     m_used = half == 0 ? m1 : m2;
                     m_own = m2;
+                    if (qtr == 0) sm.m_mid[mr][row] = m1;
                 }
-                sm.m_pub[grp][row] = m_own;
-                __syncwarp();
-                if (lane == 0) mbar_arrive(smem_u32(&sm.bar_m_ready[grp]));
-                // S buffer b is free once the PV of tile gt - kSBufs has finished (long ago, as a rule)
+                // S buffer b is free once the PV of tile gt - kSBufs has finished (long ago, as a rule).  The wait stands ahead
+                // of the running maximum: with it the epilogue warps are never a whole ring of maxima behind.
                 if (gt >= (uint32_t)kSBufs) {
                     const uint32_t g = gt - kSBufs;
                     MXDSA_WAIT_POLL(sm.bar_pv_done[g % kScStages], (g / kScStages) & 1, 52);
                 }
+                if (qtr == 0) {   // the same value in all four warps of the row
+                    sm.m_pub[mr][row] = m_own;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&sm.bar_m_ready[mr]));
+                }
                 // probabilities, key-scaled, re-quantised per 32 keys and stored
                 const float2 negm2 = make_float2(-m_used, -m_used);
-                const float4* tok4 = reinterpret_cast<const float4*>(&sm.tok_scale[sc][half * 64]);
+                const float4* tok4 = reinterpret_cast<const float4*>(&sm.tok_scale[sc][qtr * 32]);
                 uint8_t* srow = sm.s[b];
                 float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
-                uint32_t e_bytes = 0;
+                float am0 = 0.f, am1 = 0.f;
 #pragma unroll
-                for (int g = 0; g < 2; ++g) {
-                    uint32_t s8[8];
-                    uint32_t e;
-                    float am0 = 0.f, am1 = 0.f;
-                    float* xg = x + 32 * g;
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        const float4 tk = tok4[g * 8 + i / 4];
-                        float2 a = f2_fma(make_float2(xg[i], xg[i + 1]), scale2, negm2);
-                        float2 c = f2_fma(make_float2(xg[i + 2], xg[i + 3]), scale2, negm2);
-                        a = make_float2(ex2_approx(a.x), ex2_approx(a.y));
-                        c = make_float2(ex2_approx(c.x), ex2_approx(c.y));
-                        sum2[0] = f2_add(sum2[0], a);
-                        sum2[1] = f2_add(sum2[1], c);
-                        a = f2_mul(a, make_float2(tk.x, tk.y));
-                        c = f2_mul(c, make_float2(tk.z, tk.w));
-                        am0 = fmax3(am0, a.x, a.y);
-                        am1 = fmax3(am1, c.x, c.y);
-                        xg[i] = a.x; xg[i + 1] = a.y; xg[i + 2] = c.x; xg[i + 3] = c.y;
-                    }
-                    const float am = fmaxf(am0, am1);
-                    e = cvt_ue8m0_roundup(am > 0.f ? __fdividef(am, 448.0f) : 1.0f);
-                    e = max(e, 61u);
-                    const float mulf = __uint_as_float((254u - e) << 23);
-                    const float2 mul2 = make_float2(mulf, mulf);
-#pragma unroll
-                    for (int i = 0; i < 32; i += 4) {
-                        const float2 a = f2_mul(make_float2(xg[i], xg[i + 1]), mul2);
-                        const float2 c = f2_mul(make_float2(xg[i + 2], xg[i + 3]), mul2);
-                        s8[i / 4] = (uint32_t)cvt_e4m3x2(a.x, a.y) | ((uint32_t)cvt_e4m3x2(c.x, c.y) << 16);
-                    }
-                    e_bytes |= e << (8 * g);
-                    *reinterpret_cast<uint4*>(srow + swz128(row, half * 64 + g * 32)) = make_uint4(s8[0], s8[1], s8[2], s8[3]);
-                    *reinterpret_cast<uint4*>(srow + swz128(row, half * 64 + g * 32 + 16)) = make_uint4(s8[4], s8[5], s8[6], s8[7]);
+                for (int i = 0; i < 32; i += 4) {
+                    const float4 tk = tok4[i / 4];
+                    float2 a = f2_fma(make_float2(x[i], x[i + 1]), scale2, negm2);
+                    float2 c = f2_fma(make_float2(x[i + 2], x[i + 3]), scale2, negm2);
+                    a = make_float2(ex2_approx(a.x), ex2_approx(a.y));
+                    c = make_float2(ex2_approx(c.x), ex2_approx(c.y));
+                    sum2[0] = f2_add(sum2[0], a);
+                    sum2[1] = f2_add(sum2[1], c);
+                    a = f2_mul(a, make_float2(tk.x, tk.y));
+                    c = f2_mul(c, make_float2(tk.z, tk.w));
+                    am0 = fmax3(am0, a.x, a.y);
+                    am1 = fmax3(am1, c.x, c.y);
+                    x[i] = a.x; x[i + 1] = a.y; x[i + 2] = c.x; x[i + 3] = c.y;
                 }
-                // scale rows: row (row%32) and its copy at +32; word row/32; bytes 2*half, 2*half+1
-                reinterpret_cast<uint16_t*>(&sm.s_sf[b][(row % 32) * 4 + row / 32])[half] = (uint16_t)e_bytes;
-                reinterpret_cast<uint16_t*>(&sm.s_sf[b][(32 + row % 32) * 4 + row / 32])[half] = (uint16_t)e_bytes;
+                const float am = fmaxf(am0, am1);
+                uint32_t e = cvt_ue8m0_roundup(am > 0.f ? __fdividef(am, 448.0f) : 1.0f);
+                e = max(e, 61u);
+                const float mulf = __uint_as_float((254u - e) << 23);
+                const float2 mul2 = make_float2(mulf, mulf);
+                uint32_t s8[8];
+#pragma unroll
+                for (int i = 0; i < 32; i += 4) {
+                    const float2 a = f2_mul(make_float2(x[i], x[i + 1]), mul2);
+                    const float2 c = f2_mul(make_float2(x[i + 2], x[i + 3]), mul2);
+                    s8[i / 4] = (uint32_t)cvt_e4m3x2(a.x, a.y) | ((uint32_t)cvt_e4m3x2(c.x, c.y) << 16);
+                }
+                *reinterpret_cast<uint4*>(srow + swz128(row, qtr * 32)) = make_uint4(s8[0], s8[1], s8[2], s8[3]);
+                *reinterpret_cast<uint4*>(srow + swz128(row, qtr * 32 + 16)) = make_uint4(s8[4], s8[5], s8[6], s8[7]);
+                // scale rows: row (row%32) and its copy at +32; word row/32; byte qtr
+                reinterpret_cast<uint8_t*>(&sm.s_sf[b][(row % 32) * 4 + row / 32])[qtr] = (uint8_t)e;
+                reinterpret_cast<uint8_t*>(&sm.s_sf[b][(32 + row % 32) * 4 + row / 32])[qtr] = (uint8_t)e;
                 const float2 s2 = f2_add(sum2[0], sum2[1]);
                 const float sum = s2.x + s2.y;
                 // l bookkeeping: every update of m rescales all partial sums of the row
@@ -1172,28 +1177,10 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     if (half == 0) l = fmaf(l * sprev, scale0, sum) * scale1;
                     else l = fmaf(l * sprev * scale0, scale1, sum);
                 }
-                // O rescale before the first key half is accumulated (this thread: its whole lane)
-                if (grow0 && t > 0)
-                {
-                    MXDSA_WAIT_POLL(sm.bar_pv_done[(gt - 1) % kScStages], ((gt - 1) / kScStages) & 1, 53);
-                    tc_fence_after();
-                    rescale_o(lane_addr, scale0);
-                    tc_fence_before();
-                }
                 fence_proxy_async_smem();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(s_full0 + (b * 2 + 0) * 8);
-                if constexpr (NT == 64) {
-                    if (grow1) {
-                        MXDSA_WAIT_POLL(sm.bar_pv_half[b], bph, 54);
-                        tc_fence_after();
-                        rescale_o(lane_addr, scale1);
-                        tc_fence_before();
-                    }
-                }
-                __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive_cluster(s_full0 + (b * 2 + 1) * 8);
+                    mbar_arrive_cluster(s_full0 + b * 8);
                     mbar_arrive(smem_u32(&sm.bar_tok_empty[sc]));
                 }
             }
@@ -1202,26 +1189,25 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             float m_fin = m_own;
             const int last_grp = (int)(last % kGroups);
             if (last_grp != grp) {
-                MXDSA_WAIT_POLL(sm.bar_m_ready[last_grp], (last / kGroups) & 1, 59);
-                m_fin = sm.m_pub[last_grp][row];
+                MXDSA_WAIT_POLL(sm.bar_m_ready[last % kMRing], (last / kMRing) & 1, 59);
+                m_fin = sm.m_pub[last % kMRing][row];
                 l *= (m_own == m_fin) ? 1.f : ex2_approx(m_own - m_fin);
             }
-            sm.xl[grp * 128 + L] = l;
-            sm.xr[grp * 128 + L] = real_m;
-            named_bar_sync(1 + kGroups, kGroups * 128);
-            const float* xl = sm.xl;
-            const float* xr = sm.xr;
-            float l_tot = (xl[row] + xl[64 + row]) + (xl[128 + row] + xl[192 + row]);
-            float real_all = fmaxf(fmaxf(xr[row], xr[64 + row]), fmaxf(xr[128 + row], xr[192 + row]));
-            if constexpr (kGroups == 3) {
-                l_tot += xl[256 + row] + xl[320 + row];
-                real_all = fmaxf(real_all, fmaxf(xr[256 + row], xr[320 + row]));
+            sm.xl[grp][qtr][row] = l;
+            if (qtr == 0) sm.xr[grp][row] = real_m;   // the same in all four warps of the row
+            named_bar_sync(1 + kGroups, kGroups * kGroupWarps * 32);
+            float l_tot = 0.f, real_all = 0.f;
+            if (warp < 14) {
+#pragma unroll
+                for (int g = 0; g < kGroups; ++g)
+                    l_tot += (sm.xl[g][0][row] + sm.xl[g][1][row]) + (sm.xl[g][2][row] + sm.xl[g][3][row]);
+                real_all = fmaxf(sm.xr[0][row], sm.xr[1][row]);
             }
-            named_bar_sync(1 + kGroups, kGroups * 128);   // everybody has read the exchange area before the next pair writes it
+            named_bar_sync(1 + kGroups, kGroups * kGroupWarps * 32);   // everybody has read the exchange area before the next pair writes it
             // The first two warps of group 0 (one thread per row) turn the row sums into what the epilogue warps
             // need, write lse / max_logits, and every softmax warp goes straight on to the next pair: O is drained
             // by warps of its own while the next pair's tiles are worked on.
-            if (grp == 0 && half == 0) {
+            if (warp < 14) {
                 float m = m_fin;
                 if (real_all == -CUDART_INF_F) {
                     l_tot = 0.f;
@@ -1254,7 +1240,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             ++gw;
         }
     } else {
-        if constexpr (kRebalanceRegs) setmaxnreg_dec<kRegsEpi>();
+        setmaxnreg_inc<kRegsEpi>();
         // ===================== epilogue (last four warps): O -> out =====================
         // A thread drains its tensor-memory lane: row L%64, the 256 dims of half L/64, 32 columns at a time,
         // multiplied by the row's oscale.  Unsplit work goes to `out` as bf16, split decode work to the fp32
@@ -1266,24 +1252,70 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         const int half = L / 64;
         const uint32_t lane_addr = tmem + (uint32_t(q4 * 32) << 16);
         const uint32_t o_empty0 = map_to_cta(smem_u32(&sm.bar_o_empty), 0);
+        const uint32_t o_ready0 = map_to_cta(smem_u32(&sm.bar_o_ready[0][0]), 0);
         cluster_wait();
         WorkIter<DECODE> it(p);
         WorkItem w;
+        uint32_t gt = 0, gw = 0, later = 0;   // tiles, pairs, tiles that were not their pair's first
         // O is free for the next pair's first PV as soon as this warp has READ its last columns; the stores of
         // those columns (which may have to wait for a staging tile) follow after the release.  Nothing is signalled where
         // no pair follows: CTA 0 may be gone before an arrival that nobody waits for has come.
+        auto rescale = [&](int col, int cols, float f) {
+            tc_fence_after();
+            rescale_o(lane_addr + kColO + col, cols, f);
+        };
+        auto o_is_ready = [&](int step, uint32_t n) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(o_ready0 + (step * kScStages + n % kScStages) * 8);
+        };
         auto release_o = [&]() {
             tc_fence_before();
             __syncwarp();
             if (lane == 0 && !it.done()) mbar_arrive_cluster(o_empty0);
         };
-        uint32_t gt = 0, gw = 0;
         uint32_t round = 0;   // output rounds of this warp so far (staging tile = round % kOutTiles)
 #pragma unroll 1
         while (it.template next<NT>(w)) {
             const int ntiles = (w.blk_end - w.blk_begin + 1) / 2;
             if (ntiles <= 0) continue;  // never produced by the scheduler; keeps the roles in step
-            gt += ntiles;
+            float m_cur = 0.f;
+#pragma unroll 1
+            for (int t = 0; t < ntiles; ++t, ++gt) {
+                const uint32_t mr = gt % kMRing, before = gt - 1;
+                MXDSA_WAIT(sm.bar_m_ready[mr], (gt / kMRing) & 1, 61);
+                const float m_new = sm.m_pub[mr][row];
+                if constexpr (NT == 128) {
+                    if (t > 0) {
+                        const bool grew = __any_sync(0xffffffffu, m_new != m_cur);
+                        const float f = ex2_approx(m_cur - m_new);
+#pragma unroll 1
+                        for (int n = 0; n < 2; ++n) {
+                            if (grew) {
+                                const uint32_t pv = smem_u32(n == 0 ? &sm.bar_pv_half[before % kScStages] : &sm.bar_pv_done[before % kScStages]);
+                                MXDSA_WAIT_ADDR_(MXDSA_POLL_BACKOFF_NS, pv, (before / kScStages) & 1, 53);
+                                rescale(n * 128, 128, f);
+                            }
+                            o_is_ready(n, later);
+                        }
+                    }
+                } else {
+                    const float m_mid = sm.m_mid[mr][row];
+#pragma unroll 1
+                    for (int h = t > 0 ? 0 : 1; h < 2; ++h) {
+                        const float from = h == 0 ? m_cur : m_mid, to = h == 0 ? m_mid : m_new;
+                        if (__any_sync(0xffffffffu, from != to)) {
+                            const uint32_t g = h == 0 ? before : gt;
+                            const uint32_t pv = smem_u32(h == 0 ? &sm.bar_pv_done[g % kScStages] : &sm.bar_pv_half[g % kScStages]);
+                            MXDSA_WAIT_ADDR_(MXDSA_POLL_BACKOFF_NS, pv, (g / kScStages) & 1, 54);
+                            rescale(0, 256, ex2_approx(from - to));
+                        }
+                        o_is_ready(h, h == 0 ? later : gt);
+                    }
+                }
+                m_cur = m_new;
+                if (t > 0) ++later;
+            }
             const uint32_t last = gt - 1;
             MXDSA_WAIT(sm.bar_os_full[gw & 1], (gw >> 1) & 1, 60);
             const float oscale = sm.oscale[gw & 1][row];
@@ -1382,7 +1414,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             ++gw;
         }
         // CTA 0 signals this one for every tile, whether a maximum grew or not
-        if (NT == 64 && gt > 0) MXDSA_WAIT(sm.bar_pv_half[(gt - 1) % kSBufs], ((gt - 1) / kSBufs) & 1, 57);
+        if (gt > 0) MXDSA_WAIT(sm.bar_pv_half[(gt - 1) % kScStages], ((gt - 1) / kScStages) & 1, 57);
     }
 
 done:
@@ -1395,8 +1427,8 @@ done:
     // completes the exchange barrier for those still parked on it (they fail their next wait and
     // follow).  In a normal exit the arrivals are harmless: nobody waits on that barrier any more.
     if (warp >= 12 && warp < 12 + 4 * G) {
-        named_bar_arrive(1 + ((warp - 12) >> 2), 128);
-        named_bar_arrive(1 + kGroups, kGroups * 128);
+        named_bar_arrive(1 + (warp - 12) / kGroupWarps, 32 * kGroupWarps);
+        named_bar_arrive(1 + kGroups, kGroups * kGroupWarps * 32);
     }
     tc_fence_before();
     // Nobody leaves while the peer may still signal it: the cluster barrier's release orders every arrival on a barrier of

@@ -129,29 +129,20 @@ int make_out_map(CUtensorMap* map, void* base, uint64_t tokens) {
 
 constexpr size_t kSmemBytes = sizeof(mxdsa::SmemPlan) + 1024;
 
-#ifndef MXDSA_GROUPS_PREFILL
-#define MXDSA_GROUPS_PREFILL 3
-#endif
-#ifndef MXDSA_GROUPS_DECODE
-#define MXDSA_GROUPS_DECODE 3
-#endif
-
-// `groups` = softmax groups of the instantiation (the template's G): it fixes the block size and the register
-// allocation that the kernel's setmaxnreg budget assumes.
 template <typename K>
-int launch_pairs(K kernel, int groups, dim3 grid, cudaStream_t stream, const mxdsa::AttnParams& ap,
+int launch_pairs(K kernel, dim3 grid, cudaStream_t stream, const mxdsa::AttnParams& ap,
                  const mxdsa::TensorMaps& maps) {
     static_assert(kSmemBytes <= 227 * 1024, "shared-memory plan exceeds the 227 KB per-CTA limit");
-    // The kernel re-balances registers between its roles against a pool of launch_regs(groups) per thread.
+    // The kernel re-balances registers between its roles against a pool of kLaunchRegs per thread.
     // If this build of the kernel was given a different number (another toolkit or flag set), an increase
     // beyond the pool would block in hardware for ever: refuse to launch instead.
     cudaFuncAttributes fa;
     MX_CUDA(cudaFuncGetAttributes(&fa, kernel));
-    if (fa.numRegs != mxdsa::launch_regs(groups)) return MXDSA_ERR_DEVICE;
+    if (fa.numRegs != mxdsa::kLaunchRegs) return MXDSA_ERR_DEVICE;
     MX_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(mxdsa::kBaseThreads + 128 * groups);
+    cfg.blockDim = dim3(mxdsa::kThreads);
     cfg.dynamicSmemBytes = kSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[2]{};
@@ -555,9 +546,8 @@ int mxdsa_prefill_fwd(const mxdsa_prefill_params* p) {
     const int clusters = ap.num_pairs < d->sm_count / 2 ? ap.num_pairs : d->sm_count / 2;
     const dim3 grid(2 * clusters, 1, 1);
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-    constexpr int G = MXDSA_GROUPS_PREFILL;
-    if (p->topk >= 512) return launch_pairs(mxdsa::mxdsa_attn_kernel<false, 128, G>, G, grid, stream, ap, maps);
-    return launch_pairs(mxdsa::mxdsa_attn_kernel<false, 64, G>, G, grid, stream, ap, maps);
+    if (p->topk >= 512) return launch_pairs(mxdsa::mxdsa_attn_kernel<false, 128>, grid, stream, ap, maps);
+    return launch_pairs(mxdsa::mxdsa_attn_kernel<false, 64>, grid, stream, ap, maps);
 }
 
 int mxdsa_num_sm_parts(int device, int s_q) {
@@ -702,7 +692,7 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
 
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
     const dim3 grid(2 * ((p->s_q + 1) / 2), p->num_sm_parts, 1);
-    st = launch_pairs(mxdsa::mxdsa_attn_kernel<true, 64, MXDSA_GROUPS_DECODE>, MXDSA_GROUPS_DECODE, grid, stream, ap, maps);
+    st = launch_pairs(mxdsa::mxdsa_attn_kernel<true, 64>, grid, stream, ap, maps);
     if (st != MXDSA_OK) return st;
     if (!combine) return MXDSA_OK;
     // programmatic dependent launch: the combine grid is set up while the attention grid drains (the attention
