@@ -21,13 +21,16 @@
 // it in one sweep of the row and selects exactly among those (rows of many equal scores are counted instead); where there
 // are fewer rows than SMs it divides a row among the CTAs of a cluster.
 //
-// Counting every key: exact radix selection on the order-preserving 32-bit image of the float, three histogram
-// passes (11 + 11 + 10 bits) with shared-memory atomics, keys of a row held in registers (one HBM read
+// Counting every key: exact radix selection on the order-preserving 32-bit image of the float, up to three histogram
+// passes (11 + 11 + 10 bits) with shared-memory atomics, ended where a whole bin is taken (after two, as a rule), keys of a row held in registers (one HBM read
 // per score for rows of up to 16 384 keys; longer rows are swept again from L2).  No pass branches per
 // key: the first counts every key, the later ones send keys outside the current prefix to a per-lane
 // spare bin.  Packed per-chunk counts and two block scans then give every selected key its output
 // position; the row is staged in shared memory and written in whole lines.  No sort, no global atomics,
-// deterministic.
+// deterministic.  A row costs what its own length costs: chunks of 2 048 keys past it are neither loaded nor counted, and
+// the third pass is rarely needed, because the 22-bit bin of the threshold holds one key or two.  Before, every row cost
+// 16 384 keys and three passes: 2 048 pairs of 16 384 keys, half to full length, topk 2048 93.9 -> 73.1 us (the passes alone
+// 85.4), 1 951 pairs of 3 172 keys 71.7 -> 40.0, 27 pairs of 4 464 keys 8.4 -> 7.8.
 //
 // Bound: HBM on paper (group * s_kv * 4 bytes read + topk * 4 written per row); in practice the integer and
 // shared-memory pipes (counting every key: about 25 instructions and three shared atomics per key), so every step is
@@ -70,19 +73,26 @@ __device__ __forceinline__ uint32_t score_key(float s) {
 // One sweep of a row into registers.  All loads of a batch are issued before the first conversion, so a
 // sweep exposes one memory latency (two with GROUP == 2, whose two score rows are taken in two batches
 // of four chunks to stay inside the register budget), not one per load.
+// Chunks that lie past the row's length altogether are not loaded, and their registers hold nothing: whoever walks the
+// keys stops at live_chunks(), which is the same for all threads.
+__device__ __forceinline__ int live_chunks(int sweep, int len) {
+    return min((len - sweep * kSweep + kThreads * 4 - 1) / (kThreads * 4), kChunks);
+}
 template <int GROUP>
 __device__ __forceinline__ void load_keys(const float* __restrict__ row0, const float* __restrict__ row1, int sweep,
-                                          int s_kv, int len, uint32_t (&key)[kKpt]) {
+                                          int len, uint32_t (&key)[kKpt]) {
+    const int live = live_chunks(sweep, len);
     constexpr int kBatch = GROUP == 2 ? kChunks / 2 : kChunks;
 #pragma unroll
     for (int c0 = 0; c0 < kChunks; c0 += kBatch) {
+        if (c0 >= live) break;
         float4 a[kBatch], b[GROUP == 2 ? kBatch : 1];
 #pragma unroll
         for (int c = 0; c < kBatch; ++c) {
             const int j = sweep * kSweep + ((c0 + c) * kThreads + (int)threadIdx.x) * 4;
             a[c] = make_float4(0.f, 0.f, 0.f, 0.f);
             if (GROUP == 2) b[c] = a[c];
-            if (j < s_kv) {
+            if (j < len) {               // (rows are whole groups of four)
                 a[c] = __ldg(reinterpret_cast<const float4*>(row0 + j));
                 if (GROUP == 2) b[c] = __ldg(reinterpret_cast<const float4*>(row1 + j));
             }
@@ -154,12 +164,13 @@ __device__ __forceinline__ uint32_t find_bin(TopkShared& sm, uint32_t k_or_cap, 
 // cover the eight chunks (a warp's inclusive total per chunk is at most 128).
 template <bool TIES, bool STAGED>
 __device__ __forceinline__ void emit_sweep(TopkShared& sm, const uint32_t (&key)[kKpt], uint32_t thr, uint32_t need_eq,
-                                           int32_t* __restrict__ out, int32_t off, int sw, uint32_t& base_gt,
-                                           uint32_t& base_eq) {
+                                           int32_t* __restrict__ out, int32_t off, int sw, int live,
+                                           uint32_t& base_gt, uint32_t& base_eq) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     uint32_t own_a[2] = {0u, 0u}, own_e[2] = {0u, 0u};   // a: key > thr (TIES) or key >= thr; e: key == thr
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
+        if (c >= live) break;
         uint32_t na = 0, ne = 0;
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
@@ -193,6 +204,7 @@ __device__ __forceinline__ void emit_sweep(TopkShared& sm, const uint32_t (&key)
     __syncthreads();
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {
+        if (c >= live) break;
         const uint32_t before = sm.chunk_tot[c * kWarps + warp];
         const int sh = 8 * (c & 3);
         uint32_t a = base_gt + (before & 0xffffu) + ((inc_a[c >> 2] >> sh) & 0xffu) - ((own_a[c >> 2] >> sh) & 0xffu);
@@ -233,19 +245,18 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
                        int32_t* __restrict__ topk_length, int rows, int s_kv, int topk) {
     __shared__ __align__(16) TopkShared sm;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int nsweeps = (s_kv + kSweep - 1) / kSweep;
-    for (int r = blockIdx.x; r < rows; r += gridDim.x) {
+    int len = s_kv;
+    if (lengths != nullptr && (int)blockIdx.x < rows) len = min(max(__ldg(lengths + blockIdx.x), 0), s_kv);
+    for (int r = blockIdx.x, next_len; r < rows; r += gridDim.x, len = next_len) {
         const float* row0 = scores + (long long)r * GROUP * score_stride;
         const float* row1 = row0 + score_stride;
-        int len = s_kv;
-        if (lengths != nullptr) len = min(max(__ldg(lengths + r), 0), s_kv);
+        const int nsweeps = (len + kSweep - 1) / kSweep;
+        // the row this CTA takes next: its length is loaded now and its scores are asked into L2 once this row's are in
+        // registers, so that its loads do not wait for HBM
+        const int next = r + (int)gridDim.x;
+        next_len = s_kv;
+        if (lengths != nullptr && next < rows) next_len = min(max(__ldg(lengths + next), 0), s_kv);
         uint32_t key[kKpt];
-        // the row this CTA takes next: ask L2 for it now, so that its loads do not wait for HBM
-        if (r + (int)gridDim.x < rows && tid * 32 < s_kv && nsweeps == 1) {
-            const float* nx = scores + (long long)(r + (int)gridDim.x) * GROUP * score_stride + tid * 32;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(nx));
-            if (GROUP == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + score_stride));
-        }
 
         // ---- three radix passes: prefix = the bits of the threshold key found so far
         uint32_t prefix = 0, k = (uint32_t)topk, n_sel = 0;
@@ -259,21 +270,36 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
                 // every key takes part (non-candidates fall into bins 0-3, which find_bin ignores)
 #pragma unroll 1
                 for (int sw = 0; sw < nsweeps; ++sw) {
-                    load_keys<GROUP>(row0, row1, sw, s_kv, len, key);
+                    load_keys<GROUP>(row0, row1, sw, len, key);
+                    const int live = live_chunks(sw, len);
 #pragma unroll
-                    for (int i = 0; i < kKpt; ++i) atomicAdd(&sm.hist[key[i] >> 21], 1u);
+                    for (int c = 0; c < kChunks; ++c) {
+                        if (c >= live) break;
+#pragma unroll
+                        for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[key[i] >> 21], 1u);
+                    }
                 }
             } else {
                 // keys outside the prefix add to a per-lane spare bin: no branch, no bank conflict
 #pragma unroll 1
                 for (int sw = 0; sw < nsweeps; ++sw) {
-                    if (nsweeps > 1) load_keys<GROUP>(row0, row1, sw, s_kv, len, key);
+                    if (nsweeps > 1) load_keys<GROUP>(row0, row1, sw, len, key);
                     // distance from the first key of the prefix: inside the prefix it is below 2^hi and its top
                     // bits are the digit; everything else (wrapped or large) is clamped onto the spare bins
                     const uint32_t first = prefix << hi, spare = (uint32_t)((kBins >> (pass - 1)) + lane);   // 2048 / 1024 digits
+                    const int live = live_chunks(sw, len);
 #pragma unroll
-                    for (int i = 0; i < kKpt; ++i) atomicAdd(&sm.hist[min((key[i] - first) >> lo, spare)], 1u);
+                    for (int c = 0; c < kChunks; ++c) {
+                        if (c >= live) break;
+#pragma unroll
+                        for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[min((key[i] - first) >> lo, spare)], 1u);
+                    }
                 }
+            }
+            if (pass == 0 && next < rows && next_len <= kSweep && tid * 32 < next_len) {
+                const float* nx = scores + (long long)next * GROUP * score_stride + tid * 32;
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx));
+                if (GROUP == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + score_stride));
             }
             __syncthreads();
             uint32_t k_now;
@@ -282,6 +308,10 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
             if (total == 0u || k_now == 0u) { n_sel = 0; break; }
             prefix = pass == 0 ? sm.sel_bin : ((prefix << (hi - lo)) | sm.sel_bin);
             k = k_now - sm.sel_above;                // rank inside the chosen bin, 1-based
+            if (k == sm.sel_count) {                 // the whole bin is taken: its first key is a threshold as good as any in it
+                prefix <<= lo;
+                break;
+            }
         }
         // all threads agree on n_sel (computed from shared totals); prefix is now the full threshold key
         const uint32_t thr = prefix, need_eq = k;    // take `need_eq` keys equal to thr, smallest index first
@@ -296,9 +326,9 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
             uint32_t base_gt = 0, base_eq = 0;
 #pragma unroll 1
             for (int sw = 0; sw < nsweeps; ++sw) {
-                if (nsweeps > 1) load_keys<GROUP>(row0, row1, sw, s_kv, len, key);
-                if (!ties) emit_sweep<false, STAGED>(sm, key, thr, need_eq, out, off, sw, base_gt, base_eq);
-                else emit_sweep<true, STAGED>(sm, key, thr, need_eq, out, off, sw, base_gt, base_eq);
+                if (nsweeps > 1) load_keys<GROUP>(row0, row1, sw, len, key);
+                if (!ties) emit_sweep<false, STAGED>(sm, key, thr, need_eq, out, off, sw, live_chunks(sw, len), base_gt, base_eq);
+                else emit_sweep<true, STAGED>(sm, key, thr, need_eq, out, off, sw, live_chunks(sw, len), base_gt, base_eq);
             }
         }
         if (STAGED) {                                // topk <= kStage: positions were staged in shared memory
