@@ -287,12 +287,20 @@ std::tuple<at::Tensor, at::Tensor, OptTensor, OptTensor> decode_fwd_whole(
                        extra_kv, extra_indices, extra_topk_length, d_qk, d_v, sm_scale, w1, w2, true);
 }
 
-// Launches of the pack and selection kernels for mxdsa_b200.quantize and mxdsa_b200.indexer, which check the arguments:
-// a small call is bound by its host side, and building the parameters here instead of with ctypes takes most of it away
-// (64 pages of 64 rows: 15.6 us through ctypes, 8.7 us here).
-at::Tensor pack_q_rows(const at::Tensor& src, bool paired_storage) {
+// The pack operators of mxdsa_b200.quantize, and the launch of the selection kernel for mxdsa_b200.indexer (which checks the
+// arguments).  A small call is bound by its host side: 64 pages of 64 rows took 15.6 us with the parameters built by
+// ctypes, 8.9 us with them built here, 5.4 us with the checks and the result's shape here too.
+at::Tensor pack_source(const at::Tensor& t, const char* name) {
+    TORCH_CHECK(t.is_cuda(), name, " must be on CUDA");
+    TORCH_CHECK(t.scalar_type() == at::kBFloat16 || t.scalar_type() == at::kFloat, name, " must be bf16 or fp32");
+    TORCH_CHECK(t.dim() >= 2 && t.size(-1) == kDim, name, " must have a last dimension of ", kDim);
+    return t.contiguous();
+}
+
+at::Tensor pack_q_rows(const at::Tensor& q, bool paired_storage) {
+    const at::Tensor src = pack_source(q, "q");
     c10::cuda::CUDAGuard guard(src.device());
-    std::vector<int64_t> shape = src.sizes().vec();
+    c10::DimVector shape(src.sizes());
     shape.back() = kRow;
     at::Tensor out = at::empty(shape, src.options().dtype(at::kByte));
     mxdsa_pack_q_params p{};
@@ -308,9 +316,10 @@ at::Tensor pack_q_rows(const at::Tensor& src, bool paired_storage) {
     return out;
 }
 
-at::Tensor pack_kv_rows(const at::Tensor& src, int64_t pages, int64_t rows_per_page) {
+at::Tensor pack_kv_rows(const at::Tensor& kv, int64_t pages, int64_t rows_per_page, at::IntArrayRef shape) {
+    const at::Tensor src = pack_source(kv, "kv");
     c10::cuda::CUDAGuard guard(src.device());
-    at::Tensor out = at::empty({pages, rows_per_page * kRow}, src.options().dtype(at::kByte));
+    at::Tensor out = at::empty(shape, src.options().dtype(at::kByte));
     mxdsa_pack_kv_params p{};
     p.rows = pages * rows_per_page;
     p.src = src.data_ptr();
@@ -322,6 +331,14 @@ at::Tensor pack_kv_rows(const at::Tensor& src, int64_t pages, int64_t rows_per_p
     p.stream = at::cuda::getCurrentCUDAStream().stream();
     if (p.rows > 0) require_status(mxdsa_pack_kv(&p), "mxdsa_pack_kv");
     return out;
+}
+at::Tensor pack_prefill_kv(const at::Tensor& kv) {
+    TORCH_CHECK(kv.dim() == 3 && kv.size(1) == 1, "kv must have shape [s_kv, 1, 512]");
+    return pack_kv_rows(kv, 1, kv.size(0), {kv.size(0), 1, kRow});
+}
+at::Tensor pack_decode_kv_pages(const at::Tensor& kv) {
+    TORCH_CHECK(kv.dim() == 4 && kv.size(2) == 1, "kv must have shape [pages, page_size, 1, 512]");
+    return pack_kv_rows(kv, kv.size(0), kv.size(1), {kv.size(0), kv.size(1), 1, kRow});
 }
 
 std::tuple<at::Tensor, at::Tensor> topk_rows(const at::Tensor& scores, int64_t topk, const OptTensor& lengths, int64_t group,
@@ -359,7 +376,8 @@ static void define_module(pybind11::module_& m) {
     m.def("dual_mxfp8_sparse_decode_fwd", &decode_fwd);
     m.def("dual_mxfp8_sparse_decode_fwd_whole", &decode_fwd_whole);
     m.def("pack_q_rows", &pack_q_rows);
-    m.def("pack_kv_rows", &pack_kv_rows);
+    m.def("pack_prefill_kv", &pack_prefill_kv);
+    m.def("pack_decode_kv_pages", &pack_decode_kv_pages);
     m.def("topk_rows", &topk_rows);
     m.def("device_fault", &device_fault);
 }

@@ -15,6 +15,17 @@ from typing import Optional, Tuple
 import torch
 
 
+_module = None
+
+
+def _ext():
+    global _module
+    if _module is None:
+        from . import ext      # the package binds it after this module may have been imported
+        _module = ext()
+    return _module
+
+
 def _score_rows(scores: torch.Tensor) -> torch.Tensor:
     """`scores` [n, s_kv] with the strides that the kernel is to read it by.  It takes a row stride of 0 for s_kv, so a
     row that is broadcast over n is copied out; the stride of a single row means nothing and is set to s_kv."""
@@ -55,5 +66,4 @@ def select_topk_indices(scores: torch.Tensor, topk: int, lengths: Optional[torch
         return t.contiguous()
 
     lengths, row_offset = opt(lengths, "lengths"), opt(row_offset, "row_offset")
-    from . import ext
-    return ext().topk_rows(scores, topk, lengths, group, row_offset)
+    return _ext().topk_rows(scores, topk, lengths, group, row_offset)

@@ -11,44 +11,30 @@ from __future__ import annotations
 
 import torch
 
-D = 512
-ROW = 528
-
-
-def _src(t: torch.Tensor, name: str) -> torch.Tensor:
-    if not t.is_cuda:
-        raise RuntimeError(f"{name} must be on CUDA")
-    if t.dtype not in (torch.bfloat16, torch.float32):
-        raise RuntimeError(f"{name} must be bf16 or fp32")
-    if t.dim() < 2 or t.size(-1) != D:
-        raise RuntimeError(f"{name} must have a last dimension of {D}")
-    return t.contiguous()
+_module = None
 
 
 def _ext():
-    from . import ext      # the package binds it after this module may have been imported
-    return ext()
+    global _module
+    if _module is None:
+        from . import ext      # the package binds it after this module may have been imported
+        _module = ext()
+    return _module
 
 
 def pack_dual_q64(q: torch.Tensor, paired_storage: bool = False) -> torch.Tensor:
     """q [..., 64, 512] -> u8 [..., 64, 528]: 512 E4M3 bytes + 8 UE8M0 scale bytes stored twice; scale g is
     shared by dims [32g,32g+32) and [256+32g,256+32g+32) (reference pack_dual_q64)."""
-    return _ext().pack_q_rows(_src(q, "q"), bool(paired_storage))
+    return _ext().pack_q_rows(q, bool(paired_storage))
 
 
 def pack_dual_prefill_kv64(kv: torch.Tensor) -> torch.Tensor:
     """kv [s_kv, 1, 512] -> u8 [s_kv, 1, 528] view of one flat buffer: all data rows, then all 16-byte scale
     slots; scale g covers dims [64g,64g+64) (reference pack_dual_prefill_kv64)."""
-    if kv.dim() != 3 or kv.size(1) != 1:
-        raise RuntimeError("kv must have shape [s_kv, 1, 512]")
-    n = kv.size(0)
-    return _ext().pack_kv_rows(_src(kv, "kv"), 1, n).view(n, 1, ROW)
+    return _ext().pack_prefill_kv(kv)
 
 
 def pack_dual_decode_kv_pages(kv: torch.Tensor) -> torch.Tensor:
     """kv [pages, page_size, 1, 512] -> u8 [pages, page_size, 1, 528]: per page, page_size*512 data bytes and
     then page_size 16-byte scale slots (reference pack_dual_decode_kv_pages)."""
-    if kv.dim() != 4 or kv.size(2) != 1:
-        raise RuntimeError("kv must have shape [pages, page_size, 1, 512]")
-    pages, psz = kv.size(0), kv.size(1)
-    return _ext().pack_kv_rows(_src(kv, "kv"), pages, psz).view(pages, psz, 1, ROW)
+    return _ext().pack_decode_kv_pages(kv)
