@@ -48,7 +48,10 @@
 // and a rescale 1 250 more; now 2 400 and none.  Per pass, that form / now, timed in turn: 256 tokens at topk 128 14.1 /
 // 12.9 us, decode of 64 requests at 640 keys 46.6 / 44.2, of 128 requests at 4224 keys 354 / 336, of 37 requests of two
 // tokens 22.7 / 21.6; prefill of 4 096 tokens at topk 2048 unchanged (672 / 680): there the chip is at its power limit
-// (990 W, 1 590 of 1 965 MHz), fewer cycles buy a lower clock.
+// (990 W, 1 590 of 1 965 MHz), fewer cycles buy a lower clock.  For the same reason an instruction counts wherever it is:
+// key positions that advance by addition, groups that visit their own tiles alone, rings indexed by a power of two and the
+// row sums rescaled only where a maximum moved took another 3 to 5 % off prefill (65 536 tokens at topk 4096 20.4 / 19.4 ms,
+// 4 096 tokens at topk 2048 688 / 659 us) and 2.7 % off decode of 64 requests (43.8 / 42.6 us).
 //
 // Numerical contract (identical to the reference kernels, reference file:line in brackets)
 //   * keys are consumed in numerical tiles of NT = 128 (prefill, topk >= 512) or 64 keys
@@ -113,7 +116,8 @@ static constexpr int G = kGroups * kGroupWarps / 4;   // softmax warps in fours:
 static constexpr int kThreads = 32 * (12 + 4 * G + 4);   // warps 0-11: K producers, V producers, control; then softmax; then four epilogue warps
 static constexpr int kLaunchRegs = 64;     // registers per thread of the launch: 65536 / kThreads
 static constexpr uint32_t kBarTmem = 7;    // named barrier: tensor memory allocated (warp 10 -> warps 12-15)
-static constexpr int kMRing = 6;         // ring of running maxima by tile, see the epilogue warps
+static constexpr int kMRing = 4;         // ring of running maxima by tile
+static_assert(kMRing > kSBufs && kMRing == kScStages, "a maximum is overwritten kMRing tiles later, see the softmax warps");
 
 // tensor-memory columns
 static constexpr uint32_t kColO = 0;      // 256 columns
@@ -313,50 +317,118 @@ template <bool DECODE> struct WorkIter {
 };
 
 
-// Position in the sequence of 128-key tiles that a CTA pair walks: work item after work item.
-template <bool DECODE, int NT> struct TileCursor {
-    WorkIter<DECODE> it;
-    WorkItem w;
-    int t, ntiles;
-    bool live;
-    __device__ TileCursor(const AttnParams& params) : it(params), t(0), ntiles(0) { live = fetch(); }
-    __device__ bool fetch() {
-        while (it.template next<NT>(w)) {
-            ntiles = (w.blk_end - w.blk_begin + 1) / 2;
-            if (ntiles > 0) {   // empty items are never produced by the scheduler; skipping keeps the roles in step
-                t = 0;
-                return true;
-            }
-        }
-        return false;
-    }
-    __device__ void advance() {
-        if (++t >= ntiles) live = fetch();
-    }
-};
-
-// Key at position `j` (0..63) of 64-key block `blk` of a work item, in two steps so that callers can
-// keep the index load and the loads that depend on it in flight for different tiles.
-// Step 1: the raw index (-1 when the position does not exist, or nothing `exists`).  The load is predicated by hand: as a
-// conditional expression it became a load, a wait for it and a selection, which held the copying warps for its latency.
+// The raw index at `at`, -1 where nothing `exists`.  The load is predicated by hand: as a conditional expression it became
+// a load, a wait for it and a selection, which held the copying warps for its latency.
 __device__ __forceinline__ int load_index_if(bool exists, const int* at) {
     int v = -1;
     asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, 0;\n@p ld.global.nc.s32 %0, [%2];\n}"
                  : "+r"(v) : "r"((uint32_t)exists), "l"(at));
     return v;
 }
-template <bool DECODE>
-__device__ __forceinline__ int key_index(const AttnParams& p, const WorkItem& w, bool exists, int blk, int j) {
-    exists = exists && blk < w.blk_end;
-    if constexpr (!DECODE) {
-        const int pos = blk * 64 + j;
-        return load_index_if(exists && pos < p.topk, w.row + pos);
-    } else {
-        const bool extra = blk >= w.n_main_blocks;
-        const int pos = (extra ? blk - w.n_main_blocks : blk) * 64 + j;
-        return load_index_if(exists && pos < (extra ? p.extra_topk : p.topk), (extra ? w.erow : w.row) + pos);
+static constexpr uint32_t kNoRow = 0xffffffffu;
+// One lane's key through the sequence of 128-key tiles that a CTA pair walks, work item after work item: the lane looks
+// after position `key` of every tile.  What depends on the list that the position lies in (main or extra) is worked out
+// where the list changes, not per tile.
+template <bool DECODE, int NT> struct KeyWalk {
+    const AttnParams& p;
+    WorkIter<DECODE> it;
+    WorkItem w;
+    const int key;
+    int left;                    // tiles of the work item from the current one on
+    bool live;
+    int v;                       // position, counted through the item's 64-key blocks, main blocks first
+    const int* at;               // at[v] is the raw index ...
+    int v_exists, v_attended;    // ... which exists below, and is attended below
+    // decode: the store of the current list
+    bool extra;
+    uint32_t pool, gap, page_size;
+    int page_shift;
+    const uint8_t* base;
+
+    __device__ KeyWalk(const AttnParams& params, int k) : p(params), it(params), key(k) { live = fetch(); }
+    __device__ bool fetch() {
+        while (it.template next<NT>(w)) {
+            left = (w.blk_end - w.blk_begin + 1) / 2;
+            if (left > 0) {      // empty items are never produced by the scheduler; skipping keeps the roles in step
+                v = w.blk_begin * 64 + key;
+                at = w.row;
+                v_exists = min(w.blk_end * 64, p.topk);
+                v_attended = w.len;
+                if constexpr (DECODE) {
+                    v_exists = min(v_exists, w.n_main_blocks * 64);
+                    extra = false;
+                    pool = p.pool_rows32;
+                    gap = p.row_gap;
+                    page_size = p.page_size;
+                    page_shift = p.page_shift;
+                    base = p.kv;
+                    change_list();
+                }
+                return true;
+            }
+        }
+        return false;
     }
-}
+    __device__ __forceinline__ void change_list() {
+        const int first = w.n_main_blocks * 64;
+        if (!extra && v >= first) {
+            extra = true;
+            at = w.erow - first;
+            v_exists = min(w.blk_end * 64, first + p.extra_topk);
+            v_attended = first + w.elen;
+            pool = p.extra_pool_rows32;
+            gap = p.extra_row_gap;
+            page_size = p.extra_page_size;
+            page_shift = p.extra_page_shift;
+            base = p.extra_kv;
+        }
+    }
+    __device__ __forceinline__ void advance() {
+        if (--left == 0) live = fetch();
+        else {
+            v += kTileKeys;
+            if constexpr (DECODE) change_list();
+        }
+    }
+    __device__ __forceinline__ int index() const { return load_index_if(live && v < v_exists, at + v); }
+    // The coordinate of the key with raw index `idx` in the view of its store as rows of 512 bytes (kNoRow = no row: the
+    // operand rows are zero-filled) and whether the key is attended.  An index outside the store (stale or corrupt) is
+    // treated like -1: not attended, nothing dereferenced (one unsigned compare: a negative index is a huge unsigned one).
+    __device__ __forceinline__ uint32_t row(int idx, bool& attended) const {
+        if constexpr (!DECODE) {
+            const bool there = (uint32_t)idx < (uint32_t)p.s_kv;
+            attended = there && v < v_attended;
+            return there ? (uint32_t)idx : kNoRow;
+        } else {
+            attended = (uint32_t)idx < pool && v < v_attended;
+            // row = page * rows_per_block + slot in page = idx + page * (rows_per_block - page_size)
+            return attended ? (uint32_t)idx + page(idx) * gap : kNoRow;
+        }
+    }
+    __device__ __forceinline__ uint32_t page(int idx) const {   // pages are powers of two as a rule: no division then
+        return __builtin_expect(page_shift >= 0, 1) ? (uint32_t)idx >> page_shift : (uint32_t)idx / page_size;
+    }
+    // the 16-byte scale slot of a key that has a row
+    __device__ __forceinline__ const uint8_t* slot(int idx, uint32_t r) const {
+        if constexpr (!DECODE) return p.kv_scales + (unsigned long long)r * 16;
+        else {   // behind the data rows of the page, whose first row is r - in_page
+            const uint32_t in_page = (uint32_t)idx - page(idx) * page_size;
+            return base + (unsigned long long)(r - in_page + page_size) * kDim + in_page * 16;
+        }
+    }
+    // base of the store, the same for all lanes whose keys lie in half `h` of the tile
+    __device__ __forceinline__ const uint8_t* store(int h) const {
+        if constexpr (!DECODE) return p.kv;
+        else return v - key + 64 * h >= w.n_main_blocks * 64 && p.extra_topk > 0 ? p.extra_kv : p.kv;
+    }
+    // the tensor map over it, for lanes whose own key lies in the same half
+    __device__ __forceinline__ const void* map(const TensorMaps& maps) const {
+        if constexpr (!DECODE) return &maps.kv;
+        // without an extra pool there is no second map: positions past the main list have no row anyway
+        else return extra && p.extra_topk > 0 ? &maps.ekv : &maps.kv;
+    }
+};
+
 // Ask for the index lines of the two 64-key blocks blk, blk + 1 into L2: lane 0..3 takes 128-byte line lane % 2 of
 // block blk + lane / 2 (nothing where the block or the position does not exist).
 template <bool DECODE>
@@ -372,69 +444,6 @@ __device__ __forceinline__ void prefetch_index_lines(const AttnParams& p, const 
         if (pos < (extra ? p.extra_topk : p.topk)) prefetch_l2((extra ? w.erow : w.row) + pos);
     }
 }
-// Step 2: is the key attended, where is its 16-byte scale slot, and -- returned -- the coordinate of its data in the view
-// of the KV store as rows of 512 bytes (kNoRow = no row: the operand rows are zero-filled, the slot is null).
-static constexpr uint32_t kNoRow = 0xffffffffu;
-template <bool DECODE>
-__device__ __forceinline__ uint32_t key_resolve(const AttnParams& p, const WorkItem& w, int blk, int j, int idx, bool& valid,
-                                                const uint8_t*& slot) {
-    valid = false;
-    slot = nullptr;
-    if (blk >= w.blk_end) return kNoRow;
-    if constexpr (!DECODE) {
-        const int pos = blk * 64 + j;
-        if (idx < 0 || idx >= p.s_kv) return kNoRow;
-        valid = pos < w.len;
-        slot = p.kv_scales + (long long)idx * 16;
-        return (uint32_t)idx;
-    } else {
-        const bool extra = blk >= w.n_main_blocks;
-        const int pos = (extra ? blk - w.n_main_blocks : blk) * 64 + j;
-        // an index outside the pool (stale or corrupt) is treated like -1: not attended, nothing dereferenced
-        // (one unsigned compare: a negative index is a huge unsigned one)
-        valid = (unsigned)idx < (extra ? p.extra_pool_rows32 : p.pool_rows32) && pos < (extra ? w.elen : w.len);
-        if (!valid) return kNoRow;
-        const unsigned psz = extra ? p.extra_page_size : p.page_size;
-        const int sh = extra ? p.extra_page_shift : p.page_shift;   // pages are powers of two as a rule: no division then
-        const unsigned page = __builtin_expect(sh >= 0, 1) ? (unsigned)idx >> sh : (unsigned)idx / psz;
-        const unsigned in_page = (unsigned)idx - page * psz;
-        slot = (extra ? p.extra_kv : p.kv) + (long long)page * (extra ? p.extra_stride_block : p.stride_block) + psz * kDim + in_page * 16;
-        return (unsigned)idx + page * (extra ? p.extra_row_gap : p.row_gap);
-    }
-}
-// Base of the store that the rows of 64-key block `blk` come from.
-template <bool DECODE>
-__device__ __forceinline__ const uint8_t* key_store(const AttnParams& p, const WorkItem& w, int blk) {
-    if constexpr (!DECODE) return p.kv;
-    else return (blk >= w.n_main_blocks && p.extra_topk > 0) ? p.extra_kv : p.kv;
-}
-// Row coordinate of one key in the 2-D view {512 B, rows} of its KV store (-1 = no row: the copy engine fills
-// zeros), from the key's raw index.
-template <bool DECODE>
-__device__ __forceinline__ int key_row(const AttnParams& p, const WorkItem& w, int blk, int j, int idx) {
-    if (blk >= w.blk_end) return -1;
-    if constexpr (!DECODE) {
-        return (idx >= 0 && idx < p.s_kv) ? idx : -1;
-    } else {
-        const bool extra = blk >= w.n_main_blocks;
-        const int pos = (extra ? blk - w.n_main_blocks : blk) * 64 + j;
-        if ((unsigned)idx >= (extra ? p.extra_pool_rows32 : p.pool_rows32) || pos >= (extra ? w.elen : w.len)) return -1;
-        // row = page * rows_per_block + slot in page = idx + page * (rows_per_block - page_size)
-        const int sh = extra ? p.extra_page_shift : p.page_shift;
-        const unsigned gap = extra ? p.extra_row_gap : p.row_gap;
-        const unsigned page = __builtin_expect(sh >= 0, 1) ? (unsigned)idx >> sh
-                                                           : (unsigned)idx / (unsigned)(extra ? p.extra_page_size : p.page_size);
-        return (int)((unsigned)idx + page * gap);
-    }
-}
-// The tensor map that the rows of 64-key block `blk` are gathered through.
-template <bool DECODE>
-__device__ __forceinline__ const void* key_map(const AttnParams& p, const TensorMaps& maps, const WorkItem& w, int blk) {
-    if constexpr (!DECODE) return &maps.kv;
-    // without an extra pool there is no second map: positions past the main list have no row anyway
-    else return (blk >= w.n_main_blocks && p.extra_topk > 0) ? &maps.ekv : &maps.kv;
-}
-
 // packed fp32 pairs (one instruction for two lanes of data)
 __device__ __forceinline__ float2 f2_fma(float2 a, float2 b, float2 c) {
     float2 d;
@@ -654,7 +663,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     // to launch unless the compiled kernel really has kLaunchRegs registers.  The copy and control warps hand
     // most of theirs back so that the softmax warps (32 logits per thread in registers) work without spilling.
     // Each setmaxnreg is executed by the four warps of one aligned warp group with the same value.
-    constexpr int kRegsCopy = 48, kRegsGather = 32, kRegsCtl = 48, kRegsEpi = 96, kRegsSoftmax = 72;
+    constexpr int kRegsCopy = DECODE ? 48 : 40, kRegsGather = 40, kRegsCtl = DECODE ? 40 : 48, kRegsEpi = 96, kRegsSoftmax = 72;
     static_assert(4 * 32 * (kRegsCopy + kRegsGather + kRegsCtl + kRegsEpi) + kGroups * kGroupWarps * 32 * kRegsSoftmax <= kThreads * kLaunchRegs,
                   "register budget must fit in the launch allocation");
     if (warp < 8) {
@@ -669,23 +678,23 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             // issues in order, so an address computed at load time would hold the warp until the load is back.
             const int pw = warp;
             const int key = lane < 16 ? 64 * (int)cta + 16 * pw + lane : 64 * (1 - (int)cta) + 16 * pw + (lane - 16);
-            TileCursor<DECODE, NT> ck(p);
+            KeyWalk<DECODE, NT> ck(p, key);
             uint32_t kt = 0;
-            int idx = key_index<DECODE>(p, ck.w, ck.live, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64);
+            int idx = ck.index();
             // row 16 pw of chunk lane/8, 16-byte column lane%8; bits 4-6 are free for the swizzle's exclusive or
             const uint32_t k_dst0 = smem_u32(sm.kv[0]) + (lane / 8) * 8192 + 16 * pw * 128 + (lane & 7) * 16;
+            const uint32_t k_sf0 = smem_u32(&sm.k_sf[0][((key >> 6) * 32 + (key & 31)) * 4 + ((key >> 5) & 1)]);
             // Where the key's row and scale slot are is worked out as soon as the tile's index is back, before the
             // wait for a free stage: the wait then covers what is left of the index load's latency.
-            uint32_t krow = kNoRow;
+            uint32_t krow = kNoRow, vbits = 0;
             const uint8_t* src0 = p.kv;      // lane's column of row 0 of the store that this warp's rows come from
-            const uint8_t* slot = nullptr;
-            uint32_t vbits = 0;
+            const uint8_t* slot = p.kv;
             auto resolve_tile = [&]() {
-                bool valid;
-                const int blk = ck.w.blk_begin + 2 * ck.t;
-                krow = key_resolve<DECODE>(p, ck.w, blk + key / 64, key % 64, idx, valid, slot);
-                src0 = key_store<DECODE>(p, ck.w, blk + (int)cta) + lane * 16;
-                vbits = __ballot_sync(0xffffffffu, valid);
+                bool attended;
+                krow = ck.row(idx, attended);
+                slot = krow != kNoRow ? ck.slot(idx, krow) : p.kv;
+                src0 = ck.store((int)cta) + lane * 16;
+                vbits = __ballot_sync(0xffffffffu, attended);
             };
             if (ck.live) resolve_tile();
             cluster_wait();
@@ -700,12 +709,12 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 // warp ask for the 512 bytes that a tile further on will need, so that the index loads of all three
                 // roles that read them (these warps, the V producers, the stager) come back from L2, not from HBM.
                 if constexpr (MXDSA_INDEX_AHEAD > 0) {
-                    if (pw == 0 && cta == 0 && lane < 4 && ck.t + MXDSA_INDEX_AHEAD < ck.ntiles)
-                        prefetch_index_lines<DECODE>(p, ck.w, ck.w.blk_begin + 2 * (ck.t + MXDSA_INDEX_AHEAD), lane);
+                    if (pw == 0 && cta == 0 && lane < 4 && ck.left > MXDSA_INDEX_AHEAD)
+                        prefetch_index_lines<DECODE>(p, ck.w, (ck.v - key) / 64 + 2 * MXDSA_INDEX_AHEAD, lane);
                 }
                 // the next tile's indices: the loads run while this tile's rows are issued
                 ck.advance();
-                idx = key_index<DECODE>(p, ck.w, ck.live, ck.w.blk_begin + 2 * ck.t + key / 64, key % 64);
+                idx = ck.index();
                 // Four instructions a row: the coordinate by shuffle, one multiply-add to its address, one exclusive or
                 // for the swizzle, the copy.
                 const uint32_t dst = k_dst0 + s * 32768;
@@ -723,9 +732,9 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 // the key's 8 scale bytes go straight into the row layout that tcgen05.cp wants: row (key/64)*32 +
                 // key%32 holds {bytes0-3[k], bytes0-3[k+32], bytes4-7[k], bytes4-7[k+32]} of keys k and k+32
                 {
-                    const uint32_t sf = smem_u32(&sm.k_sf[s][((key >> 6) * 32 + (key & 31)) * 4 + ((key >> 5) & 1)]);
-                    cp_async4(sf, slot ? slot : p.kv, slot ? 4u : 0u);
-                    cp_async4(sf + 8, slot ? slot + 4 : p.kv, slot ? 4u : 0u);
+                    const uint32_t bytes = krow != kNoRow ? 4u : 0u;
+                    cp_async4(k_sf0 + s * 1024, slot, bytes);
+                    cp_async4(k_sf0 + s * 1024 + 8, slot + 4, bytes);
                 }
                 cp_async_arrive(smem_u32(&sm.bar_k_landed[s]));
                 if (lane == 0) {   // validity of the warp's 32 keys: a plain store, released by a plain arrival
@@ -748,48 +757,46 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             // 65 536 tokens at topk 4096 21.9 -> 21.0 ms, both trees timed in turn; decode of 128 requests at 4224 keys 386 ->
             // 370 us, within the spread of either's runs.
             // Lanes 0-7 of every warp request four keys x 128 bytes each (measured: the copy engine takes requests
-            // fastest from a few lanes of several warps).  Rows that do not exist (index -1, position beyond the list,
+            // fastest from a few lanes of several warps; sixteen lanes of two warps made decode of 128 requests 18 % slower).  Rows that do not exist (index -1, position beyond the list,
             // row outside the store) get a coordinate outside the tensor map, which the copy engine fills with zeros.
             // The bytes of both CTAs complete on ONE barrier of CTA 0, where the PV issuer waits; nothing else needs
             // to know that V has landed.  Every lane turns one index into a row coordinate, ahead of the wait for
             // "QK done", and the index load it needs is issued before the requests of the tile before it.
             const int pw = warp - 4;
             const int other = 1 - (int)cta;              // the 64-key half of a tile that the peer CTA holds
-            const int jl = 16 * pw + (lane & 15);        // the key of that half whose row this lane works out
-            TileCursor<DECODE, NT> cv(p);
+            KeyWalk<DECODE, NT> cv(p, 64 * other + 16 * pw + (lane & 15));
             uint32_t vt = 0;
             const uint32_t v_full0 = map_to_cta(smem_u32(&sm.bar_v_full[0]), 0);
             const int col = 256 * (int)cta + 128 * (lane & 1);
-            const uint32_t v_dst0 = smem_u32(sm.kv[0]) + (2 * other + (lane & 1)) * 8192 + (16 * pw + 4 * ((lane >> 1) & 3)) * 128;
+            const int quad = (lane >> 1) & 3;
+            const uint32_t v_dst0 = smem_u32(sm.kv[0]) + (2 * other + (lane & 1)) * 8192 + (16 * pw + 4 * quad) * 128;
             int row = -1;
             const void* map = &maps.kv;
             auto locate = [&](int idx) {
-                const int blk = cv.w.blk_begin + 2 * cv.t + other;
-                row = key_row<DECODE>(p, cv.w, blk, jl, idx);
-                map = key_map<DECODE>(p, maps, cv.w, blk);
+                bool attended;
+                row = (int)cv.row(idx, attended);
+                map = cv.map(maps);
             };
-            bool live = cv.live;
-            if (live) locate(key_index<DECODE>(p, cv.w, true, cv.w.blk_begin + 2 * cv.t + other, jl));
+            if (cv.live) locate(cv.index());
             cluster_wait();
 #pragma unroll 1
-            while (live) {
+            while (cv.live) {
                 const uint32_t s = vt % kStages;
                 const void* map_cur = map;
                 int r[4];
 #pragma unroll
-                for (int i = 0; i < 4; ++i) r[i] = __shfl_sync(0xffffffffu, row, 4 * ((lane >> 1) & 3) + i);
+                for (int i = 0; i < 4; ++i) r[i] = __shfl_sync(0xffffffffu, row, 4 * quad + i);
                 cv.advance();
-                live = cv.live;
-                const int idx = key_index<DECODE>(p, cv.w, live, cv.w.blk_begin + 2 * cv.t + other, jl);
+                const int idx = cv.index();
                 // the half that is about to be overwritten has been read once the tile's QK is done
-                MXDSA_WAIT(sm.bar_qk_done[vt % kScStages], (vt / kScStages) & 1, 11);
+                MXDSA_WAIT(sm.bar_qk_done[s], (vt / kScStages) & 1, 11);
                 if (lane == 0) mbar_expect_tx_cluster(v_full0 + s * 8, 16 * 256);
                 __syncwarp();
                 if (lane < 8)
                     tma_gather4_pair(v_dst0 + s * 32768, map_cur, col, r[0], r[1], r[2], r[3], v_full0 + s * 8, MXDSA_V_HINT);
                 __syncwarp();
                 ++vt;
-                if (live) locate(idx);
+                if (cv.live) locate(idx);
             }
         }
     } else if (warp < 12) {
@@ -807,7 +814,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             const uint32_t e = __shfl_sync(0xffffffffu, warp - 8, 0);   // tile parity = P buffer = scale column set
             WorkIter<DECODE> it(p);
             WorkItem w;
-            uint32_t gt = 0, gw = 0;
+            uint32_t gt0 = 0, gw = 0;
             const uint32_t q_empty_peer = map_to_cta(smem_u32(&sm.bar_q_empty), 1);
             const uint64_t a_base = smem_desc(desc_k128, smem_u32(sm.q));
             const uint32_t d_p = tmem + kColP + e * 64, sfa0 = tmem + kColQs + 4 * e, sfb0 = tmem + kColKs + 4 * e;
@@ -822,8 +829,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 MXDSA_WAIT_TIGHT(sm.bar_q_full, gw & 1, 20);
                 bool mine = false;
 #pragma unroll 1
-                for (int t = 0; t < ntiles; ++t, ++gt) {
-                    if ((gt & 1) != e) continue;
+                for (uint32_t t = (gt0 & 1) ^ e; t < (uint32_t)ntiles; t += 2) {
+                    const uint32_t gt = gt0 + t;
                     const uint32_t s = gt % kStages;
                     const uint32_t sc = gt % kScStages, sph = (gt / kScStages) & 1;
                     const uint32_t bph = (gt >> 1) & 1;
@@ -853,6 +860,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     __syncwarp();
                     mine = true;
                 }
+                gt0 += ntiles;
                 // Q may be overwritten once both issuers' QKs of this pair have finished
                 if (elect_one()) {
                     if (mine) {
@@ -1050,30 +1058,30 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
         }
         WorkIter<DECODE> it(p);
         WorkItem w;
-        uint32_t gt = 0, gw = 0;
+        uint32_t gt0 = 0, gw = 0;                // tiles and pairs so far
+        uint32_t b = grp;                        // S buffer of the group's next tile
+        const uint32_t p_addr = lane_addr + kColP + grp * 64 + part * 32;
+        const uint32_t s_dst = swz128(row, qtr * 32);
 #pragma unroll 1
         while (it.template next<NT>(w)) {
-            const int ntiles = (w.blk_end - w.blk_begin + 1) / 2;
-            if (ntiles <= 0) continue;  // never produced by the scheduler; keeps the roles in step
+            const uint32_t ntiles = (uint32_t)max((w.blk_end - w.blk_begin + 1) / 2, 0);
+            if (ntiles == 0) continue;  // never produced by the scheduler; keeps the roles in step
             float m_own = -1e30f;   // running max after this group's latest tile of the pair
             float l = 0.f, real_m = -CUDART_INF_F;
 #pragma unroll 1
-            for (int t = 0; t < ntiles; ++t, ++gt) {
-                if ((int)(gt % kGroups) != grp) continue;
-                const uint32_t sc = gt % kScStages, sph = (gt / kScStages) & 1;
-                const uint32_t pb = gt & 1;                              // P buffer
-                const uint32_t b = gt % kSBufs;                          // S buffer
-                const uint32_t mr = gt % kMRing, mr_prev = (gt + kMRing - 1) % kMRing;
+            for (uint32_t t = (gt0 ^ grp) & 1; t < ntiles; t += kGroups) {
+                const uint32_t gt = gt0 + t, sc = gt % kScStages, sph = (gt / kScStages) & 1;
+                const uint32_t prev = (gt - 1) % kScStages, prev_ph = ((gt - 1) / kScStages) & 1;
                 MXDSA_WAIT_POLL(sm.bar_tok_full[sc], sph, 50);
                 const uint32_t vbits = sm.valid[sc][qtr];
                 MXDSA_WAIT_POLL(sm.bar_qk_done[sc], sph, 51);
                 tc_fence_after();
                 float x[32];
-                tmem_ld32(lane_addr + kColP + pb * 64 + part * 32, reinterpret_cast<uint32_t*>(x));
+                tmem_ld32(p_addr, reinterpret_cast<uint32_t*>(x));
                 tmem_wait_ld();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_cluster(p_empty0 + pb * 8);
+                if (lane == 0) mbar_arrive_cluster(p_empty0 + grp * 8);
                 if (vbits != 0xffffffffu) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) x[i] = ((vbits >> i) & 1u) ? x[i] : -CUDART_INF_F;
@@ -1091,49 +1099,43 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 xm[qtr][row] = own_max;
                 named_bar_sync(1 + grp, 32 * kGroupWarps);
                 const float half0_max = fmaxf(xm[0][row], xm[1][row]), half1_max = fmaxf(xm[2][row], xm[3][row]);
-                // the running maximum handed over by the group before (value ignored on a pair's first
-                // tile, but every phase of that barrier is observed)
-                if (gt > 0) MXDSA_WAIT_POLL(sm.bar_m_ready[mr_prev], ((gt - 1) / kMRing) & 1, 58);
-                const float m_prev = t == 0 ? -1e30f : sm.m_pub[mr_prev][row];
-                const float sprev = (m_own == m_prev) ? 1.f : ex2_approx(m_own - m_prev);
-                // numerical tiles: NT = 128 -> one per tensor-core tile; NT = 64 -> key half 0 then 1
-                float m_used, scale0 = 1.f, scale1 = 1.f;
-                if constexpr (NT == 128) {
-                    const float tmax = fmaxf(half0_max, half1_max);
-                    real_m = fmaxf(real_m, tmax);
-                    const bool grow0 = __any_sync(0xffffffffu, tmax - m_prev > 6.0f);
-                    const float nm = grow0 ? fmaxf(m_prev, tmax) : m_prev;
-                    scale0 = grow0 ? ex2_approx(m_prev - nm) : 1.f;
-                    m_own = nm;
-                    m_used = nm;
-                } else {
-                    const float t0 = half0_max, t1 = half1_max;
-                    real_m = fmaxf(real_m, fmaxf(t0, t1));
-                    const bool grow0 = __any_sync(0xffffffffu, t0 - m_prev > 6.0f);
-                    const float m1 = grow0 ? fmaxf(m_prev, t0) : m_prev;
-                    scale0 = grow0 ? ex2_approx(m_prev - m1) : 1.f;
-                    const bool grow1 = __any_sync(0xffffffffu, t1 - m1 > 6.0f);
-                    const float m2 = grow1 ? fmaxf(m1, t1) : m1;
-                    scale1 = grow1 ? ex2_approx(m1 - m2) : 1.f;
-                    m_used = half == 0 ? m1 : m2;
-                    m_own = m2;
-                    if (qtr == 0) sm.m_mid[mr][row] = m1;
-                }
                 // S buffer b is free once the PV of tile gt - kSBufs has finished (long ago, as a rule).  The wait stands ahead
                 // of the running maximum: with it the epilogue warps are never a whole ring of maxima behind.
                 if (gt >= (uint32_t)kSBufs) {
                     const uint32_t g = gt - kSBufs;
                     MXDSA_WAIT_POLL(sm.bar_pv_done[g % kScStages], (g / kScStages) & 1, 52);
                 }
-                if (qtr == 0) {   // the same value in all four warps of the row
-                    sm.m_pub[mr][row] = m_own;
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(smem_u32(&sm.bar_m_ready[mr]));
+                // the running maximum handed over by the group before (value ignored on a pair's first
+                // tile, but every phase of that barrier is observed)
+                if (gt > 0) MXDSA_WAIT_POLL(sm.bar_m_ready[prev], prev_ph, 58);
+                const float m_prev = t == 0 ? -1e30f : sm.m_pub[prev][row];
+                // numerical tiles: NT = 128 -> one per tensor-core tile; NT = 64 -> key half 0 then 1
+                const float tmax = fmaxf(half0_max, half1_max);
+                real_m = fmaxf(real_m, tmax);
+                float m_mid, m_new;   // the maximum after the first 64-key tile, and after the whole tile
+                if constexpr (NT == 128) {
+                    m_new = __any_sync(0xffffffffu, tmax - m_prev > 6.0f) ? fmaxf(m_prev, tmax) : m_prev;
+                    m_mid = m_new;
+                } else {
+                    m_mid = __any_sync(0xffffffffu, half0_max - m_prev > 6.0f) ? fmaxf(m_prev, half0_max) : m_prev;
+                    m_new = __any_sync(0xffffffffu, half1_max - m_mid > 6.0f) ? fmaxf(m_mid, half1_max) : m_mid;
                 }
+                if (qtr == 0) {   // the same value in all four warps of the row
+                    if (NT == 64) sm.m_mid[sc][row] = m_mid;
+                    sm.m_pub[sc][row] = m_new;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&sm.bar_m_ready[sc]));
+                }
+                // every update of m rescales the partial sum
+                if (__any_sync(0xffffffffu, m_new != m_own)) {
+                    if (m_new != m_own) l *= ex2_approx(m_own - m_new);
+                    m_own = m_new;
+                }
+                const float m_used = half == 0 ? m_mid : m_new;
                 // probabilities, key-scaled, re-quantised per 32 keys and stored
                 const float2 negm2 = make_float2(-m_used, -m_used);
                 const float4* tok4 = reinterpret_cast<const float4*>(&sm.tok_scale[sc][qtr * 32]);
-                uint8_t* srow = sm.s[b];
+                uint8_t* srow = sm.s[b] + s_dst;
                 float2 sum2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
                 float am0 = 0.f, am1 = 0.f;
 #pragma unroll
@@ -1163,29 +1165,28 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     const float2 c = f2_mul(make_float2(x[i + 2], x[i + 3]), mul2);
                     s8[i / 4] = (uint32_t)cvt_e4m3x2(a.x, a.y) | ((uint32_t)cvt_e4m3x2(c.x, c.y) << 16);
                 }
-                *reinterpret_cast<uint4*>(srow + swz128(row, qtr * 32)) = make_uint4(s8[0], s8[1], s8[2], s8[3]);
-                *reinterpret_cast<uint4*>(srow + swz128(row, qtr * 32 + 16)) = make_uint4(s8[4], s8[5], s8[6], s8[7]);
+                // (the second 16 bytes: the swizzle is an exclusive or above bit 4)
+                *reinterpret_cast<uint4*>(srow) = make_uint4(s8[0], s8[1], s8[2], s8[3]);
+                *reinterpret_cast<uint4*>(sm.s[b] + (s_dst ^ 16u)) = make_uint4(s8[4], s8[5], s8[6], s8[7]);
                 // scale rows: row (row%32) and its copy at +32; word row/32; byte qtr
                 reinterpret_cast<uint8_t*>(&sm.s_sf[b][(row % 32) * 4 + row / 32])[qtr] = (uint8_t)e;
                 reinterpret_cast<uint8_t*>(&sm.s_sf[b][(32 + row % 32) * 4 + row / 32])[qtr] = (uint8_t)e;
                 const float2 s2 = f2_add(sum2[0], sum2[1]);
                 const float sum = s2.x + s2.y;
-                // l bookkeeping: every update of m rescales all partial sums of the row
-                if constexpr (NT == 128) {
-                    l = fmaf(l * sprev, scale0, sum);
-                } else {
-                    if (half == 0) l = fmaf(l * sprev, scale0, sum) * scale1;
-                    else l = fmaf(l * sprev * scale0, scale1, sum);
-                }
+                if (NT == 64 && half == 0 && m_mid != m_new) l = fmaf(sum, ex2_approx(m_mid - m_new), l);
+                else l += sum;
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
                     mbar_arrive_cluster(s_full0 + b * 8);
                     mbar_arrive(smem_u32(&sm.bar_tok_empty[sc]));
                 }
+                b += kGroups;
+                if (b >= (uint32_t)kSBufs) b -= kSBufs;
             }
+            gt0 += ntiles;
             // ---------------- end of the pair: final m, the four partial l of each row, drain O
-            const uint32_t last = gt - 1;
+            const uint32_t last = gt0 - 1;
             float m_fin = m_own;
             const int last_grp = (int)(last % kGroups);
             if (last_grp != grp) {
