@@ -14,7 +14,7 @@
 //   holds row L%64, and column half L/64 (P: keys 64*(L/64).., O: dims 256*(L/64)..).
 //
 // Roles (warp-specialised, 32 warps per CTA; the launch gives every thread 64 registers, re-balanced with
-// setmaxnreg to 48 / 32 / 48 / 72 / 96 for the five kinds of warp below)
+// setmaxnreg to 48 / 40 / 40 / 72 / 96 for the five kinds of warp below, in prefill 40 / 40 / 48 / 72 / 96)
 //   warps 0-3   K producers: read key indices one tile ahead and copy the selected rows of this CTA's 64 keys
 //               into the tile ring with 16-byte cp.async; one warp instruction moves one 512-byte row straight
 //               into the 128-byte-swizzled operand layout.  The same warps gather the 8 scale bytes of all 128
@@ -906,6 +906,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     MXDSA_WAIT_TIGHT(sm.bar_s_full[b], bph, 33);
                     // Two steps, each of which waits for its part of O.  128-key tiles: dim chunk 0, then 1, so that one chunk is
                     // rescaled while the other is being accumulated.  64-key tiles: key half 0, then 1, O being rescaled in between.
+                    // A step costs this warp 300 to 400 cycles: with one for 128-key tiles prefill took 1 to 2 % longer, with four
+                    // for 64-key tiles (half x chunk) decode 2 to 10 %.
 #pragma unroll
                     for (int h = 0; h < 2; ++h) {
                         if (t > 0 || (NT == 64 && h == 1)) {
