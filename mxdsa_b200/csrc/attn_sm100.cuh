@@ -565,6 +565,17 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
 #define MXDSA_WAIT_TIGHT(bar, parity, code) MXDSA_WAIT_ADDR_(0, smem_u32(&(bar)), parity, code)
 #define MXDSA_WAIT(bar, parity, code) MXDSA_WAIT_ADDR_(-1, smem_u32(&(bar)), parity, code)
 
+// Behind the softmax warps' exchange barrier.  A named barrier's wait has no limit.  A warp that abandons a wait arrives in
+// the tear-down in its own place, once on each of the two barriers that it takes part in, after the abort word was set; whoever
+// that arrival lets through sees the word here and leaves as well, and nobody comes to an exchange that a warp which has
+// left would be needed for a second time.  A group's barrier needs no look: its next use but one lies behind a wait for
+// what the missing warp would have signalled ("P copied" of its last tile, or "stage read").
+// All lanes read the same word: the warp stays together.
+#define MXDSA_LEAVE_IF_ABORTED()                                  \
+    do {                                                          \
+        if (*(volatile int*)&sm.abort_word != 0) goto done;       \
+    } while (0)
+
 // A wait was abandoned: mark both CTAs of the pair and the device fault record.
 template <typename Plan> __device__ __noinline__ void raise_fault(Plan& sm, int code) {
     sm.abort_word = 1;
@@ -1199,6 +1210,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             sm.xl[grp][qtr][row] = l;
             if (qtr == 0) sm.xr[grp][row] = real_m;   // the same in all four warps of the row
             named_bar_sync(1 + kGroups, kGroups * kGroupWarps * 32);
+            MXDSA_LEAVE_IF_ABORTED();
             float l_tot = 0.f, real_all = 0.f;
             if (warp < 14) {
 #pragma unroll
@@ -1207,6 +1219,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 real_all = fmaxf(sm.xr[0][row], sm.xr[1][row]);
             }
             named_bar_sync(1 + kGroups, kGroups * kGroupWarps * 32);   // everybody has read the exchange area before the next pair writes it
+            MXDSA_LEAVE_IF_ABORTED();
             // The first two warps of group 0 (one thread per row) turn the row sums into what the epilogue warps
             // need, write lse / max_logits, and every softmax warp goes straight on to the next pair: O is drained
             // by warps of its own while the next pair's tiles are worked on.
@@ -1426,9 +1439,9 @@ done:
     // stores still reading this CTA's shared memory must have done so before the CTA may end
     if (warp >= 12 + 4 * G && lane == 0) tma_store_wait_read<0>();
 #endif
-    // After a fault, softmax threads leave at different points; one extra arrival per leaving thread
-    // completes the exchange barrier for those still parked on it (they fail their next wait and
-    // follow).  In a normal exit the arrivals are harmless: nobody waits on that barrier any more.
+    // After a fault the softmax warps leave at different points: each arrives on its group's barrier and on the exchange
+    // barrier in place of the sync that it will not come to, and those parked there follow it, see MXDSA_LEAVE_IF_ABORTED.
+    // In a normal exit the arrivals are harmless: nobody waits on these barriers any more.
     if (warp >= 12 && warp < 12 + 4 * G) {
         named_bar_arrive(1 + (warp - 12) / kGroupWarps, 32 * kGroupWarps);
         named_bar_arrive(1 + kGroups, kGroups * kGroupWarps * 32);
