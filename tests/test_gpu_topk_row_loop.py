@@ -1,0 +1,41 @@
+"""GPU: index selection by counting with more rows than CTAs (two per SM), so that every CTA takes several rows in turn: a
+row's length, its number of sweeps and the chunks that hold keys differ from those of the row before, whose keys are still in
+registers.  Bit for bit against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import mxdsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+def _check(rows_a_cta, s_kv, topk, pair, lengths):
+    """`lengths` are dealt out so that the rows of a CTA (r, r + grid, ...) have different ones, longer and shorter."""
+    from mxdsa_b200.indexer import select_topk_indices
+    grid = 2 * torch.cuda.get_device_properties(0).multi_processor_count
+    rows = (rows_a_cta - 1) * grid + grid // 3
+    r = np.arange(rows)
+    ln = np.array(lengths, np.int32)[(r + 5 * (r // grid)) % len(lengths)]
+    rng = np.random.default_rng(rows + s_kv + topk)
+    s = rng.standard_normal((rows * (2 if pair else 1), s_kv), dtype=np.float32)
+    idx, cnt = select_topk_indices(torch.from_numpy(s).cuda(), topk, torch.from_numpy(ln).cuda(), pair, None)
+    ri, rc = O.topk_select_ref(s, topk, ln, pair, None)
+    assert np.array_equal(cnt.cpu().numpy(), rc) and np.array_equal(idx.cpu().numpy(), ri)
+
+
+# lengths around the chunks of 2 048 keys (14 336: seven of eight), around topk, none at all, the whole row
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("topk", [2048, 4096, 6000])          # the last: written without staging
+def test_rows_of_one_sweep(topk, pair):
+    _check(3, 16384, topk, pair, [16384, 0, topk - 1, 1, 8193, 2047, topk, 2048, 14336, 2049, topk + 1, 14337, 16381])
+
+
+@pytest.mark.parametrize("pair", [False, True])
+def test_short_rows(pair):
+    _check(4, 4100, 300, pair, [4100, 0, 4096, 1, 2048, 299, 2049, 300, 4097, 301])
+
+
+@pytest.mark.parametrize("pair", [False, True])
+def test_rows_of_several_sweeps(pair):                         # lists of more than 4 096 keys are counted whatever the length
+    _check(2, 40000, 5000, pair, [40000, 20, 16384, 32769, 0, 16385, 4999, 32768, 5001, 39999, 18432])
