@@ -29,7 +29,7 @@
 // position; the row is staged in shared memory and written in whole lines.  No sort, no global atomics,
 // deterministic.  A row costs what its own length costs: chunks of 2 048 keys past it are neither loaded nor counted, and
 // the third pass is rarely needed, because the 22-bit bin of the threshold holds one key or two.  Before, every row cost
-// 16 384 keys and three passes: 2 048 pairs of 16 384 keys, half to full length, topk 2048 93.9 -> 73.1 us (the passes alone
+// 16 384 keys and three passes: 2 048 pairs of 16 384 keys, half to full length, topk 2048 93.9 -> 70.5 us (the passes alone
 // 85.4), 1 951 pairs of 3 172 keys 71.7 -> 40.0, 27 pairs of 4 464 keys 8.4 -> 7.8.
 //
 // Bound: HBM on paper (group * s_kv * 4 bytes read + topk * 4 written per row); in practice the integer and
@@ -77,6 +77,24 @@ __device__ __forceinline__ uint32_t score_key(float s) {
 // keys stops at live_chunks(), which is the same for all threads.
 __device__ __forceinline__ int live_chunks(int sweep, int len) {
     return min((len - sweep * kSweep + kThreads * 4 - 1) / (kThreads * 4), kChunks);
+}
+// f(c) for the chunks of a sweep that hold keys; STRAIGHT: in one straight line where that is all eight.  A branch per chunk
+// keeps the work of one from overlapping the next's, which shows where a CTA has its SM to itself; more code shows too, in short
+// rows.  So the histogram passes of pairs are straight where positions are staged (without, registers run out), and the
+// first pass of single rows.  Device time in us, warm L2, of three passes over all keys / a branch per chunk everywhere /
+// this: topk 2048 of 16 384 keys 1 row 7.7 / 8.2 / 7.8, 20 pairs 8.2 / 8.45 / 8.25, 2 048 pairs half to full length 94.3 / 72.7 /
+// 70.2; 20 rows of 32 768 keys 16.5 / 17.3 / 16.4; 2 048 rows of 4 096, topk 512 66.2 / 41.8 / 41.7 (straight everywhere: 42.9).
+template <bool STRAIGHT, typename F> __device__ __forceinline__ void for_live_chunks(int live, const F& f) {
+    if (STRAIGHT && live == kChunks) {
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) f(c);
+    } else {
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+            if (c >= live) break;
+            f(c);
+        }
+    }
 }
 template <int GROUP>
 __device__ __forceinline__ void load_keys(const float* __restrict__ row0, const float* __restrict__ row1, int sweep,
@@ -270,13 +288,20 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
                 // every key takes part (non-candidates fall into bins 0-3, which find_bin ignores)
 #pragma unroll 1
                 for (int sw = 0; sw < nsweeps; ++sw) {
-                    load_keys<GROUP>(row0, row1, sw, len, key);
                     const int live = live_chunks(sw, len);
-#pragma unroll
-                    for (int c = 0; c < kChunks; ++c) {
-                        if (c >= live) break;
+                    auto count = [&](int c) {
 #pragma unroll
                         for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[key[i] >> 21], 1u);
+                    };
+                    // single rows: no branch behind the loads either, a chunk is counted while others are on their way (pairs
+                    // are loaded in two batches anyway and lose by it: 2 048 of 8 192 keys +3 %)
+                    if (GROUP == 1 && live == kChunks) {
+                        load_keys<GROUP>(row0, row1, sw, len, key);
+#pragma unroll
+                        for (int c = 0; c < kChunks; ++c) count(c);
+                    } else {
+                        load_keys<GROUP>(row0, row1, sw, len, key);
+                        for_live_chunks<GROUP == 2 && STAGED>(live, count);
                     }
                 }
             } else {
@@ -288,12 +313,10 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
                     // bits are the digit; everything else (wrapped or large) is clamped onto the spare bins
                     const uint32_t first = prefix << hi, spare = (uint32_t)((kBins >> (pass - 1)) + lane);   // 2048 / 1024 digits
                     const int live = live_chunks(sw, len);
-#pragma unroll
-                    for (int c = 0; c < kChunks; ++c) {
-                        if (c >= live) break;
+                    for_live_chunks<GROUP == 2 && STAGED>(live, [&](int c) {
 #pragma unroll
                         for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[min((key[i] - first) >> lo, spare)], 1u);
-                    }
+                    });
                 }
             }
             if (pass == 0 && next < rows && next_len <= kSweep && tid * 32 < next_len) {
