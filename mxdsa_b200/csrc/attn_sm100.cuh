@@ -576,7 +576,11 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
         if (*(volatile int*)&sm.abort_word != 0) goto done;       \
     } while (0)
 
-// A wait was abandoned: mark both CTAs of the pair and the device fault record.
+// A wait was abandoned: mark both CTAs of the pair and the device fault record, then hold the tear-down, whose cluster
+// barrier needs this warp, for a while.  Copies and matrix instructions may be on their way that nobody will wait for any
+// more, into shared or tensor memory of either CTA, and roles that have not run into a wait yet issue a ring's worth of tiles
+// at most; none of these waits for anything, so time is all they need before a CTA ends or its tensor memory goes.
+// (Two sleeps of about a millisecond, not a loop by the clock: this function may use next to no registers.)
 template <typename Plan> __device__ __noinline__ void raise_fault(Plan& sm, int code) {
     sm.abort_word = 1;
     // tell the peer CTA so that its roles stop waiting as well
@@ -585,6 +589,8 @@ template <typename Plan> __device__ __noinline__ void raise_fault(Plan& sm, int 
     // an epilogue warp arrives at the tear-down's cluster barrier without a release: this store must not outlive the peer
     asm volatile("fence.acq_rel.cluster;" ::: "memory");
     if (atomicCAS(&sm.fault->flag, 0, 1) == 0) sm.fault->where = code;
+    __nanosleep(1000000);
+    __nanosleep(1000000);
 }
 
 template <bool DECODE, int NT>

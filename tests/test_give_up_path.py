@@ -4,11 +4,12 @@ behind in a named barrier, the one kind of wait of theirs that has no limit.
 The sequence of waits, barriers, arrivals and looks at the abort word is read off the kernel's source; a model of two softmax
 groups of two warps walks it in every order, any warp abandoning any of its waits at any time.  What the other roles do is taken
 to follow at once: a later answer is a warp that is scheduled later, and none at all is an abandoned wait."""
+import os
 import re
 
 import pytest
 
-from test_kernel_ordering import body
+from test_kernel_ordering import CSRC, body
 
 GROUPS, WARPS = 2, 2                       # warp 0 of a group publishes the maxima, and in group 0 the row sums
 RING, S_BUFS = 4, 3
@@ -158,3 +159,19 @@ def test_no_softmax_warp_is_left_in_a_named_barrier(pairs):
     stuck, states = stuck_states(pairs)
     assert states > 1000
     assert not stuck, (len(stuck), states, stuck[0])
+
+
+def test_copies_in_flight_get_time_to_land():
+    """A role that gives up leaves copies and matrix instructions behind it; the CTA pair may not end, nor give its tensor
+    memory back, in the moment it was abandoned.  Whoever abandons a wait holds the tear-down for a time that is bounded."""
+    with open(os.path.join(CSRC, "attn_sm100.cuh")) as f:
+        text = f.read()
+    wait = text[text.index("#define MXDSA_WAIT_LIMITED_"): text.index("#define MXDSA_WAIT_ADDR_")]
+    leaves = re.findall(r"(\w+)\(.*\);\s*\\\n\s*goto done;", wait)
+    assert leaves == ["raise_fault"] * 2 and wait.count("goto done;") == 2
+    raised = text[text.index("void raise_fault("):]
+    raised = raised[: raised.index("\n}\n")]
+    assert raised.index("abort_word = 1") < raised.index("st.shared::cluster") < raised.index("__nanosleep(1000000)")
+    done = body("attn_sm100.cuh", "mxdsa_attn_kernel")
+    done = done[done.index("done:"):]
+    assert done.index("cluster_arrive") < done.index("cluster_wait()") < done.index("tmem_dealloc")
