@@ -11,6 +11,9 @@ from __future__ import annotations
 
 import torch
 
+D = 512       # elements of a row
+ROW = 528     # bytes of a packed row: the elements and a 16-byte slot of scales
+
 _module = None
 
 

@@ -67,3 +67,8 @@ def test_strides_and_no_rows_are_taken(op, shape, name, dtype):
     assert torch.equal(op(x.clone().requires_grad_()), want)
     if name == "kv":                                                    # (no rows of q: refused by the library)
         assert op(x[:0]).shape == (0,) + shape[1:-1] + (528,)
+
+
+def test_row_constants():
+    from mxdsa_b200 import packing
+    assert Z.D == packing.D_HEAD and Z.ROW == packing.D_HEAD + 16
