@@ -117,6 +117,9 @@ static constexpr int kThreads = 32 * (12 + 4 * G + 4);   // warps 0-11: K produc
 static constexpr int kLaunchRegs = 64;     // registers per thread of the launch: 65536 / kThreads
 static constexpr uint32_t kBarTmem = 7;    // named barrier: tensor memory allocated (warp 10 -> warps 12-15)
 static constexpr int kMRing = 4;         // ring of running maxima by tile
+static_assert(kGroups == 2, "tile parity names a group, its P buffer and its QK issuer");
+static_assert(kSBufs >= kGroups, "group g starts with S buffer g");
+static_assert(kStages == kScStages, "the V producers use one ring position for the tile's stage and its barriers");
 static_assert(kMRing > kSBufs && kMRing == kScStages, "a maximum is overwritten kMRing tiles later, see the softmax warps");
 
 // tensor-memory columns
@@ -156,11 +159,10 @@ struct AttnParams {
     const uint8_t* kv_scales; // prefill: start of the 16-byte slot plane (kv = data rows)
     // decode
     int b;
-    int page_size, rows_per_block;            // rows_per_block = stride_block / 512
-    int extra_topk, extra_page_size, extra_rows_per_block;
+    int page_size;
+    int extra_topk, extra_page_size;
     const uint8_t* kv;        // prefill: data rows; decode: pool base (slots live inside the pages)
     const uint8_t* extra_kv;
-    long long stride_block, extra_stride_block; // bytes
     const int* extra_indices;
     long long eidx_stride_row, eidx_stride_b;
     const int* extra_topk_length;
@@ -170,7 +172,7 @@ struct AttnParams {
     float* lse_accum;         // [splits][s_q][64]
     int page_shift, extra_page_shift;         // log2(page size) when it is a power of two, else -1
     unsigned pool_rows32, extra_pool_rows32;  // decode: keys in each pool (num_blocks * page_size, at most 2^31); indices beyond are skipped
-    unsigned row_gap, extra_row_gap;          // rows_per_block - page_size: rows of the 512-byte view that a page's scale slots take
+    unsigned row_gap, extra_row_gap;          // rows of 512 bytes from the end of a page's data to the next page (its scale slots)
 };
 
 struct TensorMaps {
@@ -401,7 +403,7 @@ template <bool DECODE, int NT> struct KeyWalk {
             return there ? (uint32_t)idx : kNoRow;
         } else {
             attended = (uint32_t)idx < pool && v < v_attended;
-            // row = page * rows_per_block + slot in page = idx + page * (rows_per_block - page_size)
+            // row = page * (page_size + gap) + slot in page = idx + page * gap
             return attended ? (uint32_t)idx + page(idx) * gap : kNoRow;
         }
     }

@@ -642,15 +642,11 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     ap.fault = d->fault;
     ap.b = p->b;
     ap.page_size = p->page_block_size;
-    ap.rows_per_block = (int)(p->stride_kv_block / 512);
     ap.kv = static_cast<const uint8_t*>(p->kv);
-    ap.stride_block = p->stride_kv_block;
     ap.extra_topk = has_extra ? p->extra_topk : 0;
     if (has_extra) {
         ap.extra_page_size = p->extra_page_block_size;
-        ap.extra_rows_per_block = (int)(p->stride_extra_kv_block / 512);
         ap.extra_kv = static_cast<const uint8_t*>(p->extra_kv);
-        ap.extra_stride_block = p->stride_extra_kv_block;
         ap.extra_indices = p->extra_indices;
         ap.eidx_stride_row = p->stride_extra_indices_s;
         ap.eidx_stride_b = p->stride_extra_indices_b;
@@ -665,8 +661,9 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     };
     ap.pool_rows32 = rows32(p->num_blocks, p->page_block_size);
     ap.extra_pool_rows32 = has_extra ? rows32(p->extra_num_blocks, p->extra_page_block_size) : 0u;
-    ap.row_gap = (unsigned)(ap.rows_per_block - p->page_block_size);
-    ap.extra_row_gap = has_extra ? (unsigned)(ap.extra_rows_per_block - p->extra_page_block_size) : 0u;
+    const int rows_per_block = (int)(p->stride_kv_block / 512), extra_rows_per_block = (int)(p->stride_extra_kv_block / 512);
+    ap.row_gap = (unsigned)(rows_per_block - p->page_block_size);
+    ap.extra_row_gap = has_extra ? (unsigned)(extra_rows_per_block - p->extra_page_block_size) : 0u;
     ap.sched_meta = p->sched_meta;
     ap.num_splits = p->num_splits;
     ap.o_accum = o_accum;
@@ -679,10 +676,10 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     if (st != MXDSA_OK) return st;
     // the last page of a pool may be shorter than the page stride: only its data rows are in the view
     st = make_kv_map(&maps.kv, p->kv,
-                     (uint64_t)(p->num_blocks - 1) * (uint64_t)ap.rows_per_block + (uint64_t)p->page_block_size);
+                     (uint64_t)(p->num_blocks - 1) * (uint64_t)rows_per_block + (uint64_t)p->page_block_size);
     if (st != MXDSA_OK) return st;
     if (has_extra) {
-        st = make_kv_map(&maps.ekv, p->extra_kv, (uint64_t)(p->extra_num_blocks - 1) * (uint64_t)ap.extra_rows_per_block +
+        st = make_kv_map(&maps.ekv, p->extra_kv, (uint64_t)(p->extra_num_blocks - 1) * (uint64_t)extra_rows_per_block +
                                                      (uint64_t)p->extra_page_block_size);
         if (st != MXDSA_OK) return st;
     }
