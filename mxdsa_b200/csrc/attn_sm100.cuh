@@ -578,11 +578,7 @@ __device__ __forceinline__ float fmax3(float a, float b, float c) {
         if (*(volatile int*)&sm.abort_word != 0) goto done;       \
     } while (0)
 
-// A wait was abandoned: mark both CTAs of the pair and the device fault record, then hold the tear-down, whose cluster
-// barrier needs this warp, for a while.  Copies and matrix instructions may be on their way that nobody will wait for any
-// more, into shared or tensor memory of either CTA, and roles that have not run into a wait yet issue a ring's worth of tiles
-// at most; none of these waits for anything, so time is all they need before a CTA ends or its tensor memory goes.
-// (Two sleeps of about a millisecond, not a loop by the clock: this function may use next to no registers.)
+// A wait was abandoned: mark both CTAs of the pair and the device fault record.
 template <typename Plan> __device__ __noinline__ void raise_fault(Plan& sm, int code) {
     sm.abort_word = 1;
     // tell the peer CTA so that its roles stop waiting as well
@@ -591,8 +587,13 @@ template <typename Plan> __device__ __noinline__ void raise_fault(Plan& sm, int 
     // an epilogue warp arrives at the tear-down's cluster barrier without a release: this store must not outlive the peer
     asm volatile("fence.acq_rel.cluster;" ::: "memory");
     if (atomicCAS(&sm.fault->flag, 0, 1) == 0) sm.fault->where = code;
-    __nanosleep(1000000);
-    __nanosleep(1000000);
+}
+
+// About a millisecond, with a limit of its own.
+__device__ __noinline__ void let_copies_land() {
+    const long long start = clock64();
+#pragma unroll 1
+    for (int i = 0; i < (1 << 16) && clock64() - start < 2000000; ++i) __nanosleep(1000);
 }
 
 template <bool DECODE, int NT>
@@ -1461,7 +1462,14 @@ done:
     if (warp >= 12 + 4 * G) cluster_arrive_relaxed();
     else cluster_arrive();
     cluster_wait();
-    if (warp == 10) tmem_dealloc<2>(tmem, kTmemCols);
+    if (warp == 10) {
+        // After a fault copies and matrix instructions may be on their way that nobody has waited for, into shared or tensor
+        // memory of either CTA.  No role issues any more and they wait for nothing, so time is all they need, and a CTA and
+        // its tensor memory last as long as this warp.  (Held here, not where the wait was abandoned: two sleeps in
+        // raise_fault made decode of 128 requests 2 % slower, the compiler arranges every wait around that call.)
+        if (*(volatile int*)&sm.abort_word != 0) let_copies_land();
+        tmem_dealloc<2>(tmem, kTmemCols);
+    }
 }
 
 // ----------------------------------------------------------------------------------------------

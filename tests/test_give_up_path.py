@@ -163,15 +163,14 @@ def test_no_softmax_warp_is_left_in_a_named_barrier(pairs):
 
 def test_copies_in_flight_get_time_to_land():
     """A role that gives up leaves copies and matrix instructions behind it; the CTA pair may not end, nor give its tensor
-    memory back, in the moment it was abandoned.  Whoever abandons a wait holds the tear-down for a time that is bounded."""
-    with open(os.path.join(CSRC, "attn_sm100.cuh")) as f:
-        text = f.read()
-    wait = text[text.index("#define MXDSA_WAIT_LIMITED_"): text.index("#define MXDSA_WAIT_ADDR_")]
-    leaves = re.findall(r"(\w+)\(.*\);\s*\\\n\s*goto done;", wait)
-    assert leaves == ["raise_fault"] * 2 and wait.count("goto done;") == 2
-    raised = text[text.index("void raise_fault("):]
-    raised = raised[: raised.index("\n}\n")]
-    assert raised.index("abort_word = 1") < raised.index("st.shared::cluster") < raised.index("__nanosleep(1000000)")
+    memory back, in the moment it was abandoned.  The warp that gives it back stays, and with it the CTA, for a time that is
+    bounded, once no role of either CTA issues any more."""
     done = body("attn_sm100.cuh", "mxdsa_attn_kernel")
     done = done[done.index("done:"):]
-    assert done.index("cluster_arrive") < done.index("cluster_wait()") < done.index("tmem_dealloc")
+    last = re.search(r"if \(warp == 10\) \{\s*if \(\*\(volatile int\*\)&sm\.abort_word != 0\) let_copies_land\(\);\s*tmem_dealloc", done)
+    assert last and done.index("cluster_arrive") < done.index("cluster_wait()") < last.start()
+    with open(os.path.join(CSRC, "attn_sm100.cuh")) as f:
+        text = f.read()
+    pause = text[text.index("void let_copies_land()"):]
+    pause = pause[: pause.index("\n}\n")]
+    assert re.search(r"for \(int i = 0; i < \(1 << 16\) && clock64\(\) - start < 2000000; \+\+i\) __nanosleep", pause)
