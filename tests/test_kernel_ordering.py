@@ -51,3 +51,30 @@ def test_nobody_leaves_ahead_of_the_peers_last_arrivals():
         role = b[b.index(role_from): b.index(role_to)]
         last_item = role.rindex("++gw;")        # a role's loop over its work items ends by counting one
         assert re.search(r"MXDSA_WAIT\(sm\." + barrier, role[last_item:]), barrier
+
+
+def test_every_phase_of_o_is_ready_is_waited_for():
+    """The epilogue warps of both CTAs arrive on CTA 0's "O is ready" without a release behind it.  That is safe because the PV
+    issuer of CTA 0 waits for each of these phases ahead of the step that it is for, the last tile's too: nothing is left on its
+    way when CTA 0 comes to the tear-down."""
+    b = body("attn_sm100.cuh", "mxdsa_attn_kernel")
+    pv = b[b.index("else if (warp == 10)"): b.index("else if (warp == 11)")]
+    epilogue = b[b.index("o_is_ready = ["): b.index("done:")]
+    # which phases: (step, ring index) of a tile
+    assert re.search(r"for \(int h = 0; h < 2; \+\+h\) \{\s*if \(t > 0 \|\| \(NT == 64 && h == 1\)\) \{\s*"
+                     r"const uint32_t n = NT == 64 && h == 1 \? gt : later;\s*MXDSA_WAIT_TIGHT\(sm\.bar_o_ready\[h\]\[n % kScStages\]", pv)
+    wide, narrow = epilogue[epilogue.index("if constexpr (NT == 128)"):].split("} else {", 1)
+    assert re.search(r"if \(t > 0\) \{.*for \(int n = 0; n < 2; \+\+n\) \{.*o_is_ready\(n, later\);", wide, re.S)
+    assert re.search(r"for \(int h = t > 0 \? 0 : 1; h < 2; \+\+h\) \{.*o_is_ready\(h, h == 0 \? later : gt\);", narrow, re.S)
+    for role in (pv, epilogue):
+        assert role.count("if (t > 0) ++later;") == 1
+    for nt in (64, 128):
+        for tiles in ([1], [1, 1, 1], [4, 1, 2], [3, 3]):
+            waited, signalled, gt, later = [], [], 0, 0
+            for count in tiles:
+                for t in range(count):
+                    waited += [(h, gt if nt == 64 and h == 1 else later) for h in (0, 1) if t > 0 or (nt == 64 and h == 1)]
+                    signalled += ([(n, later) for n in (0, 1)] if t > 0 else []) if nt == 128 else \
+                                 [(h, later if h == 0 else gt) for h in range(0 if t > 0 else 1, 2)]
+                    gt, later = gt + 1, later + (t > 0)
+            assert waited == signalled
