@@ -42,13 +42,15 @@
 //               on the next pair; only that pair's first PV waits, and only until the last columns have been read.
 //
 // What bounds a tile: latency.  A tile's way (K rows, QK, softmax, PV, its stage freed) is longer than four stages of the
-// ring at the tensor core's pace, and a warp gets to issue an instruction every 7 cycles or so (four to eight warps of a
-// scheduler are at work, 50 to 60 % of the issue slots taken).  Hence warps with little to do each: with three groups of
-// four warps, 64 keys a thread, and O rescaled by the softmax warps the softmax of a tile took 3 050 cycles from P to S
-// and a rescale 1 250 more; now 2 400 and none.  Per pass, that form / now, timed in turn: 256 tokens at topk 128 14.1 /
-// 12.9 us, decode of 64 requests at 640 keys 46.6 / 44.2, of 128 requests at 4224 keys 354 / 336, of 37 requests of two
-// tokens 22.7 / 21.6; prefill of 4 096 tokens at topk 2048 unchanged (672 / 680): there the chip is at its power limit
-// (990 W, 1 590 of 1 965 MHz), fewer cycles buy a lower clock.  For the same reason an instruction counts wherever it is:
+// ring at the tensor core's pace: a stage is held for 7 800 to 8 400 cycles in prefill, 10 000 in decode, a tile comes by
+// every 1 900 to 2 050 and 2 550.  Issue slots are taken to 62 % in prefill, 48 % in decode: of a scheduler's eight warps
+// three to four wait at a barrier, and one that does not gets to issue once in about 7 cycles.  Hence warps with little to do
+// each: with three groups of four warps, 64 keys a thread, and O rescaled by the softmax warps the softmax of a tile took
+// 3 050 cycles from P to S and a rescale 1 250 more; now 2 350 and none.  Per pass, that form / this one when it came, timed in
+// turn: 256 tokens at topk 128 14.1 / 12.9 us, decode of 64 requests at 640 keys 46.6 / 44.2, of 128 requests at 4224 keys
+// 354 / 336, of 37 requests of two tokens 22.7 / 21.6.  Long prefill paid for it, 4 096 tokens at topk 2048 672 / 680 us and
+// 65 536 at 4096 19.4 / 20.0 ms: there the chip is at its power limit (990 W, 1 590 of 1 965 MHz), fewer cycles of latency buy a
+// lower clock, and sixteen warps execute more instructions than twelve.  For that reason an instruction counts wherever it is:
 // key positions that advance by addition, groups that visit their own tiles alone, rings indexed by a power of two and the
 // row sums rescaled only where a maximum moved took another 3 to 5 % off prefill (65 536 tokens at topk 4096 20.4 / 19.4 ms,
 // 4 096 tokens at topk 2048 688 / 659 us) and 2.7 % off decode of 64 requests (43.8 / 42.6 us).
@@ -1458,7 +1460,8 @@ done:
     tc_fence_before();
     // Nobody leaves while the peer may still signal it: the cluster barrier's release orders every arrival on a barrier of
     // the peer ahead of the peer's exit.  The epilogue warps arrive without a release, which would wait for their global
-    // stores of the last pair: all that they signal the peer, "O drained", is waited for by CTA 0's PV issuer.
+    // stores of the last pair.  What they signal the peer is waited for by CTA 0's PV issuer: "O drained", which they leave out
+    // where no pair follows, and "O is ready", every phase of which it waits for ahead of a PV step, the last tile's too.
     if (warp >= 12 + 4 * G) cluster_arrive_relaxed();
     else cluster_arrive();
     cluster_wait();

@@ -33,8 +33,8 @@
 // 85.4), 1 951 pairs of 3 172 keys 71.7 -> 40.0, 27 pairs of 4 464 keys 8.4 -> 7.8.
 //
 // Bound: HBM on paper (group * s_kv * 4 bytes read + topk * 4 written per row); in practice the integer and
-// shared-memory pipes (counting every key: about 25 instructions and three shared atomics per key), so every step is
-// written to save instructions, not bytes.
+// shared-memory pipes (counting every key: two shared atomics per key as a rule, 25 executed instructions per score,
+// half of the ALU's cycles taken), so every step is written to save instructions, not bytes.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <math_constants.h>
@@ -366,8 +366,8 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 
 // ------------------------------------------------------------------------------------------------ selection by pivot
 //
-// For rows of more than 16 384 keys the kernel above sweeps the row four times and spends three shared-memory atomics
-// on every key.  Here
+// For rows of more than 16 384 keys the kernel above sweeps the row three or four times and spends two or three
+// shared-memory atomics on every key.  Here
 //   1. every eighth key is a sample; two histogram passes over the samples give a pivot: the lower edge, to 22 bits, of the
 //      rank'th largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that about 8 rank keys reach it (1.46 topk of them at
 //      topk 4096, 1.66 at 2048, 5.5 at 64).  Independent scores would do with half the margin; but neighbouring keys have
@@ -383,8 +383,8 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 // A row where the list overflows or falls short (heavy ties, a sample that misled) is counted, see recount_row.  Rows of
 // up to kShortRow keys skip the sampling: every usable key is listed.
 //
-// Measured against the kernel above (cold L2, us): 2048 rows of 32 768 keys, topk 2048 195.6 -> 134.2 (pairs 257 -> 183),
-// of 65 536 keys 355 -> 196; 64 rows of 65 536 keys, half to full length 28.7 -> 20.5; one pair of 131 072 keys 72.7 -> 24.6.
+// Measured against the kernel above (us per call among calls of its kind), topk 2048: 2048 rows of 32 768 keys 162 / 137 (pairs
+// 212 / 185), of 65 536 301 / 201 (pairs 552 / 306); 74 rows of 65 536 keys, half to full length 28.7 / 20.5; one row 28.7 / 16.4.
 // Bound: latency of the phases between barriers and, with many rows, instruction issue (54 % of the slots, about 1 650
 // instructions per warp and 16 384 keys of a pair), not HBM.
 //
@@ -1068,8 +1068,11 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
         return MXDSA_ERR_CUDA;
     const cudaStream_t s = static_cast<cudaStream_t>(p->stream);
     // By pivot where a row does not fit the registers of a CTA (16 384 keys) and the list fits with its margin.  Shorter
-    // rows are read and counted once by the other kernel, which is the faster one there for the lists in use: 2048 rows of
-    // 16 384 keys, topk 2048 81 us against 84 by pivot (pairs 101 against 120); 20 rows of 16 384 keys 11 against 19.
+    // rows are read once by the other kernel and counted from registers, which is faster there throughout: 2048 rows of
+    // 16 384 keys, topk 2048 70 us against 105 by pivot (pairs 76 against 127), 20 rows 8.2 against 15.6.  Longer ones are swept
+    // again for every pass: 2048 rows of 16 388 keys 142 against 119 (pairs 154 against 146).  The line is drawn by s_kv, as lengths
+    // are on the device; where they leave most rows within 16 384 keys counting would still be the faster (those
+    // 2048 rows, half to full length: 65 against 106).
     // Few rows are divided among CTAs.  A division in two, four or eight is taken while every CTA of the call finds an SM of
     // its own; clusters of four and eight leave some SMs over (33 rows by four, 15 by eight are resident at once, one more
     // makes a second wave: 34 rows of 36 864 keys 15.3 -> 17.6 us).  With two CTAs on an SM a division gains only where the
@@ -1077,8 +1080,9 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     // 38.7; 16 rows by eight of 262 144 31.0 against 28.3 by four, of 524 288 40.6 against 41.6.  There, too, what does not
     // fit at once must not be started: 74 rows by four of 49 152 keys 31.2 us, by two 20.2, counted 23.6.  A row is divided in
     // any case where a CTA could not hold the samples of its part.
-    // The steps between the CTAs of a row cost more than a second sweep (one row of 32 768 keys, topk 2048, events around the
-    // call: 20.5 us counted, 24.5 divided), less than the further ones (65 536 keys: 32.8 against 22.6), hence the two lines.
+    // The steps between the CTAs of a row cost about as much as a second sweep (topk 2048, one row of 20 480 keys 12.3 us counted,
+    // 14.4 divided, of 32 768 14.4 and 14.9; 148 rows of 32 768 19.2 and 15.3, a line that more rows would put lower), less
+    // than the further ones (one row of 65 536 keys 28.7 against 16.4), hence the two lines.
     int parts = 1;
     while (parts < 8) {
         const int next = 2 * parts, over = next == 8 ? 28 : (next == 4 ? 16 : 0);      // SMs left over
