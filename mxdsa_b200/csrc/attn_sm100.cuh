@@ -48,9 +48,10 @@
 // each: with three groups of four warps, 64 keys a thread, and O rescaled by the softmax warps the softmax of a tile took
 // 3 050 cycles from P to S and a rescale 1 250 more; now 2 350 and none.  Per pass, that form / this one when it came, timed in
 // turn: 256 tokens at topk 128 14.1 / 12.9 us, decode of 64 requests at 640 keys 46.6 / 44.2, of 128 requests at 4224 keys
-// 354 / 336, of 37 requests of two tokens 22.7 / 21.6.  Long prefill paid for it, 4 096 tokens at topk 2048 672 / 680 us and
-// 65 536 at 4096 19.4 / 20.0 ms: there the chip is at its power limit (990 W, 1 590 of 1 965 MHz), fewer cycles of latency buy a
-// lower clock, and sixteen warps execute more instructions than twelve.  For that reason an instruction counts wherever it is:
+// 354 / 336, of 37 requests of two tokens 22.7 / 21.6, prefill of 16 384 tokens at topk 512 841 / 782.  Long lists paid for it,
+// 4 096 tokens at topk 2048 672 / 680 us and 65 536 at 4096 19.5 / 20.0 ms: there the chip is at its power limit (990 W, 1 590 of
+// 1 965 MHz), fewer cycles of latency buy a lower clock, and what a tile executes grew.  For that reason an instruction counts
+// wherever it is:
 // key positions that advance by addition, groups that visit their own tiles alone, rings indexed by a power of two and the
 // row sums rescaled only where a maximum moved took another 3 to 5 % off prefill (65 536 tokens at topk 4096 20.4 / 19.4 ms,
 // 4 096 tokens at topk 2048 688 / 659 us) and 2.7 % off decode of 64 requests (43.8 / 42.6 us).
