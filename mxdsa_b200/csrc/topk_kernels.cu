@@ -16,8 +16,10 @@
 //     (-0 and +0 tie);
 //   * written in ascending j (+ row_offset[r]), then -1 up to topk; topk_length[r] = number selected.
 //
-// Two kernels.  mxdsa_topk_rows_kernel counts every key.  mxdsa_topk_pivot_kernel, for rows of more than 16 384 keys,
-// finds a score that a little more than topk keys reach from a sample of every eighth key, lists the keys at or above
+// Three kernels.  mxdsa_topk_held_kernel, for rows of up to 16 384 keys, counts within an interval that a sample points at,
+// with the row in registers.  mxdsa_topk_rows_kernel counts every key; it has the rows that neither of the others takes
+// (lists longer than 4096, pairs of short rows of which most keys are taken, up to 148 rows of 16 388 to 32 768 keys).
+// mxdsa_topk_pivot_kernel, for rows of more than 16 384 keys, finds a score that a little more than topk keys reach from a sample of every eighth key, lists the keys at or above
 // it in one sweep of the row and selects exactly among those (rows of many equal scores are counted instead); where there
 // are fewer rows than SMs it divides a row among the CTAs of a cluster.
 //
@@ -1052,6 +1054,352 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
     }
 }
 
+// ------------------------------------------------------------------------------------------------ rows held in registers
+//
+// For rows of up to 16 384 keys.  The row is read once and stays in registers; what each key costs in instructions is the
+// bound, so that as few steps as possible look at all of them:
+//   1. a histogram of every eighth key by its 11 highest bits gives a score that a little more than topk keys reach: the lower
+//      edge of the bin of the rank'th largest, rank = topk/8 + 4 sqrt(topk/8) + 4; the same barriers give the row's maximum;
+//   2. every key becomes its distance from the maximum (one subtraction of bit patterns where that score is positive),
+//      which needs one comparison to be sorted in or out, and those within the interval are counted in 2048 bins
+//      that span just the interval: a bin then holds a handful of keys where scores are in use;
+//   3. the bin of the topk-th key: taken as a whole, or its few keys ranked among themselves, or counted again in finer bins
+//      (many equal scores; ties go to the smaller position).  A bit per key then says what is selected.
+// A sample that misled (fewer keys than topk reach the score) is answered by counting once more from the lowest score on, from
+// registers, which is why the margin of the rank is smaller than where a row would be read again.
+// A warp owns a contiguous piece of the row, 128 keys a chunk, so that positions follow from counts within the warp and one
+// sum over the warps ahead of it; the pieces share the row's own length evenly.
+//
+// Bound: latency between barriers and instruction issue, about half each: 1 190 instructions per warp for a pair of
+// 12 288 keys, two of them per cycle and SM.  Counting all keys twice (mxdsa_topk_rows_kernel) took 1 440.  Per call, that kernel /
+// this one, us, topk 2048 unless said: 2 048 pairs of 16 384 keys, half to full length 69.8 / 63.5, 2 048 single rows 66.0 / 56.2,
+// 20 of them 7.6 / 6.3; 1 951 pairs of 3 172 keys, topk 512, 36.5 / 32.6; 8 000 rows of 1 024, topk 256, 134 / 110; 2 048 of 4 096,
+// topk 512, 40.7 / 29.5.  Tried and left out: a pair's first score row through shared memory as well, or a single row (one row
+// 6.2 -> 7.0 us: a latency more where there is no row ahead); keys turned into distances in place (one more pass over
+// them); additions of the histogram's addresses by multiply-add (no change; for the marks below it gave 3 %).
+struct __align__(16) RowShared {
+    uint32_t sample[kBins], hist[kBins + 32];      // + a bin per lane that nobody reads
+    uint32_t warp_tot[kWarps], warp_max[kWarps], warp_gt[kWarps], warp_in[kWarps];
+    uint32_t sel_bin, sel_ahead, sel_count;
+    uint32_t few_n;
+    uint2 few[32];                                 // (distance, position) of the keys of a bin of up to 32
+    __align__(16) int32_t stage[kStage];
+};
+
+// The bin of the k-th entry counted from bin 0 (from the last bin: TOP), from the histogram `hist`; sel_*.  Returns the
+// total; nothing is selected where it is below k.  Ends with a barrier.
+template <bool TOP>
+__device__ __forceinline__ uint32_t row_locate(RowShared& sm, const uint32_t* hist, uint32_t k) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int at = TOP ? kBins / 4 - 1 - tid : tid;
+    const uint4 h = *reinterpret_cast<const uint4*>(&hist[4 * at]);
+    const uint32_t b[4] = {TOP ? h.w : h.x, TOP ? h.z : h.y, TOP ? h.y : h.z, TOP ? h.x : h.w};
+    const uint32_t local = h.x + h.y + h.z + h.w;
+    const uint32_t inc = warp_inclusive_scan(local, lane);
+    if (lane == 31) sm.warp_tot[warp] = inc;
+    __syncthreads();
+    const uint32_t wt = lane < kWarps ? sm.warp_tot[lane] : 0u;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, wt);
+    uint32_t run = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u) + inc - local;
+    if (run < k && run + local >= k) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (run < k && run + b[i] >= k) {
+                sm.sel_bin = TOP ? 4 * at + 3 - i : 4 * at + i;
+                sm.sel_ahead = run;
+                sm.sel_count = b[i];
+            }
+            run += b[i];
+        }
+    }
+    __syncthreads();
+    return total;
+}
+
+// Predicated by hand: a branch per key would cost more than what it skips.
+__device__ __forceinline__ void put_position(uint32_t& to, uint32_t on, int pos) {
+    asm volatile("{\n.reg .pred p;\nsetp.ne.u32 p, %1, 0;\n@p st.shared.b32 [%0], %2;\n@p add.u32 %0, %0, 4;\n}"
+                 : "+r"(to) : "r"(on), "r"(pos) : "memory");
+}
+
+// v[i] of a register array
+__device__ __forceinline__ float register_at(const float (&v)[kKpt], uint32_t i) {
+    float t[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) t[k] = i & 16u ? v[16 + k] : v[k];
+#pragma unroll
+    for (int w = 8; w > 0; w >>= 1) {
+#pragma unroll
+        for (int k = 0; k < w; ++k) t[k] = i & (uint32_t)w ? t[w + k] : t[k];
+    }
+    return t[0];
+}
+
+// counts of a bit mask's eight nibbles, a byte each: nibbles 0, 2, 4, 6 and 1, 3, 5, 7
+__device__ __forceinline__ uint2 nibble_counts(uint32_t mask) {
+    uint32_t n = mask - ((mask >> 1) & 0x55555555u);
+    n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
+    return make_uint2(n & 0x0f0f0f0fu, (n >> 4) & 0x0f0f0f0fu);
+}
+
+template <int GROUP>
+__global__ void __launch_bounds__(kThreads, 2)
+mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
+                       const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
+                       int32_t* __restrict__ topk_length, int rows, int s_kv, int topk, uint32_t sample_rank) {
+    extern __shared__ __align__(16) uint8_t topk_smem[];
+    RowShared& sm = *reinterpret_cast<RowShared*>(topk_smem);
+    const uint32_t stage0 = (uint32_t)__cvta_generic_to_shared(sm.stage);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    int len = s_kv;
+    if (lengths != nullptr && (int)blockIdx.x < rows) len = min(max(__ldg(lengths + blockIdx.x), 0), s_kv);
+    // A pair's second score row comes through shared memory, asked for while the row before is worked on; a thread copies
+    // what it will read itself.
+    float4* ahead = reinterpret_cast<float4*>(topk_smem + sizeof(RowShared)) + tid;
+    const auto ask = [&](int row, int n) {
+        const int per_warp = 128 * ((n + 2047) >> 11), j = warp * per_warp + 4 * lane, end = min(n, (warp + 1) * per_warp);
+        const float* from = scores + ((long long)row * 2 + 1) * score_stride + j;
+        const uint32_t to = (uint32_t)__cvta_generic_to_shared(ahead);
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c)
+            if (j + 128 * c < end)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + c * kThreads * 16), "l"(from + 128 * c) : "memory");
+    };
+    if (GROUP == 2 && (int)blockIdx.x < rows) ask(blockIdx.x, len);
+    for (int r = blockIdx.x, next_len; r < rows; r += gridDim.x, len = next_len) {
+        const int next = r + (int)gridDim.x;
+        next_len = s_kv;
+        if (lengths != nullptr && next < rows) next_len = min(max(__ldg(lengths + next), 0), s_kv);
+
+        *reinterpret_cast<uint4*>(&sm.sample[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        if (tid == 0) sm.few_n = 0u;
+
+        // ---- the row: chunk c of this thread holds keys j0 + 128 c .. + 3
+        const int chunks = (len + 2047) >> 11;       // the same for all warps
+        const int j0 = warp * 128 * chunks + 4 * lane;
+        const int limit = min(len, (warp + 1) * 128 * chunks);
+        float key[kKpt];                             // (from chunk `chunks` rounded up to two on: nothing)
+        const float4* from = reinterpret_cast<const float4*>(scores + (long long)r * GROUP * score_stride + j0);
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+            if (j0 + 128 * c < limit) {              // past it the registers hold anything until below
+                const float4 f = __ldg(from + 32 * c);
+                key[4 * c] = f.x; key[4 * c + 1] = f.y; key[4 * c + 2] = f.z; key[4 * c + 3] = f.w;
+            }
+        }
+        if (GROUP == 2) {
+            asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c) {
+                if (c >= chunks) break;
+                const float4 f = ahead[c * kThreads];
+                key[4 * c] = fmaxf(key[4 * c], f.x);
+                key[4 * c + 1] = fmaxf(key[4 * c + 1], f.y);
+                key[4 * c + 2] = fmaxf(key[4 * c + 2], f.z);
+                key[4 * c + 3] = fmaxf(key[4 * c + 3], f.w);
+            }
+            if (next < rows) ask(next, next_len);
+        }
+        if ((warp + 1) * 128 * chunks > len) {       // the warps that the row ends in, or ahead of
+#pragma unroll
+            for (int i = 0; i < kKpt; ++i)
+                if (j0 + 128 * (i >> 2) + (i & 3) >= len) key[i] = -CUDART_INF_F;
+        }
+#pragma unroll
+        for (int c = 1; c < kChunks; c += 2) {       // chunks are worked on two by two
+            if (c == chunks) {
+#pragma unroll
+                for (int i = 4 * c; i < 4 * c + 4; ++i) key[i] = -CUDART_INF_F;
+            }
+        }
+        __syncthreads();                             // the histograms are clear
+
+        // ---- 1. the sample, and the maximum.  Even lanes look at one of their four keys in even chunks, odd ones in odd
+        // chunks, another one in each pair of chunks: 16 keys of every 128, of every residue modulo 8.  What is no
+        // candidate falls into bins 0 to 3, below all others.
+        float top = -CUDART_INF_F;
+#pragma unroll
+        for (int c = 0; c < kChunks; c += 2) {
+            if (c >= chunks) break;
+            atomicAdd(&sm.sample[score_key(lane & 1 ? key[4 * c + 4 + (c >> 1)] : key[4 * c + (c >> 1)]) >> 21], 1u);
+#pragma unroll
+            for (int i = 4 * c; i < 4 * c + 8; i += 2) top = fmax3(top, key[i], key[i + 1]);
+        }
+        const uint32_t warp_top = __reduce_max_sync(0xffffffffu, score_key(top));
+        if (lane == 0) sm.warp_max[warp] = warp_top;
+        if (next < rows && tid * 32 < next_len)      // the other scores of the next row are asked into L2
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(scores + (long long)next * GROUP * score_stride + tid * 32));
+        __syncthreads();
+        const uint32_t top_key = __reduce_max_sync(0xffffffffu, lane < kWarps ? sm.warp_max[lane] : 0u);
+        uint32_t pivot = kMinKey;
+        if (row_locate<true>(sm, sm.sample, sample_rank) >= sample_rank) pivot = max(sm.sel_bin << 21, kMinKey);
+        uint32_t n_sel = 0u;
+
+        // ---- 2. distances from the maximum and their histogram, 3. the bin of the topk-th
+        uint32_t lo = 0u, last = 0u, need = 0u, in_bin = 0u;       // all nearer than `lo` are selected, and `need` of the in_bin in lo .. last
+        if (top_key >= kMinKey) {                    // otherwise there is no candidate at all
+            const uint32_t top_bits = __float_as_uint(key_score(top_key)), farthest = top_key - kMinKey;
+            uint32_t span = top_key - min(pivot, top_key);
+            need = (uint32_t)topk;
+            n_sel = need;
+            bool first = true;
+#pragma unroll 1
+            while (true) {
+                if (!first) {
+                    *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+                    __syncthreads();
+                }
+                const int sh = max(21 - __clz(span), 0);
+                const uint32_t spare = (uint32_t)(kBins + lane);
+                // Bit patterns of positive scores are in the order of the scores.  What else there is (negative scores,
+                // zeros, NaNs) is farther from a positive maximum than its own bit pattern, so they are out of the way where the
+                // bins do not reach as far.
+                if (top_key > 0x80000000u && lo + ((unsigned long long)kBins << sh) <= top_bits) {
+                    const uint32_t from = top_bits - lo;
+#pragma unroll
+                    for (int c = 0; c < kChunks; c += 2) {
+                        if (c >= chunks) break;
+#pragma unroll
+                        for (int i = 4 * c; i < 4 * c + 8; ++i)
+                            atomicAdd(&sm.hist[min((from - __float_as_uint(key[i])) >> sh, spare)], 1u);
+                    }
+                } else {
+#pragma unroll
+                    for (int c = 0; c < kChunks; c += 2) {
+                        if (c >= chunks) break;
+#pragma unroll
+                        for (int i = 4 * c; i < 4 * c + 8; ++i) {
+                            float v = key[i];
+                            asm volatile("" : "+f"(v));          // worked out here, not ahead of the loop and kept
+                            const uint32_t d = top_key - score_key(v);
+                            atomicAdd(&sm.hist[d <= farthest ? min((d - lo) >> sh, spare) : spare], 1u);
+                        }
+                    }
+                }
+                __syncthreads();
+                const uint32_t total = row_locate<false>(sm, sm.hist, need);
+                first = false;
+                if (total < need) {                  // only while the interval is the first one
+                    if (span < farthest) {
+                        span = farthest;             // the sample misled: from the lowest score on
+                        continue;
+                    }
+                    n_sel = need = in_bin = total;   // fewer candidates than topk: all of them
+                    last = farthest;
+                    break;
+                }
+                lo += sm.sel_bin << sh;
+                last = min(lo + (1u << sh) - 1u, farthest);
+                need -= sm.sel_ahead;
+                in_bin = sm.sel_count;
+                if (in_bin == need || in_bin <= 32u || sh == 0) break;
+                span = last - lo;
+                // (the next pass's barriers stand between these reads of sel_* and their next writes)
+            }
+        }
+
+        // ---- what is selected, a bit per key; positions
+        int32_t* out = indices + (long long)r * index_stride;
+        const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
+        if (n_sel > 0u) {
+            const bool whole = in_bin == need;
+            uint32_t one = 1u;
+            asm volatile("" : "+r"(one));
+            uint32_t sel = 0u, within = 0u;          // nearer than lo | up to last
+            const float at_lo = key_score(top_key - lo + 1u), at_last = key_score(top_key - last);     // (beyond +inf: a NaN)
+#pragma unroll
+            for (int c = 0; c < kChunks; c += 2) {
+                if (c >= chunks) break;
+#pragma unroll
+                for (int i = 4 * c; i < 4 * c + 8; ++i) {
+                    if (key[i] >= at_lo) sel += one << i;
+                    if (key[i] >= at_last) within += one << i;
+                }
+            }
+            if (whole) sel = within;
+            within &= ~sel;
+            const bool few = !whole && in_bin <= 32u;
+            if (few) {
+                for (uint32_t m = within; m != 0u; m &= m - 1u) {
+                    const uint32_t i = __ffs(m) - 1;
+                    sm.few[atomicAdd(&sm.few_n, 1u)] = make_uint2(top_key - score_key(register_at(key, i)), (uint32_t)j0 + 128u * (i >> 2) + (i & 3u));
+                }
+            }
+            const uint32_t n_gt = __reduce_add_sync(0xffffffffu, __popc(sel));
+            if (lane == 0) sm.warp_gt[warp] = n_gt;
+            if (!whole && !few) {
+                const uint32_t n_in = __reduce_add_sync(0xffffffffu, __popc(within));
+                if (lane == 0) sm.warp_in[warp] = n_in;
+            }
+            __syncthreads();
+            uint32_t base = __reduce_add_sync(0xffffffffu, lane < warp ? sm.warp_gt[lane & (kWarps - 1)] : 0u);
+            if (few) {                               // rank the few among themselves; every warp for itself
+                const uint2 own = lane < (int)in_bin ? sm.few[lane] : make_uint2(0xffffffffu, 0xffffffffu);
+                uint32_t better = 0u;
+#pragma unroll 4
+                for (uint32_t i = 0; i < in_bin; ++i) {
+                    const uint2 o = sm.few[i];
+                    better += (o.x < own.x || (o.x == own.x && o.y < own.y)) ? 1u : 0u;
+                }
+                const bool taken = lane < (int)in_bin && better < need;
+                const uint32_t begin = (uint32_t)(warp * 128 * chunks), rel = own.y - begin;
+                base += __popc(__ballot_sync(0xffffffffu, taken && own.y < begin));
+                for (uint32_t m = __ballot_sync(0xffffffffu, taken && rel < 128u * (uint32_t)chunks); m != 0u; m &= m - 1u) {
+                    const uint32_t at = __shfl_sync(0xffffffffu, rel, __ffs(m) - 1);
+                    if (lane == (int)((at >> 2) & 31u)) sel |= 1u << ((at >> 7) * 4 + (at & 3u));
+                }
+            } else if (!whole) {                     // equal keys: the first `need` of the row
+                uint32_t q = __reduce_add_sync(0xffffffffu, lane < warp ? sm.warp_in[lane & (kWarps - 1)] : 0u);
+                base += min(q, need);
+                const uint2 own = nibble_counts(within);
+                const uint2 inc = make_uint2(warp_inclusive_scan(own.x, lane), warp_inclusive_scan(own.y, lane));
+                const uint2 all = make_uint2(__shfl_sync(0xffffffffu, inc.x, 31), __shfl_sync(0xffffffffu, inc.y, 31));
+#pragma unroll
+                for (int c = 0; c < kChunks; ++c) {
+                    const int s8 = 8 * (c >> 1);
+                    const uint32_t ahead = q + (((c & 1 ? inc.y - own.y : inc.x - own.x) >> s8) & 0xffu);
+                    uint32_t nib = (within >> (4 * c)) & 15u;
+                    for (uint32_t n = ahead + __popc(nib); n > need && nib != 0u; --n) nib ^= 1u << (31 - __clz(nib));
+                    sel |= nib << (4 * c);
+                    q += ((c & 1 ? all.y : all.x) >> s8) & 0xffu;
+                }
+            }
+            const uint2 own = nibble_counts(sel);
+            const uint2 inc = make_uint2(warp_inclusive_scan(own.x, lane), warp_inclusive_scan(own.y, lane));
+            const uint2 all = make_uint2(__shfl_sync(0xffffffffu, inc.x, 31), __shfl_sync(0xffffffffu, inc.y, 31));
+#pragma unroll
+            for (int c = 0; c < kChunks; ++c) {
+                if (c >= chunks) break;
+                const int s8 = 8 * (c >> 1);
+                uint32_t a = base + (((c & 1 ? inc.y - own.y : inc.x - own.x) >> s8) & 0xffu);
+                base += ((c & 1 ? all.y : all.x) >> s8) & 0xffu;
+                uint32_t to = stage0 + 4u * a;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    put_position(to, sel & (1u << (4 * c + e)), j0 + 128 * c + e + off);
+                }
+            }
+        }
+        __syncthreads();                             // (the next row clears the histograms and few_n behind it)
+        if (((topk | (int)(index_stride & 3) | (int)((uintptr_t)indices >> 2 & 3)) & 3) == 0) {      // rows of whole, aligned fours
+            for (uint32_t pos = 4 * tid; pos < (uint32_t)topk; pos += 4 * kThreads) {
+                int4 v = *reinterpret_cast<const int4*>(&sm.stage[pos]);
+                if (pos + 4 > n_sel) {
+                    v.x = pos < n_sel ? v.x : -1;
+                    v.y = pos + 1 < n_sel ? v.y : -1;
+                    v.z = pos + 2 < n_sel ? v.z : -1;
+                    v.w = -1;
+                }
+                *reinterpret_cast<int4*>(&out[pos]) = v;
+            }
+        } else {
+            for (uint32_t pos = tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = pos < n_sel ? sm.stage[pos] : -1;
+        }
+        if (topk_length != nullptr && tid == 0) topk_length[r] = (int32_t)n_sel;
+    }
+}
+
 thread_local int tl_topk_cuda_error = 0;
 
 }  // namespace
@@ -1068,9 +1416,9 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
         return MXDSA_ERR_CUDA;
     const cudaStream_t s = static_cast<cudaStream_t>(p->stream);
     // By pivot where a row does not fit the registers of a CTA (16 384 keys) and the list fits with its margin.  Shorter
-    // rows are read once by the other kernel and counted from registers, which is faster there throughout: 2048 rows of
-    // 16 384 keys, topk 2048 70 us against 105 by pivot (pairs 76 against 127), 20 rows 8.2 against 15.6.  Longer ones are swept
-    // again for every pass: 2048 rows of 16 388 keys 142 against 119 (pairs 154 against 146).  The line is drawn by s_kv, as lengths
+    // rows are read once and selected from registers, which is faster there throughout: 2048 rows of 16 384 keys, topk 2048
+    // 56 us against 105 by pivot (pairs 69 against 127), 20 rows 6.3 against 15.6.  Longer ones are swept again by counting
+    // for every pass: 2048 rows of 16 388 keys 142 against 119 (pairs 154 against 146).  The line is drawn by s_kv, as lengths
     // are on the device; where they leave most rows within 16 384 keys counting would still be the faster (those
     // 2048 rows, half to full length: 65 against 106).
     // Few rows are divided among CTAs.  A division in two, four or eight is taken while every CTA of the call finds an SM of
@@ -1095,6 +1443,14 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     }
     const int each = (int)((((long long)p->s_kv + parts - 1) / parts + 3) & ~3LL);      // the longest part of a row
     const bool pivot = p->topk <= kStage && p->s_kv > (p->rows <= sms ? 2 : 1) * kSweep && each <= kMaxSweeps * kSweep;
+    // Rows that a CTA's registers hold: counted within an interval that a sample points at.  Pairs of which most keys
+    // are taken stay with the other kernel: where the sample points at the lower quarter of the keys, next to all of them are
+    // counted anyway, and the interval reaches across zero, where bit patterns are far apart (2 000 pairs of 1 024 keys,
+    // topk 512 33.2 us there, 41.8 here; single rows 34.3 and 30.5).  Lists that are not staged gain nothing either (2 000 rows of
+    // 16 384 keys, topk 8 000 76.4, 83.9).
+    const float sample_mean = p->topk * 0.125f;
+    const uint32_t held_rank = (uint32_t)(sample_mean + 4.0f * sqrtf(sample_mean) + 4.0f);
+    const bool held = p->s_kv <= kSweep && p->topk <= kStage && (p->group == 1 || held_rank <= 3 * (uint32_t)p->s_kv / 32);
     cudaError_t e = cudaSuccess;
     if (pivot) {
         const bool multi = each > kSweep;
@@ -1122,6 +1478,14 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
             e = cudaLaunchKernelEx(&cfg, kern, p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length,
                                    p->rows, p->s_kv, p->topk, rank);
         }
+    } else if (held) {
+        const int grid = p->rows < sms * 2 ? p->rows : sms * 2;      // two resident CTAs of 512 threads per SM
+        auto kern = p->group == 2 ? mxdsa_topk_held_kernel<2> : mxdsa_topk_held_kernel<1>;
+        const int smem = (int)(sizeof(RowShared) + (p->group == 2 ? kSweep * sizeof(float) : 0));
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e == cudaSuccess)
+            kern<<<grid, kThreads, smem, s>>>(p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows,
+                                              p->s_kv, p->topk, held_rank);
     } else {
         const int grid = p->rows < sms * 2 ? p->rows : sms * 2;      // two resident CTAs of 512 threads per SM
         auto kern = p->topk <= kStage ? (p->group == 2 ? mxdsa_topk_rows_kernel<2, true> : mxdsa_topk_rows_kernel<1, true>)

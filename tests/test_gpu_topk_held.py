@@ -1,0 +1,70 @@
+"""Selection of rows that are held in registers (run with -m gpu): a sample points at an interval, keys are counted within it.
+Bit for bit against the oracle where that can go wrong: rows that end at the edges of chunks, warps and groups of four; scores of
+either sign, around zero, of few values and of very different size; samples that mislead; more rows than resident CTAs."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import mxdsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+LENGTHS = [0, 1, 3, 127, 128, 129, 1021, 2047, 2048, 2049, 4095, 4096, 6143, 6146, 8192, 8195, 14336, 14339, 16383, 16384]
+
+
+def _check(scores, topk, lengths=None, pair=False, offset=None):
+    from mxdsa_b200.indexer import select_topk_indices
+    dev = "cuda:0"
+    t = lambda a: None if a is None else torch.from_numpy(np.asarray(a, np.int32)).to(dev)
+    idx, cnt = select_topk_indices(torch.from_numpy(scores).to(dev), topk, t(lengths), pair, t(offset))
+    ri, rc = O.topk_select_ref(scores, topk, lengths, pair, offset)
+    assert np.array_equal(cnt.cpu().numpy(), rc) and np.array_equal(idx.cpu().numpy(), ri)
+
+
+def _scores(kind, n, s_kv, rng):
+    x = rng.standard_normal((n, s_kv)).astype(np.float32)
+    if kind == "negative":
+        x = x - np.float32(50)
+    elif kind == "zeros":              # most keys are zeros of either sign
+        x[rng.random(x.shape) < 0.9] = 0.0
+        x[rng.random(x.shape) < 0.5] *= np.float32(-1)
+    elif kind == "few":                # five values
+        x = np.round(x).clip(-2, 2)
+    elif kind == "sizes":              # 1e-40 to 1e38, some infinite, some NaN
+        x = (x * 10.0 ** rng.integers(-40, 39, x.shape)).astype(np.float32)
+        x[rng.random(x.shape) < 0.01] = np.inf
+        x[rng.random(x.shape) < 0.05] = np.nan
+        x[rng.random(x.shape) < 0.05] = -np.nan
+    elif kind == "misled":             # the best keys lie where no sample does, in adjacent pieces
+        x[:, s_kv // 3: s_kv // 3 + 100] += np.float32(9)
+        x[:, 1::8] = np.where(np.arange(s_kv)[1::8] % 256 < 128, x[:, 1::8] + np.float32(20), x[:, 1::8])
+    elif kind == "close":              # differ in the last bits
+        x = np.float32(3) + rng.integers(0, 40, x.shape).astype(np.float32) * np.float32(2.0 ** -22)
+    return x
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("kind", ["normal", "negative", "zeros", "few", "sizes", "misled", "close"])
+@pytest.mark.parametrize("s_kv,topk", [(16384, 2048), (16384, 33), (8196, 1), (2052, 130), (260, 64), (1536, 1200)])
+def test_against_the_oracle(s_kv, topk, kind, pair):
+    rng = np.random.default_rng(s_kv + topk)
+    with np.errstate(over="ignore"):
+        scores = _scores(kind, 6 if pair else 5, s_kv, rng)
+    _check(scores, topk, pair=pair)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("topk", [64, 1030, 4096])
+def test_rows_that_end_anywhere(topk, pair):
+    rng = np.random.default_rng(topk)
+    n = len(LENGTHS)
+    _check(rng.standard_normal((n * (2 if pair else 1), 16384)).astype(np.float32), topk, LENGTHS, pair,
+           np.arange(n, dtype=np.int32) * 16384)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+def test_more_rows_than_ctas(pair):
+    rng = np.random.default_rng(7)
+    rows = 700
+    lengths = rng.integers(0, 2561, rows)
+    _check(rng.standard_normal((rows * (2 if pair else 1), 2560)).astype(np.float32), 200, lengths, pair)
