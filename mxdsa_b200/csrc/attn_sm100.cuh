@@ -120,6 +120,7 @@ static constexpr int kThreads = 32 * (12 + 4 * G + 4);   // warps 0-11: K produc
 static constexpr int kLaunchRegs = 64;     // registers per thread of the launch: 65536 / kThreads
 static constexpr uint32_t kBarTmem = 7;    // named barrier: tensor memory allocated (warp 10 -> warps 12-15)
 static constexpr int kMRing = 4;         // ring of running maxima by tile
+static_assert(8 % kOutTiles == 0, "a pair's output takes 8 or 16 rounds: each pair may begin with the first staging tile");
 static_assert(kGroups == 2, "tile parity names a group, its P buffer and its QK issuer");
 static_assert(kSBufs >= kGroups, "group g starts with S buffer g");
 static_assert(kStages == kScStages, "the V producers use one ring position for the tile's stage and its barriers");
@@ -182,6 +183,7 @@ struct TensorMaps {
     CUtensorMap q;        // 5-D {128 B, 64 heads, 4 chunks, tokens, requests}
     CUtensorMap kv;       // 2-D {512 B, rows}: data rows of the (main) KV store, row pitch 512 B; gather4 source for V
     CUtensorMap ekv;      // decode: the same over the extra pool
+    CUtensorMap part;     // decode 2: 2-D {512 fp32, partials x 64 heads} over the split partials; one store box = 16 columns of 32 rows
     CUtensorMap out;      // 2-D {512 bf16, tokens x 64 heads} over the output; one store box = 32 columns of 32 rows
 };
 
@@ -246,7 +248,10 @@ struct __align__(1024) SmemPlan {
 // ----------------------------------------------------------------------------------------------
 // The roles walk the schedule independently.  What an iterator keeps in registers is its position alone: the schedule
 // record is read again (from L1) where it is needed, because every role holds its iterator across the tile loop.
-template <bool DECODE> struct WorkIter {
+// DECODE: 0 prefill, 1 decode, 2 decode of short parts, where what counts is how soon the last output has left: split
+// partials go through staging tiles and tiled stores, the last work item's output through the idle ring of KV tiles.  An
+// instantiation of its own, because long parts lose by it and because a register more in any role can make another one spill.
+template <int DECODE> struct WorkIter {
     const AttnParams& p;
     int next_pair, pair_step;      // prefill
     int req, end_req;              // decode
@@ -334,7 +339,7 @@ static constexpr uint32_t kNoRow = 0xffffffffu;
 // One lane's key through the sequence of 128-key tiles that a CTA pair walks, work item after work item: the lane looks
 // after position `key` of every tile.  What depends on the list that the position lies in (main or extra) is worked out
 // where the list changes, not per tile.
-template <bool DECODE, int NT> struct KeyWalk {
+template <int DECODE, int NT> struct KeyWalk {
     const AttnParams& p;
     WorkIter<DECODE> it;
     WorkItem w;
@@ -436,7 +441,7 @@ template <bool DECODE, int NT> struct KeyWalk {
 
 // Ask for the index lines of the two 64-key blocks blk, blk + 1 into L2: lane 0..3 takes 128-byte line lane % 2 of
 // block blk + lane / 2 (nothing where the block or the position does not exist).
-template <bool DECODE>
+template <int DECODE>
 __device__ __forceinline__ void prefetch_index_lines(const AttnParams& p, const WorkItem& w, int blk, int lane) {
     const int b = blk + (lane >> 1);
     if (b >= w.blk_end) return;
@@ -599,7 +604,7 @@ __device__ __noinline__ void let_copies_land() {
     for (int i = 0; i < (1 << 16) && clock64() - start < 2000000; ++i) __nanosleep(1000);
 }
 
-template <bool DECODE, int NT>
+template <int DECODE, int NT>
 __global__ void __launch_bounds__(kThreads, 1)
 mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ TensorMaps maps) {
     extern __shared__ uint8_t smem_raw[];
@@ -745,6 +750,10 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
                         cp_async16((dst ^ ((i & 7) << 4)) + i * 128, src0 + (unsigned long long)__shfl_sync(0xffffffffu, krow, i) * kDim);
+                } else if (DECODE == 2 && !__any_sync(0xffffffffu, lane < 16 && krow != kNoRow)) {
+                    // the half of a tile that a part's single block leaves empty: zeros, with no look at the rows
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) cp_async16((dst ^ ((i & 7) << 4)) + i * 128, p.kv, 0u);
                 } else {
 #pragma unroll 1
                     for (int i = 0; i < 16; ++i) {
@@ -1354,6 +1363,9 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             const int tok_idx = 2 * w.pair + (int)cta;
             const bool store = tok_idx < p.s_q;
             const WorkOutput wo = it.output(w);
+            // Decode of short parts: behind the last work item the ring of KV tiles is idle, and its 128 KB hold all of the output:
+            // no round waits for a staging tile.
+            [[maybe_unused]] const uint32_t tile_mask = DECODE == 2 && it.done() ? 31u : kOutTiles - 1;
             if (!DECODE || !wo.split) {
 #if MXDSA_TMA_EPILOGUE
                 // 32 columns at a time: one load becomes 32 rows x 64 bytes of the warp's staging area (16-byte
@@ -1363,7 +1375,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 // SM writes about 32 bytes per clock to global memory at best, and only with stores kept in flight
                 // (measured alone: 64 KB in 2470 cycles this way, 3330 with one tile, 3890 with 32-byte stores
                 // from the lanes).
-                const uint32_t stage0 = smem_u32(sm.o_stage[q4]);
+                const uint32_t stage0 = DECODE != 2 || tile_mask < 16 ? smem_u32(sm.o_stage[q4]) : smem_u32(sm.kv[q4]);
                 const int out_row0 = (w.req * p.s_q + tok_idx) * kHeads + (q4 & 1) * 32;
 #pragma unroll 1
                 for (int c = 0; c < 256; c += 32) {
@@ -1371,10 +1383,13 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     tmem_ld32(lane_addr + kColO + c, reinterpret_cast<uint32_t*>(o));
                     tmem_wait_ld();
                     if (c == 256 - 32) release_o();   // the last columns are in registers: the next pair's PV may go
-                    const uint32_t tile = stage0 + (round % kOutTiles) * 2048;   // tiles rotate across pairs too
-                    ++round;
-                    if (lane == 0) tma_store_wait_read<kOutTiles - 1>();   // the tile written kOutTiles rounds ago has been read
-                    __syncwarp();
+                    // tiles rotate; across pairs too, or (decode of short parts: a register less) each pair begins with the first
+                    const uint32_t tile = stage0 + (DECODE == 2 ? (uint32_t)c / 32 & tile_mask : round % kOutTiles) * 2048;
+                    if (DECODE != 2) ++round;
+                    if (DECODE != 2 || tile_mask < 16) {
+                        if (DECODE == 2 ? elect_one() : lane == 0) tma_store_wait_read<kOutTiles - 1>();   // the tile written kOutTiles rounds ago has been read
+                        __syncwarp();
+                    }
 #pragma unroll
                     for (int i = 0; i < 32; i += 8) {
                         uint32_t u[4];
@@ -1387,7 +1402,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0) {   // a group per round, empty when nothing is stored, keeps "kOutTiles - 1 pending" exact
+                    if (DECODE == 2 ? elect_one() : lane == 0) {   // a group per round, empty when nothing is stored, keeps "kOutTiles - 1 pending" exact
                         if (store) tma_store_2d(&maps.out, tile, half * 256 + c, out_row0);
                         tma_store_commit();
                     }
@@ -1418,6 +1433,36 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     }
                 }
 #endif
+            } else if constexpr (DECODE == 2) {
+                // Partials in fp32 through the same staging tiles, 16 columns to one.  32-byte stores from the lanes, one lane a row,
+                // take 7 700 cycles for a token's 128 KB with nothing else on the SM, 4 100 is what the SM can write.  Us per call, one
+                // token over 2176 keys / 30 requests of one token over 2176: lane stores 15.6 / 40.2, tiled stores 14.9 / 38.2,
+                // without a row-by-row pass over the half tile that does not exist 14.6 / 38.4, stores by an elected lane 14.4 / 37.5,
+                // the last item's by way of the KV ring 13.9 / 36.9.
+                const uint32_t stage0 = tile_mask < 16 ? smem_u32(sm.o_stage[q4]) : smem_u32(sm.kv[q4]);
+                const int part_row0 = (wo.split_idx * p.s_q + tok_idx) * kHeads + (q4 & 1) * 32;
+#pragma unroll 1
+                for (int c = 0; c < 256; c += 16) {
+                    float o[16];
+                    tmem_ld16(lane_addr + kColO + c, reinterpret_cast<uint32_t*>(o));
+                    tmem_wait_ld();
+                    if (c == 256 - 16) release_o();   // the last columns are in registers: the next pair's PV may go
+                    const uint32_t tile = stage0 + (c / 16 & tile_mask) * 2048;
+                    if (tile_mask < 16) {
+                        if (elect_one()) tma_store_wait_read<kOutTiles - 1>();
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        st_shared_16B(tile + lane * 64 + ((i ^ ((lane >> 1) & 3)) << 4), __float_as_uint(o[4 * i] * oscale),
+                                      __float_as_uint(o[4 * i + 1] * oscale), __float_as_uint(o[4 * i + 2] * oscale), __float_as_uint(o[4 * i + 3] * oscale));
+                    fence_proxy_async_smem();
+                    __syncwarp();
+                    if (elect_one()) {
+                        if (store) tma_store_2d(&maps.part, tile, half * 256 + c, part_row0);
+                        tma_store_commit();
+                    }
+                }
             } else {
                 float* dst = p.o_accum + (((long long)wo.split_idx * p.s_q + tok_idx) * kHeads + row) * kDim + half * 256;
 #pragma unroll 1
@@ -1449,7 +1494,7 @@ done:
     // ------------------------------------------------------------------ tear-down
 #if MXDSA_TMA_EPILOGUE
     // stores still reading this CTA's shared memory must have done so before the CTA may end
-    if (warp >= 12 + 4 * G && lane == 0) tma_store_wait_read<0>();
+    if (warp >= 12 + 4 * G && (DECODE == 2 ? elect_one() : lane == 0)) tma_store_wait_read<0>();
 #endif
     // After a fault the softmax warps leave at different points: each arrives on its group's barrier and on the exchange
     // barrier in place of the sync that it will not come to, and those parked there follow it, see MXDSA_LEAVE_IF_ABORTED.

@@ -127,6 +127,23 @@ int make_out_map(CUtensorMap* map, void* base, uint64_t tokens) {
     return MXDSA_OK;
 }
 
+// 2-D map over the fp32 split partials viewed as {512 columns, partials x 64 heads}: boxes of 16 columns x 32 rows out of the
+// same 64-byte-swizzled staging tiles.
+int make_part_map(CUtensorMap* map, void* base, uint64_t partials) {
+    cuuint64_t dims[2] = {MXDSA_DIM, partials * MXDSA_HEADS};
+    cuuint64_t strides[1] = {MXDSA_DIM * 4};
+    cuuint32_t box[2] = {16, 32};
+    cuuint32_t es[2] = {1, 1};
+    CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, base, dims, strides, box, es,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) {
+        tl_last_cuda_error = (int)r;
+        return MXDSA_ERR_CUDA;
+    }
+    return MXDSA_OK;
+}
+
 constexpr size_t kSmemBytes = sizeof(mxdsa::SmemPlan) + 1024;
 
 template <typename K>
@@ -546,8 +563,8 @@ int mxdsa_prefill_fwd(const mxdsa_prefill_params* p) {
     const int clusters = ap.num_pairs < d->sm_count / 2 ? ap.num_pairs : d->sm_count / 2;
     const dim3 grid(2 * clusters, 1, 1);
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-    if (p->topk >= 512) return launch_pairs(mxdsa::mxdsa_attn_kernel<false, 128>, grid, stream, ap, maps);
-    return launch_pairs(mxdsa::mxdsa_attn_kernel<false, 64>, grid, stream, ap, maps);
+    if (p->topk >= 512) return launch_pairs(mxdsa::mxdsa_attn_kernel<0, 128>, grid, stream, ap, maps);
+    return launch_pairs(mxdsa::mxdsa_attn_kernel<0, 64>, grid, stream, ap, maps);
 }
 
 int mxdsa_num_sm_parts(int device, int s_q) {
@@ -686,10 +703,23 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
 
     st = make_out_map(&maps.out, p->out, (uint64_t)p->b * (uint64_t)p->s_q);
     if (st != MXDSA_OK) return st;
+    if (combine) {
+        st = make_part_map(&maps.part, o_accum, splits * (uint64_t)p->s_q);
+        if (st != MXDSA_OK) return st;
+    }
 
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
     const dim3 grid(2 * ((p->s_q + 1) / 2), p->num_sm_parts, 1);
-    st = launch_pairs(mxdsa::mxdsa_attn_kernel<true, 64>, grid, stream, ap, maps);
+    // Short parts, up to 16 blocks of 64 keys on average, are mostly start-up and the drain of their last output.  Us per call, the
+    // kernel for long parts / for short ones: one token over 2176 keys 15.6 / 13.9, 8 requests of one token over 640 keys 25.6 /
+    // 22.8, 30 over 2176 keys (7 blocks to a part) 40.2 / 36.9, 30 of three tokens over 1152 (11) 46.5 / 42.9, 64 of one over 2176
+    // (15) 52.2 / 50.9; 64 of six over 640 (27) 41.3 / 41.1, 128 of one over 2176 (29) 63 / 73, 128 of six over 4224 (352) 325 / 347:
+    // there tiled stores of the partials wait behind the copies of the tiles that follow.
+    const long long blocks = (long long)p->b * ((p->topk + 63) / 64 + (ap.extra_topk + 63) / 64);
+    if (blocks <= 16ll * p->num_sm_parts)
+        st = launch_pairs(mxdsa::mxdsa_attn_kernel<2, 64>, grid, stream, ap, maps);
+    else
+        st = launch_pairs(mxdsa::mxdsa_attn_kernel<1, 64>, grid, stream, ap, maps);
     if (st != MXDSA_OK) return st;
     if (!combine) return MXDSA_OK;
     // programmatic dependent launch: the combine grid is set up while the attention grid drains (the attention
