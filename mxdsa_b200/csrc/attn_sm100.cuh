@@ -607,6 +607,11 @@ __device__ __noinline__ void let_copies_land() {
 template <int DECODE, int NT>
 __global__ void __launch_bounds__(kThreads, 1)
 mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ TensorMaps maps) {
+    // The last work item's output goes by way of the ring of KV tiles, which is idle by then, and empty halves of tiles are filled
+    // without a look at their rows: decode of short parts, and prefill in tiles of 128 keys, where it is worth most in calls of a
+    // few pairs to a CTA pair and costs nothing in long ones (us per call: 100 tokens at topk 512 12.3 / 11.7, 256 at 700 23.0 / 22.6,
+    // 2 048 at 512 111.2 / 110.3, 16 384 at 512 816 / 804, 4 096 at 2048 655.5 / 655.8).  Prefill in tiles of 64 keys loses 2 %.
+    constexpr bool kRingOut = DECODE == 2 || (DECODE == 0 && NT == 128);
     extern __shared__ uint8_t smem_raw[];
     // The plan starts at the first 1024-byte boundary.  The pointer is formed by adding an offset to
     // the shared array (not by rounding an integer), so the compiler still knows that every access
@@ -750,7 +755,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
 #pragma unroll
                     for (int i = 0; i < 16; ++i)
                         cp_async16((dst ^ ((i & 7) << 4)) + i * 128, src0 + (unsigned long long)__shfl_sync(0xffffffffu, krow, i) * kDim);
-                } else if (DECODE == 2 && !__any_sync(0xffffffffu, lane < 16 && krow != kNoRow)) {
+                } else if (kRingOut && !__any_sync(0xffffffffu, lane < 16 && krow != kNoRow)) {
                     // the half of a tile that a part's single block leaves empty: zeros, with no look at the rows
 #pragma unroll
                     for (int i = 0; i < 16; ++i) cp_async16((dst ^ ((i & 7) << 4)) + i * 128, p.kv, 0u);
@@ -1365,7 +1370,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             const WorkOutput wo = it.output(w);
             // Decode of short parts: behind the last work item the ring of KV tiles is idle, and its 128 KB hold all of the output:
             // no round waits for a staging tile.
-            [[maybe_unused]] const uint32_t tile_mask = DECODE == 2 && it.done() ? 31u : kOutTiles - 1;
+            [[maybe_unused]] const uint32_t tile_mask = kRingOut && it.done() ? 31u : kOutTiles - 1;
             if (!DECODE || !wo.split) {
 #if MXDSA_TMA_EPILOGUE
                 // 32 columns at a time: one load becomes 32 rows x 64 bytes of the warp's staging area (16-byte
@@ -1375,7 +1380,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 // SM writes about 32 bytes per clock to global memory at best, and only with stores kept in flight
                 // (measured alone: 64 KB in 2470 cycles this way, 3330 with one tile, 3890 with 32-byte stores
                 // from the lanes).
-                const uint32_t stage0 = DECODE != 2 || tile_mask < 16 ? smem_u32(sm.o_stage[q4]) : smem_u32(sm.kv[q4]);
+                const uint32_t stage0 = !kRingOut || tile_mask < 16 ? smem_u32(sm.o_stage[q4]) : smem_u32(sm.kv[q4]);
                 const int out_row0 = (w.req * p.s_q + tok_idx) * kHeads + (q4 & 1) * 32;
 #pragma unroll 1
                 for (int c = 0; c < 256; c += 32) {
@@ -1384,10 +1389,10 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     tmem_wait_ld();
                     if (c == 256 - 32) release_o();   // the last columns are in registers: the next pair's PV may go
                     // tiles rotate; across pairs too, or (decode of short parts: a register less) each pair begins with the first
-                    const uint32_t tile = stage0 + (DECODE == 2 ? (uint32_t)c / 32 & tile_mask : round % kOutTiles) * 2048;
-                    if (DECODE != 2) ++round;
-                    if (DECODE != 2 || tile_mask < 16) {
-                        if (DECODE == 2 ? elect_one() : lane == 0) tma_store_wait_read<kOutTiles - 1>();   // the tile written kOutTiles rounds ago has been read
+                    const uint32_t tile = stage0 + (kRingOut ? (uint32_t)c / 32 & tile_mask : round % kOutTiles) * 2048;
+                    if (!kRingOut) ++round;
+                    if (!kRingOut || tile_mask < 16) {
+                        if (kRingOut ? elect_one() : lane == 0) tma_store_wait_read<kOutTiles - 1>();   // the tile written kOutTiles rounds ago has been read
                         __syncwarp();
                     }
 #pragma unroll
@@ -1402,7 +1407,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (DECODE == 2 ? elect_one() : lane == 0) {   // a group per round, empty when nothing is stored, keeps "kOutTiles - 1 pending" exact
+                    if (kRingOut ? elect_one() : lane == 0) {   // a group per round, empty when nothing is stored, keeps "kOutTiles - 1 pending" exact
                         if (store) tma_store_2d(&maps.out, tile, half * 256 + c, out_row0);
                         tma_store_commit();
                     }
@@ -1494,7 +1499,7 @@ done:
     // ------------------------------------------------------------------ tear-down
 #if MXDSA_TMA_EPILOGUE
     // stores still reading this CTA's shared memory must have done so before the CTA may end
-    if (warp >= 12 + 4 * G && (DECODE == 2 ? elect_one() : lane == 0)) tma_store_wait_read<0>();
+    if (warp >= 12 + 4 * G && (kRingOut ? elect_one() : lane == 0)) tma_store_wait_read<0>();
 #endif
     // After a fault the softmax warps leave at different points: each arrives on its group's barrier and on the exchange
     // barrier in place of the sync that it will not come to, and those parked there follow it, see MXDSA_LEAVE_IF_ABORTED.
