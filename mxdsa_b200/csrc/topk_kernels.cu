@@ -370,9 +370,13 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 //
 // For rows of more than 16 384 keys the kernel above sweeps the row three or four times and spends two or three
 // shared-memory atomics on every key.  Here
-//   1. every eighth key is a sample; two histogram passes over the samples give a pivot: the lower edge, to 22 bits, of the
-//      rank'th largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that about 8 rank keys reach it (1.46 topk of them at
-//      topk 4096, 1.66 at 2048, 5.5 at 64).  Independent scores would do with half the margin; but neighbouring keys have
+//   1. every eighth key is a sample; a histogram of their 12 highest bits gives a pivot: the lower edge of the bin of the rank'th
+//      largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that a little more than 8 rank keys reach it (8 rank is 1.46 topk
+//      at topk 4096, 1.66 at 2048, 5.5 at 64).  Where the bin holds so many that the list might not, its next 11 bits are
+//      looked at as well.  Only the half of the histogram with the sign of the rank'th is added up over the CTAs of a row.
+//      (With a second histogram in every case, 22 bits: 64 rows of 65 536 keys, topk 2048 18.3 us, now 16.4; one row 14.4 / 12.0,
+//      8 rows of 131 072 18.6 / 15.8, 300 of 32 768 27.9 / 25.5, 2048 of 32 768 136 / 123; scores that take the second look as
+//      before.)  Independent scores would do with half the margin; but neighbouring keys have
 //      similar scores in earnest, a sample of 16 adjacent keys then tells little more than one of them, and a row that
 //      falls short costs a second time.  (With 128 adjacent keys per sample and the smaller margin, 64 rows of 65 536
 //      keys, topk 2048, equal in runs of 128, took 59.9 us, by counting 29.4, now 20.5; in runs of 64 60.6, 29.3, 21.1;
@@ -871,7 +875,7 @@ __device__ __forceinline__ void emit_part(PivotShared& sm, const float* __restri
     }
 }
 
-// All CTAs of the row call it; pivot_key: the lower edge, to 22 bits, of the interval the sample pointed at.  True, with
+// All CTAs of the row call it; pivot_key: the lower edge, to 22 bits, of what the sample pointed at.  True, with
 // nothing written, where the keys above the interval are enough and the list can hold them (RELIST).  Out of line: inlined, the
 // kernel spills and the rows that never come here take 3 to 6 % longer.
 template <int GROUP, bool RELIST, bool CLUSTER>
@@ -977,28 +981,35 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
                 }
             }
             __syncthreads();
-            uint32_t prefix = 0, k = sample_rank;
-            bool found = true;
-#pragma unroll 1
-            for (int pass = 0; pass < 2; ++pass) {
-                uint32_t* hist = &sm.hist[pass * kBins];
-                const int lo = pass == 0 ? 21 : 10;
-                const uint32_t first = pass == 0 ? 0u : prefix << 21;
+            // The 12 highest bits, the sign among them: an eighth of a power of two to a bin.  Where that many samples come with the
+            // rank'th, its bin's lower edge is the pivot, otherwise its next 11 bits are looked at (fewer usable samples than
+            // the rank: every usable key is listed).  All CTAs of the cluster decide alike.
 #pragma unroll
-                for (int i = 0; i < kSamples; ++i) {
-                    const uint32_t bin = (smp[i] - first) >> lo;
-                    if (smp[i] >= kMinKey && bin < (uint32_t)kBins) atomicAdd(&hist[bin], 1u);
-                }
-                if (locate(sm, row_bins<CLUSTER>(hist, parts), k) < k) {               // fewer usable samples than that: list every usable key
-                    found = false;                        // (decided in the first pass, by all CTAs of the cluster alike)
-                    break;
-                }
-                prefix = pass == 0 ? sm.sel_bin : (prefix << 11) | sm.sel_bin;
-                k -= sm.sel_above;
+            for (int i = 0; i < kSamples; ++i)
+                if (smp[i] >= kMinKey) atomicAdd(&sm.hist[smp[i] >> 20], 1u);
+            uint32_t k = sample_rank, half = kBins, total = locate(sm, row_bins<CLUSTER>(sm.hist + kBins, parts), k);
+            if (total < k) {                              // the rank'th is negative
+                k -= total;
+                half = 0u;
+                total = locate(sm, row_bins<CLUSTER>(sm.hist, parts), k);
             }
-            if (found) {
-                pivot_key = max(prefix << 10, kMinKey);
-                listed = 8u * (sample_rank - k + sm.sel_count) <= (uint32_t)kList;     // samples above the interval and inside it
+            if (total >= k) {
+                uint32_t edge = (half + sm.sel_bin) << 20, above = sample_rank - k + sm.sel_above, inside = sm.sel_count;
+                if (8u * (above + inside) > (uint32_t)kList * 5 / 8) {
+                    if (CLUSTER) cluster_barrier();       // the peers have read the histogram
+                    else __syncthreads();
+                    *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+                    __syncthreads();
+#pragma unroll
+                    for (int i = 0; i < kSamples; ++i)
+                        if (smp[i] - edge < 1u << 20) atomicAdd(&sm.hist[(smp[i] - edge) >> 9], 1u);
+                    locate(sm, row_bins<CLUSTER>(sm.hist, parts), sample_rank - above);
+                    edge += sm.sel_bin << 9;
+                    above += sm.sel_above;
+                    inside = sm.sel_count;
+                }
+                pivot_key = max(edge & ~1023u, kMinKey);
+                listed = 8u * (above + inside) <= (uint32_t)kList;
             }
         }
         int32_t* out = indices + (long long)r * index_stride;

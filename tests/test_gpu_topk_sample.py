@@ -1,0 +1,36 @@
+"""Selection by pivot (run with -m gpu): the sample's first look, the second one at scores that lie close together, ranks that are
+negative, rows divided among CTAs and not.  Bit for bit against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import mxdsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kind", ["normal", "close", "negative", "mixed", "zeros", "runs"])
+@pytest.mark.parametrize("rows,s_kv,topk,pair", [(1, 65536, 2048, False), (3, 40000, 300, True), (20, 36864, 4096, False),
+                                                 (150, 16400, 1000, False), (150, 20004, 64, True)])
+def test_against_the_oracle(rows, s_kv, topk, pair, kind):
+    from mxdsa_b200.indexer import select_topk_indices
+    rng = np.random.default_rng(rows + s_kv)
+    n = rows * (2 if pair else 1)
+    x = rng.standard_normal((n, s_kv), dtype=np.float32)
+    if kind == "close":              # one bin of the first look holds all
+        x = np.float32(100) + x * np.float32(0.5)
+    elif kind == "negative":
+        x = x - np.float32(30)
+    elif kind == "mixed":            # the rank'th lies at zero
+        x = x * np.float32(1e-3)
+        x[:, topk:] -= np.abs(x[:, topk:]) * np.float32(2)
+        x = rng.permuted(x, axis=1)
+    elif kind == "zeros":
+        x[rng.random(x.shape) < 0.99] = 0.0
+    elif kind == "runs":             # runs of 64 equal keys
+        x = np.repeat(x[:, : (s_kv + 63) // 64], 64, axis=1)[:, :s_kv]
+    x = np.ascontiguousarray(x)
+    lengths = rng.integers(s_kv // 2, s_kv + 1, rows).astype(np.int32)
+    idx, cnt = select_topk_indices(torch.from_numpy(x).cuda(), topk, torch.from_numpy(lengths).cuda(), pair)
+    ri, rc = O.topk_select_ref(x, topk, lengths, pair)
+    assert np.array_equal(cnt.cpu().numpy(), rc) and np.array_equal(idx.cpu().numpy(), ri)
