@@ -623,8 +623,12 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
 
     // ------------------------------------------------------------------ set-up
     // A programmatic dependent of whatever precedes it on the stream: its CTAs may be resident before that grid has ended,
-    // and nothing in global memory is touched before the wait.  Prefill sets up its barriers ahead of the wait; decode
-    // waits first, because a part without work (few requests on many parts) leaves before it sets anything up.
+    // and nothing in global memory is touched before the wait.  Barriers are set up ahead of it, except in decode of long
+    // parts: where a CTA's predecessor on the SM leaves late there is nothing to gain, and a part without work leaves at once.
+    // In decode of short parts this start overlaps the combine grid of the call before, which releases its dependents too (us per
+    // call, the wait first and no release / so): one token over 2176 keys 14.9 / 14.0, over 192 11.4 / 10.8, 8 requests of one token
+    // over 640 22.9 / 21.8, 37 whole requests of two over 128 to 1128 21.4 / 20.6, 64 of one over 2176 50.2 / 49.3; two and four
+    // requests of one token over 2176 lose, 15.6 / 16.2 and 14.8 / 15.5.  Neither of the two alone gains.
     // Dependents of this grid are released by warp 10, once the CTA has passed the wait AND holds its tensor memory: a
     // dependent that reads data older than this grid ahead of its own wait then finds it complete, and one that
     // allocates tensor memory cannot take what this grid still needs.
@@ -633,7 +637,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     // it, the first row was asked for 8 000 cycles after the start; now 4 500.  With the launch overlap: 256 tokens at
     // topk 128 18.4 -> 14.2 us per call, 37 requests of 2 tokens 25.3 -> 21.7 us, one request of one token 19.8 -> 15.7, each
     // among calls of its own kind; a single pass on new inputs gains factors of 1.06 and 1.07.
-    if constexpr (DECODE) {
+    if constexpr (DECODE == 1) {
         grid_dependency_wait();
         const int4 rec = WorkIter<DECODE>::record(p, 0);   // a volatile load: it stays behind the wait
         if (rec.x >= p.b || rec.x > rec.y) return;   // the same for both CTAs of the pair
@@ -680,7 +684,14 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     // From here a role may use this CTA's barriers; the peer's, and its tensor memory, only after cluster_wait().
     // Every role makes its first global loads (schedule, lengths, indices: three dependent latencies) in between.
     cluster_arrive();
-    if constexpr (!DECODE) grid_dependency_wait();
+    if constexpr (DECODE != 1) grid_dependency_wait();
+    if constexpr (DECODE == 2) {
+        const int4 rec = WorkIter<DECODE>::record(p, 0);
+        if (rec.x >= p.b || rec.x > rec.y) {   // the same for both CTAs of the pair
+            cluster_wait();
+            return;
+        }
+    }
 
     const uint64_t desc_k128 = smem_desc_base(16, 1024, 2);   // K-major, 128-byte swizzle
     const uint64_t desc_v = smem_desc_base(8192, 1024, 2);    // MN-major, 128-byte swizzle
