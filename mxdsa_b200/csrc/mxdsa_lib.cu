@@ -706,13 +706,6 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
 
     st = make_out_map(&maps.out, p->out, (uint64_t)p->b * (uint64_t)p->s_q);
     if (st != MXDSA_OK) return st;
-    if (combine) {
-        st = make_part_map(&maps.part, o_accum, splits * (uint64_t)p->s_q);
-        if (st != MXDSA_OK) return st;
-    }
-
-    cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-    const dim3 grid(2 * ((p->s_q + 1) / 2), p->num_sm_parts, 1);
     // Short parts, up to 16 blocks of 64 keys on average, are mostly start-up and the drain of their last output.  Us per call, the
     // kernel for long parts / for short ones: one token over 2176 keys 15.6 / 13.9, 8 requests of one token over 640 keys 25.6 /
     // 22.8, 30 over 2176 keys (7 blocks to a part) 40.2 / 36.9, 30 of three tokens over 1152 (11) 46.5 / 42.9, 64 of one over 2176
@@ -720,6 +713,13 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     // there tiled stores of the partials wait behind the copies of the tiles that follow.
     const long long blocks = (long long)p->b * ((p->topk + 63) / 64 + (ap.extra_topk + 63) / 64);
     const bool short_parts = blocks <= 16ll * p->num_sm_parts;
+    if (short_parts && combine) {
+        st = make_part_map(&maps.part, o_accum, splits * (uint64_t)p->s_q);
+        if (st != MXDSA_OK) return st;
+    }
+
+    cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
+    const dim3 grid(2 * ((p->s_q + 1) / 2), p->num_sm_parts, 1);
     if (short_parts)
         st = launch_pairs(mxdsa::mxdsa_attn_kernel<2, 64>, grid, stream, ap, maps);
     else
