@@ -1091,6 +1091,7 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 struct __align__(16) RowShared {
     uint32_t sample[kBins], hist[kBins + 32];      // + a bin per lane that nobody reads
     uint32_t warp_tot[kWarps], warp_max[kWarps], warp_gt[kWarps], warp_in[kWarps];
+    uint32_t warp_min[kWarps];                     // (not warp_in: no barrier stands between its reads and the counts of equal keys)
     uint32_t sel_bin, sel_ahead, sel_count;
     uint32_t few_n;
     uint2 few[32];                                 // (distance, position) of the keys of a bin of up to 32
@@ -1324,14 +1325,14 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                 const uint32_t warp_least = __reduce_min_sync(0xffffffffu, score_key(least));
                 if (lane == 0) {
                     sm.warp_max[warp] = warp_most;
-                    sm.warp_in[warp] = warp_least;
+                    sm.warp_min[warp] = warp_least;
                 }
                 __syncthreads();
                 lo = top_key - __reduce_max_sync(0xffffffffu, lane < kWarps ? sm.warp_max[lane] : 0u);
-                last = top_key - __reduce_min_sync(0xffffffffu, lane < kWarps ? sm.warp_in[lane] : 0xffffffffu);
+                last = top_key - __reduce_min_sync(0xffffffffu, lane < kWarps ? sm.warp_min[lane] : 0xffffffffu);
                 if (lo == last) break;
                 span = last - lo;
-                // (the next pass's barriers stand between these reads and the next writes)
+                // (the barriers of the next pass, or of the next row, stand between these reads and the next writes)
             }
         }
 

@@ -1,0 +1,145 @@
+"""What warps tell one another through shared memory in selection from held rows, followed on the CPU along every path of the
+kernel's source: between a warp's write and another's read of the same array, and between the read and the next write, there
+stands a barrier.  A run on a GPU shows a missing one only where a warp happens to be late by a hundred instructions."""
+import os
+import re
+
+import pytest
+
+from test_kernel_ordering import CSRC, body
+
+SHARED = re.compile(r"(?P<barrier>__syncthreads\(\))|(?P<locate>row_locate<)|(?P<add>atomicAdd\(&)?sm\.(?P<name>warp_\w+|sel_\w+|few_n|few)\b")
+HEAD = re.compile(r"\s*(if constexpr|if|else|for|while)\b")
+
+
+def _close(text, at):
+    """The place behind the bracket that closes the one at `at`."""
+    depth = 0
+    for i in range(at, len(text)):
+        depth += (text[i] in "({[") - (text[i] in ")}]")
+        if depth == 0:
+            return i + 1
+    raise AssertionError(text[at: at + 80])
+
+
+def _statement(text, at):
+    """(node, place behind it): ("block", nodes), ("if", events, then, else), ("loop", events, body, endless), ("do", events) or a jump."""
+    at += len(text[at:]) - len(text[at:].lstrip())
+    if text[at] == "{":
+        end = _close(text, at)
+        return ("block", _nodes(text[at + 1: end - 1])), end
+    m = HEAD.match(text, at)
+    if m:
+        end = _close(text, text.index("(", m.end()))
+        head = text[m.end(): end]
+        then, end = _statement(text, end)
+        if m[1] in ("for", "while"):
+            return ("loop", _events(head), then, head.strip() == "(true)"), end
+        other, rest = ("block", []), re.match(r"\s*else\b", text[end:])
+        if rest:
+            other, end = _statement(text, end + rest.end())
+        return ("if", _events(head), then, other), end
+    end = at
+    while text[end] != ";":
+        end = _close(text, end) if text[end] in "({[" else end + 1
+    word = text[at:end].strip()
+    return (word,) if word in ("break", "continue") else ("do", _events(word)), end + 1
+
+
+def _nodes(text):
+    text = re.sub(r"(?m)^\s*#.*$", "", text)      # pragmas
+    out, at = [], 0
+    while text[at:].strip():
+        node, at = _statement(text, at)
+        out.append(node)
+    return out
+
+
+def _events(text):
+    out = []
+    for m in SHARED.finditer(text):
+        if m["name"]:
+            index = _close(text, m.end()) if text[m.end():m.end() + 1] == "[" else m.end()
+            out.append(("w" if m["add"] or re.match(r"\s*=[^=]", text[index:]) else "r", m["name"]))
+        else:
+            out.append("barrier" if m["barrier"] else "locate")
+    return out
+
+
+def _follow(nodes, state, found, locate):
+    """`state`: accesses since the last barrier on some path here, None where none leads here.  -> (state behind, at breaks, at continues)."""
+    join = lambda a, b: b if a is None else a if b is None else a | b
+    breaks = continues = None
+
+    def events(evs, state):
+        for e in evs:
+            if state is None:
+                break
+            if e == "barrier":
+                state = frozenset()
+            elif e == "locate":
+                state = _follow(locate, state, found, None)[0]
+            else:
+                if ({"r": "w", "w": "r"}[e[0]], e[1]) in state:
+                    found.add(e[1])
+                state = state | {e}
+        return state
+
+    for n in nodes:
+        if state is None:
+            break
+        if n[0] == "do":
+            state = events(n[1], state)
+        elif n[0] == "break":
+            breaks, state = join(breaks, state), None
+        elif n[0] == "continue":
+            continues, state = join(continues, state), None
+        elif n[0] == "block":
+            state, b, c = _follow(n[1], state, found, locate)
+            breaks, continues = join(breaks, b), join(continues, c)
+        elif n[0] == "if":
+            state = events(n[1], state)
+            one, two = (_follow([x], state, found, locate) for x in n[2:4])
+            state, breaks, continues = join(one[0], two[0]), join(join(breaks, one[1]), two[1]), join(join(continues, one[2]), two[2])
+        else:
+            entry, out = events(n[1], state), None
+            while True:
+                end, b, c = _follow([n[2]], entry, found, locate)
+                again = join(end, c)
+                out = join(out, b)
+                following = join(entry, None if again is None else events(n[1], again))
+                if following == entry:
+                    break
+                entry = following
+            state = out if n[3] else join(entry, out)
+    return state, breaks, continues
+
+
+def races(kernel, locate=""):
+    found = set()
+    _follow(_nodes(kernel), frozenset(), found, _nodes(locate))
+    return found
+
+
+@pytest.mark.parametrize("code,expected", [
+    ("sm.warp_in[warp] = a; __syncthreads(); b = sm.warp_in[lane];", set()),
+    ("sm.warp_in[warp] = a; if (c) { __syncthreads(); } b = sm.warp_in[lane];", {"warp_in"}),
+    ("while (true) { sm.warp_in[warp] = a; __syncthreads(); b = sm.warp_in[lane]; if (b == a) break; __syncthreads(); }", set()),
+    ("while (true) { sm.warp_in[warp] = a; __syncthreads(); b = sm.warp_in[lane]; if (b == a) break; }", {"warp_in"}),
+    ("while (true) { sm.warp_in[warp] = a; __syncthreads(); b = sm.warp_in[lane]; if (b == a) break; __syncthreads(); } sm.warp_in[warp] = c;",
+     {"warp_in"}),
+    ("for (int r = 0; r < n; ++r) { if (r) { f(sm.few[lane]); } else continue; __syncthreads(); sm.few[atomicAdd(&sm.few_n, 1u)] = v; }", {"few"}),
+])
+def test_what_the_check_finds(code, expected):
+    assert races(code) == expected
+
+
+def test_a_barrier_stands_between_the_warps_of_held_rows():
+    with open(os.path.join(CSRC, "topk_kernels.cu")) as f:
+        text = re.sub(r"//[^\n]*", "", f.read())
+    at = text.index("{", text.index("uint32_t row_locate("))
+    locate = text[at + 1: _close(text, at) - 1]
+    kernel = body("topk_kernels.cu", "mxdsa_topk_held_kernel")[1:-1]
+    events = str(_nodes(kernel))
+    assert "'w', 'warp_max'" in events and "'r', 'warp_max'" in events and "'locate'" in events      # otherwise there is nothing to look at
+    assert races(kernel, locate) == set()
