@@ -68,3 +68,23 @@ def test_more_rows_than_ctas(pair):
     rows = 700
     lengths = rng.integers(0, 2561, rows)
     _check(rng.standard_normal((rows * (2 if pair else 1), 2560)).astype(np.float32), 200, lengths, pair)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("top", [0x3f7fffff, 0x3fffffff, 0x40000000, 0x7f7fffff, 0x7f800000])
+def test_thresholds_just_below_zero(top, pair):
+    """-0 and +0 are one score, which leaves a gap in the keys' integer images just below zero.  With a maximum of many low one
+    bits the threshold's bin begins in the gap: negative subnormals by the hundred, zeros in the bin ahead of it."""
+    rng = np.random.default_rng(top)
+    best = np.uint32(top).view(np.float32)
+    equal = np.full((2, 1024), -5, np.float32)
+    equal[:, 10:60], equal[:, 200:300] = 0.0, np.float32(-1e-40)
+    equal[:, 30:40] = np.float32(-0.0)
+    mixed = np.zeros((2, 2048), np.float32)
+    mixed[:, :100] = rng.random((2, 100))
+    mixed[:, 548:] = -rng.integers(1, 5000, (2, 1500)).astype(np.uint32).view(np.float32)
+    mixed = rng.permuted(mixed, axis=1)
+    for x, topk in ((equal, 100), (mixed, 1000), (mixed, 700), (mixed, 140)):
+        x = np.ascontiguousarray(np.repeat(x, 2, axis=0) if pair else x)
+        x[:, 0] = best
+        _check(x, topk, pair=pair)
