@@ -78,17 +78,12 @@
 
 #include "sm100_ptx.cuh"
 
-
 #ifndef MXDSA_V_HINT
 #define MXDSA_V_HINT kEvictLast
 #endif
 // How many tiles ahead of the copies the index rows are asked into L2 (0: never)
 #ifndef MXDSA_INDEX_AHEAD
 #define MXDSA_INDEX_AHEAD 4
-#endif
-// 1: the epilogue warps write bf16 output through shared memory and tiled TMA stores; 0: 32-byte stores per lane
-#ifndef MXDSA_TMA_EPILOGUE
-#define MXDSA_TMA_EPILOGUE 1
 #endif
 #ifndef MXDSA_OUT_TILES
 #define MXDSA_OUT_TILES 2
@@ -207,9 +202,7 @@ struct __align__(1024) SmemPlan {
     uint8_t q[4 * 64 * 128];                       // [chunk][head][128 B], 128-byte swizzle
     uint8_t kv[kStages][4 * 64 * 128];             // K: [chunk][key of this CTA][128 B]; V after the exchange of one half
     uint8_t s[kSBufs][64 * 128];                        // [row][128 keys], 128-byte swizzle
-#if MXDSA_TMA_EPILOGUE
-    uint8_t o_stage[4][kOutTiles][32 * 64];        // per epilogue warp: tiles of 32 rows x 32 bf16 on their way out, 64-byte swizzle
-#endif
+    uint8_t o_stage[4][kOutTiles][32 * 64];        // per epilogue warp: tiles of 32 rows x 32 bf16 (16 fp32) on their way out, 64-byte swizzle
     __align__(16) uint16_t kvalid[kStages][8];      // validity bits of the tile's keys, 16 per entry
     __align__(128) uint32_t q_sf[64 * 4];          // scale rows for tcgen05.cp (64 rows x 16 B)
     __align__(128) uint32_t k_sf[kStages][64 * 4];    // per stage: K scale rows for tcgen05.cp, gathered by the producers with the rows
@@ -1383,7 +1376,6 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             // no round waits for a staging tile.
             [[maybe_unused]] const uint32_t tile_mask = kRingOut && it.done() ? 31u : kOutTiles - 1;
             if (!DECODE || !wo.split) {
-#if MXDSA_TMA_EPILOGUE
                 // 32 columns at a time: one load becomes 32 rows x 64 bytes of the warp's staging area (16-byte
                 // chunk c of row r sits at chunk c ^ ((r / 2) % 4), the 64-byte swizzle that the tensor map undoes
                 // and that keeps the eight lanes of a store phase on different banks), then one tiled store.  The
@@ -1423,32 +1415,6 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                         tma_store_commit();
                     }
                 }
-#else
-                __nv_bfloat16* dst = p.out + (((long long)w.req * p.s_q + tok_idx) * kHeads + row) * kDim + half * 256;
-#pragma unroll 1
-                for (int c = 0; c < 256; c += 32) {
-                    float o[32];
-                    tmem_ld32(lane_addr + kColO + c, reinterpret_cast<uint32_t*>(o));
-                    tmem_wait_ld();
-                    if (c == 256 - 32) release_o();   // the last columns are in registers: the next pair's PV may go
-                    if (store) {
-                        // 32 columns -> 64 bytes of bf16: two 32-byte stores per lane (whole sectors; sixteen-byte
-                        // stores from 32 lanes to 32 rows touch every sector twice and took twice as long)
-#pragma unroll
-                        for (int i = 0; i < 32; i += 16) {
-                            unsigned long long u[4];
-#pragma unroll
-                            for (int j = 0; j < 4; ++j) {
-                                const __nv_bfloat162 lo = __floats2bfloat162_rn(o[i + 4 * j] * oscale, o[i + 4 * j + 1] * oscale);
-                                const __nv_bfloat162 hi = __floats2bfloat162_rn(o[i + 4 * j + 2] * oscale, o[i + 4 * j + 3] * oscale);
-                                u[j] = (unsigned long long)(*reinterpret_cast<const uint32_t*>(&lo)) |
-                                       ((unsigned long long)(*reinterpret_cast<const uint32_t*>(&hi)) << 32);
-                            }
-                            st_global_32B(dst + c + i, u);
-                        }
-                    }
-                }
-#endif
             } else if constexpr (DECODE == 2) {
                 // Partials in fp32 through the same staging tiles, 16 columns to one.  32-byte stores from the lanes, one lane a row,
                 // take 7 700 cycles for a token's 128 KB with nothing else on the SM, 4 100 is what the SM can write.  Us per call, one
@@ -1508,10 +1474,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
 
 done:
     // ------------------------------------------------------------------ tear-down
-#if MXDSA_TMA_EPILOGUE
     // stores still reading this CTA's shared memory must have done so before the CTA may end
     if (warp >= 12 + 4 * G && (kRingOut ? elect_one() : lane == 0)) tma_store_wait_read<0>();
-#endif
     // After a fault the softmax warps leave at different points: each arrives on its group's barrier and on the exchange
     // barrier in place of the sync that it will not come to, and those parked there follow it, see MXDSA_LEAVE_IF_ABORTED.
     // In a normal exit the arrivals are harmless: nobody waits on these barriers any more.
