@@ -1252,6 +1252,7 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
         uint32_t lo = 0u, last = 0u, need = 0u, in_bin = 0u;       // all nearer than `lo` are selected, and `need` of the in_bin in lo .. last
         if (top_key >= kMinKey) {                    // otherwise there is no candidate at all
             const uint32_t top_bits = __float_as_uint(key_score(top_key)), farthest = top_key - kMinKey;
+            const bool negative = top_key < 0x80000000u;
             uint32_t span = top_key - min(pivot, top_key);
             need = (uint32_t)topk;
             n_sel = need;
@@ -1264,17 +1265,19 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                 }
                 const int sh = max(21 - __clz(span), 0);
                 const uint32_t spare = (uint32_t)(kBins + lane);
-                // Bit patterns of positive scores are in the order of the scores.  What else there is (negative scores,
-                // zeros, NaNs) is farther from a positive maximum than its own bit pattern, so they are out of the way where the
-                // bins do not reach as far.
-                if (top_key > 0x80000000u && lo + ((unsigned long long)kBins << sh) <= top_bits) {
-                    const uint32_t from = top_bits - lo;
+                // Bit patterns of positive scores are in the order of the scores, those of negative ones in the reverse.  What else there
+                // is (scores of the other sign, zeros, NaNs, -inf) is farther from the maximum than the end of its sign's, by
+                // its own bit pattern, so it is out of the way where the bins do not reach as far.  (One multiply-add for either sign.
+                // Rows of 16 384 scores around -50, topk 2048, by counting / with negative maxima left to the general form below / so:
+                // 2 048 pairs 79.4 / 87.5 / 79.8 us, 2 048 rows 77.1 / 75.9 / 68.6, 64 rows 8.9 / 8.2 / 7.6, one row 7.7 / 8.4 / 7.6.)
+                if (lo + ((unsigned long long)kBins << sh) <= (negative ? 0xff800000u - top_bits : top_bits)) {
+                    const uint32_t sign = negative ? 1u : 0xffffffffu, from = 0u - sign * top_bits - lo;
 #pragma unroll
                     for (int c = 0; c < kChunks; c += 2) {
                         if (c >= chunks) break;
 #pragma unroll
                         for (int i = 4 * c; i < 4 * c + 8; ++i)
-                            atomicAdd(&sm.hist[min((from - __float_as_uint(key[i])) >> sh, spare)], 1u);
+                            atomicAdd(&sm.hist[min((sign * __float_as_uint(key[i]) + from) >> sh, spare)], 1u);
                     }
                 } else {
 #pragma unroll

@@ -88,3 +88,24 @@ def test_thresholds_just_below_zero(top, pair):
         x = np.ascontiguousarray(np.repeat(x, 2, axis=0) if pair else x)
         x[:, 0] = best
         _check(x, topk, pair=pair)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("largest,smallest", [(-1.0, -3.0), (-1e-45, -1e-42), (-1e-45, -1.0), (-1e-3, -3.4e38), (-3.4028235e38, -3.4028235e38),
+                                              (-3.4028233e38, -3.4028235e38), (-0.0, -2.0)])
+def test_no_score_is_positive(largest, smallest, pair):
+    """Negative maxima near and far from the ends of the negative scores, with what must not pass for one of them: NaNs of either
+    sign, -inf, and the keys behind the row's end."""
+    rng = np.random.default_rng(11)
+    ends = np.array([largest, smallest], np.float32).view(np.uint32).astype(np.int64)
+    for s_kv, topk, lengths in ((2052, 300, [2052, 2051, 1025, 700]), (16384, 2048, [16384, 16381, 9000, 2049])):
+        bits = rng.integers(min(ends), max(ends) + 1, (4, s_kv)).astype(np.uint32)      # even over the bit patterns
+        x = bits.view(np.float32).copy()
+        x[:, 5] = np.float32(largest)
+        for at, what in ((0, np.uint32(0x7fc00000)), (1, np.uint32(0xffc00000)), (2, np.uint32(0xffffffff)), (3, np.uint32(0x7f800001)),
+                         (4, np.uint32(0xff800000))):
+            x[:, 8 + at:: 64] = what.view(np.float32)
+        if pair:
+            x = np.repeat(x, 2, axis=0)
+            x[1::2] = np.roll(x[1::2], 64, axis=1)
+        _check(np.ascontiguousarray(x), topk, lengths, pair)
