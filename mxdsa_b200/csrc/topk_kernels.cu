@@ -1088,7 +1088,9 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 // topk 512, 40.7 / 29.5.  Tried and left out: a pair's first score row through shared memory as well, or a single row (one row
 // 6.2 -> 7.0 us: a latency more where there is no row ahead); keys turned into distances in place (one more pass over
 // them); additions of the histogram's addresses by multiply-add (no change; for the marks below it gave 3 %).
-struct __align__(16) RowShared {
+// (A pair's second score row is staged behind it: at 80 bytes behind a 128-byte boundary 2 048 pairs of 16 384 keys, half to full
+// length, take 66.2 us, at 16 64.1, on a boundary 61.7; 64 full pairs 7.5, 7.25, 6.9.)
+struct __align__(128) RowShared {
     uint32_t sample[kBins], hist[kBins + 32];      // + a bin per lane that nobody reads
     uint32_t warp_tot[kWarps], warp_max[kWarps], warp_gt[kWarps], warp_in[kWarps];
     uint32_t warp_min[kWarps];                     // (not warp_in: no barrier stands between its reads and the counts of equal keys)
