@@ -1071,9 +1071,10 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 // bound, so that as few steps as possible look at all of them:
 //   1. a histogram of every eighth key by its 11 highest bits gives a score that a little more than topk keys reach: the lower
 //      edge of the bin of the rank'th largest, rank = topk/8 + 4 sqrt(topk/8) + 4; the same barriers give the row's maximum;
-//   2. every key becomes its distance from the maximum (one subtraction of bit patterns where that score is positive),
-//      which needs one comparison to be sorted in or out, and those within the interval are counted in 2048 bins
-//      that span just the interval: a bin then holds a handful of keys where scores are in use;
+//   2. every key becomes its distance from the maximum (one subtraction of bit patterns where maximum and interval have one
+//      sign, by value where the interval reaches across zero), which needs one comparison to be sorted in or out, and
+//      those within the interval are counted in 2048 bins that span just the interval: a bin then holds a handful of
+//      keys where scores are in use;
 //   3. the bin of the topk-th key: taken as a whole, or its few keys ranked among themselves, or counted again in finer bins
 //      (many equal scores; ties go to the smaller position).  A bit per key then says what is selected.
 // A sample that misled (fewer keys than topk reach the score) is answered by counting once more from the lowest score on, from
@@ -1154,6 +1155,48 @@ __device__ __forceinline__ uint2 nibble_counts(uint32_t mask) {
     uint32_t n = mask - ((mask >> 1) & 0x55555555u);
     n = (n & 0x33333333u) + ((n >> 2) & 0x33333333u);
     return make_uint2(n & 0x0f0f0f0fu, (n >> 4) & 0x0f0f0f0fu);
+}
+
+// Where the interval reaches to zero or across it, keys are counted by value: bit patterns are far apart there, a bin of them an eighth
+// or a quarter of a power of two, so that the threshold's held too many keys and rows were counted twice.  zero - key * by is one
+// multiply-add and rounds once, hence the bins are in the order of the scores whatever `by` is.  It rounds down and a negative key
+// comes one bin later, which leaves zeros a bin of their own: there may be many.  Bin 0 or 1 for the maximum, 2046 at most for the
+// interval's other end, more below it; -inf and NaN come behind all bins.
+// 2 000 rows of N(0, 1) scores, us by counting every key / by bit patterns here / by value: 1 024 keys at topk 614 35.6 / 38.4 / 30.7,
+// 2 048 at 800 35.8 / 39.0 / 29.3, 6 144 at 2 700 43.7 / 51.4 / 40.4, 5 120 at 4 096 44.4 / 56.4 / 41.3, 8 000 rows of 1 024 at 256, some of
+// which need it, 131 / 111 / 103; 64 rows of 1 024 at 614 4.7 / 5.3 / 4.5; 2 048 rows of 16 384 at 2 048, all but 1.4 % zero, 86.1 / 83.4 / 76.8.
+// (Marks by value everywhere, behind a flag: rows that never come here 1 to 2 % slower.)
+struct ByValue {
+    float by, zero;
+    __device__ __forceinline__ ByValue(uint32_t top_key, uint32_t pivot) {
+        const float top = key_score(top_key);
+        by = __fdividef(2044.0f, top - key_score(pivot));
+        zero = fmaf(top, by, 8388609.0f);
+    }
+    __device__ __forceinline__ uint32_t operator()(float key) const {
+        return __float_as_uint(__fmaf_rd(-key, by, zero)) - 0x4b000000u + (__float_as_uint(key + 0.0f) >> 31);
+    }
+    // (up to -FLT_MAX: a sample that says nothing; a reach of infinity, or a subnormal one, has no scale)
+    static __device__ __forceinline__ bool takes(uint32_t top_key, uint32_t pivot) {
+        if (pivot > 0x80000000u || top_key <= 0x80000000u || pivot <= kMinKey) return false;
+        const float reach = key_score(top_key) - key_score(pivot);
+        return reach >= 1e-30f && reach < CUDART_INF_F;
+    }
+};
+
+// What the keys of a bin span, distances from the maximum, from each thread's largest and smallest of them.  One barrier.
+__device__ __forceinline__ void row_span(RowShared& sm, uint32_t top_key, float most, float least, uint32_t& lo, uint32_t& last) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t warp_most = __reduce_max_sync(0xffffffffu, score_key(most));
+    const uint32_t warp_least = __reduce_min_sync(0xffffffffu, score_key(least));
+    if (lane == 0) {
+        sm.warp_max[warp] = warp_most;
+        sm.warp_min[warp] = warp_least;
+    }
+    __syncthreads();
+    lo = top_key - __reduce_max_sync(0xffffffffu, lane < kWarps ? sm.warp_max[lane] : 0u);
+    last = top_key - __reduce_min_sync(0xffffffffu, lane < kWarps ? sm.warp_min[lane] : 0xffffffffu);
+    // (the barriers of the next pass, or of the next row, stand between these reads and the next writes)
 }
 
 template <int GROUP>
@@ -1252,6 +1295,8 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
 
         // ---- 2. distances from the maximum and their histogram, 3. the bin of the topk-th
         uint32_t lo = 0u, last = 0u, need = 0u, in_bin = 0u;       // all nearer than `lo` are selected, and `need` of the in_bin in lo .. last
+        uint32_t sel = 0u, within = 0u;              // a bit per key: nearer than lo | up to last
+        bool marked = false;
         if (top_key >= kMinKey) {                    // otherwise there is no candidate at all
             const uint32_t top_bits = __float_as_uint(key_score(top_key)), farthest = top_key - kMinKey;
             const bool negative = top_key < 0x80000000u;
@@ -1269,17 +1314,74 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                 const uint32_t spare = (uint32_t)(kBins + lane);
                 // Bit patterns of positive scores are in the order of the scores, those of negative ones in the reverse.  What else there
                 // is (scores of the other sign, zeros, NaNs, -inf) is farther from the maximum than the end of its sign's, by
-                // its own bit pattern, so it is out of the way where the bins do not reach as far.  (One multiply-add for either sign.
-                // Rows of 16 384 scores around -50, topk 2048, by counting / with negative maxima left to the general form below / so:
-                // 2 048 pairs 79.4 / 87.5 / 79.8 us, 2 048 rows 77.1 / 75.9 / 68.6, 64 rows 8.9 / 8.2 / 7.6, one row 7.7 / 8.4 / 7.6.)
-                if (lo + ((unsigned long long)kBins << sh) <= (negative ? 0xff800000u - top_bits : top_bits)) {
-                    const uint32_t sign = negative ? 1u : 0xffffffffu, from = 0u - sign * top_bits - lo;
+                // its own bit pattern, so it is out of the way where the bins do not reach as far.  (Rows of 16 384 scores around
+                // -50, topk 2048, by counting every key / with negative maxima left to the general form below / so: 2 048 pairs 79.4 /
+                // 87.5 / 75.6 us, 2 048 rows 77.1 / 75.9 / 68.4, 64 rows 9.0 / 8.2 / 7.5, one row 7.7 / 8.4 / 7.5.)
+                if (top_key > 0x80000000u && lo + ((unsigned long long)kBins << sh) <= top_bits) {
+                    const uint32_t from = top_bits - lo;
 #pragma unroll
                     for (int c = 0; c < kChunks; c += 2) {
                         if (c >= chunks) break;
 #pragma unroll
                         for (int i = 4 * c; i < 4 * c + 8; ++i)
-                            atomicAdd(&sm.hist[min((sign * __float_as_uint(key[i]) + from) >> sh, spare)], 1u);
+                            atomicAdd(&sm.hist[min((from - __float_as_uint(key[i])) >> sh, spare)], 1u);
+                    }
+                } else if (first && ByValue::takes(top_key, pivot)) {
+                    const ByValue bin(top_key, pivot);
+#pragma unroll
+                    for (int c = 0; c < kChunks; c += 2) {
+                        if (c >= chunks) break;
+#pragma unroll
+                        for (int i = 4 * c; i < 4 * c + 8; ++i)
+                            atomicAdd(&sm.hist[min(bin(key[i]), spare)], 1u);
+                    }
+                    __syncthreads();
+                    first = false;
+                    if (row_locate<false>(sm, sm.hist, need) < need) {
+                        span = farthest;             // the sample misled
+                        continue;
+                    }
+                    const uint32_t at = sm.sel_bin;
+                    need -= sm.sel_ahead;
+                    in_bin = sm.sel_count;
+                    marked = in_bin == need || in_bin <= 32u;
+                    if (marked) {                    // `lo` and `last` have no say any more
+#pragma unroll
+                        for (int c = 0; c < kChunks; c += 2) {
+                            if (c >= chunks) break;
+#pragma unroll
+                            for (int i = 4 * c; i < 4 * c + 8; ++i) {
+                                const uint32_t b = bin(key[i]);
+                                if (b < at) sel += 1u << i;
+                                if (b <= at) within += 1u << i;
+                            }
+                        }
+                        break;
+                    }
+                    float most = -CUDART_INF_F, least = CUDART_INF_F;
+#pragma unroll
+                    for (int c = 0; c < kChunks; c += 2) {
+                        if (c >= chunks) break;
+#pragma unroll
+                        for (int i = 4 * c; i < 4 * c + 8; ++i) {
+                            if (bin(key[i]) == at) {
+                                most = fmaxf(most, key[i]);
+                                least = fminf(least, key[i]);
+                            }
+                        }
+                    }
+                    row_span(sm, top_key, most, least, lo, last);
+                    if (lo == last) break;           // equal keys, as a rule
+                    span = last - lo;
+                    continue;
+                } else if (negative && lo + ((unsigned long long)kBins << sh) <= 0xff800000u - top_bits) {
+                    const uint32_t from = top_bits + lo;
+#pragma unroll
+                    for (int c = 0; c < kChunks; c += 2) {
+                        if (c >= chunks) break;
+#pragma unroll
+                        for (int i = 4 * c; i < 4 * c + 8; ++i)
+                            atomicAdd(&sm.hist[min((__float_as_uint(key[i]) - from) >> sh, spare)], 1u);
                     }
                 } else {
 #pragma unroll
@@ -1328,18 +1430,9 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                         }
                     }
                 }
-                const uint32_t warp_most = __reduce_max_sync(0xffffffffu, score_key(most));
-                const uint32_t warp_least = __reduce_min_sync(0xffffffffu, score_key(least));
-                if (lane == 0) {
-                    sm.warp_max[warp] = warp_most;
-                    sm.warp_min[warp] = warp_least;
-                }
-                __syncthreads();
-                lo = top_key - __reduce_max_sync(0xffffffffu, lane < kWarps ? sm.warp_max[lane] : 0u);
-                last = top_key - __reduce_min_sync(0xffffffffu, lane < kWarps ? sm.warp_min[lane] : 0xffffffffu);
+                row_span(sm, top_key, most, least, lo, last);
                 if (lo == last) break;
                 span = last - lo;
-                // (the barriers of the next pass, or of the next row, stand between these reads and the next writes)
             }
         }
 
@@ -1348,17 +1441,18 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
         const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
         if (n_sel > 0u) {
             const bool whole = in_bin == need;
-            uint32_t one = 1u;
-            asm volatile("" : "+r"(one));
-            uint32_t sel = 0u, within = 0u;          // nearer than lo | up to last
-            const float at_lo = key_score(top_key - lo + 1u), at_last = key_score(top_key - last);     // (beyond +inf: a NaN)
+            if (!marked) {
+                uint32_t one = 1u;
+                asm volatile("" : "+r"(one));
+                const float at_lo = key_score(top_key - lo + 1u), at_last = key_score(top_key - last);     // (beyond +inf: a NaN)
 #pragma unroll
-            for (int c = 0; c < kChunks; c += 2) {
-                if (c >= chunks) break;
+                for (int c = 0; c < kChunks; c += 2) {
+                    if (c >= chunks) break;
 #pragma unroll
-                for (int i = 4 * c; i < 4 * c + 8; ++i) {
-                    if (key[i] >= at_lo) sel += one << i;
-                    if (key[i] >= at_last) within += one << i;
+                    for (int i = 4 * c; i < 4 * c + 8; ++i) {
+                        if (key[i] >= at_lo) sel += one << i;
+                        if (key[i] >= at_last) within += one << i;
+                    }
                 }
             }
             if (whole) sel = within;

@@ -109,3 +109,28 @@ def test_no_score_is_positive(largest, smallest, pair):
             x = np.repeat(x, 2, axis=0)
             x[1::2] = np.roll(x[1::2], 64, axis=1)
         _check(np.ascontiguousarray(x), topk, lengths, pair)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("scale", [1e-44, 1e-38, 1e-30, 1.0, 1e30, 1e38])
+def test_intervals_across_zero(scale, pair):
+    """Lists of which the sample points below zero while the maximum is positive: scores are counted by value, at scales where the
+    distance across is subnormal, ordinary and beyond the largest float, also with many zeros, an infinite maximum, and one that
+    leaves all others in one bin."""
+    rng = np.random.default_rng(5)
+    x = rng.standard_normal((4, 4100)).astype(np.float64) * scale
+    x[1] = np.maximum(x[1], 0)
+    x[2] = np.round(x[2] / scale * 2) / 2 * scale
+    with np.errstate(over="ignore"):
+        x = np.clip(x, -3.4028234e38, 3.4028234e38).astype(np.float32)
+    x[:, 7::50] = np.nan
+    x[:, 9::50] = -np.inf
+    x[:, 11::50] = np.float32(-0.0)
+    for best in (None, np.inf, np.float32(3.4028234e38)):
+        if best is not None:
+            x[:, 77] = best
+        y = np.ascontiguousarray(np.repeat(x, 2, axis=0) if pair else x)
+        if pair:
+            y[1::2] = np.roll(y[1::2], 1000, axis=1)
+        for topk in (1400, 1650, 2050, 2300, 3000, 3900):
+            _check(y, topk, [4100, 4097, 3400, 2051], pair)

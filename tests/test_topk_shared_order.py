@@ -8,7 +8,7 @@ import pytest
 
 from test_kernel_ordering import CSRC, body
 
-SHARED = re.compile(r"(?P<barrier>__syncthreads\(\))|(?P<locate>row_locate<)|(?P<add>atomicAdd\(&)?sm\.(?P<name>warp_\w+|sel_\w+|few_n|few)\b")
+SHARED = re.compile(r"(?P<barrier>__syncthreads\(\))|(?P<call>row_locate|row_span)[<(]|(?P<add>atomicAdd\(&)?sm\.(?P<name>warp_\w+|sel_\w+|few_n|few)\b")
 HEAD = re.compile(r"\s*(if constexpr|if|else|for|while)\b")
 
 
@@ -62,11 +62,11 @@ def _events(text):
             index = _close(text, m.end()) if text[m.end():m.end() + 1] == "[" else m.end()
             out.append(("w" if m["add"] or re.match(r"\s*=[^=]", text[index:]) else "r", m["name"]))
         else:
-            out.append("barrier" if m["barrier"] else "locate")
+            out.append("barrier" if m["barrier"] else ("call", m["call"]))
     return out
 
 
-def _follow(nodes, state, found, locate):
+def _follow(nodes, state, found, called):
     """`state`: accesses since the last barrier on some path here, None where none leads here.  -> (state behind, at breaks, at continues)."""
     join = lambda a, b: b if a is None else a if b is None else a | b
     breaks = continues = None
@@ -77,8 +77,8 @@ def _follow(nodes, state, found, locate):
                 break
             if e == "barrier":
                 state = frozenset()
-            elif e == "locate":
-                state = _follow(locate, state, found, None)[0]
+            elif e[0] == "call":
+                state = _follow(called[e[1]], state, found, called)[0]
             else:
                 if ({"r": "w", "w": "r"}[e[0]], e[1]) in state:
                     found.add(e[1])
@@ -95,16 +95,16 @@ def _follow(nodes, state, found, locate):
         elif n[0] == "continue":
             continues, state = join(continues, state), None
         elif n[0] == "block":
-            state, b, c = _follow(n[1], state, found, locate)
+            state, b, c = _follow(n[1], state, found, called)
             breaks, continues = join(breaks, b), join(continues, c)
         elif n[0] == "if":
             state = events(n[1], state)
-            one, two = (_follow([x], state, found, locate) for x in n[2:4])
+            one, two = (_follow([x], state, found, called) for x in n[2:4])
             state, breaks, continues = join(one[0], two[0]), join(join(breaks, one[1]), two[1]), join(join(continues, one[2]), two[2])
         else:
             entry, out = events(n[1], state), None
             while True:
-                end, b, c = _follow([n[2]], entry, found, locate)
+                end, b, c = _follow([n[2]], entry, found, called)
                 again = join(end, c)
                 out = join(out, b)
                 following = join(entry, None if again is None else events(n[1], again))
@@ -115,9 +115,9 @@ def _follow(nodes, state, found, locate):
     return state, breaks, continues
 
 
-def races(kernel, locate=""):
+def races(kernel, called={}):
     found = set()
-    _follow(_nodes(kernel), frozenset(), found, _nodes(locate))
+    _follow(_nodes(kernel), frozenset(), found, {name: _nodes(text) for name, text in called.items()})
     return found
 
 
@@ -137,9 +137,12 @@ def test_what_the_check_finds(code, expected):
 def test_a_barrier_stands_between_the_warps_of_held_rows():
     with open(os.path.join(CSRC, "topk_kernels.cu")) as f:
         text = re.sub(r"//[^\n]*", "", f.read())
-    at = text.index("{", text.index("uint32_t row_locate("))
-    locate = text[at + 1: _close(text, at) - 1]
+    called = {}
+    for name in ("row_locate", "row_span"):
+        at = text.index("{", re.search(r"__device__ __forceinline__ \w+ " + name + r"\(", text).end())
+        called[name] = text[at + 1: _close(text, at) - 1]
     kernel = body("topk_kernels.cu", "mxdsa_topk_held_kernel")[1:-1]
-    events = str(_nodes(kernel))
-    assert "'w', 'warp_max'" in events and "'r', 'warp_max'" in events and "'locate'" in events      # otherwise there is nothing to look at
-    assert races(kernel, locate) == set()
+    events = str([_nodes(kernel)] + [_nodes(t) for t in called.values()])
+    for seen in ("'w', 'warp_max'", "'r', 'warp_max'", "'w', 'warp_min'", "'r', 'warp_min'", "'call', 'row_locate'", "'call', 'row_span'"):
+        assert seen in events                      # otherwise there is nothing to look at
+    assert races(kernel, called) == set()
