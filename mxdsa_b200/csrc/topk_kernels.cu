@@ -1581,14 +1581,18 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     }
     const int each = (int)((((long long)p->s_kv + parts - 1) / parts + 3) & ~3LL);      // the longest part of a row
     const bool pivot = p->topk <= kStage && p->s_kv > (p->rows <= sms ? 2 : 1) * kSweep && each <= kMaxSweeps * kSweep;
-    // Rows that a CTA's registers hold: counted within an interval that a sample points at.  Pairs of which most keys
-    // are taken stay with the other kernel: where the sample points at the lower quarter of the keys, next to all of them are
-    // counted anyway, and the interval reaches across zero, where bit patterns are far apart (2 000 pairs of 1 024 keys,
-    // topk 512 33.2 us there, 41.8 here; single rows 34.3 and 30.5).  Lists that are not staged gain nothing either (2 000 rows of
-    // 16 384 keys, topk 8 000 76.4, 83.9).
+    // Rows that a CTA's registers hold: counted within an interval that a sample points at.  Where the sample cannot hold the rank
+    // the interval is all there is, up to -FLT_MAX, and says nothing: such rows stay with the other kernel, pairs already where the rank
+    // comes to three quarters of the sample (next to all keys are within the interval then, and the two score rows have to come through
+    // shared memory).  N(0, 1) scores, us, counting / this kernel, rank within a single row's sample and just beyond it: 2 000 rows
+    // of 512 keys, topk 290 34.6 / 30.3, at 307 35.0 / 36.5; 1 024 at 665 35.5 / 30.8, at 716 36.0 / 42.4; 2 048 at 1 536 36.8 / 30.2, at 1 638
+    // 36.9 / 42.0; 4 096 at 3 276 42.3 / 34.5, at 3 481 42.5 / 44.8; 64 rows of 1 024 at 614 4.7 / 4.5, at 768 4.7 / 5.3.  2 000 pairs, rank at 0.7 and
+    // at 0.9 of the sample: 1 024 keys at 448 33.6 / 31.5 and at 615 33.0 / 33.9, 4 096 at 2 297 38.2 / 35.1 and at 3 032 37.3 / 38.7.  All scores
+    // negative: 4 096 keys at 3 481 48.4 / 43.8, but what the scores are is known on the device alone.  Lists that are not staged gain
+    // nothing (2 000 rows of 16 384 keys, topk 8 000 76.4, 83.9).
     const float sample_mean = p->topk * 0.125f;
     const uint32_t held_rank = (uint32_t)(sample_mean + 4.0f * sqrtf(sample_mean) + 4.0f);
-    const bool held = p->s_kv <= kSweep && p->topk <= kStage && (p->group == 1 || held_rank <= 3 * (uint32_t)p->s_kv / 32);
+    const bool held = p->s_kv <= kSweep && p->topk <= kStage && held_rank <= (p->group == 1 ? 4u : 3u) * (uint32_t)p->s_kv / 32;
     cudaError_t e = cudaSuccess;
     if (pivot) {
         const bool multi = each > kSweep;

@@ -134,3 +134,17 @@ def test_intervals_across_zero(scale, pair):
             y[1::2] = np.roll(y[1::2], 1000, axis=1)
         for topk in (1400, 1650, 2050, 2300, 3000, 3900):
             _check(y, topk, [4100, 4097, 3400, 2051], pair)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("s_kv", [260, 512, 1028, 2052, 4096])
+def test_either_side_of_the_line(s_kv, pair):
+    """Rows of which most keys are taken go to the counting kernel: both sides of the line, scores that the interval reaches
+    across zero for, negative ones, and lists as long as the row."""
+    rank = lambda topk: int(topk / 8 + 4 * (topk / 8) ** 0.5 + 4)
+    most = max(t for t in range(s_kv) if rank(t) <= (3 if pair else 4) * s_kv // 32)
+    rng = np.random.default_rng(s_kv)
+    scores = rng.standard_normal((8 if pair else 4, s_kv)).astype(np.float32)
+    for topk in (most - 1, most, most + 1, most + 40, s_kv):
+        for x in (scores, np.maximum(scores, 0), scores - 30):
+            _check(x, topk, [s_kv, s_kv - 3, s_kv // 2, 1], pair)
