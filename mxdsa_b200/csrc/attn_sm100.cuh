@@ -599,7 +599,7 @@ __device__ __noinline__ void let_copies_land() {
 
 template <int DECODE, int NT>
 __global__ void __launch_bounds__(kThreads, 1)
-mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ TensorMaps maps) {
+mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ TensorMaps maps, const int resident_pairs) {
     // The last work item's output goes by way of the ring of KV tiles, which is idle by then, and empty halves of tiles are filled
     // without a look at their rows: decode of short parts, and prefill in tiles of 128 keys, where it is worth most in calls of a
     // few pairs to a CTA pair and costs nothing in long ones (us per call: 100 tokens at topk 512 12.3 / 11.7, 256 at 700 23.0 / 22.6,
@@ -620,8 +620,12 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     // parts: where a CTA's predecessor on the SM leaves late there is nothing to gain, and a part without work leaves at once.
     // In decode of short parts this start overlaps the combine grid of the call before, which releases its dependents too (us per
     // call, the wait first and no release / so): one token over 2176 keys 14.9 / 14.0, over 192 11.4 / 10.8, 8 requests of one token
-    // over 640 22.9 / 21.8, 37 whole requests of two over 128 to 1128 21.4 / 20.6, 64 of one over 2176 50.2 / 49.3; two and four
-    // requests of one token over 2176 lose, 15.6 / 16.2 and 14.8 / 15.5.  Neither of the two alone gains.
+    // over 640 22.9 / 21.8, 37 whole requests of two over 128 to 1128 21.4 / 20.6, 64 of one over 2176 50.2 / 49.3.  Neither of the two
+    // alone gains.
+    // Short parts that find no SM at the start (the second half of 148 with one token to a request) wait first all the same: they come
+    // when the wait is long over, and where they have no work the few SMs left over see them one after the other.  Us per call, the
+    // wait first everywhere / nowhere / in these: whole requests of one token, 16 over 128 keys 10.5 / 11.5 / 10.8, 64 over 128 12.1 / 13.5 /
+    // 12.3, 64 over 1128 24.2 / 25.5 / 24.3; divided, 64 over 128 11.9 / 13.1 / 11.7, two over 2176 15.8 / 16.4 / 15.3, four 15.1 / 15.7 / 14.7.
     // Dependents of this grid are released by warp 10, once the CTA has passed the wait AND holds its tensor memory: a
     // dependent that reads data older than this grid ahead of its own wait then finds it complete, and one that
     // allocates tensor memory cannot take what this grid still needs.
@@ -630,7 +634,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
     // it, the first row was asked for 8 000 cycles after the start; now 4 500.  With the launch overlap: 256 tokens at
     // topk 128 18.4 -> 14.2 us per call, 37 requests of 2 tokens 25.3 -> 21.7 us, one request of one token 19.8 -> 15.7, each
     // among calls of its own kind; a single pass on new inputs gains factors of 1.06 and 1.07.
-    if constexpr (DECODE == 1) {
+    if (DECODE == 1 || (DECODE == 2 && (int)(blockIdx.y * gridDim.x + blockIdx.x) / 2 >= resident_pairs)) {
         grid_dependency_wait();
         const int4 rec = WorkIter<DECODE>::record(p, 0);   // a volatile load: it stays behind the wait
         if (rec.x >= p.b || rec.x > rec.y) return;   // the same for both CTAs of the pair

@@ -147,7 +147,7 @@ int make_part_map(CUtensorMap* map, void* base, uint64_t partials) {
 constexpr size_t kSmemBytes = sizeof(mxdsa::SmemPlan) + 1024;
 
 template <typename K>
-int launch_pairs(K kernel, dim3 grid, cudaStream_t stream, const mxdsa::AttnParams& ap,
+int launch_pairs(K kernel, dim3 grid, int sms, cudaStream_t stream, const mxdsa::AttnParams& ap,
                  const mxdsa::TensorMaps& maps) {
     static_assert(kSmemBytes <= 227 * 1024, "shared-memory plan exceeds the 227 KB per-CTA limit");
     // The kernel re-balances registers between its roles against a pool of kLaunchRegs per thread.
@@ -169,7 +169,7 @@ int launch_pairs(K kernel, dim3 grid, cudaStream_t stream, const mxdsa::AttnPara
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    MX_CUDA(cudaLaunchKernelEx(&cfg, kernel, ap, maps));
+    MX_CUDA(cudaLaunchKernelEx(&cfg, kernel, ap, maps, sms / 2));     // (one CTA to an SM)
     return MXDSA_OK;
 }
 
@@ -566,8 +566,8 @@ int mxdsa_prefill_fwd(const mxdsa_prefill_params* p) {
     const int clusters = ap.num_pairs < d->sm_count / 2 ? ap.num_pairs : d->sm_count / 2;
     const dim3 grid(2 * clusters, 1, 1);
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
-    if (p->topk >= 512) return launch_pairs(mxdsa::mxdsa_attn_kernel<0, 128>, grid, stream, ap, maps);
-    return launch_pairs(mxdsa::mxdsa_attn_kernel<0, 64>, grid, stream, ap, maps);
+    if (p->topk >= 512) return launch_pairs(mxdsa::mxdsa_attn_kernel<0, 128>, grid, d->sm_count, stream, ap, maps);
+    return launch_pairs(mxdsa::mxdsa_attn_kernel<0, 64>, grid, d->sm_count, stream, ap, maps);
 }
 
 int mxdsa_num_sm_parts(int device, int s_q) {
@@ -721,9 +721,9 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
     const dim3 grid(2 * ((p->s_q + 1) / 2), p->num_sm_parts, 1);
     if (short_parts)
-        st = launch_pairs(mxdsa::mxdsa_attn_kernel<2, 64>, grid, stream, ap, maps);
+        st = launch_pairs(mxdsa::mxdsa_attn_kernel<2, 64>, grid, d->sm_count, stream, ap, maps);
     else
-        st = launch_pairs(mxdsa::mxdsa_attn_kernel<1, 64>, grid, stream, ap, maps);
+        st = launch_pairs(mxdsa::mxdsa_attn_kernel<1, 64>, grid, d->sm_count, stream, ap, maps);
     if (st != MXDSA_OK) return st;
     if (!combine) return MXDSA_OK;
     // programmatic dependent launch: the combine grid is set up while the attention grid drains (the attention

@@ -29,11 +29,32 @@ def test_attention_releases_its_dependents_behind_its_wait():
     b = body("attn_sm100.cuh", "mxdsa_attn_kernel")
     waits = [m.start() for m in re.finditer(r"grid_dependency_wait\(\)", b)]
     release = [m.start() for m in re.finditer(r"grid_launch_dependents\(\)", b)]
-    assert len(waits) == 2 and len(release) == 1        # one wait for each instantiation
+    assert len(waits) == 2 and len(release) == 1        # ahead of the set-up (long parts, late ones) and behind it (all others)
     assert max(waits) < release[0]
     assert b.index("tmem_alloc<2>") < release[0]        # the CTA holds its tensor memory before a dependent may start
     ahead = b[: waits[0]]
     assert not re.search(r"\bp\.|__ldg|WorkIter", ahead), ahead      # decode: nothing at all is touched ahead of the wait
+
+
+def test_set_up_ahead_of_the_wait_touches_no_global_memory():
+    """Prefill and decode of short parts set up their barriers while the grid ahead may still run, its schedule and outputs half
+    written.  Between the block that waits first and the wait behind the set-up nothing is read through a pointer; the
+    schedule is read behind either wait, and the CTAs of a pair decide alike whether to leave."""
+    b = body("attn_sm100.cuh", "mxdsa_attn_kernel")
+    first, second = [m.start() for m in re.finditer(r"grid_dependency_wait\(\)", b)]
+    early = b[: first].rstrip()
+    assert early.endswith("if (DECODE == 1 || (DECODE == 2 && (int)(blockIdx.y * gridDim.x + blockIdx.x) / 2 >= resident_pairs)) {")
+    end = b.index("}", first)
+    assert re.fullmatch(r"grid_dependency_wait\(\);\s*const int4 rec = WorkIter<DECODE>::record\(p, 0\);\s*"
+                        r"if \(rec\.x >= p\.b \|\| rec\.x > rec\.y\) return;\s*\}", b[first: end + 1])
+    between = b[end + 1: second]
+    assert between.rstrip().endswith("if constexpr (DECODE != 1)")
+    assert re.findall(r"\bp\.\w+", between) == ["p.fault"] and re.findall(r"\bmaps\.\w+", between) == ["maps.q"]      # addresses, not read through
+    assert "sm.fault = p.fault;" in between and "prefetch_tensormap(&maps.q)" in between
+    assert not re.search(r"__ldg|WorkIter|KeyWalk|prefetch_index|ld_global|st_global|tma_|cp_async|\*\s*\(|->|atomic", between), between
+    behind = b[second:]
+    assert re.match(r"grid_dependency_wait\(\);\s*if constexpr \(DECODE == 2\) \{\s*const int4 rec = WorkIter<DECODE>::record\(p, 0\);\s*"
+                    r"if \(rec\.x >= p\.b \|\| rec\.x > rec\.y\) \{\s*cluster_wait\(\);\s*return;", behind)
 
 
 def test_nobody_leaves_ahead_of_the_peers_last_arrivals():
