@@ -373,7 +373,7 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 //   1. every eighth key is a sample; a histogram of their 12 highest bits gives a pivot: the lower edge of the bin of the rank'th
 //      largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that a little more than 8 rank keys reach it (8 rank is 1.46 topk
 //      at topk 4096, 1.66 at 2048, 5.5 at 64).  Where the bin holds so many that the list might not, its next 11 bits are
-//      looked at as well.  Only the half of the histogram with the sign of the rank'th is added up over the CTAs of a row.
+//      looked at as well.  Only the half of the histogram with the sign of the rank'th is added up over the CTAs of a row, as a rule.
 //      (With a second histogram in every case, 22 bits: 64 rows of 65 536 keys, topk 2048 18.3 us, now 16.4; one row 14.4 / 12.0,
 //      8 rows of 131 072 18.6 / 15.8, 300 of 32 768 27.9 / 25.5, 2048 of 32 768 136 / 123; scores that take the second look as
 //      before.)  Independent scores would do with half the margin; but neighbouring keys have
@@ -407,6 +407,7 @@ struct PivotShared {
     uint32_t chunk_tot[kChunks * kWarps];
     uint32_t sel_bin, sel_above, sel_count;
     uint32_t list_n;                               // entries of this CTA's list; kList + 1: it did not fit
+    uint32_t negative;                             // warps of which all samples are negative
     uint32_t key_max;                              // largest key of this CTA's part
     uint32_t warp_gt[kWarps], warp_eq[kWarps];
     uint4 part_count[2];                           // recount: this CTA's keys above | inside an interval, smallest and largest inside
@@ -724,23 +725,27 @@ __device__ __forceinline__ void select_from_list(PivotShared& sm, uint32_t n, ui
 constexpr int kRecountChunks = 4;                  // chunks of keys per step: half a sweep, to stay inside the register budget
 constexpr int kRecountStep = kRecountChunks * kThreads * 4;
 
-// Sum over the CTAs of the row of this thread's four bins; a barrier (of the cluster) stands ahead of it.
+// Sum over the CTAs of the row of this thread's four bins; row_bins: a barrier (of the cluster) stands ahead of it.
 template <bool CLUSTER>
-__device__ __forceinline__ uint4 row_bins(const uint32_t* hist, uint32_t parts) {
+__device__ __forceinline__ uint4 sum_bins(const uint32_t* hist, uint32_t parts) {
     const int tid = threadIdx.x;
     uint4 h;
     if (CLUSTER) {
-        cluster_barrier();
         h = make_uint4(0u, 0u, 0u, 0u);
         for (uint32_t c = 0; c < parts; ++c) {
             const uint4 o = peer_load4(peer_address(&hist[4 * tid], c));
             h.x += o.x; h.y += o.y; h.z += o.z; h.w += o.w;
         }
     } else {
-        __syncthreads();
         h = *reinterpret_cast<const uint4*>(&hist[4 * tid]);
     }
     return h;
+}
+template <bool CLUSTER>
+__device__ __forceinline__ uint4 row_bins(const uint32_t* hist, uint32_t parts) {
+    if (CLUSTER) cluster_barrier();
+    else __syncthreads();
+    return sum_bins<CLUSTER>(hist, parts);
 }
 
 // Counts this CTA's keys from `hi` on and those in [lo, hi) into sm.part_count[slot], with the smallest and largest of the
@@ -958,6 +963,7 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
         if (len > kShortRow) {                        // the same for all CTAs of the cluster
 #pragma unroll
             for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(&sm.hist[i * kBins + 4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+            if (CLUSTER && tid == 0) sm.negative = 0u;
             constexpr int kSamples = MULTI ? 4 * kMaxSweeps : 4;
             uint32_t smp[kSamples];
             if (MULTI) {
@@ -987,11 +993,28 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 #pragma unroll
             for (int i = 0; i < kSamples; ++i)
                 if (smp[i] >= kMinKey) atomicAdd(&sm.hist[smp[i] >> 20], 1u);
-            uint32_t k = sample_rank, half = kBins, total = locate(sm, row_bins<CLUSTER>(sm.hist + kBins, parts), k);
+            // Reading a half of the peers' histograms costs more than a barrier.  Where no warp of the row has a positive sample the
+            // positive half is empty; a CTA that has none itself looks at the others.  (Scores around -50, two looks of 11 bits in every
+            // case / the positive half read first / so, us: one row of 131 072 keys, topk 2048 18.1 / 20.9 / 18.0, 8 rows of 262 144 23.2 / 25.2 /
+            // 22.3, 32 pairs of 65 536 16.5 / 18.3 / 17.3; scores around zero, 64 rows of 65 536, topk 400 16.2 / 14.4 / 14.5.)
+            uint32_t k = sample_rank, half = kBins, total = 0u;
+            bool empty = false;
+            if (CLUSTER) {
+                uint32_t any = smp[0];
+#pragma unroll
+                for (int i = 1; i < kSamples; ++i) any |= smp[i];
+                if (!__any_sync(0xffffffffu, any >= 0x80000000u) && lane == 0) atomicAdd(&sm.negative, 1u);
+                cluster_barrier();
+                if (sm.negative == (uint32_t)kWarps)
+                    empty = __reduce_min_sync(0xffffffffu, lane < (int)parts ? peer_load(peer_address(&sm.negative, lane)) : (uint32_t)kWarps) == (uint32_t)kWarps;
+            } else {
+                __syncthreads();
+            }
+            if (!empty) total = locate(sm, sum_bins<CLUSTER>(sm.hist + kBins, parts), k);
             if (total < k) {                              // the rank'th is negative
                 k -= total;
                 half = 0u;
-                total = locate(sm, row_bins<CLUSTER>(sm.hist, parts), k);
+                total = locate(sm, sum_bins<CLUSTER>(sm.hist, parts), k);
             }
             if (total >= k) {
                 uint32_t edge = (half + sm.sel_bin) << 20, above = sample_rank - k + sm.sel_above, inside = sm.sel_count;

@@ -34,3 +34,25 @@ def test_against_the_oracle(rows, s_kv, topk, pair, kind):
     idx, cnt = select_topk_indices(torch.from_numpy(x).cuda(), topk, torch.from_numpy(lengths).cuda(), pair)
     ri, rc = O.topk_select_ref(x, topk, lengths, pair)
     assert np.array_equal(cnt.cpu().numpy(), rc) and np.array_equal(idx.cpu().numpy(), ri)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("rows,s_kv", [(1, 131072), (20, 65536), (70, 36864)])
+def test_parts_that_hold_no_positive_score(rows, s_kv, pair):
+    """Divided rows of which some CTAs see no positive score and others do, down to a single one, and none at all."""
+    from mxdsa_b200.indexer import select_topk_indices
+    rng = np.random.default_rng(rows)
+    x = -np.abs(rng.standard_normal((rows, s_kv), dtype=np.float32)) - np.float32(0.01)
+    for r in range(rows):
+        n = (0, 1, 40, 3000)[r % 4]
+        at = rng.choice(s_kv // 8, n, replace=False) + (s_kv - s_kv // 8 if r % 3 else 0)
+        x[r, at] *= np.float32(-1)
+    if rows == 1:
+        x[0, 100:140] *= np.float32(-1)
+    if pair:
+        x = np.repeat(x, 2, axis=0)
+        x[1::2] -= np.float32(0.5)
+    for topk in (64, 2048):
+        idx, cnt = select_topk_indices(torch.from_numpy(np.ascontiguousarray(x)).cuda(), topk, None, pair)
+        ri, rc = O.topk_select_ref(x, topk, None, pair)
+        assert np.array_equal(cnt.cpu().numpy(), rc) and np.array_equal(idx.cpu().numpy(), ri)
