@@ -1376,8 +1376,8 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             const int tok_idx = 2 * w.pair + (int)cta;
             const bool store = tok_idx < p.s_q;
             const WorkOutput wo = it.output(w);
-            // Decode of short parts: behind the last work item the ring of KV tiles is idle, and its 128 KB hold all of the output:
-            // no round waits for a staging tile.
+            // kRingOut (decode of short parts, prefill in tiles of 128 keys): behind the last work item the ring of KV tiles is idle, and
+            // its 128 KB hold all of the output, fp32 partials too: no round waits for a staging tile.
             [[maybe_unused]] const uint32_t tile_mask = kRingOut && it.done() ? 31u : kOutTiles - 1;
             if (!DECODE || !wo.split) {
                 // 32 columns at a time: one load becomes 32 rows x 64 bytes of the warp's staging area (16-byte
@@ -1395,7 +1395,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     tmem_ld32(lane_addr + kColO + c, reinterpret_cast<uint32_t*>(o));
                     tmem_wait_ld();
                     if (c == 256 - 32) release_o();   // the last columns are in registers: the next pair's PV may go
-                    // tiles rotate; across pairs too, or (decode of short parts: a register less) each pair begins with the first
+                    // tiles rotate; across pairs too, or (kRingOut: a register less) each pair begins with the first
                     const uint32_t tile = stage0 + (kRingOut ? (uint32_t)c / 32 & tile_mask : round % kOutTiles) * 2048;
                     if (!kRingOut) ++round;
                     if (!kRingOut || tile_mask < 16) {

@@ -17,11 +17,12 @@
 //   * written in ascending j (+ row_offset[r]), then -1 up to topk; topk_length[r] = number selected.
 //
 // Three kernels.  mxdsa_topk_held_kernel, for rows of up to 16 384 keys, counts within an interval that a sample points at,
-// with the row in registers.  mxdsa_topk_rows_kernel counts every key; it has the rows that neither of the others takes
-// (lists longer than 4096, pairs of short rows of which most keys are taken, up to 148 rows of 16 388 to 32 768 keys).
-// mxdsa_topk_pivot_kernel, for rows of more than 16 384 keys, finds a score that a little more than topk keys reach from a sample of every eighth key, lists the keys at or above
-// it in one sweep of the row and selects exactly among those (rows of many equal scores are counted instead); where there
-// are fewer rows than SMs it divides a row among the CTAs of a cluster.
+// with the row in registers.  mxdsa_topk_pivot_kernel, for rows of more than 16 384 keys, finds a score that somewhat more than
+// topk keys reach from a sample of every eighth key, lists the keys at or above it in one sweep of the row and selects exactly
+// among those (rows of many equal scores are counted instead); where there are fewer rows than SMs it divides a row among the
+// CTAs of a cluster.  mxdsa_topk_rows_kernel counts every key; it has the rows that neither of the others takes: lists
+// longer than 4096, rows of up to 16 384 keys of which most are taken, up to 148 rows of 16 388 to 32 768 keys, and rows
+// of more than 131 072 keys in calls of so many that they cannot be divided.
 //
 // Counting every key: exact radix selection on the order-preserving 32-bit image of the float, up to three histogram
 // passes (11 + 11 + 10 bits) with shared-memory atomics, ended where a whole bin is taken (after two, as a rule), keys of a row held in registers (one HBM read
@@ -32,7 +33,7 @@
 // deterministic.  A row costs what its own length costs: chunks of 2 048 keys past it are neither loaded nor counted, and
 // the third pass is rarely needed, because the 22-bit bin of the threshold holds one key or two.  Before, every row cost
 // 16 384 keys and three passes: 2 048 pairs of 16 384 keys, half to full length, topk 2048 93.9 -> 70.5 us (the passes alone
-// 85.4), 1 951 pairs of 3 172 keys 71.7 -> 40.0, 27 pairs of 4 464 keys 8.4 -> 7.8.
+// 85.4), 1 951 pairs of 3 172 keys 71.7 -> 40.0, 27 pairs of 4 464 keys 8.4 -> 7.8 (calls that went this way then).
 //
 // Bound: HBM on paper (group * s_kv * 4 bytes read + topk * 4 written per row); in practice the integer and
 // shared-memory pipes (counting every key: two shared atomics per key as a rule, 25 executed instructions per score,
@@ -84,8 +85,9 @@ __device__ __forceinline__ int live_chunks(int sweep, int len) {
 // keeps the work of one from overlapping the next's, which shows where a CTA has its SM to itself; more code shows too, in short
 // rows.  So the histogram passes of pairs are straight where positions are staged (without, registers run out), and the
 // first pass of single rows.  Device time in us, warm L2, of three passes over all keys / a branch per chunk everywhere /
-// this: topk 2048 of 16 384 keys 1 row 7.7 / 8.2 / 7.8, 20 pairs 8.2 / 8.45 / 8.25, 2 048 pairs half to full length 94.3 / 72.7 /
-// 70.2; 20 rows of 32 768 keys 16.5 / 17.3 / 16.4; 2 048 rows of 4 096, topk 512 66.2 / 41.8 / 41.7 (straight everywhere: 42.9).
+// this: 20 rows of 32 768 keys, topk 2048 16.5 / 17.3 / 16.4.  Of calls that have another kernel now, then: topk 2048 of 16 384
+// keys 1 row 7.7 / 8.2 / 7.8, 20 pairs 8.2 / 8.45 / 8.25, 2 048 pairs half to full length 94.3 / 72.7 / 70.2; 2 048 rows of 4 096, topk 512
+// 66.2 / 41.8 / 41.7 (straight everywhere: 42.9).
 template <bool STRAIGHT, typename F> __device__ __forceinline__ void for_live_chunks(int live, const F& f) {
     if (STRAIGHT && live == kChunks) {
 #pragma unroll
@@ -371,9 +373,11 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 // For rows of more than 16 384 keys the kernel above sweeps the row three or four times and spends two or three
 // shared-memory atomics on every key.  Here
 //   1. every eighth key is a sample; a histogram of their 12 highest bits gives a pivot: the lower edge of the bin of the rank'th
-//      largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that a little more than 8 rank keys reach it (8 rank is 1.46 topk
-//      at topk 4096, 1.66 at 2048, 5.5 at 64).  Where the bin holds so many that the list might not, its next 11 bits are
-//      looked at as well.  Only the half of the histogram with the sign of the rank'th is added up over the CTAs of a row, as a rule.
+//      largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that 8 rank keys reach it, 1.46 topk at topk 4096, 1.66 at 2048, 5.5 at
+//      64, and what else the bin holds, an eighth of a power of two (131 072 N(0, 1) scores at topk 1000: 2 980 keys, 8 rank
+//      is 1 952; at topk 64 up to about twice 8 rank).  Where that comes to more than 5 120 keys by the sample, of the 8 192 that
+//      the list can hold, the bin's next 11 bits are looked at as well.  Only the half of the histogram with the sign of the
+//      rank'th is added up over the CTAs of a row, as a rule.
 //      (With a second histogram in every case, 22 bits: 64 rows of 65 536 keys, topk 2048 18.3 us, now 16.4; one row 14.4 / 12.0,
 //      8 rows of 131 072 18.6 / 15.8, 300 of 32 768 27.9 / 25.5, 2048 of 32 768 136 / 123; scores that take the second look as
 //      before.)  Independent scores would do with half the margin; but neighbouring keys have
@@ -389,7 +393,7 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 // A row where the list overflows or falls short (heavy ties, a sample that misled) is counted, see recount_row.  Rows of
 // up to kShortRow keys skip the sampling: every usable key is listed.
 //
-// Measured against the kernel above (us per call among calls of its kind), topk 2048: 2048 rows of 32 768 keys 162 / 137 (pairs
+// Measured against the kernel above, with two looks in every case (us per call among calls of its kind), topk 2048: 2048 rows of 32 768 keys 162 / 137 (pairs
 // 212 / 185), of 65 536 301 / 201 (pairs 552 / 306); 74 rows of 65 536 keys, half to full length 28.7 / 20.5; one row 28.7 / 16.4.
 // Bound: latency of the phases between barriers and, with many rows, instruction issue (54 % of the slots, about 1 650
 // instructions per warp and 16 384 keys of a pair), not HBM.
@@ -1105,11 +1109,12 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 // A warp owns a contiguous piece of the row, 128 keys a chunk, so that positions follow from counts within the warp and one
 // sum over the warps ahead of it; the pieces share the row's own length evenly.
 //
-// Bound: latency between barriers and instruction issue, about half each: 1 190 instructions per warp for a pair of
-// 12 288 keys, two of them per cycle and SM.  Counting all keys twice (mxdsa_topk_rows_kernel) took 1 440.  Per call, that kernel /
-// this one, us, topk 2048 unless said: 2 048 pairs of 16 384 keys, half to full length 69.8 / 63.5, 2 048 single rows 66.0 / 56.2,
-// 20 of them 7.6 / 6.3; 1 951 pairs of 3 172 keys, topk 512, 36.5 / 32.6; 8 000 rows of 1 024, topk 256, 134 / 110; 2 048 of 4 096,
-// topk 512, 40.7 / 29.5.  Tried and left out: a pair's first score row through shared memory as well, or a single row (one row
+// Bound: latency between barriers and instruction issue, about half each: 1 210 instructions per warp for a pair of
+// 12 288 keys, 2.2 of them per cycle and SM.  Counting all keys twice (mxdsa_topk_rows_kernel) takes 1 440.  Per call, that kernel /
+// this one, us, topk 2048 unless said: 2 048 pairs of 16 384 keys, half to full length 69.3 / 61.1, 2 048 single rows 64.5 / 56.3,
+// 20 of them, topk 512 7.1 / 5.7; 1 951 pairs of 3 172 keys, topk 512, 37.0 / 32.6; 8 000 rows of 1 024, topk 256, 131 / 103; 300 of 4 096,
+// topk 512, 9.1 / 7.6.  In one wave of rows an extra step shows: 64 rows in runs of 64 equal keys 6.3 / 7.1, 64 such pairs 6.7 / 8.0 (2 048 of
+// them 59.6 / 53.0 and 72.9 / 64.7).  Tried and left out: a pair's first score row through shared memory as well, or a single row (one row
 // 6.2 -> 7.0 us: a latency more where there is no row ahead); keys turned into distances in place (one more pass over
 // them); additions of the histogram's addresses by multiply-add (no change; for the marks below it gave 3 %).
 // (A pair's second score row is staged behind it: at 80 bytes behind a 128-byte boundary 2 048 pairs of 16 384 keys, half to full
@@ -1437,7 +1442,7 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                 in_bin = sm.sel_count;
                 if (in_bin == need || in_bin <= 32u) break;
                 // Many keys in one bin: equal ones as a rule.  What they span, from the registers, instead of the bin's width
-                // (2 048 rows of which all but 1.4 % are zero: 114 us with two more histograms, now 84).
+                // (2 048 rows of which all but 1.4 % are zero, before they were counted by value: 114 us with two more histograms, 84 so).
                 // (0x7fffffff, the image of -0 if it had one, is no key's: decoded, it would let the zeros of the bin ahead in again.)
                 if (top_key - lo == 0x7fffffffu) ++lo;
                 const float best = key_score(top_key - lo), worst = key_score(top_key - last);
