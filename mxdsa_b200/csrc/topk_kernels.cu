@@ -16,13 +16,15 @@
 //     (-0 and +0 tie);
 //   * written in ascending j (+ row_offset[r]), then -1 up to topk; topk_length[r] = number selected.
 //
-// Three kernels.  mxdsa_topk_held_kernel, for rows of up to 16 384 keys, counts within an interval that a sample points at,
-// with the row in registers.  mxdsa_topk_pivot_kernel, for rows of more than 16 384 keys, finds a score that somewhat more than
+// Four kernels.  mxdsa_topk_held_kernel, for rows of up to 16 384 keys and, with 1 024 threads, 32 768, counts within an interval that
+// a sample points at, with the row in registers.  mxdsa_topk_spread_kernel, for rows of up to 131 072 keys in calls of so few that two or
+// four CTAs to a row find SMs of their own, does so with the row in the shared memory of a cluster.  mxdsa_topk_pivot_kernel, for
+// other rows of more than 16 384 keys, finds a score that somewhat more than
 // topk keys reach from a sample of every eighth key, lists the keys at or above it in one sweep of the row and selects exactly
 // among those (rows of many equal scores are counted instead); where there are fewer rows than SMs it divides a row among the
-// CTAs of a cluster.  mxdsa_topk_rows_kernel counts every key; it has the rows that neither of the others takes: lists
-// longer than 4096, rows of up to 16 384 keys of which most are taken, up to 148 rows of 16 388 to 32 768 keys, and rows
-// of more than 131 072 keys in calls of so many that they cannot be divided.
+// CTAs of a cluster.  mxdsa_topk_rows_kernel counts every key; it has the rows that none of the others takes: lists
+// longer than 4096, rows of up to 16 384 keys of which most are taken, and rows of more than 131 072 keys in calls of so many
+// that they cannot be divided.
 //
 // Counting every key: exact radix selection on the order-preserving 32-bit image of the float, up to three histogram
 // passes (11 + 11 + 10 bits) with shared-memory atomics, ended where a whole bin is taken (after two, as a rule), keys of a row held in registers (one HBM read
@@ -53,6 +55,8 @@ constexpr int kChunks = 8;                         // float4 loads per thread an
 constexpr int kKpt = kChunks * 4;                  // keys per thread and sweep
 constexpr int kSweep = kThreads * kKpt;            // 16 384 keys
 constexpr int kBins = 2048;
+constexpr int kWide = 1024;                        // threads of the CTAs for longer rows
+constexpr int kHeld = kWide * kKpt;                // 32 768 keys
 constexpr int kStage = 4096;                       // rows of up to this many indices are staged in shared memory
 
 struct TopkShared {
@@ -85,7 +89,7 @@ __device__ __forceinline__ int live_chunks(int sweep, int len) {
 // keeps the work of one from overlapping the next's, which shows where a CTA has its SM to itself; more code shows too, in short
 // rows.  So the histogram passes of pairs are straight where positions are staged (without, registers run out), and the
 // first pass of single rows.  Device time in us, warm L2, of three passes over all keys / a branch per chunk everywhere /
-// this: 20 rows of 32 768 keys, topk 2048 16.5 / 17.3 / 16.4.  Of calls that have another kernel now, then: topk 2048 of 16 384
+// this, of calls that have another kernel now: 20 rows of 32 768 keys, topk 2048 16.5 / 17.3 / 16.4; topk 2048 of 16 384
 // keys 1 row 7.7 / 8.2 / 7.8, 20 pairs 8.2 / 8.45 / 8.25, 2 048 pairs half to full length 94.3 / 72.7 / 70.2; 2 048 rows of 4 096, topk 512
 // 66.2 / 41.8 / 41.7 (straight everywhere: 42.9).
 template <bool STRAIGHT, typename F> __device__ __forceinline__ void for_live_chunks(int live, const F& f) {
@@ -370,7 +374,7 @@ mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride,
 
 // ------------------------------------------------------------------------------------------------ selection by pivot
 //
-// For rows of more than 16 384 keys the kernel above sweeps the row three or four times and spends two or three
+// For the rows of more than 16 384 keys that the two kernels below leave.  The kernel above sweeps the row three or four times and spends two or three
 // shared-memory atomics on every key.  Here
 //   1. every eighth key is a sample; a histogram of their 12 highest bits gives a pivot: the lower edge of the bin of the rank'th
 //      largest, rank = topk/8 + 10 sqrt(topk/8) + 8, so that 8 rank keys reach it, 1.46 topk at topk 4096, 1.66 at 2048, 5.5 at
@@ -885,9 +889,9 @@ __device__ __forceinline__ void emit_part(PivotShared& sm, const float* __restri
 }
 
 // All CTAs of the row call it; pivot_key: the lower edge, to 22 bits, of what the sample pointed at.  True, with
-// nothing written, where the keys above the interval are enough and the list can hold them (RELIST).  Out of line: inlined, the
+// nothing written, where the keys above the interval are enough and the list can hold them.  Out of line: inlined, the
 // kernel spills and the rows that never come here take 3 to 6 % longer.
-template <int GROUP, bool RELIST, bool CLUSTER>
+template <int GROUP, bool CLUSTER>
 __device__ __noinline__ bool recount_row(const float* __restrict__ row0, const float* __restrict__ row1, int begin, int end,
                                          uint32_t parts, uint32_t part, uint32_t pivot_key, int topk,
                                          int32_t* __restrict__ out, int32_t off, int32_t* __restrict__ count) {
@@ -897,7 +901,7 @@ __device__ __noinline__ bool recount_row(const float* __restrict__ row0, const f
     count_part<GROUP>(sm, 0, row0, row1, begin, end, key_score(pivot_key), key_score(pivot_key + 1024u));
     const uint4 all = row_counts<CLUSTER>(sm, 0, parts, part, ahead);
     uint32_t n_sel = (uint32_t)topk, need = n_sel - all.x, key = all.z;
-    const bool inside = all.x < n_sel && all.x + all.y >= n_sel, list = RELIST && all.x >= n_sel && all.x <= (uint32_t)kList;
+    const bool inside = all.x < n_sel && all.x + all.y >= n_sel, list = all.x >= n_sel && all.x <= (uint32_t)kList;
     if (list) n_sel = 0u;
     else if (!inside || all.z != all.w) {
         // digits of 11, 11 and 10 bits of the distance from the smallest usable key, or the last one alone; the histograms
@@ -933,7 +937,7 @@ __device__ __noinline__ bool recount_row(const float* __restrict__ row0, const f
     return list;
 }
 
-template <int GROUP, bool MULTI, bool CLUSTER>
+template <int GROUP, bool CLUSTER>
 __global__ void __launch_bounds__(kThreads, 2)
 mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
                         const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
@@ -957,39 +961,28 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
             begin = min((int)part * each, len);      // an empty part begins at len, multiple of four or not: it loads nothing
             end = min(begin + each, len);
         }
-        const int nsweeps = MULTI ? (end - begin + kSweep - 1) / kSweep : 1;
+        const int nsweeps = (end - begin + kSweep - 1) / kSweep;
 
         // ---- 1. the pivot
-        float s[kKpt];                                // MULTI: the samples first, then a sweep at a time
-        if (!MULTI) load_scores<GROUP, kChunks>(row0, row1, begin, end, s);
+        float s[kKpt];                                // the samples first, then a sweep at a time
         uint32_t pivot_key = kMinKey;
         bool listed = true;                           // the list is expected to hold what reaches the pivot
         if (len > kShortRow) {                        // the same for all CTAs of the cluster
 #pragma unroll
             for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(&sm.hist[i * kBins + 4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
             if (CLUSTER && tid == 0) sm.negative = 0u;
-            constexpr int kSamples = MULTI ? 4 * kMaxSweeps : 4;
+            constexpr int kSamples = 4 * kMaxSweeps;
             uint32_t smp[kSamples];
-            if (MULTI) {
-                // Four threads take 16 adjacent keys (64 bytes) out of 128, another eighth in each 128 and sweep: a row is looked
-                // at evenly wherever it ends, where good scores come with a period, and where they are neighbours.
+            // Four threads take 16 adjacent keys (64 bytes) out of 128, another eighth in each 128 and sweep: a row is looked
+            // at evenly wherever it ends, where good scores come with a period, and where they are neighbours.
 #pragma unroll
-                for (int sw = 0; sw < kMaxSweeps; ++sw) {
-                    const int j = begin + sw * kSweep + (tid >> 2) * 128 + ((5 * (tid >> 2) + 3 * warp + sw) & 7) * 16 + 4 * (tid & 3);
-                    const float4 v = load_scores4<GROUP>(row0, row1, j, end);
-                    s[4 * sw] = v.x; s[4 * sw + 1] = v.y; s[4 * sw + 2] = v.z; s[4 * sw + 3] = v.w;
-                }
-#pragma unroll
-                for (int i = 0; i < kSamples; ++i) smp[i] = score_key(s[i % kKpt]);
-            } else {                                  // one of four keys of every other chunk, even or odd by warp
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float* c0 = &s[8 * i];
-                    const float a = warp & 1 ? c0[4] : c0[0], b = warp & 1 ? c0[5] : c0[1];
-                    const float c = warp & 1 ? c0[6] : c0[2], d = warp & 1 ? c0[7] : c0[3];
-                    smp[i] = score_key(lane & 2 ? (lane & 1 ? d : c) : (lane & 1 ? b : a));
-                }
+            for (int sw = 0; sw < kMaxSweeps; ++sw) {
+                const int j = begin + sw * kSweep + (tid >> 2) * 128 + ((5 * (tid >> 2) + 3 * warp + sw) & 7) * 16 + 4 * (tid & 3);
+                const float4 v = load_scores4<GROUP>(row0, row1, j, end);
+                s[4 * sw] = v.x; s[4 * sw + 1] = v.y; s[4 * sw + 2] = v.z; s[4 * sw + 3] = v.w;
             }
+#pragma unroll
+            for (int i = 0; i < kSamples; ++i) smp[i] = score_key(s[i]);
             __syncthreads();
             // The 12 highest bits, the sign among them: an eighth of a power of two to a bin.  Where that many samples come with the
             // rank'th, its bin's lower edge is the pivot, otherwise its next 11 bits are looked at (fewer usable samples than
@@ -1052,7 +1045,7 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
                 bool fits = true;
 #pragma unroll 1
                 for (int sw = 0; sw < nsweeps && fits; ++sw) {
-                    if (MULTI) load_scores<GROUP, kChunks>(row0, row1, begin + sw * kSweep, end, s);
+                    load_scores<GROUP, kChunks>(row0, row1, begin + sw * kSweep, end, s);
                     fits = list_sweep(sm, s, pivot, begin + sw * kSweep, end, n);
                 }
                 key_max = sm.key_max;
@@ -1083,9 +1076,7 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
                 else __syncthreads();
                 break;
             }
-            // (a row that is held in registers is not listed twice: it would have to be kept there across the call)
-            if (!recount_row<GROUP, MULTI, CLUSTER>(row0, row1, begin, end, parts, part, pivot_key, topk, out, off, count)) break;
-            if (!MULTI) break;
+            if (!recount_row<GROUP, CLUSTER>(row0, row1, begin, end, parts, part, pivot_key, topk, out, off, count)) break;
             pivot_key += 1024u;
             listed = true;
         }
@@ -1094,7 +1085,7 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 
 // ------------------------------------------------------------------------------------------------ rows held in registers
 //
-// For rows of up to 16 384 keys.  The row is read once and stays in registers; what each key costs in instructions is the
+// For rows of up to 16 384 keys, or 32 768 with twice the threads.  The row is read once and stays in registers; what each key costs in instructions is the
 // bound, so that as few steps as possible look at all of them:
 //   1. a histogram of every eighth key by its 11 highest bits gives a score that a little more than topk keys reach: the lower
 //      edge of the bin of the rank'th largest, rank = topk/8 + 4 sqrt(topk/8) + 4; the same barriers give the row's maximum;
@@ -1113,13 +1104,15 @@ mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride
 // 12 288 keys, 2.2 of them per cycle and SM.  Counting all keys twice (mxdsa_topk_rows_kernel) takes 1 440.  Per call, that kernel /
 // this one, us, topk 2048 unless said: 2 048 pairs of 16 384 keys, half to full length 69.3 / 61.1, 2 048 single rows 64.5 / 56.3,
 // 20 of them, topk 512 7.1 / 5.7; 1 951 pairs of 3 172 keys, topk 512, 37.0 / 32.6; 8 000 rows of 1 024, topk 256, 131 / 103; 300 of 4 096,
-// topk 512, 9.1 / 7.6.  In one wave of rows an extra step shows: 64 rows in runs of 64 equal keys 6.3 / 7.1, 64 such pairs 6.7 / 8.0 (2 048 of
+// topk 512, 9.1 / 7.6.  With 1 024 threads, by counting or by pivot / so: 148 rows of 32 768 keys 16.7 / 9.5, pairs 19.9 / 11.2, 2 048 rows 122 / 107,
+// pairs 173 / 128 (more at the dispatch).  In one wave of rows an extra step shows: 64 rows in runs of 64 equal keys 6.3 / 7.1, 64 such pairs 6.7 / 8.0 (2 048 of
 // them 59.6 / 53.0 and 72.9 / 64.7).  Tried and left out: a pair's first score row through shared memory as well, or a single row (one row
 // 6.2 -> 7.0 us: a latency more where there is no row ahead); keys turned into distances in place (one more pass over
 // them); additions of the histogram's addresses by multiply-add (no change; for the marks below it gave 3 %).
 // (A pair's second score row is staged behind it: at 80 bytes behind a 128-byte boundary 2 048 pairs of 16 384 keys, half to full
 // length, take 66.2 us, at 16 64.1, on a boundary 61.7; 64 full pairs 7.5, 7.25, 6.9.)
-struct __align__(128) RowShared {
+template <int THREADS> struct __align__(128) RowShared {
+    static constexpr int kWarps = THREADS / 32;
     uint32_t sample[kBins], hist[kBins + 32];      // + a bin per lane that nobody reads
     uint32_t warp_tot[kWarps], warp_max[kWarps], warp_gt[kWarps], warp_in[kWarps];
     uint32_t warp_min[kWarps];                     // (not warp_in: no barrier stands between its reads and the counts of equal keys)
@@ -1131,16 +1124,18 @@ struct __align__(128) RowShared {
 
 // The bin of the k-th entry counted from bin 0 (from the last bin: TOP), from the histogram `hist`; sel_*.  Returns the
 // total; nothing is selected where it is below k.  Ends with a barrier.
-template <bool TOP>
-__device__ __forceinline__ uint32_t row_locate(RowShared& sm, const uint32_t* hist, uint32_t k) {
+template <bool TOP, int THREADS>
+__device__ __forceinline__ uint32_t row_locate(RowShared<THREADS>& sm, const uint32_t* hist, uint32_t k) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int at = TOP ? kBins / 4 - 1 - tid : tid;
-    const uint4 h = *reinterpret_cast<const uint4*>(&hist[4 * at]);
+    uint4 h = make_uint4(0u, 0u, 0u, 0u);
+    if (THREADS == kBins / 4 || tid < kBins / 4) h = *reinterpret_cast<const uint4*>(&hist[4 * at]);
     const uint32_t b[4] = {TOP ? h.w : h.x, TOP ? h.z : h.y, TOP ? h.y : h.z, TOP ? h.x : h.w};
     const uint32_t local = h.x + h.y + h.z + h.w;
     const uint32_t inc = warp_inclusive_scan(local, lane);
     if (lane == 31) sm.warp_tot[warp] = inc;
     __syncthreads();
+    constexpr int kWarps = THREADS / 32;
     const uint32_t wt = lane < kWarps ? sm.warp_tot[lane] : 0u;
     const uint32_t total = __reduce_add_sync(0xffffffffu, wt);
     uint32_t run = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u) + inc - local;
@@ -1213,7 +1208,9 @@ struct ByValue {
 };
 
 // What the keys of a bin span, distances from the maximum, from each thread's largest and smallest of them.  One barrier.
-__device__ __forceinline__ void row_span(RowShared& sm, uint32_t top_key, float most, float least, uint32_t& lo, uint32_t& last) {
+template <int THREADS>
+__device__ __forceinline__ void row_span(RowShared<THREADS>& sm, uint32_t top_key, float most, float least, uint32_t& lo, uint32_t& last) {
+    constexpr int kWarps = THREADS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t warp_most = __reduce_max_sync(0xffffffffu, score_key(most));
     const uint32_t warp_least = __reduce_min_sync(0xffffffffu, score_key(least));
@@ -1227,28 +1224,114 @@ __device__ __forceinline__ void row_span(RowShared& sm, uint32_t top_key, float 
     // (the barriers of the next pass, or of the next row, stand between these reads and the next writes)
 }
 
+// A row of up to 8 192 keys by a CTA of kWide threads: eight adjacent keys to a thread, every key counted by its 11 highest bits
+// and the threshold's bin again by the next 11 and 10.  A sample says little of such a row, and chunks of 4 096 keys leave most warps without
+// any.  Out of line, so that rows that never come here keep their registers.  148 rows of up to 4 096 keys in calls of s_kv 32 768, us, by
+// counting / by sample as longer rows / so: topk 64 5.4 / 6.6 / 6.2, 512 5.2 / 7.8 / 5.8, 2 048 5.2 / 7.9 / 6.1, 4 096 4.8 / 6.4 / 5.8.
+// (The same two shortcuts within the kernel for held rows, or the lowest sample as a pivot: rows that never need them 2 to 5 % slower.)
+constexpr int kShortHeld = 8192;
 template <int GROUP>
-__global__ void __launch_bounds__(kThreads, 2)
+__device__ __noinline__ void short_row(const float* __restrict__ row0, const float* __restrict__ row1, int len, int topk,
+                                       int32_t* __restrict__ out, int32_t off, int32_t* __restrict__ count) {
+    constexpr int THREADS = kWide;
+    extern __shared__ __align__(16) uint8_t topk_smem[];
+    RowShared<THREADS>& sm = *reinterpret_cast<RowShared<THREADS>*>(topk_smem);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, j = 8 * tid;
+    uint32_t key[8];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+        const float4 f = load_scores4<GROUP>(row0, row1, j + 4 * h, len);
+        key[4 * h] = score_key(f.x); key[4 * h + 1] = score_key(f.y); key[4 * h + 2] = score_key(f.z); key[4 * h + 3] = score_key(f.w);
+    }
+    uint32_t threshold = kMinKey, need = 0xffffffffu, equal = need;      // all candidates
+    if (len > topk) {
+        if (tid < kBins / 4) {
+            *reinterpret_cast<uint4*>(&sm.sample[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        __syncthreads();
+        if (j < len) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) atomicAdd(&sm.sample[key[i] >> 21], 1u);      // (what is no candidate: bins 0 to 3)
+        }
+        __syncthreads();
+        row_locate<true>(sm, sm.sample, (uint32_t)topk);
+        if (sm.sel_bin >= 4u) {
+            threshold = sm.sel_bin << 21;
+            need = (uint32_t)topk - sm.sel_ahead;
+            equal = sm.sel_count;
+            if (equal != need) {
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    if (key[i] - threshold < 1u << 21) atomicAdd(&sm.hist[(key[i] - threshold) >> 10], 1u);
+                __syncthreads();
+                if (tid < kBins / 4) *reinterpret_cast<uint4*>(&sm.sample[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+                row_locate<true>(sm, sm.hist, need);
+                threshold += sm.sel_bin << 10;
+                need -= sm.sel_ahead;
+                equal = sm.sel_count;
+                if (equal != need) {
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (key[i] - threshold < 1u << 10) atomicAdd(&sm.sample[key[i] - threshold], 1u);
+                    __syncthreads();
+                    row_locate<true>(sm, sm.sample, need);
+                    threshold += sm.sel_bin;
+                    need -= sm.sel_ahead;
+                    equal = sm.sel_count;
+                }
+            }
+        }
+    }
+    // selected: keys from the threshold on, or those above it and the first `need` equal ones
+    const bool ties = equal != need;
+    uint32_t gt = 0u, eq = 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        gt += (ties ? key[i] > threshold : key[i] >= threshold) ? 1u : 0u;
+        eq += ties && key[i] == threshold ? 1u : 0u;
+    }
+    const uint32_t own = gt | eq << 16, upto = warp_inclusive_scan(own, lane);
+    if (lane == 31) sm.warp_gt[warp] = upto;
+    __syncthreads();
+    const uint32_t of = sm.warp_gt[lane];
+    const uint32_t ahead = __reduce_add_sync(0xffffffffu, lane < warp ? of : 0u) + upto - own, total = __reduce_add_sync(0xffffffffu, of);
+    uint32_t q = ahead >> 16, a = (ahead & 0xffffu) + min(q, need);
+    const uint32_t n_sel = (total & 0xffffu) + min(total >> 16, need);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const bool is_eq = ties && key[i] == threshold, is_gt = key[i] >= threshold && !is_eq;
+        if (is_gt || (is_eq && q < need)) out[a++] = j + i + off;
+        q += is_eq ? 1u : 0u;
+    }
+    for (uint32_t pos = n_sel + tid; pos < (uint32_t)topk; pos += THREADS) out[pos] = -1;
+    if (count != nullptr && tid == 0) *count = (int32_t)n_sel;
+    __syncthreads();
+}
+
+template <int GROUP, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
                        const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
                        int32_t* __restrict__ topk_length, int rows, int s_kv, int topk, uint32_t sample_rank) {
     extern __shared__ __align__(16) uint8_t topk_smem[];
-    RowShared& sm = *reinterpret_cast<RowShared*>(topk_smem);
+    RowShared<THREADS>& sm = *reinterpret_cast<RowShared<THREADS>*>(topk_smem);
+    constexpr int kWarps = THREADS / 32, kChunkKeys = THREADS * 4;
     const uint32_t stage0 = (uint32_t)__cvta_generic_to_shared(sm.stage);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     int len = s_kv;
     if (lengths != nullptr && (int)blockIdx.x < rows) len = min(max(__ldg(lengths + blockIdx.x), 0), s_kv);
     // A pair's second score row comes through shared memory, asked for while the row before is worked on; a thread copies
     // what it will read itself.
-    float4* ahead = reinterpret_cast<float4*>(topk_smem + sizeof(RowShared)) + tid;
+    float4* ahead = reinterpret_cast<float4*>(topk_smem + sizeof(RowShared<THREADS>)) + tid;
     const auto ask = [&](int row, int n) {
-        const int per_warp = 128 * ((n + 2047) >> 11), j = warp * per_warp + 4 * lane, end = min(n, (warp + 1) * per_warp);
+        const int per_warp = 128 * ((n + kChunkKeys - 1) / kChunkKeys), j = warp * per_warp + 4 * lane, end = min(n, (warp + 1) * per_warp);
         const float* from = scores + ((long long)row * 2 + 1) * score_stride + j;
         const uint32_t to = (uint32_t)__cvta_generic_to_shared(ahead);
 #pragma unroll
         for (int c = 0; c < kChunks; ++c)
             if (j + 128 * c < end)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + c * kThreads * 16), "l"(from + 128 * c) : "memory");
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + c * THREADS * 16), "l"(from + 128 * c) : "memory");
     };
     if (GROUP == 2 && (int)blockIdx.x < rows) ask(blockIdx.x, len);
     for (int r = blockIdx.x, next_len; r < rows; r += gridDim.x, len = next_len) {
@@ -1256,12 +1339,24 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
         next_len = s_kv;
         if (lengths != nullptr && next < rows) next_len = min(max(__ldg(lengths + next), 0), s_kv);
 
-        *reinterpret_cast<uint4*>(&sm.sample[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
-        *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        if (THREADS == kWide && len <= kShortHeld) {
+            if (GROUP == 2) {
+                asm volatile("cp.async.wait_all;" ::: "memory");
+                if (next < rows) ask(next, next_len);
+            }
+            const float* row0 = scores + (long long)r * GROUP * score_stride;
+            short_row<GROUP>(row0, row0 + score_stride, len, topk, indices + (long long)r * index_stride,
+                             row_offset != nullptr ? __ldg(row_offset + r) : 0, topk_length != nullptr ? topk_length + r : nullptr);
+            continue;
+        }
+        if (THREADS == kBins / 4 || tid < kBins / 4) {
+            *reinterpret_cast<uint4*>(&sm.sample[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+            *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        }
         if (tid == 0) sm.few_n = 0u;
 
         // ---- the row: chunk c of this thread holds keys j0 + 128 c .. + 3
-        const int chunks = (len + 2047) >> 11;       // the same for all warps
+        const int chunks = (len + kChunkKeys - 1) / kChunkKeys;       // the same for all warps
         const int j0 = warp * 128 * chunks + 4 * lane;
         const int limit = min(len, (warp + 1) * 128 * chunks);
         float key[kKpt];                             // (from chunk `chunks` rounded up to two on: nothing)
@@ -1278,7 +1373,7 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
 #pragma unroll
             for (int c = 0; c < kChunks; ++c) {
                 if (c >= chunks) break;
-                const float4 f = ahead[c * kThreads];
+                const float4 f = ahead[c * THREADS];
                 key[4 * c] = fmaxf(key[4 * c], f.x);
                 key[4 * c + 1] = fmaxf(key[4 * c + 1], f.y);
                 key[4 * c + 2] = fmaxf(key[4 * c + 2], f.z);
@@ -1335,7 +1430,7 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
 #pragma unroll 1
             while (true) {
                 if (!first) {
-                    *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+                    if (THREADS == kBins / 4 || tid < kBins / 4) *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
                     __syncthreads();
                 }
                 const int sh = max(21 - __clz(span), 0);
@@ -1549,7 +1644,7 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
         }
         __syncthreads();                             // (the next row clears the histograms and few_n behind it)
         if (((topk | (int)(index_stride & 3) | (int)((uintptr_t)indices >> 2 & 3)) & 3) == 0) {      // rows of whole, aligned fours
-            for (uint32_t pos = 4 * tid; pos < (uint32_t)topk; pos += 4 * kThreads) {
+            for (uint32_t pos = 4 * tid; pos < (uint32_t)topk; pos += 4 * THREADS) {
                 int4 v = *reinterpret_cast<const int4*>(&sm.stage[pos]);
                 if (pos + 4 > n_sel) {
                     v.x = pos < n_sel ? v.x : -1;
@@ -1560,10 +1655,538 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                 *reinterpret_cast<int4*>(&out[pos]) = v;
             }
         } else {
-            for (uint32_t pos = tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = pos < n_sel ? sm.stage[pos] : -1;
+            for (uint32_t pos = tid; pos < (uint32_t)topk; pos += THREADS) out[pos] = pos < n_sel ? sm.stage[pos] : -1;
         }
         if (topk_length != nullptr && tid == 0) topk_length[r] = (int32_t)n_sel;
     }
+}
+
+// ------------------------------------------------------------------------------------------------ rows held by a cluster
+//
+// For rows of 32 772 to 131 072 keys, few enough that two or four CTAs to a row find SMs of their own.  Each reads its part of
+// the row once and keeps it in shared memory:
+//   1. a histogram of every eighth key by its 11 highest bits, summed over the row's CTAs, gives a pivot that a little more than topk
+//      keys reach; where that comes to more than four keys a thread, the pivot's bin is looked at by the next 10 bits as well;
+//   2. the places of the keys that reach the pivot are listed in ascending order; a thread has adjacent keys, so that the order
+//      follows from one sum; from here on only the list is looked at, a few entries to a thread, in registers;
+//   3. a histogram of the list's distances from the row's maximum over just the interval down to the pivot, summed again, gives the
+//      bin of the topk-th: taken as a whole, or its few keys ranked among themselves, or narrowed to what they span; ballots
+//      turn the list into positions, each CTA writes its own.
+// Thousands of keys that even the second look does not tell apart are equal ones, as a rule: then the keys above them and the
+// first of these are selected from the bits of step 2, without a list.  A row of fewer samples than the rank has its list from the
+// lowest score on, in bins of equal width in value; a row of no more keys than topk needs none.  A sample that misled
+// costs another list and histogram.
+// What the CTAs tell one another is written into the others' shared memory ahead of a barrier of the cluster, not read from
+// there behind it: a read waits for its way there and back, a write for nothing, and nobody reads from a CTA that may have left.
+//
+// Bound: latency between the barriers (four of the cluster, 900 to 1 100 cycles each, about twelve of the CTA) and instruction issue (980
+// instructions per warp for 32 768 keys, 37 % of the slots).  64 rows of 65 536 keys, topk 2048, by pivot / as this kernel came about, us: 16.3;
+// with the keys in registers of two CTAs of 512 threads to an SM, histograms of 2 048 bins read from the peers 14.1, of 1 024 bins 12.1; keys
+// in shared memory and listed, one CTA of 1 024 threads to an SM 11.2; written to the peers instead of read 11.0.  Five values 16.5 / 11.3, all
+// but 1.4 % zero 19.0 / 12.9, scores around -50 18.4 / 12.4, runs of 64 equal ones 16.4 / 14.1.  Tried and left out: the keys of step 2 fetched
+// from shared memory ahead of the pivot (registers: 11.0 -> 11.4), bins and loops out of line or not unrolled (11.2 -> 11.6).
+constexpr int kWideWarps = kWide / 32;
+constexpr int kFine = 1024;                        // bins
+template <int PARTS> struct __align__(128) SpreadShared {
+    float row[kHeld + 32];              // this CTA's part of the row, -inf behind it
+    uint16_t list[kHeld];                          // places in it of the keys that reach the pivot, ascending
+    uint32_t bins[2 * kFine];                      // histogram of the sample; then `hist` is the first half
+    uint4 slot[2][PARTS - 1][kFine / 8];           // the other CTAs' histograms, 16 bits to a bin, in turns
+    uint32_t tops[PARTS][kWideWarps], bottoms[PARTS][kWideWarps];      // largest and smallest keys of all the row's warps
+    uint2 counts[PARTS][kWideWarps];               // nearer than the bin | in it
+    uint2 spans[PARTS][kWideWarps];                // what a bin spans
+    uint2 few[PARTS][32];                          // (distance, position) of the keys of a bin of up to 32
+    uint32_t warp_tot[kFine / 128], warp_n[kWideWarps];
+    uint32_t sel_bin, sel_ahead, sel_count;
+    uint32_t few_n;
+    uint2 cut;                                     // the last of the few that is taken ...
+    uint32_t taken[32];                            // ... and the positions of all that are
+};
+
+__device__ __forceinline__ void peer_store(uint32_t a, uint32_t v) {
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void peer_store2(uint32_t a, uint2 v) {
+    asm volatile("st.shared::cluster.v2.u32 [%0], {%1, %2};" ::"r"(a), "r"(v.x), "r"(v.y) : "memory");
+}
+__device__ __forceinline__ void peer_store4(uint32_t a, uint4 v) {
+    asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+
+// The bin of the k-th entry counted from bin 0 (from the last bin: TOP) of the histogram that the CTAs of a row have together, and
+// what lies ahead of it (sel_*).  Returns the total; nothing is selected where it is below k.  `turn` counts the calls.
+template <bool TOP, int PARTS>
+__device__ __forceinline__ uint32_t spread_locate(SpreadShared<PARTS>& sm, const uint32_t* hist, uint32_t part, uint32_t k, uint32_t& turn) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    __syncthreads();
+    if (tid < kFine / 8) {                           // (a bin holds 32 768 keys at most)
+        const uint4 a = *reinterpret_cast<const uint4*>(&hist[8 * tid]), b = *reinterpret_cast<const uint4*>(&hist[8 * tid + 4]);
+        const uint4 v = make_uint4(a.x | a.y << 16, a.z | a.w << 16, b.x | b.y << 16, b.z | b.w << 16);
+#pragma unroll
+        for (int c = 1; c < PARTS; ++c) peer_store4(peer_address(&sm.slot[turn & 1][PARTS - 1 - c][tid], (part + c) % PARTS), v);
+    }
+    cluster_barrier();
+    const int at = TOP ? kFine / 4 - 1 - tid : tid;
+    uint4 h = make_uint4(0u, 0u, 0u, 0u);
+    uint32_t inc = 0u, local = 0u;
+    if (warp < kFine / 128) {
+        h = *reinterpret_cast<const uint4*>(&hist[4 * at]);
+#pragma unroll
+        for (int c = 0; c < PARTS - 1; ++c) {
+            const uint2 o = reinterpret_cast<const uint2*>(sm.slot[turn & 1][c])[at];
+            h = make_uint4(h.x + (o.x & 0xffffu), h.y + (o.x >> 16), h.z + (o.y & 0xffffu), h.w + (o.y >> 16));
+        }
+        local = h.x + h.y + h.z + h.w;
+        inc = warp_inclusive_scan(local, lane);
+        if (lane == 31) sm.warp_tot[warp] = inc;
+    }
+    ++turn;
+    __syncthreads();
+    const uint32_t wt = lane < kFine / 128 ? sm.warp_tot[lane] : 0u;
+    const uint32_t total = __reduce_add_sync(0xffffffffu, wt);
+    if (warp < kFine / 128) {
+        uint32_t run = __reduce_add_sync(0xffffffffu, lane < warp ? wt : 0u) + inc - local;
+        if (run < k && run + local >= k) {
+            const uint32_t b[4] = {TOP ? h.w : h.x, TOP ? h.z : h.y, TOP ? h.y : h.z, TOP ? h.x : h.w};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (run < k && run + b[i] >= k) {
+                    sm.sel_bin = TOP ? 4 * at + 3 - i : 4 * at + i;
+                    sm.sel_ahead = run;
+                    sm.sel_count = b[i];
+                }
+                run += b[i];
+            }
+        }
+    }
+    __syncthreads();
+    return total;
+}
+
+template <int GROUP, int PARTS>
+__global__ void __cluster_dims__(PARTS, 1, 1) __launch_bounds__(kWide, 1)
+mxdsa_topk_spread_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
+                         const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
+                         int32_t* __restrict__ topk_length, int s_kv, int topk, uint32_t sample_rank) {
+    constexpr int kEntries = 4;                      // entries of the list that a thread keeps in registers (eight: 2 to 6 % slower)
+    extern __shared__ __align__(16) uint8_t topk_smem[];
+    SpreadShared<PARTS>& sm = *reinterpret_cast<SpreadShared<PARTS>*>(topk_smem);
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");      // peers are written to only once they run
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int part = (int)cluster_rank(), r = (int)blockIdx.x / PARTS;
+    int len = s_kv;
+    if (lengths != nullptr) len = min(max(__ldg(lengths + r), 0), s_kv);
+    // this CTA's keys: the row's own length is divided, in whole groups of four
+    const int each = ((len + PARTS - 1) / PARTS + 3) & ~3;
+    const int begin = min(part * each, len), n = min(each, len - begin);
+    const bool blind = (uint32_t)(len + 7) >> 3 < sample_rank;       // a row of fewer samples than that
+
+    if (tid < kFine / 2) *reinterpret_cast<uint4*>(&sm.bins[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+    if (tid == 0) sm.few_n = 0u;
+
+    // ---- the part into shared memory, chunk c of this thread keys 4 (c kWide + tid) .. + 3
+    const float* from = scores + (long long)r * GROUP * score_stride + begin;
+    float key[kKpt];
+    if (GROUP == 2) {
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+            const int j = 4 * (c * kWide + tid);
+            if (j < n)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(&sm.row[j])),
+                             "l"(from + score_stride + j) : "memory");
+        }
+    }
+#pragma unroll
+    for (int c = 0; c < kChunks; ++c) {
+        const int j = 4 * (c * kWide + tid);
+        if (j < n) {                                 // past it the registers hold anything until below
+            const float4 f = __ldg(reinterpret_cast<const float4*>(from + j));
+            key[4 * c] = f.x; key[4 * c + 1] = f.y; key[4 * c + 2] = f.z; key[4 * c + 3] = f.w;
+        }
+    }
+    __syncthreads();                                 // the histogram is clear
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (GROUP == 2) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < kChunks; ++c) {
+            const int j = 4 * (c * kWide + tid);
+            if (j >= n) break;
+            const float4 f = *reinterpret_cast<const float4*>(&sm.row[j]);
+            key[4 * c] = fmaxf(key[4 * c], f.x);
+            key[4 * c + 1] = fmaxf(key[4 * c + 1], f.y);
+            key[4 * c + 2] = fmaxf(key[4 * c + 2], f.z);
+            key[4 * c + 3] = fmaxf(key[4 * c + 3], f.w);
+        }
+    }
+
+    // ---- 1. the sample, and the maximum.  Even lanes look at one of their four keys in even chunks, odd ones in odd chunks
+    float top = -CUDART_INF_F, bottom = CUDART_INF_F;
+    uint32_t smp[kChunks / 2] = {};
+#pragma unroll
+    for (int c = 0; c < kChunks; c += 2) {           // chunks are worked on two by two
+        if (4 * c * kWide >= n) break;
+        const int j = 4 * (c * kWide + tid);
+        if (4 * (c + 2) * kWide > n) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (j + (e >> 2) * 4 * kWide + (e & 3) >= n) key[4 * c + e] = -CUDART_INF_F;
+        }
+        float* const to = &sm.row[j];
+        *reinterpret_cast<float4*>(to) = make_float4(key[4 * c], key[4 * c + 1], key[4 * c + 2], key[4 * c + 3]);
+        *reinterpret_cast<float4*>(to + 4 * kWide) = make_float4(key[4 * c + 4], key[4 * c + 5], key[4 * c + 6], key[4 * c + 7]);
+        smp[c >> 1] = score_key(lane & 1 ? key[4 * c + 4 + (c >> 1)] : key[4 * c + (c >> 1)]);
+        if (!blind) atomicAdd(&sm.bins[smp[c >> 1] >> 21], 1u);
+#pragma unroll
+        for (int i = 4 * c; i < 4 * c + 8; i += 2) top = fmax3(top, key[i], key[i + 1]);
+        if (blind) {
+#pragma unroll
+            for (int i = 4 * c; i < 4 * c + 8; ++i)
+                if (key[i] > -CUDART_INF_F) bottom = fminf(bottom, key[i]);
+        }
+    }
+    if (tid < 8) {                                   // (what is read of groups behind the last chunk)
+        const int j = (n + 8 * kWide - 1) / (8 * kWide) * (8 * kWide) + 4 * tid;
+        *reinterpret_cast<float4*>(&sm.row[j]) = make_float4(-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F);
+    }
+    const uint32_t warp_top = __reduce_max_sync(0xffffffffu, score_key(top));
+    if (lane < PARTS) peer_store(peer_address(&sm.tops[part][warp], lane), warp_top);
+    uint32_t turn = 0u, pivot = kMinKey, bottom_key = 0u;
+    bool heavy = false;
+    if (blind) {
+        const uint32_t warp_bottom = __reduce_min_sync(0xffffffffu, score_key(bottom));
+        if (lane < PARTS) peer_store(peer_address(&sm.bottoms[part][warp], lane), warp_bottom);
+        cluster_barrier();
+        bottom_key = 0xffffffffu;
+#pragma unroll
+        for (int c = 0; c < PARTS; ++c) bottom_key = min(bottom_key, sm.bottoms[c][lane]);
+        bottom_key = __reduce_min_sync(0xffffffffu, bottom_key);
+    } else {
+        uint32_t k = sample_rank, edge = 0x80000000u, total = spread_locate<true, PARTS>(sm, sm.bins + kFine, part, k, turn);
+        if (total < k) {
+            k -= total;
+            edge = 0u;
+            total = spread_locate<true, PARTS>(sm, sm.bins, part, k, turn);
+        }
+        if (total >= k) {
+            edge += sm.sel_bin << 21;
+            k -= sm.sel_ahead;
+            if (sample_rank - k + sm.sel_count > PARTS * kWide / 2) {
+                __syncthreads();                     // sel_* have been read
+                if (tid < kFine / 4) *reinterpret_cast<uint4*>(&sm.bins[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+                __syncthreads();
+#pragma unroll
+                for (int i = 0; i < kChunks / 2; ++i)
+                    if (smp[i] - edge < 1u << 21) atomicAdd(&sm.bins[(smp[i] - edge) >> 11], 1u);
+                spread_locate<true, PARTS>(sm, sm.bins, part, k, turn);
+                edge += sm.sel_bin << 11;
+                k -= sm.sel_ahead;
+                heavy = sm.sel_count > PARTS * kWide / 4;
+            }
+            pivot = max(edge, kMinKey);
+        }
+    }
+    uint32_t top_key = 0u;
+#pragma unroll
+    for (int c = 0; c < PARTS; ++c) top_key = max(top_key, sm.tops[c][lane]);
+    top_key = __reduce_max_sync(0xffffffffu, top_key);
+
+    // A thread has `own` adjacent groups of four keys: an odd number of them, or eight, which its neighbours then begin with another
+    // of: no bank conflicts.  Bit i of a mask is key (i + first) % 32 of the thread.
+    int groups = (n + 4 * kWide - 1) / (4 * kWide);
+    groups += groups < kChunks && (groups & 1) == 0 ? 1 : 0;
+    const int mine = 4 * groups * tid, first = groups == kChunks ? 4 * (lane & 7) : 0;
+
+    int32_t* out = indices + (long long)r * index_stride;
+    const int32_t off = (row_offset != nullptr ? __ldg(row_offset + r) : 0) + begin;
+    uint32_t n_sel = 0u;
+    bool done = top_key < kMinKey;                   // no candidate at all
+    if (heavy && !done) {
+        // ---- Thousands of keys in an interval of 2048 bit patterns: equal ones, as a rule.  Then the keys above it and the first
+        // of these are what is selected.
+        const float reach = key_score(pivot), above = key_score(pivot + 2048u);      // (beyond +inf: a NaN, which nothing reaches)
+        uint32_t mask = 0u, inside = 0u;             // above the interval | in it
+        float least = CUDART_INF_F, most = -CUDART_INF_F;
+        if (mine < n) {
+#pragma unroll
+            for (int i = 0; i < kChunks; ++i) {
+                if (i >= groups) break;
+                const float4 f = *reinterpret_cast<const float4*>(&sm.row[mine + ((4 * i + first) & 31)]);
+                const float v[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    if (v[e] >= above) mask |= 1u << (4 * i + e);
+                    else if (v[e] >= reach) {
+                        inside |= 1u << (4 * i + e);
+                        least = fminf(least, v[e]);
+                        most = fmaxf(most, v[e]);
+                    }
+                }
+            }
+            mask = __funnelshift_l(mask, mask, first);
+            inside = __funnelshift_l(inside, inside, first);
+        }
+        const uint2 count = make_uint2(__reduce_add_sync(0xffffffffu, __popc(mask)), __reduce_add_sync(0xffffffffu, __popc(inside)));
+        const uint2 span = make_uint2(__reduce_min_sync(0xffffffffu, score_key(least)), __reduce_max_sync(0xffffffffu, score_key(most)));
+        if (lane < PARTS) {
+            peer_store2(peer_address(&sm.counts[part][warp], lane), count);
+            peer_store2(peer_address(&sm.spans[part][warp], lane), span);
+        }
+        cluster_barrier();
+        uint2 all = make_uint2(0u, 0u), ahead = make_uint2(0u, 0u), range = make_uint2(0xffffffffu, 0u);
+#pragma unroll
+        for (int c = 0; c < PARTS; ++c) {
+            const uint2 x = sm.counts[c][lane], y = sm.spans[c][lane];
+            all = make_uint2(all.x + x.x, all.y + x.y);
+            if (c < part || (c == part && lane < warp)) ahead = make_uint2(ahead.x + x.x, ahead.y + x.y);
+            range = make_uint2(min(range.x, y.x), max(range.y, y.y));
+        }
+        all = make_uint2(__reduce_add_sync(0xffffffffu, all.x), __reduce_add_sync(0xffffffffu, all.y));
+        ahead = make_uint2(__reduce_add_sync(0xffffffffu, ahead.x), __reduce_add_sync(0xffffffffu, ahead.y));
+        range = make_uint2(__reduce_min_sync(0xffffffffu, range.x), __reduce_max_sync(0xffffffffu, range.y));
+        if (all.x >= (uint32_t)topk) pivot += 2048u;                                 // as good a pivot, with fewer keys
+        else if (all.x + all.y < (uint32_t)topk) pivot = kMinKey;                    // the sample misled
+        else if (range.x == range.y) {
+            n_sel = (uint32_t)topk;
+            done = true;
+            const uint32_t need = n_sel - all.x, own = __popc(mask) | __popc(inside) << 16;
+            const uint32_t before = warp_inclusive_scan(own, lane) - own;
+            uint32_t q = ahead.y + (before >> 16), a = ahead.x + (before & 0xffffu) + min(q, need);
+            for (uint32_t m = mask | inside; m != 0u; m &= m - 1u) {
+                const uint32_t i = __ffs(m) - 1;
+                const bool equal = inside >> i & 1u;
+                if (!equal || q < need) out[a++] = mine + (int)i + off;
+                q += equal ? 1u : 0u;
+            }
+        }
+    }
+    if (!done) {
+        // ---- 2. the keys that reach the pivot, a bit each, and the list of their places; their distances from the maximum and the
+        // histogram of these; 3. the bin of the topk-th
+        const uint32_t farthest = top_key - kMinKey;
+        uint32_t span = top_key - min(pivot, top_key), lo = 0u, last = 0u, need = (uint32_t)topk, in_bin = 0u;
+        uint32_t n_list = 0u, i0 = 0u, rounds = 0u;  // this warp's piece of the list begins at i0, `rounds` times 32 entries
+        uint32_t at[kEntries], d[kEntries];          // entries of the list: place, distance
+        n_sel = need;
+        // Without a sample the first bins are of equal width in value, from the maximum to the minimum.  Subtraction and product round
+        // in the order of the scores.  (A reach of infinity, or next to none, has no scale.)
+        const float top_score = key_score(top_key), reach = top_score - key_score(bottom_key);
+        bool valued = blind && reach >= 1e-30f && reach < CUDART_INF_F;
+        const float by = __fdividef(1023.0f, reach);
+        uint32_t at_bin = 0u;
+        const auto value_bin = [&](uint32_t distance) {
+            return min((uint32_t)(int)((top_score - key_score(top_key - distance)) * by), (uint32_t)kFine - 1u);
+        };
+        // entries i0 + 32 (k0 + k) + lane, k < kEntries; nothing: a distance beyond all others
+        const auto entries = [&](uint32_t k0) {
+#pragma unroll
+            for (int k = 0; k < kEntries; ++k) {
+                d[k] = 0xffffffffu;
+                if (k0 + k >= rounds) continue;
+                const uint32_t i = i0 + 32u * (k0 + k) + lane;
+                if (i < n_list) {
+                    at[k] = sm.list[i];
+                    d[k] = top_key - score_key(sm.row[at[k]]);
+                }
+            }
+        };
+        const bool everything = len <= topk;
+        bool list = true;
+#pragma unroll 1
+        while (true) {
+            __syncthreads();                         // what was in the histogram has been read
+            if (tid < kFine / 4) *reinterpret_cast<uint4*>(&sm.bins[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+            const int sh = max(22 - __clz(span), 0);
+            if (list) {
+                uint32_t mask = 0u;
+                if (mine < n) {
+                    const float reach = key_score(pivot);
+                    uint32_t one = 1u;
+                    asm volatile("" : "+r"(one));
+#pragma unroll
+                    for (int i = 0; i < kChunks; ++i) {
+                        if (i >= groups) break;
+                        const float4 f = *reinterpret_cast<const float4*>(&sm.row[mine + ((4 * i + first) & 31)]);
+                        if (f.x >= reach) mask += one << (4 * i);
+                        if (f.y >= reach) mask += one << (4 * i + 1);
+                        if (f.z >= reach) mask += one << (4 * i + 2);
+                        if (f.w >= reach) mask += one << (4 * i + 3);
+                    }
+                }
+                const uint32_t found = __popc(mask), upto = warp_inclusive_scan(found, lane);
+                if (lane == 31) sm.warp_n[warp] = upto;
+                __syncthreads();
+                const uint32_t of = sm.warp_n[lane];
+                const uint32_t place = __reduce_add_sync(0xffffffffu, lane < warp ? of : 0u) + upto - found;
+                n_list = __reduce_add_sync(0xffffffffu, of);
+                rounds = (n_list + kWide - 1) / kWide;
+                i0 = 32u * rounds * warp;
+                const uint32_t ordered = __funnelshift_l(mask, mask, first);
+                for (uint32_t m = mask; m != 0u; m &= m - 1u) {
+                    const uint32_t i = (__ffs(m) - 1 + first) & 31;
+                    sm.list[place + __popc(ordered & ((1u << i) - 1u))] = (uint16_t)(mine + i);
+                }
+                list = false;
+            }
+            __syncthreads();                         // the list is there, the histogram is clear
+            if (everything) {
+                entries(0u);
+                in_bin = need;
+                last = farthest;
+                valued = false;
+                break;
+            }
+            for (uint32_t k0 = 0; k0 < rounds; k0 += kEntries) {
+                entries(k0);
+#pragma unroll
+                for (int k = 0; k < kEntries; ++k)
+                    if (d[k] - lo <= span) atomicAdd(&sm.bins[valued ? value_bin(d[k]) : (d[k] - lo) >> sh], 1u);
+            }
+            const uint32_t total = spread_locate<false, PARTS>(sm, sm.bins, part, need, turn);
+            if (total < need) {                      // only while the interval is the first one
+                if (span < farthest) {               // the sample misled: from the lowest score on
+                    span = farthest;
+                    pivot = kMinKey;
+                    list = true;
+                    continue;
+                }
+                n_sel = need = in_bin = total;       // fewer candidates than topk: all of them
+                last = farthest;
+                valued = false;
+                break;
+            }
+            need -= sm.sel_ahead;
+            in_bin = sm.sel_count;
+            if (valued) {
+                at_bin = sm.sel_bin;
+                if (in_bin <= 32u) break;
+            } else {
+                lo += sm.sel_bin << sh;
+                last = min(lo + (1u << sh) - 1u, farthest);
+                if (in_bin == need || in_bin <= 32u) break;
+            }
+            // Many keys in one bin: equal ones as a rule.  What they span, instead of the bin's width
+            uint32_t least = 0xffffffffu, most = 0u;
+            for (uint32_t k0 = 0; k0 < rounds; k0 += kEntries) {
+                if (rounds > kEntries) entries(k0);
+#pragma unroll
+                for (int k = 0; k < kEntries; ++k) {
+                    if (valued ? d[k] <= farthest && value_bin(d[k]) == at_bin : d[k] >= lo && d[k] <= last) {
+                        least = min(least, d[k]);
+                        most = max(most, d[k]);
+                    }
+                }
+            }
+            least = __reduce_min_sync(0xffffffffu, least);
+            most = __reduce_max_sync(0xffffffffu, most);
+            if (lane < PARTS) peer_store2(peer_address(&sm.spans[part][warp], lane), make_uint2(least, most));
+            cluster_barrier();
+#pragma unroll
+            for (int c = 0; c < PARTS; ++c) {
+                const uint2 x = sm.spans[c][lane];
+                least = min(least, x.x);
+                most = max(most, x.y);
+            }
+            lo = __reduce_min_sync(0xffffffffu, least);
+            last = __reduce_max_sync(0xffffffffu, most);
+            valued = false;
+            if (lo == last) break;
+            span = last - lo;
+        }
+
+        // ---- what is selected of the list
+        const bool whole = in_bin == need && !valued, few = !whole && in_bin <= 32u;
+        uint32_t n_gt = 0u, n_eq = 0u;               // nearer than the bin | in it
+        for (uint32_t k0 = 0; k0 < rounds; k0 += kEntries) {
+            if (rounds > kEntries) entries(k0);
+#pragma unroll
+            for (int k = 0; k < kEntries; ++k) {
+                if (k0 + k >= rounds) break;
+                bool nearer = d[k] < lo, inside = d[k] >= lo && d[k] <= last;
+                if (valued) {
+                    const uint32_t b = d[k] <= farthest ? value_bin(d[k]) : (uint32_t)kFine;
+                    nearer = b < at_bin;
+                    inside = b == at_bin;
+                }
+                n_gt += __popc(__ballot_sync(0xffffffffu, nearer));
+                n_eq += __popc(__ballot_sync(0xffffffffu, inside));
+                if (few && inside) {
+                    const uint32_t slot = atomicAdd(&sm.few_n, 1u);
+#pragma unroll
+                    for (int c = 0; c < PARTS; ++c) peer_store2(peer_address(&sm.few[part][slot], c), make_uint2(d[k], (uint32_t)begin + at[k]));
+                }
+            }
+        }
+        if (lane < PARTS) peer_store2(peer_address(&sm.counts[part][warp], lane), make_uint2(n_gt, n_eq));
+        cluster_barrier();
+        if (few && warp == 0) {                      // rank the few among themselves
+            uint2 own = make_uint2(0xffffffffu, 0xffffffffu);
+            uint32_t before = 0u, m[PARTS];
+#pragma unroll
+            for (int c = 0; c < PARTS; ++c) {
+                m[c] = __reduce_add_sync(0xffffffffu, sm.counts[c][lane].y);
+                if (lane - before < m[c]) own = sm.few[c][lane - before];
+                before += m[c];
+            }
+            uint32_t better = 0u;
+#pragma unroll
+            for (int c = 0; c < PARTS; ++c) {
+                for (uint32_t i = 0; i < m[c]; ++i) {
+                    const uint2 x = sm.few[c][i];
+                    better += (x.x < own.x || (x.x == own.x && x.y < own.y)) ? 1u : 0u;
+                }
+            }
+            const bool taken = lane < (int)in_bin && better < need;
+            sm.taken[lane] = taken ? own.y : 0xffffffffu;
+            if (taken && better == need - 1u) sm.cut = own;
+        }
+        uint32_t a = 0u, q = 0u;
+#pragma unroll
+        for (int c = 0; c < PARTS; ++c) {
+            const uint2 x = sm.counts[c][lane];
+            if (c < part || (c == part && lane < warp)) {
+                a += x.x;
+                q += x.y;
+            }
+        }
+        a = __reduce_add_sync(0xffffffffu, a);
+        uint32_t d_cut = last, at_cut = 0xffffffffu;
+        if (few) {
+            __syncthreads();
+            const uint32_t begins = i0 < n_list ? (uint32_t)begin + sm.list[i0] : 0u;
+            a += __popc(__ballot_sync(0xffffffffu, sm.taken[lane] < begins));
+            d_cut = sm.cut.x;
+            at_cut = sm.cut.y;
+        } else {
+            q = __reduce_add_sync(0xffffffffu, q);
+            a += min(q, need);
+            if (everything) {
+                n_sel = 0u;
+#pragma unroll
+                for (int c = 0; c < PARTS; ++c) n_sel += sm.counts[c][lane].y;
+                n_sel = __reduce_add_sync(0xffffffffu, n_sel);
+            }
+        }
+        const uint32_t before = (1u << lane) - 1u;
+        for (uint32_t k0 = 0; k0 < rounds; k0 += kEntries) {
+            if (rounds > kEntries) entries(k0);
+#pragma unroll
+            for (int k = 0; k < kEntries; ++k) {
+                if (k0 + k >= rounds) break;
+                bool sel = d[k] < d_cut || (d[k] == d_cut && (uint32_t)begin + at[k] <= at_cut);
+                if (!whole && !few) {                // equal keys: the first `need` of the row
+                    const uint32_t equal = __ballot_sync(0xffffffffu, d[k] == last);
+                    sel = d[k] < last || (d[k] == last && q + __popc(equal & before) < need);
+                    q += __popc(equal);
+                }
+                const uint32_t ms = __ballot_sync(0xffffffffu, sel);
+                if (sel) out[a + __popc(ms & before)] = (int)at[k] + off;
+                a += __popc(ms);
+            }
+        }
+    }
+    for (uint32_t pos = n_sel + part * kWide + tid; pos < (uint32_t)topk; pos += PARTS * kWide) out[pos] = -1;
+    if (topk_length != nullptr && part == 0 && tid == 0) topk_length[r] = (int32_t)n_sel;
 }
 
 thread_local int tl_topk_cuda_error = 0;
@@ -1581,22 +2204,40 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return MXDSA_ERR_CUDA;
     const cudaStream_t s = static_cast<cudaStream_t>(p->stream);
-    // By pivot where a row does not fit the registers of a CTA (16 384 keys) and the list fits with its margin.  Shorter
-    // rows are read once and selected from registers, which is faster there throughout: 2048 rows of 16 384 keys, topk 2048
-    // 56 us against 105 by pivot (pairs 69 against 127), 20 rows 6.3 against 15.6.  Longer ones are swept again by counting
-    // for every pass: 2048 rows of 16 388 keys 142 against 119 (pairs 154 against 146).  The line is drawn by s_kv, as lengths
-    // are on the device; where they leave most rows within 16 384 keys counting would still be the faster (those
-    // 2048 rows, half to full length: 65 against 106).
-    // Few rows are divided among CTAs.  A division in two, four or eight is taken while every CTA of the call finds an SM of
+    // Rows that a CTA's registers hold (16 384 keys with 512 threads, two CTAs to an SM; 32 768 with 1 024): counted within an interval that
+    // a sample points at.  Where the sample cannot hold the rank
+    // the interval is all there is, up to -FLT_MAX, and says nothing: such rows stay with the other kernel, pairs already where the rank
+    // comes to three quarters of the sample (next to all keys are within the interval then, and the two score rows have to come through
+    // shared memory).  N(0, 1) scores, us, counting / this kernel, rank within a single row's sample and just beyond it: 2 000 rows
+    // of 512 keys, topk 290 34.6 / 30.3, at 307 35.0 / 36.5; 1 024 at 665 35.5 / 30.8, at 716 36.0 / 42.4; 2 048 at 1 536 36.8 / 30.2, at 1 638
+    // 36.9 / 42.0; 4 096 at 3 276 42.3 / 34.5, at 3 481 42.5 / 44.8; 64 rows of 1 024 at 614 4.7 / 4.5, at 768 4.7 / 5.3.  2 000 pairs, rank at 0.7 and
+    // at 0.9 of the sample: 1 024 keys at 448 33.6 / 31.5 and at 615 33.0 / 33.9, 4 096 at 2 297 38.2 / 35.1 and at 3 032 37.3 / 38.7.  All scores
+    // negative: 4 096 keys at 3 481 48.4 / 43.8, but what the scores are is known on the device alone.  Lists that are not staged gain
+    // nothing (2 000 rows of 16 384 keys, topk 8 000 76.4, 83.9).
+    const float sample_mean = p->topk * 0.125f;
+    const uint32_t held_rank = (uint32_t)(sample_mean + 4.0f * sqrtf(sample_mean) + 4.0f);
+    const bool staged = p->topk <= kStage;
+    const bool held = p->s_kv <= kSweep && staged && held_rank <= (p->group == 1 ? 4u : 3u) * (uint32_t)p->s_kv / 32;
+    // 1 024 threads for rows of 16 388 to 32 768 keys: in one wave of rows throughout, in more of them for pairs and long lists.  us, before
+    // (rows of up to an SM each counted, the others by pivot) / so: one wave, 148 rows of 32 768 at topk 64 15.7 / 8.9, 512 16.6 / 9.3, 2 048 16.7 / 9.5,
+    // 4 096 17.0 / 10.6, half to full length, topk 2 048 16.8 / 9.6, a quarter to half full 7.8 / 7.7, up to an eighth 5.2 / 6.1; 148 of 20 000 14.3 / 8.6;
+    // one row 12.9 / 8.3.  2 048 rows of 32 768 at topk 4 096 147 / 118, 2 048 122 / 107, 512 108 / 104; 600 of 26 000 at 512 31.8 / 35.3; pairs 173 / 128
+    // at 2 048, 151 / 117 at 64.
+    const bool wide = p->s_kv > kSweep && p->s_kv <= 2 * kSweep && staged && (p->rows <= sms || p->group == 2 || p->topk >= 1024);
+    // Longer rows in few: held by the CTAs of a cluster, two or four, as long as every one finds an SM of its own (33 clusters of four
+    // are resident at once).  us, by pivot / so: 64 rows of 65 536 keys, topk 2 048 16.3 / 11.0, half to full length 16.4 / 10.9, 74 at topk 512 14.7 / 10.1;
+    // 33 rows of 131 072 at 2 048 17.4 / 11.0, one 15.2 / 10.3; pairs 22.0 / 13.5.  Four rather than two where they fit: 8 rows of 65 536 at 4 096
+    // 11.2 by two, 9.8 by four.  Clusters that have to wait are slower: 74 rows of 131 072 21.5 / 29.4, 148 of 65 536 17.9 / 20.7 by two.
+    const int spread = p->s_kv <= 2 * kSweep || !staged || p->s_kv > 4 * kHeld ? 0
+                       : (long long)p->rows * 4 <= sms - 16 ? 4 : p->s_kv <= 2 * kHeld && (long long)p->rows * 2 <= sms ? 2 : 0;
+    // What is left, by pivot where the list fits with its margin.
+    // A division of a row among two, four or eight CTAs is taken while every CTA of the call finds an SM of
     // its own; clusters of four and eight leave some SMs over (33 rows by four, 15 by eight are resident at once, one more
     // makes a second wave: 34 rows of 36 864 keys 15.3 -> 17.6 us).  With two CTAs on an SM a division gains only where the
     // parts stay long: 148 rows by two, topk 2048, of 65 536 keys 24.8 us against 23.7 undivided, of 131 072 35.7 against
     // 38.7; 16 rows by eight of 262 144 31.0 against 28.3 by four, of 524 288 40.6 against 41.6.  There, too, what does not
     // fit at once must not be started: 74 rows by four of 49 152 keys 31.2 us, by two 20.2, counted 23.6.  A row is divided in
     // any case where a CTA could not hold the samples of its part.
-    // The steps between the CTAs of a row cost about as much as a second sweep (topk 2048, one row of 20 480 keys 12.3 us counted,
-    // 14.4 divided, of 32 768 14.4 and 14.9; 148 rows of 32 768 19.2 and 15.3, a line that more rows would put lower), less
-    // than the further ones (one row of 65 536 keys 28.7 against 16.4), hence the two lines.
     int parts = 1;
     while (parts < 8) {
         const int next = 2 * parts, over = next == 8 ? 28 : (next == 4 ? 16 : 0);      // SMs left over
@@ -1608,28 +2249,33 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
         parts = next;
     }
     const int each = (int)((((long long)p->s_kv + parts - 1) / parts + 3) & ~3LL);      // the longest part of a row
-    const bool pivot = p->topk <= kStage && p->s_kv > (p->rows <= sms ? 2 : 1) * kSweep && each <= kMaxSweeps * kSweep;
-    // Rows that a CTA's registers hold: counted within an interval that a sample points at.  Where the sample cannot hold the rank
-    // the interval is all there is, up to -FLT_MAX, and says nothing: such rows stay with the other kernel, pairs already where the rank
-    // comes to three quarters of the sample (next to all keys are within the interval then, and the two score rows have to come through
-    // shared memory).  N(0, 1) scores, us, counting / this kernel, rank within a single row's sample and just beyond it: 2 000 rows
-    // of 512 keys, topk 290 34.6 / 30.3, at 307 35.0 / 36.5; 1 024 at 665 35.5 / 30.8, at 716 36.0 / 42.4; 2 048 at 1 536 36.8 / 30.2, at 1 638
-    // 36.9 / 42.0; 4 096 at 3 276 42.3 / 34.5, at 3 481 42.5 / 44.8; 64 rows of 1 024 at 614 4.7 / 4.5, at 768 4.7 / 5.3.  2 000 pairs, rank at 0.7 and
-    // at 0.9 of the sample: 1 024 keys at 448 33.6 / 31.5 and at 615 33.0 / 33.9, 4 096 at 2 297 38.2 / 35.1 and at 3 032 37.3 / 38.7.  All scores
-    // negative: 4 096 keys at 3 481 48.4 / 43.8, but what the scores are is known on the device alone.  Lists that are not staged gain
-    // nothing (2 000 rows of 16 384 keys, topk 8 000 76.4, 83.9).
-    const float sample_mean = p->topk * 0.125f;
-    const uint32_t held_rank = (uint32_t)(sample_mean + 4.0f * sqrtf(sample_mean) + 4.0f);
-    const bool held = p->s_kv <= kSweep && p->topk <= kStage && held_rank <= (p->group == 1 ? 4u : 3u) * (uint32_t)p->s_kv / 32;
+    const bool pivot = staged && p->s_kv > kSweep && each <= kMaxSweeps * kSweep;
     cudaError_t e = cudaSuccess;
-    if (pivot) {
-        const bool multi = each > kSweep;
+    if (held || wide) {
+        const int resident = wide ? sms : sms * 2, grid = p->rows < resident ? p->rows : resident;
+        const auto start = [&](auto kern, size_t shared, int threads) {
+            const int smem = (int)(shared + (p->group == 2 ? (size_t)threads * kKpt * sizeof(float) : 0));
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            if (e == cudaSuccess)
+                kern<<<grid, threads, smem, s>>>(p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows,
+                                                 p->s_kv, p->topk, held_rank);
+        };
+        if (wide) start(p->group == 2 ? mxdsa_topk_held_kernel<2, kWide> : mxdsa_topk_held_kernel<1, kWide>, sizeof(RowShared<kWide>), kWide);
+        else start(p->group == 2 ? mxdsa_topk_held_kernel<2, kThreads> : mxdsa_topk_held_kernel<1, kThreads>, sizeof(RowShared<kThreads>), kThreads);
+    } else if (spread) {
+        const auto start = [&](auto kern, size_t shared) {
+            e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shared);
+            if (e == cudaSuccess)
+                kern<<<p->rows * spread, kWide, shared, s>>>(p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length,
+                                                             p->s_kv, p->topk, held_rank);
+        };
+        if (spread == 4) start(p->group == 2 ? mxdsa_topk_spread_kernel<2, 4> : mxdsa_topk_spread_kernel<1, 4>, sizeof(SpreadShared<4>));
+        else start(p->group == 2 ? mxdsa_topk_spread_kernel<2, 2> : mxdsa_topk_spread_kernel<1, 2>, sizeof(SpreadShared<2>));
+    } else if (pivot) {
         const float mean = p->topk * 0.125f;
         const uint32_t rank = (uint32_t)(mean + 10.0f * sqrtf(mean) + 8.0f);
-        auto kern = p->group == 2 ? (parts == 1 ? mxdsa_topk_pivot_kernel<2, true, false>
-                                     : multi ? mxdsa_topk_pivot_kernel<2, true, true> : mxdsa_topk_pivot_kernel<2, false, true>)
-                                  : (parts == 1 ? mxdsa_topk_pivot_kernel<1, true, false>
-                                     : multi ? mxdsa_topk_pivot_kernel<1, true, true> : mxdsa_topk_pivot_kernel<1, false, true>);
+        auto kern = p->group == 2 ? (parts == 1 ? mxdsa_topk_pivot_kernel<2, false> : mxdsa_topk_pivot_kernel<2, true>)
+                                  : (parts == 1 ? mxdsa_topk_pivot_kernel<1, false> : mxdsa_topk_pivot_kernel<1, true>);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PivotShared));
         if (e == cudaSuccess) {
             const long long want = (long long)p->rows * parts;
@@ -1648,18 +2294,10 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
             e = cudaLaunchKernelEx(&cfg, kern, p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length,
                                    p->rows, p->s_kv, p->topk, rank);
         }
-    } else if (held) {
-        const int grid = p->rows < sms * 2 ? p->rows : sms * 2;      // two resident CTAs of 512 threads per SM
-        auto kern = p->group == 2 ? mxdsa_topk_held_kernel<2> : mxdsa_topk_held_kernel<1>;
-        const int smem = (int)(sizeof(RowShared) + (p->group == 2 ? kSweep * sizeof(float) : 0));
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e == cudaSuccess)
-            kern<<<grid, kThreads, smem, s>>>(p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows,
-                                              p->s_kv, p->topk, held_rank);
     } else {
         const int grid = p->rows < sms * 2 ? p->rows : sms * 2;      // two resident CTAs of 512 threads per SM
-        auto kern = p->topk <= kStage ? (p->group == 2 ? mxdsa_topk_rows_kernel<2, true> : mxdsa_topk_rows_kernel<1, true>)
-                                      : (p->group == 2 ? mxdsa_topk_rows_kernel<2, false> : mxdsa_topk_rows_kernel<1, false>);
+        auto kern = staged ? (p->group == 2 ? mxdsa_topk_rows_kernel<2, true> : mxdsa_topk_rows_kernel<1, true>)
+                           : (p->group == 2 ? mxdsa_topk_rows_kernel<2, false> : mxdsa_topk_rows_kernel<1, false>);
         kern<<<grid, kThreads, 0, s>>>(p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows,
                                        p->s_kv, p->topk);
     }

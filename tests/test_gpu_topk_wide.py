@@ -1,0 +1,71 @@
+"""Selection from rows of 16 388 to 131 072 keys (run with -m gpu): held by one CTA of 1 024 threads, or by the CTAs of a cluster.
+Bit for bit against the oracle where that can go wrong: both sides of every line of the dispatch; rows that end at the edges of
+threads, warps, chunks and parts, or hold fewer keys than topk or than samples; scores of either sign, of few values, of very
+different size; samples that mislead; more rows than CTAs."""
+import numpy as np
+import pytest
+
+from test_gpu_topk_held import _check, _scores
+
+pytestmark = pytest.mark.gpu
+
+KINDS = ["normal", "negative", "zeros", "few", "sizes", "misled", "close", "one", "runs"]
+
+
+def _rows(kind, n, s_kv, rng):
+    if kind == "one":
+        return np.full((n, s_kv), -0.5, np.float32)
+    if kind == "runs":                 # 64 equal keys after one another
+        return np.repeat(rng.standard_normal((n, -(-s_kv // 64))).astype(np.float32), 64, 1)[:, :s_kv].copy()
+    with np.errstate(over="ignore"):
+        return _scores(kind, n, s_kv, rng)
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("kind", KINDS)
+@pytest.mark.parametrize("rows,s_kv,topk", [
+    (3, 16388, 2048), (2, 32768, 4096), (2, 20000, 33),            # one CTA
+    (3, 32772, 2048), (2, 65540, 64), (2, 131072, 4096),           # four
+    (34, 33000, 512), (34, 65536, 2048),                           # two
+])
+def test_against_the_oracle(rows, s_kv, topk, kind, pair):
+    if pair and rows == 34:
+        rows = 35
+    rng = np.random.default_rng(s_kv + topk)
+    distinct = 3                       # the oracle sorts every row: few different ones, many copies
+    scores = _rows(kind, distinct * (2 if pair else 1), s_kv, rng)
+    if rows <= distinct:
+        return _check(scores[:rows * (2 if pair else 1)], topk, pair=pair)
+    import torch
+    from mxdsa_b200.indexer import select_topk_indices
+    from oracle import mxdsa_oracle as O
+    which = np.arange(rows) % distinct
+    take = np.stack([2 * which, 2 * which + 1], 1).ravel() if pair else which
+    idx, cnt = select_topk_indices(torch.from_numpy(scores[take]).cuda(), topk, None, pair)
+    ri, rc = O.topk_select_ref(scores, topk, None, pair)
+    assert np.array_equal(cnt.cpu().numpy(), rc[which]) and np.array_equal(idx.cpu().numpy(), ri[which])
+
+
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("topk", [64, 2048, 4096])
+@pytest.mark.parametrize("s_kv", [16416, 32768, 32772, 65536, 131072])
+def test_rows_that_end_anywhere(s_kv, topk, pair):
+    """Ends around topk, the rank of the sample, 8 192 keys, the groups of a thread, the chunks of a CTA and the parts of a row."""
+    around = [0, 4, topk, 8 * (topk // 8 + 4 * int((topk // 8) ** 0.5) + 4), 4096, 8192, 12288, 16384, 24576, s_kv // 4, s_kv // 2, s_kv]
+    lengths = sorted({min(max(n + d, 0), s_kv) for n in around for d in (-5, -1, 0, 1, 3)})
+    if s_kv > 32768:                   # by four and by two
+        lengths = lengths[topk % 3::2][:33] if pair or s_kv > 65536 else lengths[:73]
+    rng = np.random.default_rng(topk)
+    n = len(lengths)
+    base = rng.standard_normal((4, s_kv)).astype(np.float32)
+    scores = base[rng.integers(0, 4, n * (2 if pair else 1))]
+    _check(scores, topk, np.asarray(lengths, np.int32), pair, np.arange(n, dtype=np.int32) * 7)
+
+
+def test_more_rows_than_ctas():
+    rng = np.random.default_rng(3)
+    lengths = rng.integers(0, 16401, 320)
+    lengths[::5] = rng.integers(0, 9000, 64)
+    base = rng.standard_normal((8, 16400)).astype(np.float32)
+    _check(base[rng.integers(0, 8, 640)], 300, lengths, True)
+    _check(base[rng.integers(0, 8, 320)], 1024, lengths)

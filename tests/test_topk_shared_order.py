@@ -8,7 +8,8 @@ import pytest
 
 from test_kernel_ordering import CSRC, body
 
-SHARED = re.compile(r"(?P<barrier>__syncthreads\(\))|(?P<call>row_locate|row_span)[<(]|(?P<add>atomicAdd\(&)?sm\.(?P<name>warp_\w+|sel_\w+|few_n|few)\b")
+SHARED = re.compile(r"(?P<barrier>__syncthreads\(\)|cluster_barrier\(\))|(?P<call>row_locate|row_span|spread_locate)[<(]|"
+                    r"(?P<add>atomicAdd\(&)?sm\.(?P<name>warp_\w+|sel_\w+|few_n|few|tops|bottoms|counts|spans|slot|list|taken|cut)\b")
 HEAD = re.compile(r"\s*(if constexpr|if|else|for|while)\b")
 
 
@@ -134,15 +135,38 @@ def test_what_the_check_finds(code, expected):
     assert races(code) == expected
 
 
-def test_a_barrier_stands_between_the_warps_of_held_rows():
+def _source(kernel, calls):
     with open(os.path.join(CSRC, "topk_kernels.cu")) as f:
         text = re.sub(r"//[^\n]*", "", f.read())
     called = {}
-    for name in ("row_locate", "row_span"):
+    for name in calls:
         at = text.index("{", re.search(r"__device__ __forceinline__ \w+ " + name + r"\(", text).end())
         called[name] = text[at + 1: _close(text, at) - 1]
-    kernel = body("topk_kernels.cu", "mxdsa_topk_held_kernel")[1:-1]
+    return body("topk_kernels.cu", kernel)[1:-1], called
+
+
+def test_a_barrier_stands_between_the_warps_of_held_rows():
+    kernel, called = _source("mxdsa_topk_held_kernel", ("row_locate", "row_span"))
     events = str([_nodes(kernel)] + [_nodes(t) for t in called.values()])
     for seen in ("'w', 'warp_max'", "'r', 'warp_max'", "'w', 'warp_min'", "'r', 'warp_min'", "'call', 'row_locate'", "'call', 'row_span'"):
         assert seen in events                      # otherwise there is nothing to look at
     assert races(kernel, called) == set()
+
+
+def test_a_barrier_stands_between_the_ctas_of_a_row():
+    """What is written into the peers' shared memory counts as written here too: every CTA does the same.  (The bins of the peers go
+    into two slots by turns, each read ahead of the barrier that the writer of its next use has passed.)"""
+    kernel, called = _source("mxdsa_topk_spread_kernel", ("spread_locate",))
+    write = lambda text: re.sub(r"peer_store\d?\(peer_address\(&sm\.(\w+)", r"f((sm.\1 = 0, x", text)
+    kernel, called = write(kernel), {name: write(text) for name, text in called.items()}
+    events = str([_nodes(kernel)] + [_nodes(t) for t in called.values()])
+    for name in ("tops", "bottoms", "counts", "spans", "slot", "few", "list", "taken", "cut", "warp_n"):
+        assert f"'w', '{name}'" in events and f"'r', '{name}'" in events
+    assert races(kernel, called) == set()
+
+
+def test_nothing_is_written_to_a_peer_behind_the_last_barrier():
+    """A CTA may end once it has passed it."""
+    kernel, _ = _source("mxdsa_topk_spread_kernel", ())
+    assert kernel.rindex("peer_store") < kernel.rindex("cluster_barrier()")
+    assert kernel.index("barrier.cluster.arrive") < kernel.index("barrier.cluster.wait") < kernel.index("peer_store")
