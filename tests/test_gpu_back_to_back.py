@@ -62,3 +62,33 @@ def test_schedule_then_decode_then_others(b, s_q):
     for key, out in got:
         n = 3 if key == "prefill" else 2
         assert all(torch.equal(a, r) for a, r in zip(out[:n], alone[key][:n])), key
+
+
+@pytest.mark.parametrize("rows,s_kv,topk", [(40, 2048, 128), (9, 20000, 512), (20, 40000, 256), (150, 36000, 64)])
+def test_pack_select_attend(rows, s_kv, topk):
+    """Each call reads what the one right ahead of it writes, into buffers that are used again."""
+    import mxdsa_b200 as M
+    from mxdsa_b200 import packing, quantize
+    from mxdsa_b200.indexer import select_topk_indices
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    kvf, w1, w2 = packing.make_rank1_kv((s_kv, 1), device="cuda", generator=g)
+    x = [torch.randn(2 * rows, 64, 512, device="cuda", generator=g, dtype=torch.bfloat16) for _ in range(2)]
+    scores = [torch.randn(2 * rows, s_kv, device="cuda", generator=g) for _ in range(2)]
+    buffer, last = torch.empty_like(scores[0]), torch.empty_like(x[0])
+
+    def step(i, wait):
+        sync = torch.cuda.synchronize if wait else lambda: None
+        buffer.copy_(scores[i]), sync()
+        last.copy_(x[i]), sync()
+        kv = quantize.pack_dual_prefill_kv64(kvf); sync()
+        q = quantize.pack_dual_q64(last); sync()
+        idx, n = select_topk_indices(buffer, topk, None, True); sync()
+        out = M.dual_mxfp8_head64_sparse_prefill_fwd(q, kv, idx.view(rows, 1, topk), SCALE, w1, w2, None, n); sync()
+        return idx, n, q, kv, *out
+
+    alone = [step(i, True) for i in range(2)]
+    got = [step(i % 2, False) for i in range(8)]
+    torch.cuda.synchronize()
+    M.device_fault()
+    for i, r in enumerate(got):
+        assert all(torch.equal(a, b) for a, b in zip(r, alone[i % 2]))

@@ -99,3 +99,15 @@ def test_every_phase_of_o_is_ready_is_waited_for():
                                  [(h, later if h == 0 else gt) for h in range(0 if t > 0 else 1, 2)]
                     gt, later = gt + 1, later + (t > 0)
             assert waited == signalled
+
+
+def test_selection_and_packers_read_behind_their_wait():
+    """Their grids start while the one ahead may still run: no pointer is used ahead of the wait, and dependents are released behind it."""
+    kernels = [("topk_kernels.cu", k) for k in ("mxdsa_topk_rows_kernel", "mxdsa_topk_pivot_kernel", "mxdsa_topk_held_kernel", "mxdsa_topk_spread_kernel")]
+    for name, kernel in kernels + [("pack_kernels.cu", "mxdsa_pack_rows_kernel")]:
+        b = body(name, kernel)
+        assert b.count("grid_start()") == 1
+        ahead = b[: b.index("grid_start()")]
+        assert not re.search(r"__ldg|\b(scores|lengths|row_offset|indices|topk_length|src|data|slots)\b|\breturn\b", ahead), (kernel, ahead)
+        with open(os.path.join(CSRC, name)) as f:
+            assert f.read().count('asm volatile("griddepcontrol.wait;\\ngriddepcontrol.launch_dependents;" ::: "memory");') == 1
