@@ -291,7 +291,7 @@ __global__ void __launch_bounds__(32) mxdsa_sched_whole_kernel(int b, int topk, 
 // A unit of work is a divided request.  With no more requests than parts the grid counts requests; otherwise it
 // counts parts, and the part in which a divided request STARTS (split 0) owns its merge (every divided request ends
 // some part while continuing into the next one).  WPH warps share a head, 512 / WPH dims each; a lane keeps eight
-// 16-byte loads in flight, the first of them issued before the weights are worked out.
+// or sixteen 16-byte loads in flight, the first of them issued before the weights are worked out.
 // Bound: latency while few requests are divided -- one request of one token over 34 splits is 64 heads x 34 rows, which
 // a warp per head with one row in flight took 14.5 us to walk, four warps per head with eight rows in flight 3.9 us (taken
 // while the schedule was still read ahead of the wait for the attention grid) --
@@ -301,12 +301,12 @@ __global__ void __launch_bounds__(32) mxdsa_sched_whole_kernel(int b, int topk, 
 constexpr int kMaxSplits = 192;
 constexpr int kCombineWarps = 8;
 
-template <int WPH>
+template <int WPH, int IN_FLIGHT>
 __global__ void __launch_bounds__(kCombineWarps * 32)
 mxdsa_combine_kernel(int b, int s_q, int by_request, int release, const int* meta, const int* num_splits, const float* o_accum,
                      const float* lse_accum, const float* sink, __nv_bfloat16* out, float* lse) {
     constexpr int kVec = 4 / WPH;        // 16-byte pieces of a partial row per lane
-    constexpr int kAhead = 8 / kVec;     // partial rows in flight
+    constexpr int kAhead = IN_FLIGHT / kVec;     // partial rows in flight
     const int unit = blockIdx.x / s_q, tok = blockIdx.x % s_q;
     const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const int head = blockIdx.y * (kCombineWarps / WPH) + warp / WPH, dim = (warp % WPH) * (512 / WPH) + lane * 4;
@@ -420,7 +420,12 @@ int launch_combine(int b, int s_q, int parts, const int* meta, const int* num_sp
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = dependent ? 1 : 0;
-    MX_CUDA(cudaLaunchKernelEx(&cfg, wide ? mxdsa_combine_kernel<4> : mxdsa_combine_kernel<1>, b, s_q, by_request, release ? 1 : 0, meta,
+    // Where an SM gets two blocks at most, registers do not count and a lane keeps sixteen loads in flight: what there is to do then
+    // is wait for one batch of rows after another.  us per call, eight / sixteen: one request of one token over 2176 keys 13.7 /
+    // 13.3, over 4224 16.8 / 16.5, two over 2176 14.9 / 14.6, two of two tokens over 4224 19.9 / 16.9, three of three over 1128 15.3 / 13.9; with more
+    // units registers keep blocks waiting: four of four over 1152 15.0 / 16.0, 30 of one over 2176 37.3 / 39.3.
+    const bool few = units * (int)(MXDSA_HEADS * 4 / kCombineWarps) <= 2 * sms;
+    MX_CUDA(cudaLaunchKernelEx(&cfg, few ? mxdsa_combine_kernel<4, 16> : wide ? mxdsa_combine_kernel<4, 8> : mxdsa_combine_kernel<1, 8>, b, s_q, by_request, release ? 1 : 0, meta,
                                num_splits, o_accum, lse_accum, sink, out, lse));
     return MXDSA_OK;
 }
