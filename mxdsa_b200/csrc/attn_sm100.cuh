@@ -597,7 +597,12 @@ __device__ __noinline__ void let_copies_land() {
     for (int i = 0; i < (1 << 16) && clock64() - start < 2000000; ++i) __nanosleep(1000);
 }
 
-template <int DECODE, int NT>
+// ALONE: one token to a request, decode of short parts.  The token is in both CTAs of the pair, which then store half of the columns
+// each: an SM writes 32 bytes a clock at best, half of a partial's 128 KB is 1.1 us of the drain.  An instantiation of its own again:
+// bounds worked out by pair cost the other short parts 0.5 to 1 % and, everywhere, decode of long parts 2 to 5 %, 256 tokens of
+// prefill at topk 128 2 %.  Us per call, one CTA storing / both: one request over 2176 keys 13.2 / 11.8, over 192 10.7 / 9.4, 8 over 640
+// 21.9 / 19.5, 30 over 2176 37.6 / 34.6, 64 over 640 33.8 / 31.3; whole requests, 8 over 640 16.2 / 14.6, 64 over 640 18.5 / 17.6.
+template <int DECODE, int NT, bool ALONE = false>
 __global__ void __launch_bounds__(kThreads, 1)
 mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ TensorMaps maps, const int resident_pairs) {
     // The last work item's output goes by way of the ring of KV tiles, which is idle by then, and empty halves of tiles are filled
@@ -1373,8 +1378,12 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             if (lane == 0) mbar_arrive(smem_u32(&sm.bar_os_empty[gw & 1]));
             MXDSA_WAIT(sm.bar_pv_done[last % kScStages], (last / kScStages) & 1, 55);
             tc_fence_after();
-            const int tok_idx = 2 * w.pair + (int)cta;
-            const bool store = tok_idx < p.s_q;
+            static_assert(!ALONE || DECODE == 2, "long parts store their partials from the lanes");
+            const int tok_idx = ALONE ? 0 : 2 * w.pair + (int)cta;
+            const bool store = ALONE || tok_idx < p.s_q;
+            const int col0 = half * 256 + (ALONE ? 128 * (int)cta : 0);      // the columns that this warp stores begin here ...
+            constexpr int kCols = ALONE ? 128 : 256;                         // ... and are so many
+            const uint32_t o_addr = lane_addr + kColO + (ALONE ? 128 * cta : 0u);
             const WorkOutput wo = it.output(w);
             // kRingOut (decode of short parts, prefill in tiles of 128 keys): behind the last work item the ring of KV tiles is idle, and
             // its 128 KB hold all of the output, fp32 partials too: no round waits for a staging tile.
@@ -1390,11 +1399,11 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 const uint32_t stage0 = !kRingOut || tile_mask < 16 ? smem_u32(sm.o_stage[q4]) : smem_u32(sm.kv[q4]);
                 const int out_row0 = (w.req * p.s_q + tok_idx) * kHeads + (q4 & 1) * 32;
 #pragma unroll 1
-                for (int c = 0; c < 256; c += 32) {
+                for (int c = 0; c < kCols; c += 32) {
                     float o[32];
-                    tmem_ld32(lane_addr + kColO + c, reinterpret_cast<uint32_t*>(o));
+                    tmem_ld32(o_addr + c, reinterpret_cast<uint32_t*>(o));
                     tmem_wait_ld();
-                    if (c == 256 - 32) release_o();   // the last columns are in registers: the next pair's PV may go
+                    if (c == kCols - 32) release_o();   // the last columns are in registers: the next pair's PV may go
                     // tiles rotate; across pairs too, or (kRingOut: a register less) each pair begins with the first
                     const uint32_t tile = stage0 + (kRingOut ? (uint32_t)c / 32 & tile_mask : round % kOutTiles) * 2048;
                     if (!kRingOut) ++round;
@@ -1415,7 +1424,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (kRingOut ? elect_one() : lane == 0) {   // a group per round, empty when nothing is stored, keeps "kOutTiles - 1 pending" exact
-                        if (store) tma_store_2d(&maps.out, tile, half * 256 + c, out_row0);
+                        if (store) tma_store_2d(&maps.out, tile, col0 + c, out_row0);
                         tma_store_commit();
                     }
                 }
@@ -1428,11 +1437,11 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                 const uint32_t stage0 = tile_mask < 16 ? smem_u32(sm.o_stage[q4]) : smem_u32(sm.kv[q4]);
                 const int part_row0 = (wo.split_idx * p.s_q + tok_idx) * kHeads + (q4 & 1) * 32;
 #pragma unroll 1
-                for (int c = 0; c < 256; c += 16) {
+                for (int c = 0; c < kCols; c += 16) {
                     float o[16];
-                    tmem_ld16(lane_addr + kColO + c, reinterpret_cast<uint32_t*>(o));
+                    tmem_ld16(o_addr + c, reinterpret_cast<uint32_t*>(o));
                     tmem_wait_ld();
-                    if (c == 256 - 16) release_o();   // the last columns are in registers: the next pair's PV may go
+                    if (c == kCols - 16) release_o();   // the last columns are in registers: the next pair's PV may go
                     const uint32_t tile = stage0 + (c / 16 & tile_mask) * 2048;
                     if (tile_mask < 16) {
                         if (elect_one()) tma_store_wait_read<kOutTiles - 1>();
@@ -1445,7 +1454,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     fence_proxy_async_smem();
                     __syncwarp();
                     if (elect_one()) {
-                        if (store) tma_store_2d(&maps.part, tile, half * 256 + c, part_row0);
+                        if (store) tma_store_2d(&maps.part, tile, col0 + c, part_row0);
                         tma_store_commit();
                     }
                 }

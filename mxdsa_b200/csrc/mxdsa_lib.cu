@@ -726,7 +726,7 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     cudaStream_t stream = static_cast<cudaStream_t>(p->stream);
     const dim3 grid(2 * ((p->s_q + 1) / 2), p->num_sm_parts, 1);
     if (short_parts)
-        st = launch_pairs(mxdsa::mxdsa_attn_kernel<2, 64>, grid, d->sm_count, stream, ap, maps);
+        st = launch_pairs(p->s_q == 1 ? mxdsa::mxdsa_attn_kernel<2, 64, true> : mxdsa::mxdsa_attn_kernel<2, 64>, grid, d->sm_count, stream, ap, maps);
     else
         st = launch_pairs(mxdsa::mxdsa_attn_kernel<1, 64>, grid, d->sm_count, stream, ap, maps);
     if (st != MXDSA_OK) return st;
