@@ -110,4 +110,6 @@ def test_selection_and_packers_read_behind_their_wait():
         ahead = b[: b.index("grid_start()")]
         assert not re.search(r"__ldg|\b(scores|lengths|row_offset|indices|topk_length|src|data|slots)\b|\breturn\b", ahead), (kernel, ahead)
         with open(os.path.join(CSRC, name)) as f:
-            assert f.read().count('asm volatile("griddepcontrol.wait;\\ngriddepcontrol.launch_dependents;" ::: "memory");') == 1
+            assert f.read().count('asm volatile("griddepcontrol.wait;\\ngriddepcontrol.launch_dependents;" : "+r"(block)::"memory");') == 1
+        # addresses follow from what the wait passes through, or the pointers do
+        assert "blockIdx" not in b or re.match(r'grid_start\(\);\s*asm volatile\("" : "\+l"\(scores\), "\+l"\(lengths\), "\+l"\(row_offset\)\);', b[len(ahead):])
