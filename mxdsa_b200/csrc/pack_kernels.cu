@@ -8,7 +8,7 @@
 // with the ceil(log2()) taken exactly from the bits of amax (see scale_byte).
 //
 // Bound: HBM.  Algorithmic bytes per row: 512 * sizeof(input element) read + 528 written.  In a long call a warp takes
-// two adjacent rows at a time: both rows' loads are in flight together, and the 1056 bytes it writes for queries begin
+// two adjacent rows of bf16 at a time: both rows' loads are in flight together, and the 1056 bytes it writes for queries begin
 // and end on whole 32-byte sectors.  A short call takes one, see launch().  What used to come before the memory was the
 // instruction count -- a 64-bit division and remainder per row, a rounded float division, two clamps per value, byte
 // stores of the slot; see the comments below for what stands in their place.
@@ -22,6 +22,7 @@ namespace {
 
 constexpr int kDim = 512;
 constexpr int kWarpsPerBlock = 8;
+constexpr int kTwoRowBlocks = 5;       // resident blocks of an SM where a warp takes two rows at a time
 
 // UE8M0 byte of 2^ceil(log2(max(amax/448, 2^-126))) and the factor 2^-e to multiply by, without the division.
 // Write amax = m * 2^e, 1 <= m < 2, and 448 = 1.75 * 2^8.  The correctly rounded quotient is at most 2^(e-8) for
@@ -44,16 +45,24 @@ __device__ __forceinline__ uint16_t e4m3x2(float lo, float hi) {
     return r;
 }
 
+// 32 bytes of an activation: one load where the rows begin on 32-byte boundaries (WIDE), two otherwise.  Two loads of 16 bytes
+// ask for every sector twice: 4 096 rows of f32 3.1 us, now 2.3, of bf16 2.34, 2.25.
+template <bool WIDE> __device__ __forceinline__ void load32(uint32_t (&w)[8], const void* src) {
+    if (WIDE) {
+        asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                     : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src));
+    } else {
+        const uint4 a = __ldg(static_cast<const uint4*>(src)), b = __ldg(static_cast<const uint4*>(src) + 1);
+        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
+        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
+    }
+}
+
 // Sixteen values of a row as they come from memory, and what is needed of them.
 template <typename T> struct Raw16;
 template <> struct Raw16<__nv_bfloat16> {
     uint32_t w[8];
-    __device__ __forceinline__ void load(const __nv_bfloat16* src) {
-        const uint4 a = __ldg(reinterpret_cast<const uint4*>(src));
-        const uint4 b = __ldg(reinterpret_cast<const uint4*>(src) + 1);
-        w[0] = a.x; w[1] = a.y; w[2] = a.z; w[3] = a.w;
-        w[4] = b.x; w[5] = b.y; w[6] = b.z; w[7] = b.w;
-    }
+    template <bool WIDE> __device__ __forceinline__ void load(const __nv_bfloat16* src) { load32<WIDE>(w, src); }
     // largest magnitude, NaNs passed over: two values per instruction
     __device__ __forceinline__ float amax() const {
         uint32_t m = w[0] & 0x7FFF7FFFu;
@@ -66,20 +75,21 @@ template <> struct Raw16<__nv_bfloat16> {
     }
 };
 template <> struct Raw16<float> {
-    float4 v[4];
-    __device__ __forceinline__ void load(const float* src) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] = __ldg(reinterpret_cast<const float4*>(src) + i);
+    uint32_t w[2][8];
+    template <bool WIDE> __device__ __forceinline__ void load(const float* src) {
+        load32<WIDE>(w[0], src);
+        load32<WIDE>(w[1], src + 8);
     }
+    __device__ __forceinline__ float at(int i) const { return __uint_as_float(w[i >> 3][i & 7]); }
     __device__ __forceinline__ float amax() const {
         float m = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            m = fmaxf(m, fmaxf(fmaxf(fabsf(v[i].x), fabsf(v[i].y)), fmaxf(fabsf(v[i].z), fabsf(v[i].w))));
+        for (int i = 0; i < 16; i += 4)
+            m = fmaxf(m, fmaxf(fmaxf(fabsf(at(i)), fabsf(at(i + 1))), fmaxf(fabsf(at(i + 2)), fabsf(at(i + 3)))));
         return m;
     }
     __device__ __forceinline__ float2 pair(int i) const {
-        return i & 1 ? make_float2(v[i >> 1].z, v[i >> 1].w) : make_float2(v[i >> 1].x, v[i >> 1].y);
+        return make_float2(at(2 * i), at(2 * i + 1));
     }
 };
 
@@ -102,8 +112,8 @@ __device__ __forceinline__ int grid_start() {
 // QGROUPS: true  -> Q rows: scale g covers dims [32g,32g+32) and [256+32g,256+32g+32)
 //          false -> KV rows: scale g covers dims [64g,64g+64)
 // Lane L owns dims [16L, 16L+16) of the ROWS rows that its warp takes at a time.
-template <typename T, bool QGROUPS, int ROWS>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+template <typename T, bool QGROUPS, int ROWS, bool WIDE>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, ROWS == 2 ? kTwoRowBlocks : sizeof(T) == 2 ? 8 : 1)
 mxdsa_pack_rows_kernel(const T* __restrict__ src, long long src_stride, long long rows, uint8_t* __restrict__ data,
                        long long data_stride, uint8_t* __restrict__ slots, long long slot_stride, int rows_per_page,
                        long long page_stride, int paired_storage) {
@@ -123,7 +133,7 @@ mxdsa_pack_rows_kernel(const T* __restrict__ src, long long src_stride, long lon
 #pragma unroll
         for (int u = 0; u < ROWS; ++u) {
             const long long r = r0 + u < rows ? r0 + u : r0;     // past the end: the row before once more, not stored
-            x[u].load(src + r * src_stride + 16 * lane);
+            x[u].template load<WIDE>(src + r * src_stride + 16 * lane);
         }
 #pragma unroll
         for (int u = 0; u < ROWS; ++u) {
@@ -174,12 +184,20 @@ int launch(const T* src, long long src_stride, long long rows, uint8_t* data, lo
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return MXDSA_ERR_CUDA;
-    // Two rows at a time pay where every warp has many: 262 144 rows of bf16 72.2 us (one at a time 72.7), 1 048 576 272
-    // (287); f32 106 (122) and 410 (478).  Below that the longer code and the higher register count (42 to 59 against 32 to
-    // 40: 4 or 5 resident CTAs of the 8 per SM that are launched, against 6 to 8) cost more: 65 536 rows of bf16 20.9 us
-    // (19.1), 4 096 4.1 (3.4), 64 2.4 (1.6); f32 16 384 rows 9.5 (9.3), 4 096 4.5 (4.2), 64 3.0 (2.3).  All from a cold L2.
-    const long long most = (long long)sms * 8, full = most * kWarpsPerBlock;     // warps of a full grid
-    const int each = rows <= full * (sizeof(T) == 2 ? 16 : 2) ? 1 : 2;
+    // bf16: two rows at a time pay where every warp has many, and where the grid is what is resident at once: with eight blocks to an SM,
+    // of which five fit, the other three came behind and 262 144 query rows took 68.4 us, now 65.0, 1 048 576 270, now 248; 262 144
+    // KV rows 69.5 / 65.4, 1 000 001 260 / 240.  Below 16 rows to a warp the longer code costs more: 65 536 rows 18.4 us against 17.0 one
+    // at a time, 131 072 34.2 against 33.3.  (Four rows at a time, four blocks: 262 144 KV rows 63.8, but 1 000 001 258; query rows slower. One row
+    // to a warp and as many warps as that takes: queries as eight blocks to an SM, KV rows 3 to 6 % slower.)
+    // f32: one row to a warp, as many warps as that takes.  us, eight blocks to an SM, two rows at a time from 2 rows to a warp on / so: 4 096 rows 3.1 / 2.4,
+    // 32 768 14.3 / 13.5, 262 144 99.5 / 94.7, 1 048 576 rows of pages 389 / 373.
+    constexpr int kMany = sizeof(T) == 2 ? 2 : 1;
+    const long long full = (long long)sms * 8 * kWarpsPerBlock;
+    const int each = rows <= full * 16 ? 1 : kMany;
+    const long long most = sizeof(T) == 4 ? 0x7fffffffLL : (long long)sms * (each == 1 ? 8 : kTwoRowBlocks);
+    const bool aligned = (((uintptr_t)src | (uintptr_t)(src_stride * (long long)sizeof(T))) & 31) == 0;
+    const auto kern = each == 1 ? (aligned ? mxdsa_pack_rows_kernel<T, Q, 1, true> : mxdsa_pack_rows_kernel<T, Q, 1, false>)
+                                : (aligned ? mxdsa_pack_rows_kernel<T, Q, kMany, true> : mxdsa_pack_rows_kernel<T, Q, kMany, false>);
     const long long want = (rows + each * kWarpsPerBlock - 1) / (each * kWarpsPerBlock);
     cudaLaunchAttribute attr[1]{};
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -190,7 +208,7 @@ int launch(const T* src, long long src_stride, long long rows, uint8_t* data, lo
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, each == 1 ? mxdsa_pack_rows_kernel<T, Q, 1> : mxdsa_pack_rows_kernel<T, Q, 2>, src, src_stride, rows,
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, src, src_stride, rows,
                                        data, data_stride, slots, slot_stride, rows_per_page, page_stride, paired);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {

@@ -158,3 +158,22 @@ def test_both_sides_of_the_row_count_at_which_a_warp_takes_two_rows(dtype, per_w
         if kind == "kv":                       # all data rows, then all slots
             parts = [torch.cat([p[: p.numel() // 528 * 512] for p in parts]), torch.cat([p[p.numel() // 528 * 512:] for p in parts])]
         assert torch.equal(got, torch.cat(parts))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("rows", [64, 3000, 152064, 152065])
+def test_rows_that_do_not_begin_on_32_bytes(rows, dtype):
+    """Loads of 32 bytes or two of 16, one row to a warp or two: the same bytes."""
+    from mxdsa_b200 import quantize as Z
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    flat = torch.randn(rows * 512 + 16, device="cuda", generator=g).to(dtype)
+    off = 16 // flat.element_size()
+    odd = flat[off: off + rows * 512]
+    even = odd.clone()
+    assert odd.data_ptr() % 32 == 16 and even.data_ptr() % 32 == 0
+    assert torch.equal(Z.pack_dual_prefill_kv64(odd.view(rows, 1, 512)), Z.pack_dual_prefill_kv64(even.view(rows, 1, 512)))
+    if rows % 64 == 0:
+        shape = (rows // 64, 64, 512)
+        for paired in (False, True):
+            assert torch.equal(Z.pack_dual_q64(odd.view(shape), paired), Z.pack_dual_q64(even.view(shape), paired))
+        assert torch.equal(Z.pack_dual_decode_kv_pages(odd.view(-1, 64, 1, 512)), Z.pack_dual_decode_kv_pages(even.view(-1, 64, 1, 512)))
