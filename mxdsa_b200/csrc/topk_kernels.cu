@@ -1326,10 +1326,16 @@ template <int GROUP, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1024 / THREADS)
 mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
                        const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
-                       int32_t* __restrict__ topk_length, int rows, int s_kv, int topk, uint32_t sample_rank) {
+                       int32_t* __restrict__ topk_length, int rows, int s_kv, int topk, uint32_t sample_rank, int resident) {
     extern __shared__ __align__(16) uint8_t topk_smem[];
     RowShared<THREADS>& sm = *reinterpret_cast<RowShared<THREADS>*>(topk_smem);
     constexpr int kWarps = THREADS / 32, kChunkKeys = THREADS * 4;
+    // Two CTAs to an SM: one CTA to a row.  The hardware gives rows to whoever is done, the other CTA's work hides a new one's start, and rows
+    // of different lengths even out.  A CTA that has the SM to itself walks rows, with the next one's scores on their way.  us, CTAs
+    // that walk rows / a CTA to a row, topk 2048: 2 048 pairs of 16 384 keys, half to full length 60.9 / 58.2, full 65.6 / 63.0 (64.2 without
+    // asking for rows ahead), single rows 54.0 / 50.5 and 58.0 / 53.9, 400 pairs 17.6 / 14.2, 8 192 pairs at topk 4 096 263 / 250, 8 000 rows of
+    // 1 024 at 256 102 / 99; with 1 024 threads 2 048 pairs of 30 000 115 / 124.
+    constexpr bool kPersistent = THREADS == kWide;
     const uint32_t stage0 = (uint32_t)__cvta_generic_to_shared(sm.stage);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int block = grid_start();
@@ -1348,8 +1354,8 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                 asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + c * THREADS * 16), "l"(from + 128 * c) : "memory");
     };
     if (GROUP == 2 && block < rows) ask(block, len);
-    for (int r = block, next_len; r < rows; r += gridDim.x, len = next_len) {
-        const int next = r + (int)gridDim.x;
+    for (int r = block, next_len; r < rows; r = kPersistent ? r + (int)gridDim.x : rows, len = next_len) {
+        const int next = r + resident;
         next_len = s_kv;
         if (lengths != nullptr && next < rows) next_len = min(max(__ldg(lengths + next), 0), s_kv);
 
@@ -1393,7 +1399,7 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
                 key[4 * c + 2] = fmaxf(key[4 * c + 2], f.z);
                 key[4 * c + 3] = fmaxf(key[4 * c + 3], f.w);
             }
-            if (next < rows) ask(next, next_len);
+            if (kPersistent && next < rows) ask(next, next_len);
         }
         if ((warp + 1) * 128 * chunks > len) {       // the warps that the row ends in, or ahead of
 #pragma unroll
@@ -1422,8 +1428,11 @@ mxdsa_topk_held_kernel(const float* __restrict__ scores, long long score_stride,
         }
         const uint32_t warp_top = __reduce_max_sync(0xffffffffu, score_key(top));
         if (lane == 0) sm.warp_max[warp] = warp_top;
-        if (next < rows && tid * 32 < next_len)      // the other scores of the next row are asked into L2
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(scores + (long long)next * GROUP * score_stride + tid * 32));
+        if ((kPersistent || GROUP == 2) && next < rows && tid * 32 < next_len) {     // a row that comes next is asked into L2
+            const float* nx = scores + (long long)next * GROUP * score_stride + tid * 32;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(nx));
+            if (!kPersistent) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + score_stride));
+        }
         __syncthreads();
         const uint32_t top_key = __reduce_max_sync(0xffffffffu, lane < kWarps ? sm.warp_max[lane] : 0u);
         uint32_t pivot = kMinKey;
@@ -2285,13 +2294,13 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     const bool pivot = staged && p->s_kv > kSweep && each <= kMaxSweeps * kSweep;
     cudaError_t e = cudaSuccess;
     if (held || wide) {
-        const int resident = wide ? sms : sms * 2, grid = p->rows < resident ? p->rows : resident;
+        const int resident = wide ? sms : sms * 2, grid = wide && p->rows > resident ? resident : p->rows;
         const auto start = [&](auto kern, size_t shared, int threads) {
             const int smem = (int)(shared + (p->group == 2 ? (size_t)threads * kKpt * sizeof(float) : 0));
             e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e == cudaSuccess)
                 e = launch(kern, grid, threads, smem, s, 1, p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows,
-                           p->s_kv, p->topk, held_rank);
+                           p->s_kv, p->topk, held_rank, wide ? resident : resident);
         };
         if (wide) start(p->group == 2 ? mxdsa_topk_held_kernel<2, kWide> : mxdsa_topk_held_kernel<1, kWide>, sizeof(RowShared<kWide>), kWide);
         else start(p->group == 2 ? mxdsa_topk_held_kernel<2, kThreads> : mxdsa_topk_held_kernel<1, kThreads>, sizeof(RowShared<kThreads>), kThreads);
