@@ -279,109 +279,96 @@ template <int GROUP, bool STAGED>
 __global__ void __launch_bounds__(kThreads, 2)
 mxdsa_topk_rows_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
                        const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
-                       int32_t* __restrict__ topk_length, int rows, int s_kv, int topk) {
+                       int32_t* __restrict__ topk_length, int s_kv, int topk) {
     __shared__ __align__(16) TopkShared sm;
     const int tid = threadIdx.x, lane = tid & 31;
-    const int block = grid_start();
+    const int r = grid_start();
     int len = s_kv;
-    if (lengths != nullptr && block < rows) len = min(max(__ldg(lengths + block), 0), s_kv);
-    for (int r = block, next_len; r < rows; r += gridDim.x, len = next_len) {
-        const float* row0 = scores + (long long)r * GROUP * score_stride;
-        const float* row1 = row0 + score_stride;
-        const int nsweeps = (len + kSweep - 1) / kSweep;
-        // the row this CTA takes next: its length is loaded now and its scores are asked into L2 once this row's are in
-        // registers, so that its loads do not wait for HBM
-        const int next = r + (int)gridDim.x;
-        next_len = s_kv;
-        if (lengths != nullptr && next < rows) next_len = min(max(__ldg(lengths + next), 0), s_kv);
-        uint32_t key[kKpt];
+    if (lengths != nullptr) len = min(max(__ldg(lengths + r), 0), s_kv);
+    const float* row0 = scores + (long long)r * GROUP * score_stride;
+    const float* row1 = row0 + score_stride;
+    const int nsweeps = (len + kSweep - 1) / kSweep;
+    uint32_t key[kKpt];
 
-        // ---- three radix passes: prefix = the bits of the threshold key found so far
-        uint32_t prefix = 0, k = (uint32_t)topk, n_sel = 0;
+    // ---- three radix passes: prefix = the bits of the threshold key found so far
+    uint32_t prefix = 0, k = (uint32_t)topk, n_sel = 0;
 #pragma unroll 1
-        for (int pass = 0; pass < 3; ++pass) {
-            const int lo = pass == 0 ? 21 : (pass == 1 ? 10 : 0);       // lowest bit of this pass's digit
-            const int hi = pass == 0 ? 32 : (pass == 1 ? 21 : 10);      // bits above the digit are the prefix
-            *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
-            __syncthreads();
-            if (pass == 0) {
-                // every key takes part (non-candidates fall into bins 0-3, which find_bin ignores)
+    for (int pass = 0; pass < 3; ++pass) {
+        const int lo = pass == 0 ? 21 : (pass == 1 ? 10 : 0);       // lowest bit of this pass's digit
+        const int hi = pass == 0 ? 32 : (pass == 1 ? 21 : 10);      // bits above the digit are the prefix
+        *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        __syncthreads();
+        if (pass == 0) {
+            // every key takes part (non-candidates fall into bins 0-3, which find_bin ignores)
 #pragma unroll 1
-                for (int sw = 0; sw < nsweeps; ++sw) {
-                    const int live = live_chunks(sw, len);
-                    auto count = [&](int c) {
+            for (int sw = 0; sw < nsweeps; ++sw) {
+                const int live = live_chunks(sw, len);
+                auto count = [&](int c) {
 #pragma unroll
-                        for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[key[i] >> 21], 1u);
-                    };
-                    // single rows: no branch behind the loads either, a chunk is counted while others are on their way (pairs
-                    // are loaded in two batches anyway and lose by it: 2 048 of 8 192 keys +3 %)
-                    if (GROUP == 1 && live == kChunks) {
-                        load_keys<GROUP>(row0, row1, sw, len, key);
+                    for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[key[i] >> 21], 1u);
+                };
+                // single rows: no branch behind the loads either, a chunk is counted while others are on their way (pairs
+                // are loaded in two batches anyway and lose by it: 2 048 of 8 192 keys +3 %)
+                if (GROUP == 1 && live == kChunks) {
+                    load_keys<GROUP>(row0, row1, sw, len, key);
 #pragma unroll
-                        for (int c = 0; c < kChunks; ++c) count(c);
-                    } else {
-                        load_keys<GROUP>(row0, row1, sw, len, key);
-                        for_live_chunks<GROUP == 2 && STAGED>(live, count);
-                    }
-                }
-            } else {
-                // keys outside the prefix add to a per-lane spare bin: no branch, no bank conflict
-#pragma unroll 1
-                for (int sw = 0; sw < nsweeps; ++sw) {
-                    if (nsweeps > 1) load_keys<GROUP>(row0, row1, sw, len, key);
-                    // distance from the first key of the prefix: inside the prefix it is below 2^hi and its top
-                    // bits are the digit; everything else (wrapped or large) is clamped onto the spare bins
-                    const uint32_t first = prefix << hi, spare = (uint32_t)((kBins >> (pass - 1)) + lane);   // 2048 / 1024 digits
-                    const int live = live_chunks(sw, len);
-                    for_live_chunks<GROUP == 2 && STAGED>(live, [&](int c) {
-#pragma unroll
-                        for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[min((key[i] - first) >> lo, spare)], 1u);
-                    });
+                    for (int c = 0; c < kChunks; ++c) count(c);
+                } else {
+                    load_keys<GROUP>(row0, row1, sw, len, key);
+                    for_live_chunks<GROUP == 2 && STAGED>(live, count);
                 }
             }
-            if (pass == 0 && next < rows && next_len <= kSweep && tid * 32 < next_len) {
-                const float* nx = scores + (long long)next * GROUP * score_stride + tid * 32;
-                asm volatile("prefetch.global.L2 [%0];" ::"l"(nx));
-                if (GROUP == 2) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + score_stride));
-            }
-            __syncthreads();
-            uint32_t k_now;
-            const uint32_t total = find_bin(sm, k, pass == 0, k_now, pass == 2 ? kBins / 2 : kBins);
-            if (pass == 0) n_sel = k_now;            // min(topk, candidates)
-            if (total == 0u || k_now == 0u) { n_sel = 0; break; }
-            prefix = pass == 0 ? sm.sel_bin : ((prefix << (hi - lo)) | sm.sel_bin);
-            k = k_now - sm.sel_above;                // rank inside the chosen bin, 1-based
-            if (k == sm.sel_count) {                 // the whole bin is taken: its first key is a threshold as good as any in it
-                prefix <<= lo;
-                break;
-            }
-        }
-        // all threads agree on n_sel (computed from shared totals); prefix is now the full threshold key
-        const uint32_t thr = prefix, need_eq = k;    // take `need_eq` keys equal to thr, smallest index first
-
-        // ---- output positions: ascending index, order (sweep, chunk, thread, element).
-        // Without surplus ties (every key equal to the threshold is taken -- the rule unless scores repeat)
-        // "selected" is key >= thr and one count per key suffices; otherwise the equal keys are ranked too.
-        int32_t* out = indices + (long long)r * index_stride;
-        const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
-        if (n_sel > 0u) {
-            const bool ties = need_eq != sm.sel_count;
-            uint32_t base_gt = 0, base_eq = 0;
+        } else {
+            // keys outside the prefix add to a per-lane spare bin: no branch, no bank conflict
 #pragma unroll 1
             for (int sw = 0; sw < nsweeps; ++sw) {
                 if (nsweeps > 1) load_keys<GROUP>(row0, row1, sw, len, key);
-                if (!ties) emit_sweep<false, STAGED>(sm, key, thr, need_eq, out, off, sw, live_chunks(sw, len), base_gt, base_eq);
-                else emit_sweep<true, STAGED>(sm, key, thr, need_eq, out, off, sw, live_chunks(sw, len), base_gt, base_eq);
+                // distance from the first key of the prefix: inside the prefix it is below 2^hi and its top
+                // bits are the digit; everything else (wrapped or large) is clamped onto the spare bins
+                const uint32_t first = prefix << hi, spare = (uint32_t)((kBins >> (pass - 1)) + lane);   // 2048 / 1024 digits
+                const int live = live_chunks(sw, len);
+                for_live_chunks<GROUP == 2 && STAGED>(live, [&](int c) {
+#pragma unroll
+                    for (int i = 4 * c; i < 4 * c + 4; ++i) atomicAdd(&sm.hist[min((key[i] - first) >> lo, spare)], 1u);
+                });
             }
         }
-        if (STAGED) {                                // topk <= kStage: positions were staged in shared memory
-            for (uint32_t pos = tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = pos < n_sel ? sm.stage[pos] : -1;
-        } else {
-            for (uint32_t pos = n_sel + tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = -1;
+        __syncthreads();
+        uint32_t k_now;
+        const uint32_t total = find_bin(sm, k, pass == 0, k_now, pass == 2 ? kBins / 2 : kBins);
+        if (pass == 0) n_sel = k_now;            // min(topk, candidates)
+        if (total == 0u || k_now == 0u) { n_sel = 0; break; }
+        prefix = pass == 0 ? sm.sel_bin : ((prefix << (hi - lo)) | sm.sel_bin);
+        k = k_now - sm.sel_above;                // rank inside the chosen bin, 1-based
+        if (k == sm.sel_count) {                 // the whole bin is taken: its first key is a threshold as good as any in it
+            prefix <<= lo;
+            break;
         }
-        if (topk_length != nullptr && tid == 0) topk_length[r] = (int32_t)n_sel;
-        __syncthreads();                             // sm.sel_* and the histogram belong to the next row from here
     }
+    // all threads agree on n_sel (computed from shared totals); prefix is now the full threshold key
+    const uint32_t thr = prefix, need_eq = k;    // take `need_eq` keys equal to thr, smallest index first
+
+    // ---- output positions: ascending index, order (sweep, chunk, thread, element).
+    // Without surplus ties (every key equal to the threshold is taken -- the rule unless scores repeat)
+    // "selected" is key >= thr and one count per key suffices; otherwise the equal keys are ranked too.
+    int32_t* out = indices + (long long)r * index_stride;
+    const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
+    if (n_sel > 0u) {
+        const bool ties = need_eq != sm.sel_count;
+        uint32_t base_gt = 0, base_eq = 0;
+#pragma unroll 1
+        for (int sw = 0; sw < nsweeps; ++sw) {
+            if (nsweeps > 1) load_keys<GROUP>(row0, row1, sw, len, key);
+            if (!ties) emit_sweep<false, STAGED>(sm, key, thr, need_eq, out, off, sw, live_chunks(sw, len), base_gt, base_eq);
+            else emit_sweep<true, STAGED>(sm, key, thr, need_eq, out, off, sw, live_chunks(sw, len), base_gt, base_eq);
+        }
+    }
+    if (STAGED) {                                // topk <= kStage: positions were staged in shared memory
+        for (uint32_t pos = tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = pos < n_sel ? sm.stage[pos] : -1;
+    } else {
+        for (uint32_t pos = n_sel + tid; pos < (uint32_t)topk; pos += kThreads) out[pos] = -1;
+    }
+    if (topk_length != nullptr && tid == 0) topk_length[r] = (int32_t)n_sel;
 }
 
 // ------------------------------------------------------------------------------------------------ selection by pivot
@@ -953,146 +940,143 @@ template <int GROUP, bool CLUSTER>
 __global__ void __launch_bounds__(kThreads, 2)
 mxdsa_topk_pivot_kernel(const float* __restrict__ scores, long long score_stride, const int32_t* __restrict__ lengths,
                         const int32_t* __restrict__ row_offset, int32_t* __restrict__ indices, long long index_stride,
-                        int32_t* __restrict__ topk_length, int rows, int s_kv, int topk, uint32_t sample_rank) {
+                        int32_t* __restrict__ topk_length, int s_kv, int topk, uint32_t sample_rank) {
     extern __shared__ __align__(16) uint8_t topk_smem[];
     PivotShared& sm = *reinterpret_cast<PivotShared*>(topk_smem);
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t parts = CLUSTER ? cluster_size() : 1u, part = CLUSTER ? cluster_rank() : 0u;
-    const int step = (int)(gridDim.x / parts);
-    const int block = grid_start();
+    const int r = grid_start() / (int)parts;
     if (tid == 0) sm.key_max = 0u;
     __syncthreads();
-    for (int r = block / (int)parts; r < rows; r += step) {
-        const float* row0 = scores + (long long)r * GROUP * score_stride;
-        const float* row1 = row0 + score_stride;
-        int len = s_kv;
-        if (lengths != nullptr) len = min(max(__ldg(lengths + r), 0), s_kv);
-        // this CTA's keys: the row's own length is divided, in whole groups of four
-        int begin = 0, end = len;
-        if (CLUSTER) {
-            const int each = ((len + (int)parts - 1) / (int)parts + 3) & ~3;
-            begin = min((int)part * each, len);      // an empty part begins at len, multiple of four or not: it loads nothing
-            end = min(begin + each, len);
-        }
-        const int nsweeps = (end - begin + kSweep - 1) / kSweep;
+    const float* row0 = scores + (long long)r * GROUP * score_stride;
+    const float* row1 = row0 + score_stride;
+    int len = s_kv;
+    if (lengths != nullptr) len = min(max(__ldg(lengths + r), 0), s_kv);
+    // this CTA's keys: the row's own length is divided, in whole groups of four
+    int begin = 0, end = len;
+    if (CLUSTER) {
+        const int each = ((len + (int)parts - 1) / (int)parts + 3) & ~3;
+        begin = min((int)part * each, len);      // an empty part begins at len, multiple of four or not: it loads nothing
+        end = min(begin + each, len);
+    }
+    const int nsweeps = (end - begin + kSweep - 1) / kSweep;
 
-        // ---- 1. the pivot
-        float s[kKpt];                                // the samples first, then a sweep at a time
-        uint32_t pivot_key = kMinKey;
-        bool listed = true;                           // the list is expected to hold what reaches the pivot
-        if (len > kShortRow) {                        // the same for all CTAs of the cluster
+    // ---- 1. the pivot
+    float s[kKpt];                                // the samples first, then a sweep at a time
+    uint32_t pivot_key = kMinKey;
+    bool listed = true;                           // the list is expected to hold what reaches the pivot
+    if (len > kShortRow) {                        // the same for all CTAs of the cluster
 #pragma unroll
-            for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(&sm.hist[i * kBins + 4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
-            if (CLUSTER && tid == 0) sm.negative = 0u;
-            constexpr int kSamples = 4 * kMaxSweeps;
-            uint32_t smp[kSamples];
-            // Four threads take 16 adjacent keys (64 bytes) out of 128, another eighth in each 128 and sweep: a row is looked
-            // at evenly wherever it ends, where good scores come with a period, and where they are neighbours.
+        for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(&sm.hist[i * kBins + 4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+        if (CLUSTER && tid == 0) sm.negative = 0u;
+        constexpr int kSamples = 4 * kMaxSweeps;
+        uint32_t smp[kSamples];
+        // Four threads take 16 adjacent keys (64 bytes) out of 128, another eighth in each 128 and sweep: a row is looked
+        // at evenly wherever it ends, where good scores come with a period, and where they are neighbours.
 #pragma unroll
-            for (int sw = 0; sw < kMaxSweeps; ++sw) {
-                const int j = begin + sw * kSweep + (tid >> 2) * 128 + ((5 * (tid >> 2) + 3 * warp + sw) & 7) * 16 + 4 * (tid & 3);
-                const float4 v = load_scores4<GROUP>(row0, row1, j, end);
-                s[4 * sw] = v.x; s[4 * sw + 1] = v.y; s[4 * sw + 2] = v.z; s[4 * sw + 3] = v.w;
-            }
+        for (int sw = 0; sw < kMaxSweeps; ++sw) {
+            const int j = begin + sw * kSweep + (tid >> 2) * 128 + ((5 * (tid >> 2) + 3 * warp + sw) & 7) * 16 + 4 * (tid & 3);
+            const float4 v = load_scores4<GROUP>(row0, row1, j, end);
+            s[4 * sw] = v.x; s[4 * sw + 1] = v.y; s[4 * sw + 2] = v.z; s[4 * sw + 3] = v.w;
+        }
 #pragma unroll
-            for (int i = 0; i < kSamples; ++i) smp[i] = score_key(s[i]);
+        for (int i = 0; i < kSamples; ++i) smp[i] = score_key(s[i]);
+        __syncthreads();
+        // The 12 highest bits, the sign among them: an eighth of a power of two to a bin.  Where that many samples come with the
+        // rank'th, its bin's lower edge is the pivot, otherwise its next 11 bits are looked at (fewer usable samples than
+        // the rank: every usable key is listed).  All CTAs of the cluster decide alike.
+#pragma unroll
+        for (int i = 0; i < kSamples; ++i)
+            if (smp[i] >= kMinKey) atomicAdd(&sm.hist[smp[i] >> 20], 1u);
+        // Reading a half of the peers' histograms costs more than a barrier.  Where no warp of the row has a positive sample the
+        // positive half is empty; a CTA that has none itself looks at the others.  (Scores around -50, two looks of 11 bits in every
+        // case / the positive half read first / so, us: one row of 131 072 keys, topk 2048 18.1 / 20.9 / 18.0, 8 rows of 262 144 23.2 / 25.2 /
+        // 22.3, 32 pairs of 65 536 16.5 / 18.3 / 17.3; scores around zero, 64 rows of 65 536, topk 400 16.2 / 14.4 / 14.5.)
+        uint32_t k = sample_rank, half = kBins, total = 0u;
+        bool empty = false;
+        if (CLUSTER) {
+            uint32_t any = smp[0];
+#pragma unroll
+            for (int i = 1; i < kSamples; ++i) any |= smp[i];
+            if (!__any_sync(0xffffffffu, any >= 0x80000000u) && lane == 0) atomicAdd(&sm.negative, 1u);
+            cluster_barrier();
+            if (sm.negative == (uint32_t)kWarps)
+                empty = __reduce_min_sync(0xffffffffu, lane < (int)parts ? peer_load(peer_address(&sm.negative, lane)) : (uint32_t)kWarps) == (uint32_t)kWarps;
+        } else {
             __syncthreads();
-            // The 12 highest bits, the sign among them: an eighth of a power of two to a bin.  Where that many samples come with the
-            // rank'th, its bin's lower edge is the pivot, otherwise its next 11 bits are looked at (fewer usable samples than
-            // the rank: every usable key is listed).  All CTAs of the cluster decide alike.
+        }
+        if (!empty) total = locate(sm, sum_bins<CLUSTER>(sm.hist + kBins, parts), k);
+        if (total < k) {                              // the rank'th is negative
+            k -= total;
+            half = 0u;
+            total = locate(sm, sum_bins<CLUSTER>(sm.hist, parts), k);
+        }
+        if (total >= k) {
+            uint32_t edge = (half + sm.sel_bin) << 20, above = sample_rank - k + sm.sel_above, inside = sm.sel_count;
+            if (8u * (above + inside) > (uint32_t)kList * 5 / 8) {
+                if (CLUSTER) cluster_barrier();       // the peers have read the histogram
+                else __syncthreads();
+                *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
+                __syncthreads();
 #pragma unroll
-            for (int i = 0; i < kSamples; ++i)
-                if (smp[i] >= kMinKey) atomicAdd(&sm.hist[smp[i] >> 20], 1u);
-            // Reading a half of the peers' histograms costs more than a barrier.  Where no warp of the row has a positive sample the
-            // positive half is empty; a CTA that has none itself looks at the others.  (Scores around -50, two looks of 11 bits in every
-            // case / the positive half read first / so, us: one row of 131 072 keys, topk 2048 18.1 / 20.9 / 18.0, 8 rows of 262 144 23.2 / 25.2 /
-            // 22.3, 32 pairs of 65 536 16.5 / 18.3 / 17.3; scores around zero, 64 rows of 65 536, topk 400 16.2 / 14.4 / 14.5.)
-            uint32_t k = sample_rank, half = kBins, total = 0u;
-            bool empty = false;
+                for (int i = 0; i < kSamples; ++i)
+                    if (smp[i] - edge < 1u << 20) atomicAdd(&sm.hist[(smp[i] - edge) >> 9], 1u);
+                locate(sm, row_bins<CLUSTER>(sm.hist, parts), sample_rank - above);
+                edge += sm.sel_bin << 9;
+                above += sm.sel_above;
+                inside = sm.sel_count;
+            }
+            pivot_key = max(edge & ~1023u, kMinKey);
+            listed = 8u * (above + inside) <= (uint32_t)kList;
+        }
+    }
+    int32_t* out = indices + (long long)r * index_stride;
+    const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
+    int32_t* count = topk_length != nullptr ? topk_length + r : nullptr;
+
+    // ---- 2. the list, and 3. the selection.  All CTAs of the cluster decide alike.
+#pragma unroll 1
+    while (true) {
+        uint32_t n = 0, key_max = 0u;
+        if (listed) {
+            const float pivot = key_score(pivot_key);
+            bool fits = true;
+#pragma unroll 1
+            for (int sw = 0; sw < nsweeps && fits; ++sw) {
+                load_scores<GROUP, kChunks>(row0, row1, begin + sw * kSweep, end, s);
+                fits = list_sweep(sm, s, pivot, begin + sw * kSweep, end, n);
+            }
+            key_max = sm.key_max;
             if (CLUSTER) {
-                uint32_t any = smp[0];
-#pragma unroll
-                for (int i = 1; i < kSamples; ++i) any |= smp[i];
-                if (!__any_sync(0xffffffffu, any >= 0x80000000u) && lane == 0) atomicAdd(&sm.negative, 1u);
+                if (tid == 0) sm.list_n = fits ? n : (uint32_t)kList + 1u;
                 cluster_barrier();
-                if (sm.negative == (uint32_t)kWarps)
-                    empty = __reduce_min_sync(0xffffffffu, lane < (int)parts ? peer_load(peer_address(&sm.negative, lane)) : (uint32_t)kWarps) == (uint32_t)kWarps;
+                const uint32_t entries = lane < (int)parts ? peer_load(peer_address(&sm.list_n, lane)) : 0u;
+                const uint32_t upto = warp_inclusive_scan(entries, lane);
+                n = __shfl_sync(0xffffffffu, upto, 31);
+                fits = n <= (uint32_t)kList;
+                if (part == 0 && fits) {          // the first CTA gathers the others' lists behind its own
+                    key_max = __reduce_max_sync(0xffffffffu, lane < (int)parts ? peer_load(peer_address(&sm.key_max, lane)) : 0u);
+                    for (uint32_t c = 1; c < parts; ++c) {
+                        const uint32_t m = __shfl_sync(0xffffffffu, entries, c), at = __shfl_sync(0xffffffffu, upto, c) - m;
+                        const uint32_t src = peer_address(sm.list, c);
+                        for (uint32_t i = tid; i < m; i += kThreads) sm.list[at + i] = peer_load2(src + 8 * i);
+                    }
+                }
+                cluster_barrier();
             } else {
                 __syncthreads();
             }
-            if (!empty) total = locate(sm, sum_bins<CLUSTER>(sm.hist + kBins, parts), k);
-            if (total < k) {                              // the rank'th is negative
-                k -= total;
-                half = 0u;
-                total = locate(sm, sum_bins<CLUSTER>(sm.hist, parts), k);
-            }
-            if (total >= k) {
-                uint32_t edge = (half + sm.sel_bin) << 20, above = sample_rank - k + sm.sel_above, inside = sm.sel_count;
-                if (8u * (above + inside) > (uint32_t)kList * 5 / 8) {
-                    if (CLUSTER) cluster_barrier();       // the peers have read the histogram
-                    else __syncthreads();
-                    *reinterpret_cast<uint4*>(&sm.hist[4 * tid]) = make_uint4(0u, 0u, 0u, 0u);
-                    __syncthreads();
-#pragma unroll
-                    for (int i = 0; i < kSamples; ++i)
-                        if (smp[i] - edge < 1u << 20) atomicAdd(&sm.hist[(smp[i] - edge) >> 9], 1u);
-                    locate(sm, row_bins<CLUSTER>(sm.hist, parts), sample_rank - above);
-                    edge += sm.sel_bin << 9;
-                    above += sm.sel_above;
-                    inside = sm.sel_count;
-                }
-                pivot_key = max(edge & ~1023u, kMinKey);
-                listed = 8u * (above + inside) <= (uint32_t)kList;
-            }
+            if (tid == 0) sm.key_max = 0u;        // everybody has read it; a barrier follows before it is raised again
+            listed = fits && (n >= (uint32_t)topk || pivot_key == kMinKey);
         }
-        int32_t* out = indices + (long long)r * index_stride;
-        const int32_t off = row_offset != nullptr ? __ldg(row_offset + r) : 0;
-        int32_t* count = topk_length != nullptr ? topk_length + r : nullptr;
-
-        // ---- 2. the list, and 3. the selection.  All CTAs of the cluster decide alike.
-#pragma unroll 1
-        while (true) {
-            uint32_t n = 0, key_max = 0u;
-            if (listed) {
-                const float pivot = key_score(pivot_key);
-                bool fits = true;
-#pragma unroll 1
-                for (int sw = 0; sw < nsweeps && fits; ++sw) {
-                    load_scores<GROUP, kChunks>(row0, row1, begin + sw * kSweep, end, s);
-                    fits = list_sweep(sm, s, pivot, begin + sw * kSweep, end, n);
-                }
-                key_max = sm.key_max;
-                if (CLUSTER) {
-                    if (tid == 0) sm.list_n = fits ? n : (uint32_t)kList + 1u;
-                    cluster_barrier();
-                    const uint32_t entries = lane < (int)parts ? peer_load(peer_address(&sm.list_n, lane)) : 0u;
-                    const uint32_t upto = warp_inclusive_scan(entries, lane);
-                    n = __shfl_sync(0xffffffffu, upto, 31);
-                    fits = n <= (uint32_t)kList;
-                    if (part == 0 && fits) {          // the first CTA gathers the others' lists behind its own
-                        key_max = __reduce_max_sync(0xffffffffu, lane < (int)parts ? peer_load(peer_address(&sm.key_max, lane)) : 0u);
-                        for (uint32_t c = 1; c < parts; ++c) {
-                            const uint32_t m = __shfl_sync(0xffffffffu, entries, c), at = __shfl_sync(0xffffffffu, upto, c) - m;
-                            const uint32_t src = peer_address(sm.list, c);
-                            for (uint32_t i = tid; i < m; i += kThreads) sm.list[at + i] = peer_load2(src + 8 * i);
-                        }
-                    }
-                    cluster_barrier();
-                } else {
-                    __syncthreads();
-                }
-                if (tid == 0) sm.key_max = 0u;        // everybody has read it; a barrier follows before it is raised again
-                listed = fits && (n >= (uint32_t)topk || pivot_key == kMinKey);
-            }
-            if (listed) {
-                if (part == 0) select_from_list(sm, n, pivot_key, key_max, topk, out, off, count);
-                else __syncthreads();
-                break;
-            }
-            if (!recount_row<GROUP, CLUSTER>(row0, row1, begin, end, parts, part, pivot_key, topk, out, off, count)) break;
-            pivot_key += 1024u;
-            listed = true;
+        if (listed) {
+            if (part == 0) select_from_list(sm, n, pivot_key, key_max, topk, out, off, count);
+            else __syncthreads();
+            break;
         }
+        if (!recount_row<GROUP, CLUSTER>(row0, row1, begin, end, parts, part, pivot_key, topk, out, off, count)) break;
+        pivot_key += 1024u;
+        listed = true;
     }
 }
 
@@ -2272,7 +2256,9 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     // 11.2 by two, 9.8 by four.  Clusters that have to wait are slower: 74 rows of 131 072 21.5 / 29.4, 148 of 65 536 17.9 / 20.7 by two.
     const int spread = p->s_kv <= 2 * kSweep || !staged || p->s_kv > 4 * kHeld ? 0
                        : (long long)p->rows * 4 <= sms - 16 ? 4 : p->s_kv <= 2 * kHeld && (long long)p->rows * 2 <= sms ? 2 : 0;
-    // What is left, by pivot where the list fits with its margin.
+    // What is left, by pivot where the list fits with its margin.  A row has its CTAs to itself, two of them to an SM: the hardware gives rows to
+    // whoever is done.  us, CTAs that walk rows / so: by pivot, topk 2 048, 400 rows of 65 536 keys 52.4 / 44.9, pairs half to full length 80.1 / 72.6,
+    // 1 000 rows 108 / 96.6, 2 048 187 / 182, 400 of 200 000 292 / 230; by counting, 400 rows of 16 384 at topk 8 000 21.3 / 16.4, 2 000 73.8 / 66.0.
     // A division of a row among two, four or eight CTAs is taken while every CTA of the call finds an SM of
     // its own; clusters of four and eight leave some SMs over (33 rows by four, 15 by eight are resident at once, one more
     // makes a second wave: 34 rows of 36 864 keys 15.3 -> 17.6 us).  With two CTAs on an SM a division gains only where the
@@ -2320,16 +2306,13 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
                                   : (parts == 1 ? mxdsa_topk_pivot_kernel<1, false> : mxdsa_topk_pivot_kernel<1, true>);
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(PivotShared));
         if (e == cudaSuccess) {
-            const long long want = (long long)p->rows * parts;
-            e = launch(kern, (unsigned)(want < sms * 2 ? want : sms * 2 / parts * parts), kThreads, sizeof(PivotShared), s, parts, p->scores, ss,
-                       p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows, p->s_kv, p->topk, rank);
+            e = launch(kern, p->rows * parts, kThreads, sizeof(PivotShared), s, parts, p->scores, ss, p->lengths, p->row_offset, p->indices, is,
+                       p->topk_length, p->s_kv, p->topk, rank);
         }
     } else {
-        const int grid = p->rows < sms * 2 ? p->rows : sms * 2;      // two resident CTAs of 512 threads per SM
         auto kern = staged ? (p->group == 2 ? mxdsa_topk_rows_kernel<2, true> : mxdsa_topk_rows_kernel<1, true>)
                            : (p->group == 2 ? mxdsa_topk_rows_kernel<2, false> : mxdsa_topk_rows_kernel<1, false>);
-        e = launch(kern, grid, kThreads, 0, s, 1, p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->rows,
-                   p->s_kv, p->topk);
+        e = launch(kern, p->rows, kThreads, 0, s, 1, p->scores, ss, p->lengths, p->row_offset, p->indices, is, p->topk_length, p->s_kv, p->topk);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
