@@ -597,11 +597,12 @@ __device__ __noinline__ void let_copies_land() {
     for (int i = 0; i < (1 << 16) && clock64() - start < 2000000; ++i) __nanosleep(1000);
 }
 
-// ALONE: one token to a request, decode of short parts.  The token is in both CTAs of the pair, which then store half of the columns
-// each: an SM writes 32 bytes a clock at best, half of a partial's 128 KB is 1.1 us of the drain.  An instantiation of its own again:
-// bounds worked out by pair cost the other short parts 0.5 to 1 % and, everywhere, decode of long parts 2 to 5 %, 256 tokens of
-// prefill at topk 128 2 %.  Us per call, one CTA storing / both: one request over 2176 keys 13.2 / 11.8, over 192 10.7 / 9.4, 8 over 640
-// 21.9 / 19.5, 30 over 2176 37.6 / 34.6, 64 over 640 33.8 / 31.3; whole requests, 8 over 640 16.2 / 14.6, 64 over 640 18.5 / 17.6.
+// ALONE: decode of one token to a request.  The token is in both CTAs of the pair, which then store half of the columns each: an SM
+// writes 32 bytes a clock at best, half of a partial's 128 KB is 1.1 us of the drain.  Instantiations of their own again: bounds worked
+// out by pair cost the other short parts 0.5 to 1 %, decode of long parts 2 to 5 %, 256 tokens of prefill at topk 128 2 %.
+// Us per call, one CTA storing / both: short parts, one request over 2176 keys 13.2 / 11.8, over 192 10.7 / 9.4, 8 over 640 21.9 / 19.5, 30 over
+// 2176 37.6 / 34.6, 64 over 640 33.8 / 31.3, whole requests, 8 over 640 16.2 / 14.6, 64 over 640 18.5 / 17.6; long parts, 64 over 4224 76.8 /
+// 70.8, 128 over 4224 113.8 / 107.6, over 2176 62.9 / 61.0, whole 60.7 / 59.0.
 template <int DECODE, int NT, bool ALONE = false>
 __global__ void __launch_bounds__(kThreads, 1)
 mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ TensorMaps maps, const int resident_pairs) {
@@ -1378,7 +1379,7 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
             if (lane == 0) mbar_arrive(smem_u32(&sm.bar_os_empty[gw & 1]));
             MXDSA_WAIT(sm.bar_pv_done[last % kScStages], (last / kScStages) & 1, 55);
             tc_fence_after();
-            static_assert(!ALONE || DECODE == 2, "long parts store their partials from the lanes");
+            static_assert(!ALONE || DECODE, "prefill has one odd pair at most");
             const int tok_idx = ALONE ? 0 : 2 * w.pair + (int)cta;
             const bool store = ALONE || tok_idx < p.s_q;
             const int col0 = half * 256 + (ALONE ? 128 * (int)cta : 0);      // the columns that this warp stores begin here ...
@@ -1459,13 +1460,13 @@ mxdsa_attn_kernel(const __grid_constant__ AttnParams p, const __grid_constant__ 
                     }
                 }
             } else {
-                float* dst = p.o_accum + (((long long)wo.split_idx * p.s_q + tok_idx) * kHeads + row) * kDim + half * 256;
+                float* dst = p.o_accum + (((long long)wo.split_idx * p.s_q + tok_idx) * kHeads + row) * kDim + col0;
 #pragma unroll 1
-                for (int c = 0; c < 256; c += 32) {
+                for (int c = 0; c < kCols; c += 32) {
                     float o[32];
-                    tmem_ld32(lane_addr + kColO + c, reinterpret_cast<uint32_t*>(o));
+                    tmem_ld32(o_addr + c, reinterpret_cast<uint32_t*>(o));
                     tmem_wait_ld();
-                    if (c == 256 - 32) release_o();   // the last columns are in registers: the next pair's PV may go
+                    if (c == kCols - 32) release_o();   // the last columns are in registers: the next pair's PV may go
                     if (store) {
 #pragma unroll
                         for (int i = 0; i < 32; i += 8) {

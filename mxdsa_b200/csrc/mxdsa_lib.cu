@@ -728,7 +728,7 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     if (short_parts)
         st = launch_pairs(p->s_q == 1 ? mxdsa::mxdsa_attn_kernel<2, 64, true> : mxdsa::mxdsa_attn_kernel<2, 64>, grid, d->sm_count, stream, ap, maps);
     else
-        st = launch_pairs(mxdsa::mxdsa_attn_kernel<1, 64>, grid, d->sm_count, stream, ap, maps);
+        st = launch_pairs(p->s_q == 1 ? mxdsa::mxdsa_attn_kernel<1, 64, true> : mxdsa::mxdsa_attn_kernel<1, 64>, grid, d->sm_count, stream, ap, maps);
     if (st != MXDSA_OK) return st;
     if (!combine) return MXDSA_OK;
     // programmatic dependent launch: the combine grid is set up while the attention grid drains (the attention

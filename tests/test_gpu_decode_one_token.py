@@ -7,7 +7,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("whole", [False, True])
-@pytest.mark.parametrize("b,extra", [(1, 0), (1, 2048), (1, 4096), (3, 700), (8, 512), (9, 1000), (30, 2048), (64, 512), (100, 64)])
+@pytest.mark.parametrize("b,extra", [(1, 0), (1, 2048), (1, 4096), (3, 700), (8, 512), (9, 1000), (30, 2048), (64, 512), (100, 64), (40, 4096), (128, 1300)])
 def test_one_token_is_half_of_two(b, extra, whole):
     import mxdsa_b200 as M
     from mxdsa_b200 import packing, quantize
