@@ -405,8 +405,8 @@ mxdsa_combine_kernel(int b, int s_q, int by_request, int release, const int* met
 }
 
 int launch_combine(int b, int s_q, int parts, const int* meta, const int* num_splits, const float* o_accum,
-                   const float* lse_accum, const float* sink, __nv_bfloat16* out, float* lse, bool dependent, bool release, int sms,
-                   cudaStream_t stream) {
+                   const float* lse_accum, const float* sink, __nv_bfloat16* out, float* lse, bool dependent, bool release, int most_splits,
+                   int sms, cudaStream_t stream) {
     const int by_request = b <= parts;
     const int units = (by_request ? b : parts) * s_q;
     // 64 heads a unit: from 16 warps an SM on a warp per head fills the SMs
@@ -423,8 +423,9 @@ int launch_combine(int b, int s_q, int parts, const int* meta, const int* num_sp
     // Where an SM gets two blocks at most, registers do not count and a lane keeps sixteen loads in flight: what there is to do then
     // is wait for one batch of rows after another.  us per call, eight / sixteen: one request of one token over 2176 keys 13.7 /
     // 13.3, over 4224 16.8 / 16.5, two over 2176 14.9 / 14.6, two of two tokens over 4224 19.9 / 16.9, three of three over 1128 15.3 / 13.9; with more
-    // units registers keep blocks waiting: four of four over 1152 15.0 / 16.0, 30 of one over 2176 37.3 / 39.3.
-    const bool few = units * (int)(MXDSA_HEADS * 4 / kCombineWarps) <= 2 * sms;
+    // units registers keep blocks waiting: four of four over 1152 15.0 / 16.0, 30 of one over 2176 37.3 / 39.3.  Up to eight blocks of keys, and so
+    // splits, to a request there is one batch anyway, and the longer code costs: four of two tokens over 128 11.5 / 11.8.
+    const bool few = units * (int)(MXDSA_HEADS * 4 / kCombineWarps) <= 2 * sms && most_splits > 8;
     MX_CUDA(cudaLaunchKernelEx(&cfg, few ? mxdsa_combine_kernel<4, 16> : wide ? mxdsa_combine_kernel<4, 8> : mxdsa_combine_kernel<1, 8>, b, s_q, by_request, release ? 1 : 0, meta,
                                num_splits, o_accum, lse_accum, sink, out, lse));
     return MXDSA_OK;
@@ -734,7 +735,7 @@ static int decode_impl(const mxdsa_decode_params* p, bool combine) {
     // programmatic dependent launch: the combine grid is set up while the attention grid drains (the attention
     // kernel releases its dependents once it runs; the combine kernel waits before it reads anything)
     return launch_combine(p->b, p->s_q, p->num_sm_parts, p->sched_meta, p->num_splits, o_accum, lse_accum, p->attn_sink,
-                          static_cast<__nv_bfloat16*>(p->out), p->lse, true, short_parts, d->sm_count, stream);
+                          static_cast<__nv_bfloat16*>(p->out), p->lse, true, short_parts, (int)(blocks / p->b), d->sm_count, stream);
 }
 
 extern "C" int mxdsa_decode_fwd(const mxdsa_decode_params* p) { return decode_impl(p, true); }
@@ -765,7 +766,7 @@ extern "C" int mxdsa_decode_combine(const mxdsa_combine_params* p) {
     const int st = device_info(&d);
     if (st != MXDSA_OK) return st;
     return launch_combine(p->b, p->s_q, p->num_sm_parts, p->sched_meta, p->num_splits, o_accum, lse_accum, p->attn_sink,
-                          static_cast<__nv_bfloat16*>(p->out), p->lse, false, false, d->sm_count,
+                          static_cast<__nv_bfloat16*>(p->out), p->lse, false, false, kMaxSplits, d->sm_count,
                           static_cast<cudaStream_t>(p->stream));
 }
 

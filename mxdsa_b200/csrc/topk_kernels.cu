@@ -2248,7 +2248,8 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
     // (rows of up to an SM each counted, the others by pivot) / so: one wave, 148 rows of 32 768 at topk 64 15.7 / 8.9, 512 16.6 / 9.3, 2 048 16.7 / 9.5,
     // 4 096 17.0 / 10.6, half to full length, topk 2 048 16.8 / 9.6, a quarter to half full 7.8 / 7.7, up to an eighth 5.2 / 6.1; 148 of 20 000 14.3 / 8.6;
     // one row 12.9 / 8.3.  2 048 rows of 32 768 at topk 4 096 147 / 118, 2 048 122 / 107, 512 108 / 104; 600 of 26 000 at 512 31.8 / 35.3; pairs 173 / 128
-    // at 2 048, 151 / 117 at 64.
+    // at 2 048, 151 / 117 at 64.  All scores negative gain less, 1 024 rows of 32 768 77.3 / 76.2, and lose where a last round is nearly empty, 1 500
+    // 101 / 113; what the scores are is known on the device alone.
     const bool wide = p->s_kv > kSweep && p->s_kv <= 2 * kSweep && staged && (p->rows <= sms || p->group == 2 || p->topk >= 1024);
     // Longer rows in few: held by the CTAs of a cluster, two or four, as long as every one finds an SM of its own (33 clusters of four
     // are resident at once).  us, by pivot / so: 64 rows of 65 536 keys, topk 2 048 16.3 / 11.0, half to full length 16.4 / 10.9, 74 at topk 512 14.7 / 10.1;
@@ -2258,7 +2259,8 @@ extern "C" int mxdsa_topk_select(const mxdsa_topk_params* p) {
                        : (long long)p->rows * 4 <= sms - 16 ? 4 : p->s_kv <= 2 * kHeld && (long long)p->rows * 2 <= sms ? 2 : 0;
     // What is left, by pivot where the list fits with its margin.  A row has its CTAs to itself, two of them to an SM: the hardware gives rows to
     // whoever is done.  us, CTAs that walk rows / so: by pivot, topk 2 048, 400 rows of 65 536 keys 52.4 / 44.9, pairs half to full length 80.1 / 72.6,
-    // 1 000 rows 108 / 96.6, 2 048 187 / 182, 400 of 200 000 292 / 230; by counting, 400 rows of 16 384 at topk 8 000 21.3 / 16.4, 2 000 73.8 / 66.0.
+    // 1 000 rows 108 / 96.6, 2 048 187 / 182, 400 of 200 000 292 / 230; by counting, 400 rows of 16 384 at topk 8 000 21.3 / 16.4, 2 000 73.8 / 66.0.  (300 rows of
+    // 65 536, four more than are resident, 36.2 / 37.2.)
     // A division of a row among two, four or eight CTAs is taken while every CTA of the call finds an SM of
     // its own; clusters of four and eight leave some SMs over (33 rows by four, 15 by eight are resident at once, one more
     // makes a second wave: 34 rows of 36 864 keys 15.3 -> 17.6 us).  With two CTAs on an SM a division gains only where the
